@@ -155,7 +155,10 @@ __global__ void kConst(const ConstTask* __restrict__ tasks, const TileRef* __res
 
 // XXH3's published secret and primes (the checksum kernels below and the
 // content-checksum block sums fused into the numeric pipeline).
-__constant__ uint8_t kXxhSecret[192] = {
+struct XxhSecret {
+    uint8_t b[192];
+};
+constexpr XxhSecret kXxhSecretBytes = { {
     0xb8, 0xfe, 0x6c, 0x39, 0x23, 0xa4, 0x4b, 0xbe, 0x7c, 0x01, 0x81, 0x2c, 0xf7, 0x21, 0xad, 0x1c,
     0xde, 0xd4, 0x6d, 0xe9, 0x83, 0x90, 0x97, 0xdb, 0x72, 0x40, 0xa4, 0xa4, 0xb7, 0xb3, 0x67, 0x1f,
     0xcb, 0x79, 0xe6, 0x4e, 0xcc, 0xc0, 0xe5, 0x78, 0x82, 0x5a, 0xd0, 0x7d, 0xcc, 0xff, 0x72, 0x21,
@@ -168,7 +171,8 @@ __constant__ uint8_t kXxhSecret[192] = {
     0x17, 0x0d, 0xdd, 0x51, 0xb7, 0xf0, 0xda, 0x49, 0xd3, 0x16, 0x55, 0x26, 0x29, 0xd4, 0x68, 0x9e,
     0x2b, 0x16, 0xbe, 0x58, 0x7d, 0x47, 0xa1, 0xfc, 0x8f, 0xf8, 0xb8, 0xd1, 0x7a, 0xd0, 0x31, 0xce,
     0x45, 0xcb, 0x3a, 0x8f, 0x95, 0x16, 0x04, 0x28, 0xaf, 0xd7, 0xfb, 0xca, 0xbb, 0x4b, 0x40, 0x7e,
-};
+} };
+__constant__ XxhSecret kXxhSecret = kXxhSecretBytes;
 
 #define XP32_1 0x9E3779B1u
 #define XP32_2 0x85EBCA77u
@@ -181,16 +185,36 @@ __constant__ uint8_t kXxhSecret[192] = {
 #define XPMX1 0x165667919E3779F9ull
 #define XPMX2 0x9FB21C651E98DF25ull
 
+// The secret as the 64-bit words that the checksum kernels index per lane:
+// at byte offsets 0, 8, ..., 184; at 121 + 8 i (the final stripe); at
+// 11 + 8 k (the merge).
+struct XxhWords {
+    uint64_t w8[24], last[8], merge[8];
+};
+constexpr XxhWords xxhWords()
+{
+    XxhWords x{};
+    for (int k = 0; k < 24; k++)
+        for (int b = 0; b < 8; b++) x.w8[k] |= uint64_t(kXxhSecretBytes.b[8 * k + b]) << (8 * b);
+    for (int k = 0; k < 8; k++)
+        for (int b = 0; b < 8; b++) {
+            x.last[k] |= uint64_t(kXxhSecretBytes.b[121 + 8 * k + b]) << (8 * b);
+            x.merge[k] |= uint64_t(kXxhSecretBytes.b[11 + 8 * k + b]) << (8 * b);
+        }
+    return x;
+}
+__constant__ XxhWords kXxhWords = xxhWords();
+
 __device__ __forceinline__ uint64_t secret64(int off)
 {
     uint64_t v = 0;
-    for (int b = 0; b < 8; b++) v |= uint64_t(kXxhSecret[off + b]) << (8 * b);
+    for (int b = 0; b < 8; b++) v |= uint64_t(kXxhSecret.b[off + b]) << (8 * b);
     return v;
 }
 __device__ __forceinline__ uint32_t secret32(int off)
 {
-    return uint32_t(kXxhSecret[off]) | (uint32_t(kXxhSecret[off + 1]) << 8) | (uint32_t(kXxhSecret[off + 2]) << 16)
-            | (uint32_t(kXxhSecret[off + 3]) << 24);
+    return uint32_t(kXxhSecret.b[off]) | (uint32_t(kXxhSecret.b[off + 1]) << 8) | (uint32_t(kXxhSecret.b[off + 2]) << 16)
+            | (uint32_t(kXxhSecret.b[off + 3]) << 24);
 }
 // ---------------------------------------------------------------------------
 // Fused numeric pipeline: source (plain elements, byte planes or LSB-first
@@ -722,7 +746,7 @@ __global__ void __launch_bounds__(kNPThreads) kNumPipe(const NumPipeTask* __rest
     TileRef const tr = tiles[g];
     NumPipeTask const t = tasks[tr.task];
     if (t.blockSums) { // the same task for the whole CTA
-        if (threadIdx.x < 24) sh.key[threadIdx.x] = secret64(int(8 * threadIdx.x));
+        if (threadIdx.x < 24) sh.key[threadIdx.x] = kXxhWords.w8[threadIdx.x];
         __syncthreads();
     }
     switch (t.w) {
@@ -1872,7 +1896,7 @@ __global__ void __launch_bounds__(256) kHashBlocks(const HashTask* __restrict__ 
                                                    const TileRef* __restrict__ blocks, uint32_t nbBlocks)
 {
     __shared__ uint64_t sKey[24]; // secret words at byte offsets 0, 8, ..., 184
-    if (threadIdx.x < 24) sKey[threadIdx.x] = secret64(int(8 * threadIdx.x));
+    if (threadIdx.x < 24) sKey[threadIdx.x] = kXxhWords.w8[threadIdx.x];
     __syncthreads();
     uint32_t const lane = threadIdx.x & 31;
     // grid-stride over the blocks, one warp per block at a time: the secret
@@ -1883,75 +1907,91 @@ __global__ void __launch_bounds__(256) kHashBlocks(const HashTask* __restrict__ 
 }
 
 
-// The block chain of accumulator lane & 7 over nb blocks (all 32 lanes of the
-// warp call it; see kHashFinish), starting from init, with key words
-// (klo, khi); sb: the warp's 264 words of shared memory. Returns the
-// accumulator after the last block. Kept out of line: compiled inside
-// kHashFinish the same loop ran slower (the chain of a 256 MiB input took
-// 5.13 ms there, 4.78 ms here).
-__device__ __noinline__ uint64_t xxhBlockChain(const uint64_t* __restrict__ bs, uint32_t nb, uint64_t init,
-                                           uint32_t klo, uint32_t khi, uint64_t* sb)
+// The block chain acc = scramble(acc + sum), scramble(x) = ((x ^ (x >> 47)) ^
+// key) * PRIME32_1, of accumulator i over nb blocks, starting from init, with
+// key words (klo, khi); bs: 8 sums a block. Returns the accumulator after the
+// last block.
+//
+// The chain is serial, so its latency per block is what bounds a long input's
+// checksum. It runs on y = acc + sum of the block about to be scrambled, in
+// 32-bit halves: x >> 47 only reaches the low half, so with t = y.lo ^
+// (y.hi >> 15) ^ key.lo and u = y.hi ^ key.hi the next y is t * P + C with
+// C = next sum + ((u * P) << 32). C needs only u and is ready before t, which
+// leaves a shift, a xor, the low product (whose addition of C.lo sets the
+// carry) and the high product with C.hi and that carry: 4 + 4 + 4 + 9 cycles
+// (dependent-issue latencies measured one by one). One 64-bit multiply-add
+// instead of the pair measured 27, and the product added to in two steps 23.
+// Each lane reads its accumulator's sums straight into registers, a batch of
+// 48 blocks ahead: 48 steps cover the load's way to L2, and no barrier or
+// shared-memory round trip stands on the path (batches of 32 measured 28.7
+// cycles a block, 48 measured 22.8).
+// 262,144 blocks (a 256 MiB input): 4.71 ms before (a warp staged the sums of
+// 32 blocks in shared memory, two-step product), 3.25 ms now.
+constexpr int kChainBatch = 48;
+constexpr uint32_t kChainAhead = 512; // blocks fetched into L2 ahead of the chain
+__device__ __forceinline__ void xxhChainStep(uint32_t& ylo, uint32_t& yhi, uint32_t klo, uint32_t khi, uint64_t nv)
 {
-    uint32_t const lane = threadIdx.x & 31, i = lane & 7;
-    uint64_t const total = 8ull * nb;
-    // batches of 32 blocks: the current one, the next, and the one after
-    // it in flight (two batches of chain steps cover an L2 round trip)
-    uint64_t cur[8], nxt[8];
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-        uint64_t const idx = uint64_t(lane) + 32u * m;
-        cur[m] = idx < total ? __ldg(bs + idx) : 0;
-        nxt[m] = idx + 256 < total ? __ldg(bs + idx + 256) : 0;
-    }
-    uint64_t const y0 = init + __shfl_sync(0xffffffffu, cur[0], int(i)); // init + sum of block 0
+    uint32_t const c = (yhi ^ khi) * XP32_1 + uint32_t(nv >> 32);
+    uint32_t const t = ylo ^ (yhi >> 15) ^ klo;
+    asm("mad.lo.cc.u32 %0, %2, %3, %4;\n\tmadc.hi.u32 %1, %2, %3, %5;"
+        : "=&r"(ylo), "=r"(yhi) : "r"(t), "r"(XP32_1), "r"(uint32_t(nv)), "r"(c));
+}
+__device__ __noinline__ uint64_t xxhBlockChain(const uint64_t* __restrict__ bs, uint32_t nb, uint64_t init,
+                                               uint32_t klo, uint32_t khi, uint32_t i)
+{
+    if (nb == 0) return init;
+    uint64_t const y0 = init + __ldg(bs + i); // init + sum of block 0
     uint32_t ylo = uint32_t(y0), yhi = uint32_t(y0 >> 32);
-    for (uint32_t b0 = 0; b0 < nb; b0 += 32) {
-        uint64_t nx2[8];
+    uint32_t const m = nb - 1; // steps that add a next sum; the last block's step adds none
+    const uint64_t* p = bs + 8 + i;
+    uint64_t cur[kChainBatch], nxt[kChainBatch];
+    uint32_t b = 0;
+    // a lane fetches one line of two blocks into L2, `ahead` blocks on
+    auto fetchL2 = [&](uint32_t from) {
+        uint32_t const blk = from + 2 * (threadIdx.x & 31);
+        if (blk < nb) asm volatile("prefetch.global.L2 [%0];" ::"l"(bs + 8ull * blk));
+    };
+    for (uint32_t f = kChainBatch; f < kChainAhead; f += 64) fetchL2(f);
+    if (m >= kChainBatch) {
 #pragma unroll
-        for (int m = 0; m < 8; m++) {
-            uint64_t const idx = 8ull * (b0 + 64) + lane + 32u * m;
-            nx2[m] = idx < total ? __ldg(bs + idx) : 0;
+        for (int k = 0; k < kChainBatch; k++) cur[k] = __ldg(p + 8 * k);
+        for (; b + 2 * kChainBatch <= m; b += kChainBatch) {
+            p += 8 * kChainBatch;
+            fetchL2(b + kChainAhead);
+#pragma unroll
+            for (int k = 0; k < kChainBatch; k++) nxt[k] = __ldg(p + 8 * k);
+#pragma unroll
+            for (int k = 0; k < kChainBatch; k++) xxhChainStep(ylo, yhi, klo, khi, cur[k]);
+#pragma unroll
+            for (int k = 0; k < kChainBatch; k++) cur[k] = nxt[k];
         }
-        uint32_t const cnt = min(32u, nb - b0);
-#pragma unroll
-        for (int m = 0; m < 8; m++) sb[lane + 32 * m] = cur[m];
-        if (lane < 8) sb[256 + lane] = nxt[0];
-        __syncwarp();
-        // one chain step with the sum of block b0 + k + 1 (0 past the last block)
-        auto step = [&](int k) {
-            uint64_t const nv = sb[8 * (k + 1) + i];
-            uint32_t const tt = ylo ^ (yhi >> 15) ^ klo;
-            uint32_t const u = yhi ^ khi;
-            uint64_t const r = uint64_t(tt) * XP32_1 + nv;
-            ylo = uint32_t(r);
-            yhi = uint32_t(r >> 32) + u * XP32_1;
-        };
-        if (cnt == 32) { // full batches without a per-block predicate
-#pragma unroll
-            for (int k = 0; k < 32; k++) step(k);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 32; k++)
-                if (uint32_t(k) < cnt) step(k);
-        }
-        __syncwarp(); // the batch's sums are read before the next batch overwrites them
-#pragma unroll
-        for (int m = 0; m < 8; m++) {
-            cur[m] = nxt[m];
-            nxt[m] = nx2[m];
-        }
+        p += 8 * kChainBatch;
     }
-    // after the last block y = acc (its next sum is 0); with no block,
-    // y = init + 0
+    // the last full batch, if any, while the sums after it load; then those
+    uint32_t const rest = m - b - (m >= kChainBatch ? kChainBatch : 0); // below kChainBatch
+#pragma unroll
+    for (int k = 0; k < kChainBatch; k++) nxt[k] = uint32_t(k) < rest ? __ldg(p + 8 * k) : 0;
+    if (m >= kChainBatch) {
+#pragma unroll
+        for (int k = 0; k < kChainBatch; k++) xxhChainStep(ylo, yhi, klo, khi, cur[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kChainBatch; k++)
+        if (uint32_t(k) <= rest) xxhChainStep(ylo, yhi, klo, khi, nxt[k]); // step `rest` adds 0: the last block
     return (uint64_t(yhi) << 32) | ylo;
 }
 
 // Phase 2: one warp per task. Lane i (and its copies i + 8, i + 16, i + 24)
 // runs the block chain of accumulator i, then the trailing partial stripes
-// and the final stripe, and lane 0 merges.
-__global__ void kHashFinish(const HashTask* __restrict__ tasks, uint32_t nbTasks, uint32_t* __restrict__ status)
+// and the final stripe, and lane 0 merges. The trailing stripes add to the
+// accumulators without a chain: the four groups of 8 lanes take every fourth
+// one (at most 15, and the final stripe as the sixteenth), loaded before the
+// chain starts.
+constexpr uint32_t kFinishWarps = 4;
+__global__ void __launch_bounds__(32 * kFinishWarps) kHashFinish(const HashTask* __restrict__ tasks, uint32_t nbTasks,
+                                                                 uint32_t* __restrict__ status)
 {
-    uint32_t const ti = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    uint32_t const ti = blockIdx.x * kFinishWarps + (threadIdx.x >> 5);
     uint32_t const lane = threadIdx.x & 31;
     if (ti >= nbTasks) return;
     HashTask const t = tasks[ti];
@@ -1961,52 +2001,37 @@ __global__ void kHashFinish(const HashTask* __restrict__ tasks, uint32_t nbTasks
         if (lane != 0) return;
         h = xxh3Short(t.data, t.len, al);
     } else {
-        uint32_t const i = lane & 7;
+        uint32_t const i = lane & 7, g = lane >> 3;
         uint64_t const init = i == 0 ? XP32_3 : i == 1 ? XP64_1 : i == 2 ? XP64_2 : i == 3 ? XP64_3
                             : i == 4 ? XP64_4 : i == 5 ? XP32_2 : i == 6 ? XP64_5 : XP32_1;
-        uint64_t const key = secret64(int(192 - 64 + 8 * i));
-        uint32_t const klo = uint32_t(key), khi = uint32_t(key >> 32);
-        // The block chain acc = scramble(acc + sum), scramble(x) = ((x ^
-        // (x >> 47)) ^ key) * PRIME32_1, is serial; its inputs are not. The
-        // warp loads the sums of 32 blocks at a time (coalesced, the next
-        // batch while the current one runs), and lane i takes the value of
-        // block k for accumulator i from lane 8 * (k % 4) + i.
-        //
-        // The chain runs on y = acc + sum of the block about to be scrambled,
-        // in 32-bit halves: x >> 47 only reaches the low half (y.hi >> 15), so
-        // with t = y.lo ^ (y.hi >> 15) ^ key.lo and u = y.hi ^ key.hi the next
-        // y is t * P + next sum (one 32x32+64-bit multiply-add) with u * P
-        // added to its high half. Per block the dependent path is a shift, a
-        // xor and two multiply-adds; the sums' additions leave it. Each batch
-        // of sums is staged in the warp's shared memory and read per block:
-        // in a micro-benchmark of the loop alone, 27 cycles a block on GB300
-        // against 38 when taken by warp shuffles.
-        // per warp: the sums of a batch of 32 blocks, then the next batch's first
-        __shared__ uint64_t sBatch[8][256 + 8];
+        uint64_t const key = kXxhWords.w8[16 + i];
         uint32_t const nb = t.nbBlocks;
-        uint64_t acc = xxhBlockChain(t.blockSums, nb, init, klo, khi, sBatch[threadIdx.x >> 5]);
         uint64_t const len = t.len;
-        uint64_t const nbStripes = ((len - 1) - uint64_t(kHashBlock) * nb) / 64;
+        uint32_t const nbStripes = uint32_t(((len - 1) - uint64_t(kHashBlock) * nb) / 64);
         const uint8_t* const last = t.data + uint64_t(kHashBlock) * nb;
-        for (uint64_t st = 0; st < nbStripes; st++) {
-            uint64_t const v = ldData(last + 64 * st + 8 * i, al);
-            uint64_t const vx = __shfl_xor_sync(0xffffffffu, v, 1);
-            uint64_t const x = v ^ secret64(int(8 * st + 8 * i));
-            acc += vx + uint64_t(uint32_t(x)) * (x >> 32);
+        uint64_t v[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) {
+            uint32_t const st = g + 4 * j;
+            const uint8_t* const p = st == 15 ? t.data + len - 64 : last + 64 * st;
+            v[j] = st < nbStripes || st == 15 ? ldData(p + 8 * i, al) : 0;
         }
-        {
-            uint64_t const v = ldData(t.data + len - 64 + 8 * i, al);
-            uint64_t const vx = __shfl_xor_sync(0xffffffffu, v, 1);
-            uint64_t const x = v ^ secret64(192 - 64 - 7 + 8 * int(i));
-            acc += vx + uint64_t(uint32_t(x)) * (x >> 32);
+        uint64_t acc = xxhBlockChain(t.blockSums, nb, init, uint32_t(key), uint32_t(key >> 32), i);
+        uint64_t part = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) {
+            uint32_t const st = g + 4 * j;
+            uint64_t const vx = __shfl_xor_sync(0xffffffffu, v[j], 1);
+            uint64_t const x = v[j] ^ (st == 15 ? kXxhWords.last[i] : kXxhWords.w8[st + i]);
+            if (st < nbStripes || st == 15) part += vx + uint64_t(uint32_t(x)) * (x >> 32);
         }
+        part += __shfl_xor_sync(0xffffffffu, part, 8);
+        part += __shfl_xor_sync(0xffffffffu, part, 16);
+        acc += part;
         // merge: pairs (2k, 2k+1) folded with secret words at 11 + 16k
         uint64_t const odd = __shfl_xor_sync(0xffffffffu, acc, 1);
-        uint64_t part = 0;
-        if (!(i & 1)) {
-            int const k = int(i >> 1);
-            part = fold128(acc ^ secret64(11 + 16 * k), odd ^ secret64(11 + 16 * k + 8));
-        }
+        part = 0;
+        if (!(i & 1)) part = fold128(acc ^ kXxhWords.merge[i], odd ^ kXxhWords.merge[i + 1]);
         part += __shfl_xor_sync(0xffffffffu, part, 2);
         part += __shfl_xor_sync(0xffffffffu, part, 4);
         if (lane != 0) return;
@@ -2167,8 +2192,8 @@ long runOneLaunch(const DeviceLayout& L, size_t li, uint8_t* dPool, uint8_t* dSc
                                                                    l.nbTiles);
                     count++;
                 }
-                uint32_t const grid = (l.nbTasks * 32 + 255) / 256;
-                kHashFinish<<<grid, 256, 0, s>>>(static_cast<const HashTask*>(tasks), l.nbTasks, dStatus);
+                uint32_t const grid = (l.nbTasks + kFinishWarps - 1) / kFinishWarps;
+                kHashFinish<<<grid, 32 * kFinishWarps, 0, s>>>(static_cast<const HashTask*>(tasks), l.nbTasks, dStatus);
                 break;
             }
             default:
@@ -2194,7 +2219,7 @@ void launchHash(const HashTask* tasks, uint32_t nbTasks, const TileRef* blocks, 
                 cudaStream_t s)
 {
     if (nbBlocks) kHashBlocks<<<hashGrid(nbBlocks), 256, 0, s>>>(tasks, blocks, nbBlocks);
-    if (nbTasks) kHashFinish<<<(nbTasks * 32 + 255) / 256, 256, 0, s>>>(tasks, nbTasks, status);
+    if (nbTasks) kHashFinish<<<(nbTasks + kFinishWarps - 1) / kFinishWarps, 32 * kFinishWarps, 0, s>>>(tasks, nbTasks, status);
 }
 
 cudaError_t xxh3Device(const uint8_t* data, uint64_t len, uint64_t* dHashOut, uint8_t* dScratch,
