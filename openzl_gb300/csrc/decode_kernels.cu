@@ -5,7 +5,9 @@
 // host planner (dec_plan.cpp) builds both. Kernels never trap: malformed
 // input sets the batch status word (first error wins) and the kernel moves
 // on. Every spin-wait is bounded.
+#include <algorithm>
 #include <cstdint>
+#include <type_traits>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -994,33 +996,51 @@ struct BitWin3 {
 };
 
 // ---------------------------------------------------------------------------
-// FSE: one lane per chunk. Each lane keeps its decoding table in shared
-// memory as two arrays over the cells: a 16-bit entry holding the cell's
-// newStateBase (bits 4-15) and nbBits (bits 0-3), and the cell's symbol byte.
-// Three bytes a cell (6 KiB at tableLog 11) let about 32 chunks reside per
-// SM. A decoder state is a cell index: a transition is one 16-bit load, the
-// symbol one byte load, and the fields of a pair of transitions come out of
-// one 32-bit window by funnel shifts.
+// FSE: one lane per chunk. A CTA keeps its streams' decoding tables in shared
+// memory, one cell per decoder state, in one of three forms:
+//  - kCells32: a 32-bit cell with nbBits in the low byte, the symbol in the
+//    next and newStateBase * 4 above; a transition is one load (8 KiB a stream
+//    at tableLog 11, 27 streams per SM);
+//  - kCells24: a symbol byte and a 16-bit entry, newStateBase above five bits
+//    of nbBits, in two arrays (6 KiB a stream, 36 streams per SM);
+//  - kCells24Wide: the same with four bits of nbBits, for tableLog 12.
 //
 // Table construction restates src/openzl/fse/decompress/fse_decompress.c:
 // 73-171; decode order restates fse_decompress.c:255-337 (state i % nbStates
 // emits symbol i; the last symbol of each state has no transition).
-constexpr uint32_t kFseCtaSmem = 224 * 1024; // up to 32 tableLog-11 lanes per CTA (one warp)
-constexpr uint32_t kFseDefaultLanes = 6;       // streams per CTA when the autotuner has not run
+enum FseCells : int { kCells32, kCells24, kCells24Wide };
+constexpr uint32_t kFseCtaSmem = 224 * 1024; // up to 32 tableLog-11 lanes per CTA (one decoding warp)
 
-constexpr int kFseRing = 16, kFseAhead = 12; // stream ring: 256 bytes per lane, 192 bytes ahead
+constexpr uint32_t kFseQuarterSmem = 56 * 1024; // four CTAs of this much fit an SM
+constexpr int kFseRing = 16, kFseAhead = 12;   // stream ring: 256 bytes per lane, 192 bytes ahead
+// The ring of a kFse stream follows a copy of its last 16 bytes: the words
+// below the ring's first one, so that a window's three words have one address.
+constexpr uint32_t kFseRingBytes = 16 + 16 * kFseRing;
+constexpr uint32_t kFseScratch = 260 * 2 + 256 * 2 + 8; // a warp's table-build scratch: cum[260], next[256]
 
-// per lane: 16-bit entries (2 << tableLog), symbols (1 << tableLog), stream
-// ring (16-byte aligned for tableLog >= 4)
-__host__ __device__ __forceinline__ uint32_t fseSlotBytes(uint32_t tlMax) { return (3u << tlMax) + 16u * kFseRing; }
-__host__ __device__ __forceinline__ uint32_t fseSmemBytes(uint32_t lanes, uint32_t tlMax)
+// warps that build a CTA's tables (the first one then decodes): a table takes
+// about 5 us, and the scratch of the builders is the rings' memory where it fits
+__host__ __device__ __forceinline__ uint32_t fseWarps(uint32_t lanes) { return lanes >= 8 ? 3 : lanes >= 2 ? 2 : 1; }
+__host__ __device__ __forceinline__ uint32_t fseRingOff(uint32_t lanes, uint32_t tlMax, int cells)
 {
-    return lanes * fseSlotBytes(tlMax);
+    return lanes * ((cells == kCells32 ? 4u : 3u) << tlMax);
 }
+// shared memory of a CTA: tables of all lanes, then the rings (kFse) or the
+// build scratch, whichever is larger
+__host__ __device__ __forceinline__ uint32_t fseSmemBytes(uint32_t lanes, uint32_t tlMax, int cells)
+{
+    uint32_t const rings = lanes * kFseRingBytes, scratch = fseWarps(lanes) * kFseScratch;
+    return fseRingOff(lanes, tlMax, cells) + (rings > scratch ? rings : scratch);
+}
+// per lane of kFse4: 16-bit entries, symbols, stream ring (16-byte aligned
+// for tableLog >= 4)
+__host__ __device__ __forceinline__ uint32_t fse4SlotBytes(uint32_t tlMax) { return (3u << tlMax) + 16u * kFseRing; }
 
-// Builds the decoding table of task t in the slot at byte `slot` of the CTA's
-// shared memory with all 32 lanes of the warp (every lane calls it); `cum`
-// and `next` are the CTA's build scratch (257 and 256 entries).
+// Builds the decoding table of task t (cells or entries at tab, newStateBase
+// above the low NB bits of an entry; symbols at symOf, for kCells32 in the
+// cells themselves) with all 32 lanes of the warp (every lane calls it); `cum`
+// and `next` are the warp's build scratch (257 and 256 entries, next 16-byte
+// aligned).
 //  - Counts: the normalized counts go to the counters; a warp scan of
 //    the positive counts gives each symbol's first occurrence (cum), and the
 //    count -1 symbols take the top cells in symbol order.
@@ -1032,13 +1052,13 @@ __host__ __device__ __forceinline__ uint32_t fseSmemBytes(uint32_t lanes, uint32
 //    the same symbol (__match_any_sync); the highest such lane advances the
 //    counter.
 // The result equals the serial construction of fse_decompress.c:73-171.
-__device__ __forceinline__ void fseBuildWarp(const FseTask& t, uint8_t* smem, uint32_t slot, uint32_t tlMax,
-                                             uint16_t* cum, uint16_t* next)
+template <int CELLS>
+__device__ __forceinline__ void fseBuildWarp(const FseTask& t, void* tab, uint8_t* symOf, uint16_t* cum,
+                                             uint16_t* next)
 {
-    uint32_t const lane = threadIdx.x;
+    constexpr uint32_t SS = CELLS == kCells32 ? 4 : 1; // bytes from one cell's symbol to the next's
+    uint32_t const lane = threadIdx.x & 31;
     uint32_t const lt = (1u << lane) - 1u;
-    uint16_t* const tab = reinterpret_cast<uint16_t*>(smem + slot);
-    uint8_t* const symOf = smem + slot + (2u << tlMax);
     uint32_t const tl = t.tableLog;
     uint32_t const size = 1u << tl, mask = size - 1;
     uint32_t const step = (size >> 1) + (size >> 3) + 3;
@@ -1076,7 +1096,7 @@ __device__ __forceinline__ void fseBuildWarp(const FseTask& t, uint8_t* smem, ui
         cum[sy] = uint16_t(c0);
         c0 += v[k] > 0 ? uint32_t(v[k]) : 0u;
         if (v[k] == -1) {
-            symOf[size - 1 - n0] = uint8_t(sy);
+            symOf[SS * (size - 1 - n0)] = uint8_t(sy);
             next[sy] = 1;
             n0++;
         }
@@ -1092,7 +1112,7 @@ __device__ __forceinline__ void fseBuildWarp(const FseTask& t, uint8_t* smem, ui
         if (valid) {
             uint32_t const occ = occBase + __popc(bal & lt);
             while (occ >= cumNext && sCur < 255) cumNext = cum[++sCur + 1];
-            symOf[pos] = uint8_t(sCur);
+            symOf[SS * pos] = uint8_t(sCur);
         }
         occBase += __popc(bal);
     }
@@ -1100,7 +1120,7 @@ __device__ __forceinline__ void fseBuildWarp(const FseTask& t, uint8_t* smem, ui
     // cells
     for (uint32_t b0 = 0; b0 < size; b0 += 32) {
         uint32_t const u = b0 + lane;
-        uint32_t const sy = symOf[u];
+        uint32_t const sy = symOf[SS * u];
         uint32_t const m = __match_any_sync(0xffffffffu, sy);
         uint32_t const base = next[sy];
         __syncwarp();
@@ -1108,111 +1128,225 @@ __device__ __forceinline__ void fseBuildWarp(const FseTask& t, uint8_t* smem, ui
         uint32_t const x = base + __popc(m & lt);
         uint32_t const nb = tl - (31 - __clz(x));
         uint32_t const ns = (x << nb) - size;
-        tab[u] = uint16_t((ns << 4) | nb);
+        if (CELLS == kCells32) static_cast<uint32_t*>(tab)[u] = (ns << 18) | (sy << 8) | nb;
+        else static_cast<uint16_t*>(tab)[u] = uint16_t((ns << (CELLS == kCells24 ? 5 : 4)) | nb);
         __syncwarp();
     }
 }
 
-__global__ void __launch_bounds__(32) kFse(const FseTask* __restrict__ tasks, uint32_t nbTasks, uint32_t lanes,
-                                           uint32_t tableLogMax, uint32_t* __restrict__ status)
+// Decodes one stream (kFse's lane). `cell0` is the lane's first cell in the
+// CTA's tables, `tabBase` the byte of the entries of cell 0 (kCells24: symbols
+// are at byte `cell`), `ring` the byte of the lane's stream ring.
+//
+// What bounds it: a stream is a serial chain and an SM's shared memory holds
+// few streams, so a four-symbol step costs its dependent latencies and, with
+// one warp a scheduler, its instructions (two cycles each on the integer
+// pipe). Both were cut:
+//  - The position is one bit index, and each step loads the three stream words
+//    at it (one masked address, the ring's wrapped words are mirrored below
+//    it) and shifts out the 64 bits below it. The load runs beside the table
+//    lookups; neither waits for the other.
+//  - Five bits of nbBits in an entry are its own shift amount (shifts take the
+//    low five bits), also summed in pairs (two fields are at most 24 bits).
+//  - Ring refills come once per 32 symbols without a branch: up to three
+//    predicated 16-byte copies for the at most 48 bytes that the steps read,
+//    one commit, and a wait that leaves the last two refills' copies in
+//    flight. (A refill per step inside a branch was taken by some lane of the
+//    warp at nearly every step; branches around the copies, and copies through
+//    registers, measured 10 to 15 cycles a step slower than the predicates.)
+//  - Four steps fill one 16-byte store.
+// Cycles per step, one stream on an SM: 275 before, 115 with kCells24, 96 with
+// kCells32.
+// 32 K symbols at tableLog 11: 1.09 ms before, 0.40 ms now. Mixed batch of 4096
+// frames, largest FSE launch (beside others): 4.65 ms before, 2.60 ms now.
+template <int CELLS, int NST>
+__device__ __forceinline__ void fseDecode(const FseTask& t, const uint8_t* smem, uint32_t cell0, uint32_t tabBase,
+                                          uint32_t ring, uint32_t* status)
 {
-    extern __shared__ __align__(16) uint8_t smemFse[];
-    __shared__ uint16_t sCum[260];
-    __shared__ __align__(16) uint16_t sNext[256];
-    uint32_t const lane = threadIdx.x;
-    // every lane of the warp builds every table of the CTA, one at a time
-    for (uint32_t k = 0; k < lanes; k++) {
-        uint32_t const tk = blockIdx.x * lanes + k;
-        if (tk >= nbTasks) break;
-        FseTask const tt = tasks[tk];
-        fseBuildWarp(tt, smemFse, k * fseSlotBytes(tableLogMax), tableLogMax, sCum, sNext);
+    const uint8_t* g16;
+    int32_t pos, end;
+    if (!streamStart(t.bits, t.bitsSize, g16, pos, end)) { reportError(status, DERR_CORRUPTION); return; }
+    uint32_t const ringAddr = uint32_t(__cvta_generic_to_shared(smem + ring));
+    // The ring holds the stream's 16-byte chunks down to the one at byte `low`
+    // of g16 (not below 0); a copy of the ring's last chunk goes to the mirror.
+    // next(goal): the next chunk below, unless `low` has reached `goal`.
+    int32_t low;
+    auto next = [&](int32_t goal) {
+        asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 s;\n\t.reg .u64 a;\n\t"
+                     "setp.gt.s32 p, %0, %1;\n\t"
+                     "@p sub.s32 %0, %0, 16;\n\t"
+                     "and.b32 s, %0, %4;\n\t"
+                     "setp.eq.and.u32 q, s, %4, p;\n\t"
+                     "add.u32 s, s, %2;\n\t"
+                     "cvt.u64.u32 a, %0;\n\t"
+                     "add.u64 a, a, %3;\n\t"
+                     "@p cp.async.ca.shared.global [s], [a], 16;\n\t"
+                     "@q cp.async.ca.shared.global [s + %5], [a], 16;\n\t}"
+                     : "+r"(low) : "r"(goal), "r"(ringAddr), "l"(g16), "n"(16 * kFseRing - 16), "n"(-16 * kFseRing) : "memory");
+    };
+    {
+        int32_t const first = ((pos - 1) >> 7) * 16, goal = max(first - 16 * kFseAhead, 0);
+        low = first + 16;
+        while (low > goal) next(goal);
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
     }
-    if (lane >= lanes) return;
-    uint32_t const ti = blockIdx.x * lanes + lane;
-    if (ti >= nbTasks) return;
-    FseTask const t = tasks[ti];
-    uint32_t const slot = lane * fseSlotBytes(tableLogMax);
-    uint32_t* const ring = reinterpret_cast<uint32_t*>(smemFse + slot + (3u << tableLogMax));
-    const uint16_t* const tab = reinterpret_cast<const uint16_t*>(smemFse + slot);
-    const uint8_t* const symOf = smemFse + slot + (2u << tableLogMax);
-    uint32_t const tl = t.tableLog;
-
-    BitWin3<kFseRing, kFseAhead> br;
-    if (!br.init(t.bits, t.bitsSize, ring)) { reportError(status, DERR_CORRUPTION); return; }
-    uint32_t const nst = t.nbStates;
-    uint32_t st0 = br.read(tl), st1 = br.read(tl), st2 = 0, st3 = 0;
-    if (nst == 4) {
-        st2 = br.read(tl);
-        st3 = br.read(tl);
+    // Keeps kFseAhead chunks below the position's in the ring, given that at
+    // most N of them were read since the last call (48 bytes for three): N + 1
+    // may be needed until the next call, and were issued at least two calls
+    // before it.
+    auto refill = [&](auto nMax) {
+        int32_t const goal = max(((pos >> 3) & ~15) - 16 * kFseAhead, 0);
+#pragma unroll
+        for (int k = 0; k < decltype(nMax)::value; k++) next(goal);
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 2;" ::: "memory");
+    };
+    using One = std::integral_constant<int, 1>;
+    using Three = std::integral_constant<int, 3>;
+    // the 64 bits below pos, most significant first
+    auto window = [&](uint32_t& hi, uint32_t& lo) {
+        uint32_t const o = ring + ((uint32_t(pos) & (128 * kFseRing - 32)) >> 3);
+        uint32_t const a = *reinterpret_cast<const uint32_t*>(smem + o);
+        uint32_t const b = *reinterpret_cast<const uint32_t*>(smem + o - 4);
+        uint32_t const c = *reinterpret_cast<const uint32_t*>(smem + o - 8);
+        hi = __funnelshift_r(b, a, uint32_t(pos));
+        lo = __funnelshift_r(c, b, uint32_t(pos));
+    };
+    // A state is its cell's index (kCells32: its byte). ent: its cell or
+    // entry; to: the state that an entry and its field lead to; amt: the
+    // entry's shift amount (low five bits); nbOf: nbBits alone.
+    uint32_t const s00 = CELLS == kCells32 ? 4 * cell0 : cell0;
+    auto state = [&](uint32_t f) -> uint32_t { return s00 + (CELLS == kCells32 ? 4 * f : f); };
+    auto ent = [&](uint32_t st) -> uint32_t {
+        if (CELLS == kCells32) return *reinterpret_cast<const uint32_t*>(smem + st);
+        return *reinterpret_cast<const uint16_t*>(smem + tabBase + 2 * st);
+    };
+    auto sym = [&](uint32_t st) -> uint32_t { return CELLS == kCells32 ? smem[st + 1] : smem[st]; };
+    auto nbOf = [](uint32_t e) -> uint32_t { return CELLS == kCells24Wide ? e & 15u : e & 31u; };
+    auto amt = [&](uint32_t e) -> uint32_t { return CELLS == kCells24Wide ? e & 15u : e; };
+    auto to = [&](uint32_t e, uint32_t f) -> uint32_t {
+        return CELLS == kCells32 ? s00 + (e >> 16) + 4 * f : s00 + (e >> (CELLS == kCells24 ? 5 : 4)) + f;
+    };
+    auto top = [](uint32_t x, uint32_t n) -> uint32_t { return __funnelshift_l(x, 0u, n); }; // top n bits
+    auto read = [&](uint32_t n) -> uint32_t { // one field
+        refill(One());
+        uint32_t hi, lo;
+        window(hi, lo);
+        pos -= int32_t(n);
+        return top(hi, n);
+    };
+    uint32_t s0 = state(read(t.tableLog)), s1 = state(read(t.tableLog)), s2 = 0, s3 = 0;
+    if (NST == 4) {
+        s2 = state(read(t.tableLog));
+        s3 = state(read(t.tableLog));
     }
     uint32_t const n = t.dstSize;
-    uint32_t const lastTr = n > nst ? n - nst : 0; // symbols [0, lastTr) have a transition
+    uint32_t const lastTr = n > NST ? n - NST : 0; // symbols [0, lastTr) have a transition
     uint8_t* const out = t.out;
-    auto ent = [&](uint32_t st) -> uint32_t { return tab[st]; };
-    auto sym = [&](uint32_t st) -> uint32_t { return symOf[st]; };
-    auto nbOf = [](uint32_t e) -> uint32_t { return e & 15u; };
-    auto nextOf = [](uint32_t e, uint32_t f) -> uint32_t { return (e >> 4) + f; };
-    // one transition: its field is the top bits of the 64-bit register window
-    // (hi, lo), which then shifts them out; four fields take at most 48 bits
-    auto take = [](uint32_t e, uint32_t& hi, uint32_t& lo) -> uint32_t {
-        uint32_t const nb = e & 15u;
-        uint32_t const f = __funnelshift_l(hi, 0u, nb);
-        hi = __funnelshift_l(lo, hi, nb);
-        lo <<= nb;
-        return (e >> 4) + f;
-    };
-    // one symbol from st0, then the states rotate
+    // one symbol from s0, then the states rotate
     auto single = [&](uint32_t i) {
-        uint32_t const e = ent(st0);
-        out[i] = uint8_t(sym(st0));
-        uint32_t ns = st0;
-        if (i < lastTr) ns = nextOf(e, br.read(nbOf(e)));
-        if (nst == 4) {
-            st0 = st1; st1 = st2; st2 = st3; st3 = ns;
+        uint32_t const e = ent(s0);
+        out[i] = uint8_t(sym(s0));
+        uint32_t ns = s0;
+        if (i < lastTr) ns = to(e, read(nbOf(e)));
+        if (NST == 4) {
+            s0 = s1; s1 = s2; s2 = s3; s3 = ns;
         } else {
-            st0 = st1; st1 = ns;
+            s0 = s1; s1 = ns;
         }
+    };
+    // four symbols with transitions, as one little-endian word
+    auto step = [&]() -> uint32_t {
+        uint32_t hi, lo, e0, e1, e2 = 0, e3 = 0, y0 = 0, y1 = 0, y2 = 0, y3 = 0;
+        window(hi, lo);
+        e0 = ent(s0);
+        e1 = ent(s1);
+        if (NST == 4) {
+            e2 = ent(s2);
+            e3 = ent(s3);
+        }
+        if (CELLS != kCells32) {
+            y0 = sym(s0);
+            y1 = sym(s1);
+            if (NST == 4) {
+                y2 = sym(s2);
+                y3 = sym(s3);
+            }
+        }
+        uint32_t const a0 = amt(e0), a1 = amt(e1), a01 = a0 + a1;
+        uint32_t const hi2 = __funnelshift_l(lo, hi, a01); // 32 bits from the second pair's fields on
+        s0 = to(e0, top(hi, a0));
+        s1 = to(e1, top(__funnelshift_l(0u, hi, a0), a1));
+        if (NST == 2) { // the second pair's lookups follow the first pair's
+            e2 = ent(s0);
+            e3 = ent(s1);
+            if (CELLS != kCells32) {
+                y2 = sym(s0);
+                y3 = sym(s1);
+            }
+        }
+        uint32_t const a2 = amt(e2), a3 = amt(e3), a23 = a2 + a3;
+        uint32_t const f2 = top(hi2, a2), f3 = top(__funnelshift_l(0u, hi2, a2), a3);
+        if (NST == 4) {
+            s2 = to(e2, f2);
+            s3 = to(e3, f3);
+        } else {
+            s0 = to(e2, f2);
+            s1 = to(e3, f3);
+        }
+        pos -= int32_t((a01 & 31u) + (a23 & 31u));
+        if (CELLS == kCells32) return __byte_perm(__byte_perm(e0, e1, 0x0051), __byte_perm(e2, e3, 0x0051), 0x5410);
+        return __byte_perm(__byte_perm(y0, y1, 0x0040), __byte_perm(y2, y3, 0x0040), 0x5410);
     };
     uint32_t i = 0;
-    uint32_t const head = min(n, uint32_t((4 - (reinterpret_cast<uintptr_t>(out) & 3)) & 3));
+    uint32_t const head = min(n, uint32_t((16 - (reinterpret_cast<uintptr_t>(out) & 15)) & 15));
     for (; i < head; i++) single(i);
-    if (nst == 4) {
-        for (; i + 4 <= lastTr; i += 4) {
-            br.prepare();
-            // the 64 bits below pos, left-aligned (g is in [0, 32])
-            uint32_t hi = __funnelshift_lc(br.b, br.a, uint32_t(br.g));
-            uint32_t lo = __funnelshift_lc(br.c, br.b, uint32_t(br.g));
-            uint32_t const ea = ent(st0), eb = ent(st1), ec = ent(st2), ed = ent(st3);
-            uint32_t const ya = sym(st0), yb = sym(st1), yc = sym(st2), yd = sym(st3);
-            st0 = take(ea, hi, lo);
-            st1 = take(eb, hi, lo);
-            st2 = take(ec, hi, lo);
-            st3 = take(ed, hi, lo);
-            br.advance(int32_t(nbOf(ea) + nbOf(eb) + nbOf(ec) + nbOf(ed)));
-            *reinterpret_cast<uint32_t*>(out + i) =
-                __byte_perm(__byte_perm(ya, yb, 0x0040), __byte_perm(yc, yd, 0x0040), 0x5410);
+    for (; i + 32 <= lastTr; i += 32) {
+        refill(Three());
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            uint4 v;
+            v.x = step();
+            v.y = step();
+            v.z = step();
+            v.w = step();
+            *reinterpret_cast<uint4*>(out + i + 16 * h) = v;
         }
-    } else {
-        for (; i + 4 <= lastTr; i += 4) {
-            br.prepare();
-            uint32_t hi = __funnelshift_lc(br.b, br.a, uint32_t(br.g));
-            uint32_t lo = __funnelshift_lc(br.c, br.b, uint32_t(br.g));
-            uint32_t const ea = ent(st0), eb = ent(st1);
-            uint32_t const ya = sym(st0), yb = sym(st1);
-            st0 = take(ea, hi, lo);
-            st1 = take(eb, hi, lo);
-            uint32_t const ec = ent(st0), ed = ent(st1);
-            uint32_t const yc = sym(st0), yd = sym(st1);
-            st0 = take(ec, hi, lo);
-            st1 = take(ed, hi, lo);
-            br.advance(int32_t(nbOf(ea) + nbOf(eb) + nbOf(ec) + nbOf(ed)));
-            *reinterpret_cast<uint32_t*>(out + i) =
-                __byte_perm(__byte_perm(ya, yb, 0x0040), __byte_perm(yc, yd, 0x0040), 0x5410);
-        }
+    }
+    for (; i + 4 <= lastTr; i += 4) {
+        refill(One());
+        *reinterpret_cast<uint32_t*>(out + i) = step();
     }
     for (; i < n; i++) single(i);
     asm volatile("cp.async.wait_all;" ::: "memory"); // no copy outlives the lane
-    if (!br.finished()) reportError(status, DERR_CORRUPTION);
+    if (pos != end) reportError(status, DERR_CORRUPTION);
+}
+
+template <int CELLS>
+__global__ void __launch_bounds__(96) kFse(const FseTask* __restrict__ tasks, uint32_t nbTasks, uint32_t lanes,
+                                           uint32_t tableLogMax, uint32_t* __restrict__ status)
+{
+    extern __shared__ __align__(16) uint8_t smemFse[];
+    uint32_t const wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t const tabBase = CELLS == kCells32 ? 0 : lanes << tableLogMax;
+    uint32_t const ringOff = fseRingOff(lanes, tableLogMax, CELLS);
+    // every warp builds its share of the CTA's tables, one at a time
+    {
+        uint16_t* const next = reinterpret_cast<uint16_t*>(smemFse + ringOff + wid * kFseScratch);
+        for (uint32_t k = wid; k < lanes; k += blockDim.x >> 5) {
+            uint32_t const tk = blockIdx.x * lanes + k;
+            if (tk >= nbTasks) break;
+            FseTask const tt = tasks[tk];
+            uint8_t* const tab = smemFse + tabBase + (k << tableLogMax) * (CELLS == kCells32 ? 4 : 2);
+            fseBuildWarp<CELLS>(tt, tab, CELLS == kCells32 ? tab + 1 : smemFse + (k << tableLogMax), next + 256, next);
+        }
+    }
+    __syncthreads();
+    uint32_t const ti = blockIdx.x * lanes + lane;
+    if (wid != 0 || lane >= lanes || ti >= nbTasks) return;
+    FseTask const t = tasks[ti];
+    uint32_t const cell0 = lane << tableLogMax, ring = ringOff + lane * kFseRingBytes + 16;
+    if (t.nbStates == 4) fseDecode<CELLS, 4>(t, smemFse, cell0, tabBase, ring, status);
+    else fseDecode<CELLS, 2>(t, smemFse, cell0, tabBase, ring, status);
 }
 
 // FSE with one lane per state: a warp decodes up to eight streams, four lanes
@@ -1241,14 +1375,15 @@ __global__ void __launch_bounds__(32) kFse4(const FseTask* __restrict__ tasks, u
         uint32_t const tk = blockIdx.x * streams + q;
         if (tk >= nbTasks) break;
         FseTask const tt = tasks[tk];
-        fseBuildWarp(tt, smemFse, q * fseSlotBytes(tableLogMax), tableLogMax, sCum, sNext);
+        uint8_t* const sl = smemFse + q * fse4SlotBytes(tableLogMax);
+        fseBuildWarp<kCells24Wide>(tt, sl, sl + (2u << tableLogMax), sCum, sNext);
     }
     uint32_t const grp = lane >> 2, k = lane & 3;
     uint32_t const ti = blockIdx.x * streams + grp;
     FseTask t{};
     bool ok = grp < streams && ti < nbTasks;
     if (ok) t = tasks[ti];
-    uint32_t const slot = grp * fseSlotBytes(tableLogMax);
+    uint32_t const slot = grp * fse4SlotBytes(tableLogMax);
     uint32_t* const ring = reinterpret_cast<uint32_t*>(smemFse + slot + (3u << tableLogMax));
     const uint16_t* const tab = reinterpret_cast<const uint16_t*>(smemFse + slot);
     const uint8_t* const symOf = smemFse + slot + (2u << tableLogMax);
@@ -2049,16 +2184,13 @@ __global__ void __launch_bounds__(32 * kFinishWarps) kHashFinish(const HashTask*
 namespace ozl {
 
 namespace {
-uint32_t fseLanes(uint32_t tlMax)
+uint32_t fseLanes(uint32_t tlMax, int cells = kCells24)
 {
     uint32_t lanes = 32;
-    while (lanes > 1 && fseSmemBytes(lanes, tlMax) > kFseCtaSmem) lanes--;
+    while (lanes > 1 && fseSmemBytes(lanes, tlMax, cells) > kFseCtaSmem) lanes--;
     return lanes;
 }
-uint32_t hufSmem(uint32_t chunks) { return hufRingOff(chunks) + 4 * chunks * 16 * kHufRing; }
-// kHashBlocks grid: one warp per block up to eight full CTAs per SM, then
-// grid-stride (any grid size is correct)
-uint32_t hashGrid(uint32_t nbBlocks)
+int smCount()
 {
     static int sms = 0;
     if (!sms) {
@@ -2067,8 +2199,45 @@ uint32_t hashGrid(uint32_t nbBlocks)
             sms = n;
         if (sms <= 0) sms = 152;
     }
+    return sms;
+}
+// Table form and streams per CTA of an FSE launch.
+// 32-bit cells step faster (96 against 115 cycles) but take a third more
+// shared memory: they are used while every stream of the launch fits the SMs
+// at once (24 per SM at tableLog 11), and for small tables; 24-bit cells where
+// the streams come in waves (32 per SM).
+// Untuned, small tables run as many lanes a CTA as fit. Large ones spread over
+// the SMs first (a stream alone in its warp steps fastest), up to what four
+// CTAs of an SM hold: one decoding warp for each of its schedulers.
+struct FseShape {
+    int cells;
+    uint32_t lanes;
+};
+FseShape fseShape(const Launch& l)
+{
+    uint32_t const sms = uint32_t(smCount()), perSm = (l.nbTasks + sms - 1) / sms;
+    auto quarter = [&](int cells) { // streams of a CTA of which four fit an SM
+        uint32_t lanes = 32;
+        while (lanes > 1 && fseSmemBytes(lanes, l.param0, cells) > kFseQuarterSmem) lanes--;
+        return lanes;
+    };
+    FseShape s;
+    s.cells = l.param0 >= 12                                          ? kCells24Wide
+              : l.param0 <= 8 || perSm <= 4 * quarter(kCells32) ? kCells32
+                                                                      : kCells24;
+    uint32_t const maxLanes = fseLanes(l.param0, s.cells);
+    s.lanes = l.tune & 0xFFu;
+    if (!s.lanes) s.lanes = l.param0 <= 8 ? maxLanes : std::min((perSm + 3) / 4, quarter(s.cells));
+    s.lanes = std::max(1u, std::min(s.lanes, maxLanes));
+    return s;
+}
+uint32_t hufSmem(uint32_t chunks) { return hufRingOff(chunks) + 4 * chunks * 16 * kHufRing; }
+// kHashBlocks grid: one warp per block up to eight full CTAs per SM, then
+// grid-stride (any grid size is correct)
+uint32_t hashGrid(uint32_t nbBlocks)
+{
     uint32_t const want = (nbBlocks + 7) / 8;
-    uint32_t const cap = uint32_t(sms) * 8;
+    uint32_t const cap = uint32_t(smCount()) * 8;
     return want < cap ? (want ? want : 1) : cap;
 }
 static_assert(2 * kHufSlotBytes >= (2u << kHufTableLog), "a tableLog-12 table fits two slots");
@@ -2076,8 +2245,11 @@ static_assert(2 * kHufSlotBytes >= (2u << kHufTableLog), "a tableLog-12 table fi
 
 cudaError_t prepareKernels()
 {
-    cudaError_t e = cudaFuncSetAttribute(kFse, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFseCtaSmem));
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
+    for (auto* const k : { kFse<kCells32>, kFse<kCells24>, kFse<kCells24Wide> }) {
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFseCtaSmem));
+        if (e != cudaSuccess) return e;
+    }
     e = cudaFuncSetAttribute(kFse4, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFseCtaSmem));
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(kHuf, cudaFuncAttributeMaxDynamicSharedMemorySize, int(hufSmem(kHufChunks)));
@@ -2088,7 +2260,7 @@ uint32_t tuneCandidates(const Launch& l, uint32_t* out, uint32_t cap)
     uint32_t n = 0;
     if (l.kind == KIND_FSE) {
         uint32_t const mx = fseLanes(l.param0);
-        for (uint32_t c : { 32u, 16u, 8u, 6u, 5u, 4u, 3u, 2u })
+        for (uint32_t c : { 32u, 17u, 11u, 8u, 6u, 5u, 4u, 2u })
             if (c <= mx && n < cap) out[n++] = c;
         for (uint32_t c : { 8u, 6u, 4u }) // kFse4: streams per warp
             if (c <= mx && n < cap) out[n++] = kFse4Variant | c;
@@ -2127,25 +2299,22 @@ long runOneLaunch(const DeviceLayout& L, size_t li, uint8_t* dPool, uint8_t* dSc
                 break;
             case KIND_FSE: {
                 uint32_t const maxLanes = fseLanes(l.param0);
-                // untuned: large tables six streams per warp, the autotuner's
-                // choice on the mixed-frame workload (wider CTAs wait on their
-                // serial table builds and leave too few warps per SM to hide
-                // latency); small tables as many as fit
                 if (l.tune & kFse4Variant) { // one lane per state, up to eight streams per warp
                     uint32_t streams = l.tune & 0xFFu;
                     if (streams > 8) streams = 8;
                     if (streams > maxLanes) streams = maxLanes;
                     if (streams == 0) streams = 1;
                     uint32_t const grid = (l.nbTasks + streams - 1) / streams;
-                    kFse4<<<grid, 32, fseSmemBytes(streams, l.param0), s>>>(static_cast<const FseTask*>(tasks), l.nbTasks,
+                    kFse4<<<grid, 32, streams * fse4SlotBytes(l.param0), s>>>(static_cast<const FseTask*>(tasks), l.nbTasks,
                                                                             streams, l.param0, dStatus);
                     break;
                 }
-                uint32_t const dflt = l.param0 <= 8 || maxLanes < kFseDefaultLanes ? maxLanes : kFseDefaultLanes;
-                uint32_t const lanes = l.tune && l.tune <= maxLanes ? l.tune : dflt;
-                uint32_t const grid = (l.nbTasks + lanes - 1) / lanes;
-                kFse<<<grid, 32, fseSmemBytes(lanes, l.param0), s>>>(static_cast<const FseTask*>(tasks), l.nbTasks,
-                                                                     lanes, l.param0, dStatus);
+                FseShape const sh = fseShape(l);
+                uint32_t const grid = (l.nbTasks + sh.lanes - 1) / sh.lanes;
+                auto* const k = sh.cells == kCells32 ? kFse<kCells32> : sh.cells == kCells24 ? kFse<kCells24>
+                                                                                              : kFse<kCells24Wide>;
+                k<<<grid, 32 * fseWarps(sh.lanes), fseSmemBytes(sh.lanes, l.param0, sh.cells), s>>>(
+                        static_cast<const FseTask*>(tasks), l.nbTasks, sh.lanes, l.param0, dStatus);
                 break;
             }
             case KIND_HUF: {

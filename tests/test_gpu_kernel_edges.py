@@ -23,3 +23,53 @@ def test_xxh3_around_the_chain_batches(gpu_lib, offset):
     for n in lengths:
         want = oracle.lib().ozo_xxh3_64(data[offset:].ctypes.data, n)
         assert oz.xxh3_64_device(dev.data_ptr() + offset, n) == want, n
+
+
+def _round_trip(arrays, recipe, width, dst_offsets):
+    """Compresses on the device, decodes to destinations at the given offsets
+    from a 16-byte boundary and returns the decoded bytes and the frames."""
+    import torch
+    import openzl_gb300 as oz
+
+    enc, n = oz.GpuEncoder(), len(arrays)
+    srcs = [torch.from_numpy(a.view(np.uint8).copy()).cuda() for a in arrays]
+    caps = [enc.bound(a.nbytes) for a in arrays]
+    dsts = [torch.zeros(c, dtype=torch.uint8, device="cuda") for c in caps]
+    sizes = enc.compress_batch([s.data_ptr() for s in srcs], [a.size for a in arrays], [width] * n, [recipe] * n,
+                               [d.data_ptr() for d in dsts], caps, checksums=True)
+    frames = [d[:s].cpu().numpy() for d, s in zip(dsts, sizes)]
+    outs = [torch.zeros(a.nbytes + 32, dtype=torch.uint8, device="cuda") for a in arrays]
+    batch = oz.GpuBatch()
+    batch.plan(frames, [d.data_ptr() for d in dsts], [o.data_ptr() + k for o, k in zip(outs, dst_offsets)],
+               [a.nbytes for a in arrays])
+    batch.run(0, graph=False)
+    batch.check(0)
+    got = [o.cpu().numpy() for o in outs]
+    for a, g, k in zip(arrays, got, dst_offsets):
+        assert not g[:k].any() and not g[k + a.nbytes:].any(), a.size  # nothing outside the destination
+    return [g[k:k + a.nbytes] for a, g, k in zip(arrays, got, dst_offsets)], frames
+
+
+def test_fse_blocks_alignments_and_table_forms(gpu_lib):
+    """Streams of every length around the 32-symbol blocks of the decoder at
+    every destination alignment, from almost no bits a symbol to near 8, then
+    more streams than the SMs hold at once, whose tables take the packed form."""
+    rng = np.random.default_rng(32)
+    arrays = []
+    for n in list(range(20, 140)) + [1000 + k for k in range(40)] + [4096 + k for k in range(36)] + [32767, 32768, 99999]:
+        kind = n % 4
+        if kind == 0:
+            a = (rng.random(n) < 0.03).astype(np.uint8)
+        elif kind == 1:
+            a = (rng.zipf(1.3, n) % 7).astype(np.uint8)
+        elif kind == 2:
+            a = np.minimum(rng.geometric(0.05, n), 255).astype(np.uint8)
+        else:
+            a = np.minimum(np.abs(rng.normal(100, 30, n)), 255).astype(np.uint8)
+        arrays.append(a)
+    out, frames = _round_trip(arrays, 7, 0, [k % 16 for k in range(len(arrays))])
+    for a, g, f in zip(arrays, out, frames):
+        assert g.tobytes() == a.tobytes() == oracle.decompress(f)[0].tobytes(), a.size
+    many = [np.minimum(rng.geometric(0.04, 4097 + k % 300), 255).astype(np.uint8) for k in range(6000)]
+    out, _ = _round_trip(many, 7, 0, [k % 16 for k in range(len(many))])
+    assert all(g.tobytes() == a.tobytes() for a, g in zip(many, out))
