@@ -915,84 +915,76 @@ __device__ __forceinline__ bool streamStart(const uint8_t* p, uint32_t size, con
     return true;
 }
 
-// Backward bit reader (FSE and Huffman decoders): three stream words in
-// registers, a (bits [cb + 64, cb + 96)) above b and c (bits [cb, cb + 32)),
-// cb = 32 * kb, and g = cb + 96 - pos, the bits of the window already read.
-// Invariant: g <= 32 at the start of every step. The four-symbol loops take
-// the 64 bits just below pos as one left-aligned register pair (hi, lo) =
-// two funnel shifts of (a, b, c), peel each field off the top of the pair,
-// and then call advance() once with the step's total. A step reads at most
-// four fields of at most 12 bits (FSE tableLog <= 12, Huffman codes <= 12
-// bits), i.e. n <= 48, so g + n <= 80 < 96 stays inside the three words, and
-// advance() drops one or two words without a branch, leaving g <= 32 again.
-// read(nb) is the one-field path (stream heads, tails and initial states):
-// it takes window(g), the 32 bits starting g bits below the top of the
-// window. prepare(), once per step, makes the next two words of the ring
-// readable. Words below the stream are never consumed by a valid stream
-// (finished() checks that the stream ends exactly at its first bit), so the
-// ring's stale contents may stand in for them.
+// Backward bit reader by position (FSE and Huffman decoders): `pos` is
+// one bit index, window() loads the three stream words at it (one masked
+// address) and shifts out the 64 bits below it. The stream's 16-byte chunks
+// lie in a ring of RING chunks at byte `ring` of shared memory, from the
+// position's down to the one at byte `low` of g16; the ring's last chunk is
+// copied to the 16 bytes below the ring too, so that a window's words never
+// wrap. Words below the stream are never consumed by a valid stream
+// (finished() checks that it ends exactly at its first bit), so the ring's
+// stale contents may stand in for them.
 template <int RING, int AHEAD>
-struct BitWin3 {
-    StreamRing<RING, AHEAD> r;
-    uint32_t a, b, c;
-    int32_t kb, g, end;
+struct PosStream {
+    static_assert((RING & (RING - 1)) == 0 && AHEAD + 4 <= RING, "ring shape");
+    static constexpr uint32_t kBytes = 16 + 16 * RING; // mirror and ring, 16-byte aligned
+    const uint8_t *g16, *smem;
+    uint32_t ring, ringAddr;
+    int32_t pos, end, low;
 
-    __device__ __forceinline__ bool init(const uint8_t* p, uint32_t size, uint32_t* ring)
+    // the next chunk below, unless `low` has reached `goal` (not below 0)
+    __device__ __forceinline__ void next(int32_t goal)
     {
-        int32_t pos;
-        if (!streamStart(p, size, r.g16, pos, end)) return false;
-        r.ring = ring;
-        r.start(pos);
-        int32_t const jt = (pos - 1) >> 5; // word of the top unread bit
-        a = r.word(jt);
-        b = r.word(jt - 1);
-        c = r.word(jt - 2);
-        kb = jt - 2;
-        g = (kb + 3) * 32 - pos; // in [0, 32)
+        asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 s;\n\t.reg .u64 a;\n\t"
+                     "setp.gt.s32 p, %0, %1;\n\t"
+                     "@p sub.s32 %0, %0, 16;\n\t"
+                     "and.b32 s, %0, %4;\n\t"
+                     "setp.eq.and.u32 q, s, %4, p;\n\t"
+                     "add.u32 s, s, %2;\n\t"
+                     "cvt.u64.u32 a, %0;\n\t"
+                     "add.u64 a, a, %3;\n\t"
+                     "@p cp.async.ca.shared.global.L2::128B [s], [a], 16;\n\t"
+                     "@q cp.async.ca.shared.global.L2::128B [s + %5], [a], 16;\n\t}"
+                     : "+r"(low) : "r"(goal), "r"(ringAddr), "l"(g16), "n"(16 * RING - 16), "n"(-16 * RING) : "memory");
+    }
+    // `area`: byte of the kBytes of shared memory
+    __device__ __forceinline__ bool init(const uint8_t* p, uint32_t size, const uint8_t* sm, uint32_t area)
+    {
+        if (!streamStart(p, size, g16, pos, end)) return false;
+        smem = sm;
+        ring = area + 16;
+        ringAddr = uint32_t(__cvta_generic_to_shared(sm + ring));
+        int32_t const first = ((pos - 1) >> 7) * 16, goal = max(first - 16 * AHEAD, 0);
+        low = first + 16;
+        while (low > goal) next(goal);
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
         return true;
     }
-    __device__ __forceinline__ void prepare()
+    // Keeps AHEAD chunks below the position's in the ring, given that at most
+    // N <= 3 of them were read since the last call: N + 1 may be needed until
+    // the next call, and were issued at least two calls before it.
+    template <int N>
+    __device__ __forceinline__ void refill()
     {
-        int32_t const m = (kb - 2) >> 2;
-        if (m < r.low) {
-            r.low = m;
-            r.issue(m - AHEAD);
-            asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
-        }
+        static_assert(3 * N + 1 <= AHEAD, "a chunk is issued two calls before it is read");
+        int32_t const goal = max(((pos >> 3) & ~15) - 16 * AHEAD, 0);
+#pragma unroll
+        for (int k = 0; k < N; k++) next(goal);
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 2;" ::: "memory");
     }
-    // the 32 bits starting o bits below the top of the window (o <= 56)
-    __device__ __forceinline__ uint32_t window(int32_t o) const
+    // the 64 bits below pos, most significant first
+    __device__ __forceinline__ void window(uint32_t& hi, uint32_t& lo) const
     {
-        uint32_t const hiPair = __funnelshift_l(b, a, uint32_t(o));      // o < 32
-        uint32_t const loPair = __funnelshift_l(c, b, uint32_t(o - 32)); // 32 <= o <= 56
-        return o < 32 ? hiPair : loPair;
+        uint32_t const o = ring + ((uint32_t(pos) & (128 * RING - 32)) >> 3);
+        uint32_t const a = *reinterpret_cast<const uint32_t*>(smem + o);
+        uint32_t const b = *reinterpret_cast<const uint32_t*>(smem + o - 4);
+        uint32_t const c = *reinterpret_cast<const uint32_t*>(smem + o - 8);
+        hi = __funnelshift_r(b, a, uint32_t(pos));
+        lo = __funnelshift_r(c, b, uint32_t(pos));
     }
-    // drops the n bits read since the start of the step (g + n <= 96)
-    __device__ __forceinline__ void advance(int32_t n)
-    {
-        uint32_t const w1 = r.ring[(kb - 1) & (4 * RING - 1)];
-        uint32_t const w2 = r.ring[(kb - 2) & (4 * RING - 1)];
-        g += n;
-        bool const one = g > 32, two = g > 64;
-        uint32_t const na = two ? c : (one ? b : a);
-        uint32_t const nb = two ? w1 : (one ? c : b);
-        uint32_t const nc = two ? w2 : (one ? w1 : c);
-        a = na;
-        b = nb;
-        c = nc;
-        int32_t const k = int32_t(one) + int32_t(two);
-        kb -= k;
-        g -= 32 * k;
-    }
-    // one field of nb bits (nb <= 12) just below pos
-    __device__ __forceinline__ uint32_t read(uint32_t nb)
-    {
-        prepare();
-        uint32_t const f = __funnelshift_l(window(g), 0u, nb);
-        advance(int32_t(nb));
-        return f;
-    }
-    __device__ __forceinline__ bool finished() const { return (kb + 3) * 32 - g == end; }
+    __device__ __forceinline__ bool finished() const { return pos == end; }
+    // ends the stream: no copy outlives the lane
+    __device__ __forceinline__ void close() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 };
 
 // ---------------------------------------------------------------------------
@@ -1013,9 +1005,8 @@ constexpr uint32_t kFseCtaSmem = 224 * 1024; // up to 32 tableLog-11 lanes per C
 
 constexpr uint32_t kFseQuarterSmem = 56 * 1024; // four CTAs of this much fit an SM
 constexpr int kFseRing = 16, kFseAhead = 12;   // stream ring: 256 bytes per lane, 192 bytes ahead
-// The ring of a kFse stream follows a copy of its last 16 bytes: the words
-// below the ring's first one, so that a window's three words have one address.
-constexpr uint32_t kFseRingBytes = 16 + 16 * kFseRing;
+using FseStream = PosStream<kFseRing, kFseAhead>;
+constexpr uint32_t kFseRingBytes = FseStream::kBytes;
 constexpr uint32_t kFseScratch = 260 * 2 + 256 * 2 + 8; // a warp's table-build scratch: cum[260], next[256]
 
 // warps that build a CTA's tables (the first one then decodes): a table takes
@@ -1136,16 +1127,15 @@ __device__ __forceinline__ void fseBuildWarp(const FseTask& t, void* tab, uint8_
 
 // Decodes one stream (kFse's lane). `cell0` is the lane's first cell in the
 // CTA's tables, `tabBase` the byte of the entries of cell 0 (kCells24: symbols
-// are at byte `cell`), `ring` the byte of the lane's stream ring.
+// are at byte `cell`), `area` the byte of the lane's stream ring.
 //
 // What bounds it: a stream is a serial chain and an SM's shared memory holds
 // few streams, so a four-symbol step costs its dependent latencies and, with
 // one warp a scheduler, its instructions (two cycles each on the integer
 // pipe). Both were cut:
-//  - The position is one bit index, and each step loads the three stream words
-//    at it (one masked address, the ring's wrapped words are mirrored below
-//    it) and shifts out the 64 bits below it. The load runs beside the table
-//    lookups; neither waits for the other.
+//  - The position is one bit index, and each step loads the stream words at it
+//    (PosStream). The loads run beside the table lookups; neither waits for
+//    the other.
 //  - Five bits of nbBits in an entry are its own shift amount (shifts take the
 //    low five bits), also summed in pairs (two fields are at most 24 bits).
 //  - Ring refills come once per 32 symbols without a branch: up to three
@@ -1161,56 +1151,10 @@ __device__ __forceinline__ void fseBuildWarp(const FseTask& t, void* tab, uint8_
 // frames, largest FSE launch (beside others): 4.65 ms before, 2.60 ms now.
 template <int CELLS, int NST>
 __device__ __forceinline__ void fseDecode(const FseTask& t, const uint8_t* smem, uint32_t cell0, uint32_t tabBase,
-                                          uint32_t ring, uint32_t* status)
+                                          uint32_t area, uint32_t* status)
 {
-    const uint8_t* g16;
-    int32_t pos, end;
-    if (!streamStart(t.bits, t.bitsSize, g16, pos, end)) { reportError(status, DERR_CORRUPTION); return; }
-    uint32_t const ringAddr = uint32_t(__cvta_generic_to_shared(smem + ring));
-    // The ring holds the stream's 16-byte chunks down to the one at byte `low`
-    // of g16 (not below 0); a copy of the ring's last chunk goes to the mirror.
-    // next(goal): the next chunk below, unless `low` has reached `goal`.
-    int32_t low;
-    auto next = [&](int32_t goal) {
-        asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 s;\n\t.reg .u64 a;\n\t"
-                     "setp.gt.s32 p, %0, %1;\n\t"
-                     "@p sub.s32 %0, %0, 16;\n\t"
-                     "and.b32 s, %0, %4;\n\t"
-                     "setp.eq.and.u32 q, s, %4, p;\n\t"
-                     "add.u32 s, s, %2;\n\t"
-                     "cvt.u64.u32 a, %0;\n\t"
-                     "add.u64 a, a, %3;\n\t"
-                     "@p cp.async.ca.shared.global [s], [a], 16;\n\t"
-                     "@q cp.async.ca.shared.global [s + %5], [a], 16;\n\t}"
-                     : "+r"(low) : "r"(goal), "r"(ringAddr), "l"(g16), "n"(16 * kFseRing - 16), "n"(-16 * kFseRing) : "memory");
-    };
-    {
-        int32_t const first = ((pos - 1) >> 7) * 16, goal = max(first - 16 * kFseAhead, 0);
-        low = first + 16;
-        while (low > goal) next(goal);
-        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-    }
-    // Keeps kFseAhead chunks below the position's in the ring, given that at
-    // most N of them were read since the last call (48 bytes for three): N + 1
-    // may be needed until the next call, and were issued at least two calls
-    // before it.
-    auto refill = [&](auto nMax) {
-        int32_t const goal = max(((pos >> 3) & ~15) - 16 * kFseAhead, 0);
-#pragma unroll
-        for (int k = 0; k < decltype(nMax)::value; k++) next(goal);
-        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 2;" ::: "memory");
-    };
-    using One = std::integral_constant<int, 1>;
-    using Three = std::integral_constant<int, 3>;
-    // the 64 bits below pos, most significant first
-    auto window = [&](uint32_t& hi, uint32_t& lo) {
-        uint32_t const o = ring + ((uint32_t(pos) & (128 * kFseRing - 32)) >> 3);
-        uint32_t const a = *reinterpret_cast<const uint32_t*>(smem + o);
-        uint32_t const b = *reinterpret_cast<const uint32_t*>(smem + o - 4);
-        uint32_t const c = *reinterpret_cast<const uint32_t*>(smem + o - 8);
-        hi = __funnelshift_r(b, a, uint32_t(pos));
-        lo = __funnelshift_r(c, b, uint32_t(pos));
-    };
+    FseStream br;
+    if (!br.init(t.bits, t.bitsSize, smem, area)) { reportError(status, DERR_CORRUPTION); return; }
     // A state is its cell's index (kCells32: its byte). ent: its cell or
     // entry; to: the state that an entry and its field lead to; amt: the
     // entry's shift amount (low five bits); nbOf: nbBits alone.
@@ -1228,10 +1172,10 @@ __device__ __forceinline__ void fseDecode(const FseTask& t, const uint8_t* smem,
     };
     auto top = [](uint32_t x, uint32_t n) -> uint32_t { return __funnelshift_l(x, 0u, n); }; // top n bits
     auto read = [&](uint32_t n) -> uint32_t { // one field
-        refill(One());
+        br.refill<1>();
         uint32_t hi, lo;
-        window(hi, lo);
-        pos -= int32_t(n);
+        br.window(hi, lo);
+        br.pos -= int32_t(n);
         return top(hi, n);
     };
     uint32_t s0 = state(read(t.tableLog)), s1 = state(read(t.tableLog)), s2 = 0, s3 = 0;
@@ -1257,7 +1201,7 @@ __device__ __forceinline__ void fseDecode(const FseTask& t, const uint8_t* smem,
     // four symbols with transitions, as one little-endian word
     auto step = [&]() -> uint32_t {
         uint32_t hi, lo, e0, e1, e2 = 0, e3 = 0, y0 = 0, y1 = 0, y2 = 0, y3 = 0;
-        window(hi, lo);
+        br.window(hi, lo);
         e0 = ent(s0);
         e1 = ent(s1);
         if (NST == 4) {
@@ -1293,7 +1237,7 @@ __device__ __forceinline__ void fseDecode(const FseTask& t, const uint8_t* smem,
             s0 = to(e2, f2);
             s1 = to(e3, f3);
         }
-        pos -= int32_t((a01 & 31u) + (a23 & 31u));
+        br.pos -= int32_t((a01 & 31u) + (a23 & 31u));
         if (CELLS == kCells32) return __byte_perm(__byte_perm(e0, e1, 0x0051), __byte_perm(e2, e3, 0x0051), 0x5410);
         return __byte_perm(__byte_perm(y0, y1, 0x0040), __byte_perm(y2, y3, 0x0040), 0x5410);
     };
@@ -1301,7 +1245,7 @@ __device__ __forceinline__ void fseDecode(const FseTask& t, const uint8_t* smem,
     uint32_t const head = min(n, uint32_t((16 - (reinterpret_cast<uintptr_t>(out) & 15)) & 15));
     for (; i < head; i++) single(i);
     for (; i + 32 <= lastTr; i += 32) {
-        refill(Three());
+        br.refill<3>();
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             uint4 v;
@@ -1313,12 +1257,12 @@ __device__ __forceinline__ void fseDecode(const FseTask& t, const uint8_t* smem,
         }
     }
     for (; i + 4 <= lastTr; i += 4) {
-        refill(One());
+        br.refill<1>();
         *reinterpret_cast<uint32_t*>(out + i) = step();
     }
     for (; i < n; i++) single(i);
-    asm volatile("cp.async.wait_all;" ::: "memory"); // no copy outlives the lane
-    if (pos != end) reportError(status, DERR_CORRUPTION);
+    br.close();
+    if (!br.finished()) reportError(status, DERR_CORRUPTION);
 }
 
 template <int CELLS>
@@ -1344,9 +1288,9 @@ __global__ void __launch_bounds__(96) kFse(const FseTask* __restrict__ tasks, ui
     uint32_t const ti = blockIdx.x * lanes + lane;
     if (wid != 0 || lane >= lanes || ti >= nbTasks) return;
     FseTask const t = tasks[ti];
-    uint32_t const cell0 = lane << tableLogMax, ring = ringOff + lane * kFseRingBytes + 16;
-    if (t.nbStates == 4) fseDecode<CELLS, 4>(t, smemFse, cell0, tabBase, ring, status);
-    else fseDecode<CELLS, 2>(t, smemFse, cell0, tabBase, ring, status);
+    uint32_t const cell0 = lane << tableLogMax, area = ringOff + lane * kFseRingBytes;
+    if (t.nbStates == 4) fseDecode<CELLS, 4>(t, smemFse, cell0, tabBase, area, status);
+    else fseDecode<CELLS, 2>(t, smemFse, cell0, tabBase, area, status);
 }
 
 // FSE with one lane per state: a warp decodes up to eight streams, four lanes
@@ -1492,64 +1436,111 @@ __global__ void __launch_bounds__(32) kFse4(const FseTask* __restrict__ tasks, u
 // ---------------------------------------------------------------------------
 // Huffman: weights -> canonical table (symbols ranked by weight then value;
 // weight w spans 2^(w-1) cells, nbBits = tableLog + 1 - w), after
-// src/openzl/fse/decompress/huf_decompress.c:342-454. One warp per CTA
-// decodes eight chunks, four lanes per chunk (one per stream of a 4X chunk;
-// lane 0 alone for 1X) sharing the chunk's table (entry: symbol |
-// nbBits << 8). Table slots hold tableLog 11, the largest the reference's
-// encoder emits (encode_entropy_binding.c:222, HUF_TABLELOG_DEFAULT); chunks
-// with tableLog 12 take two adjacent slots and are decoded in a second round
-// when their neighbour's slot is busy.
+// src/openzl/fse/decompress/huf_decompress.c:342-454. The first warp of a CTA
+// decodes up to eight chunks, four lanes per chunk (one per stream of a 4X
+// chunk; lane 0 alone for 1X) sharing the chunk's table (16-bit cells: symbol
+// << 8 | nbBits); both warps build the tables. Table slots hold tableLog 11,
+// the largest the reference's encoder emits (encode_entropy_binding.c:222,
+// HUF_TABLELOG_DEFAULT); chunks with tableLog 12 take two slots, one chunk at
+// a time after the others.
+//
+// What bounds it: a symbol's code length comes from a table lookup, so a
+// stream is a chain of lookups (shift, address, shared-memory load, shift: 35
+// cycles), and the tables limit an SM to 48 chunks, six warps of 32 streams,
+// which do not hide it. So everything else leaves the chain: the window is
+// loaded by position once per four symbols (PosStream), a cell's low five bits
+// are its shift amount, ring refills are two predicated copies per 16 symbols
+// without a branch, and 16 symbols share a store. A warp builds a table in a
+// few thousand cycles: symbols ranked 32 at a time, then one weight's cells
+// after another (one lane ranking all symbols and filling runs of unequal
+// length took longer than 1,000 symbols' decoding).
+// A 256 MiB timestamp frame (4,224 chunks of 32 KiB): 0.46 ms before, 0.33 now;
+// one chunk of about 100,000 symbols, a stream of 25,000: 1.12 and 0.75 ms.
 constexpr uint32_t kHufTableLog = 12;
 constexpr uint32_t kHufChunks = 8;
-constexpr uint32_t kHufSlotCells = 1u << 11;
-constexpr uint32_t kHufSlotBytes = kHufSlotCells * 2 + 512 + 4;
+constexpr uint32_t kHufSlotBytes = 2u << 11;
+using HufStream = PosStream<8, 4>;
+constexpr uint32_t kHufAreaBytes = 4 * HufStream::kBytes; // a chunk's four rings; the table build's scratch before
+struct HufScratch {
+    uint32_t count[16], next[16];
+    uint8_t sorted[256];
+};
+static_assert(sizeof(HufScratch) <= kHufAreaBytes && kHufAreaBytes % 16 == 0, "the scratch lies in the rings' memory");
+// tables (two slots at least, for a tableLog-12 chunk), then the rings
+__host__ __device__ __forceinline__ uint32_t hufAreaOff(uint32_t chunks) { return (chunks < 2 ? 2 : chunks) * kHufSlotBytes; }
+__host__ __device__ __forceinline__ uint32_t hufSmem(uint32_t chunks) { return hufAreaOff(chunks) + chunks * kHufAreaBytes; }
 
-__device__ bool hufRank(const uint8_t* weights, uint32_t nbW, uint16_t* first, uint32_t& tlOut)
+// Ranks the symbols by weight (every lane of the warp calls it): count[w]
+// symbols of weight w in `sorted`, from the sum of the counts below w.
+// Returns the table log, 0 if the weights are not valid.
+__device__ __forceinline__ uint32_t hufRankWarp(const uint8_t* weights, uint32_t nbW, HufScratch& S)
 {
-    uint32_t counts[13];
-#pragma unroll
-    for (int k = 0; k < 13; k++) counts[k] = 0;
-    uint32_t sum = 0;
-    if (nbW > 256) return false;
-    for (uint32_t s = 0; s < nbW; s++) {
-        uint32_t const w = weights[s];
-        if (w > 12) return false;
-#pragma unroll
-        for (int k = 1; k < 13; k++) counts[k] += (w == uint32_t(k));
-        sum += (1u << w) >> 1;
+    uint32_t const lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    if (nbW > 256) return 0;
+    if (lane < 16) S.count[lane] = 0;
+    __syncwarp();
+    bool bad = false;
+    for (uint32_t b = 0; b < nbW; b += 32) {
+        uint32_t w = b + lane < nbW ? weights[b + lane] : 0u;
+        bad |= w > kHufTableLog;
+        w &= 15u;
+        uint32_t const m = __match_any_sync(0xffffffffu, w);
+        if (lane == 31u - __clz(m)) S.count[w] += __popc(m);
+        __syncwarp();
     }
-    if (sum == 0 || (sum & (sum - 1))) return false;
+    if (__any_sync(0xffffffffu, bad)) return 0;
+    uint32_t const c = lane >= 1 && lane <= kHufTableLog ? S.count[lane] : 0u;
+    uint32_t symbols = c, cells = lane ? c << (lane - 1) : 0u;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+        uint32_t const ys = __shfl_up_sync(0xffffffffu, symbols, o), yc = __shfl_up_sync(0xffffffffu, cells, o);
+        if (lane >= uint32_t(o)) {
+            symbols += ys;
+            cells += yc;
+        }
+    }
+    if (lane <= kHufTableLog) S.next[lane] = symbols - c;
+    __syncwarp();
+    uint32_t const sum = __shfl_sync(0xffffffffu, cells, kHufTableLog), nz = __shfl_sync(0xffffffffu, symbols, kHufTableLog);
+    if (sum == 0 || (sum & (sum - 1)) || nz < 2) return 0;
     uint32_t const tl = 31 - __clz(sum);
-    if (tl > kHufTableLog) return false;
-    uint32_t nz = 0;
-#pragma unroll
-    for (int k = 1; k < 13; k++) nz += counts[k];
-    if (nz < 2) return false;
-    uint32_t start[13];
-    uint32_t p = 0;
-#pragma unroll
-    for (int k = 1; k < 13; k++) {
-        start[k] = p;
-        if (uint32_t(k) <= tl) p += counts[k] << (k - 1);
+    if (tl > kHufTableLog) return 0;
+    for (uint32_t b = 0; b < nbW; b += 32) {
+        uint32_t const w = b + lane < nbW ? weights[b + lane] : 0u;
+        uint32_t const m = __match_any_sync(0xffffffffu, w);
+        uint32_t const at = S.next[w];
+        __syncwarp();
+        if (w) {
+            if (lane == 31u - __clz(m)) S.next[w] = at + __popc(m);
+            S.sorted[at + __popc(m & lt)] = uint8_t(b + lane);
+        }
+        __syncwarp();
     }
-    for (uint32_t s = 0; s < nbW; s++) {
-        uint32_t const w = weights[s];
-        uint32_t f = 0;
-#pragma unroll
-        for (int k = 1; k < 13; k++)
-            if (w == uint32_t(k)) { f = start[k]; start[k] += 1u << (k - 1); }
-        first[s] = uint16_t(f);
-    }
-    tlOut = tl;
-    return true;
+    return tl;
 }
 
-constexpr int kHufRing = 8, kHufAhead = 5; // stream ring: 128 bytes per lane, 80 bytes ahead
-// rings after the slots and the spare ranks
-__host__ __device__ __forceinline__ uint32_t hufRingOff(uint32_t chunks) { return (chunks * kHufSlotBytes + 512 + 15) & ~15u; }
+// Fills the cells of a table from the ranked symbols, one weight after another
+// (every lane of the warp calls it); two cells a store where a symbol has them.
+__device__ __forceinline__ void hufFillWarp(const HufScratch& S, uint32_t tl, uint16_t* tab)
+{
+    uint32_t const lane = threadIdx.x & 31;
+    uint32_t base = 0, start = 0;
+    for (uint32_t w = 1; w <= tl; w++) {
+        uint32_t const c = S.count[w], nb = tl + 1 - w;
+        if (w == 1) {
+            for (uint32_t j = lane; j < c; j += 32) tab[j] = uint16_t((uint32_t(S.sorted[j]) << 8) | nb);
+        } else { // the weight's first cell is a multiple of its symbols' spans
+            uint32_t* const d = reinterpret_cast<uint32_t*>(tab + start);
+            for (uint32_t j = lane; j < c << (w - 2); j += 32)
+                d[j] = ((uint32_t(S.sorted[base + (j >> (w - 2))]) << 8) | nb) * 0x10001u;
+        }
+        base += c;
+        start += c << (w - 1);
+    }
+}
 
-__device__ __forceinline__ void hufDecodeStream(const HufTask& t, const uint16_t* dt, uint32_t tl, uint32_t sIdx,
-                                                uint32_t* ring, uint32_t* status)
+__device__ __forceinline__ void hufDecodeStream(const HufTask& t, const uint8_t* smem, uint32_t tab, uint32_t tl,
+                                                uint32_t sIdx, uint32_t area, uint32_t* status)
 {
     const uint8_t* sp;
     uint32_t ssize, n, o0;
@@ -1577,210 +1568,168 @@ __device__ __forceinline__ void hufDecodeStream(const HufTask& t, const uint16_t
         o0 = 0;
         n = t.dstSize;
     }
-    BitWin3<kHufRing, kHufAhead> br;
-    if (!br.init(sp, ssize, ring)) { reportError(status, DERR_CORRUPTION); return; }
+    HufStream br;
+    if (!br.init(sp, ssize, smem, area)) { reportError(status, DERR_CORRUPTION); return; }
     uint8_t* const out = t.out + o0;
     uint32_t const sh = 32u - tl;
-    uint32_t i = 0;
-    // one symbol; its code is at most tl <= 12 bits
-    auto single = [&]() -> uint32_t {
-        br.prepare();
-        uint32_t const e = dt[__funnelshift_lc(br.b, br.a, uint32_t(br.g)) >> sh];
-        br.advance(int32_t(e >> 8));
-        return e;
+    // the cell of the code at the top of hi; its low five bits are the shift amount
+    auto cell = [&](uint32_t hi) -> uint32_t { return *reinterpret_cast<const uint16_t*>(smem + tab + 2 * (hi >> sh)); };
+    auto four = [&]() -> uint32_t {
+        uint32_t hi, lo, c[4];
+        br.window(hi, lo);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            c[k] = cell(hi);
+            if (k < 3) {
+                hi = __funnelshift_l(lo, hi, c[k]);
+                if (k < 2) lo = __funnelshift_l(0u, lo, c[k]);
+            }
+        }
+        // lengths are at most 12, so four add up within a cell's low byte
+        br.pos -= int32_t((c[0] + c[1] + c[2] + c[3]) & 255u);
+        return __byte_perm(__byte_perm(c[0], c[1], 0x0051), __byte_perm(c[2], c[3], 0x0051), 0x5410);
     };
-    // unaligned head, then four symbols per refill and per 32-bit store: the
-    // 64 bits below pos, left-aligned in (hi, lo), hold the four codes
-    uint32_t const head = min(n, uint32_t((4 - (reinterpret_cast<uintptr_t>(out) & 3)) & 3));
-    for (; i < head; i++) out[i] = uint8_t(single());
-    for (; i + 4 <= n; i += 4) {
-        br.prepare();
-        uint32_t hi = __funnelshift_lc(br.b, br.a, uint32_t(br.g));
-        uint32_t lo = __funnelshift_lc(br.c, br.b, uint32_t(br.g));
-        uint32_t const e0 = dt[hi >> sh];
-        uint32_t const n0 = e0 >> 8;
-        hi = __funnelshift_l(lo, hi, n0);
-        lo <<= n0;
-        uint32_t const e1 = dt[hi >> sh];
-        uint32_t const n1 = e1 >> 8;
-        hi = __funnelshift_l(lo, hi, n1);
-        lo <<= n1;
-        uint32_t const e2 = dt[hi >> sh];
-        uint32_t const n2 = e2 >> 8;
-        hi = __funnelshift_l(lo, hi, n2);
-        uint32_t const e3 = dt[hi >> sh];
-        br.advance(int32_t(n0 + n1 + n2 + (e3 >> 8)));
-        *reinterpret_cast<uint32_t*>(out + i) = __byte_perm(__byte_perm(e0, e1, 0x0040), __byte_perm(e2, e3, 0x0040), 0x5410);
+    uint32_t i = 0;
+    auto single = [&]() {
+        br.refill<1>();
+        uint32_t hi, lo;
+        br.window(hi, lo);
+        uint32_t const c = cell(hi);
+        out[i] = uint8_t(c >> 8);
+        br.pos -= int32_t(c & 31u);
+    };
+    uint32_t const head = min(n, uint32_t((16 - (reinterpret_cast<uintptr_t>(out) & 15)) & 15));
+    for (; i < head; i++) single();
+    for (; i + 16 <= n; i += 16) { // eight codes are at most 12 bytes
+        uint4 v;
+        br.refill<1>();
+        v.x = four();
+        v.y = four();
+        br.refill<1>();
+        v.z = four();
+        v.w = four();
+        *reinterpret_cast<uint4*>(out + i) = v;
     }
-    for (; i < n; i++) out[i] = uint8_t(single());
-    asm volatile("cp.async.wait_all;" ::: "memory"); // no copy outlives the lane
+    for (; i < n; i++) single();
+    br.close();
     if (!br.finished()) reportError(status, DERR_CORRUPTION);
 }
 
-__global__ void __launch_bounds__(32) kHuf(const HufTask* __restrict__ tasks, uint32_t nbTasks, uint32_t chunks,
+__global__ void __launch_bounds__(64) kHuf(const HufTask* __restrict__ tasks, uint32_t nbTasks, uint32_t chunks,
                                            uint32_t* __restrict__ status)
 {
     extern __shared__ __align__(16) uint8_t smemHuf[];
     __shared__ uint32_t sTl[kHufChunks];
-    __shared__ uint8_t sOk[kHufChunks];
-    uint32_t const c = threadIdx.x >> 2;       // chunk slot in this CTA
-    uint32_t const sIdx = threadIdx.x & 3;     // stream within the chunk
-    uint32_t const ti = blockIdx.x * chunks + c;
-    bool const active = ti < nbTasks;
-    uint8_t* const slot = smemHuf + size_t(c) * kHufSlotBytes;
-    uint16_t* const first = reinterpret_cast<uint16_t*>(slot + kHufSlotCells * 2); // first cell per symbol
-    HufTask t{};
-    if (active) t = tasks[ti];
-    if (sIdx == 0) {
+    uint32_t const wid = threadIdx.x >> 5, areas = hufAreaOff(chunks);
+    for (uint32_t k = wid; k < chunks; k += 2) {
+        uint32_t const tk = blockIdx.x * chunks + k;
         uint32_t tl = 0;
-        bool const ok = active && hufRank(t.weights, t.nbWeights, first, tl);
-        sOk[c] = ok ? 1 : 0;
-        sTl[c] = tl;
-        if (active && !ok) reportError(status, DERR_CORRUPTION);
+        if (tk < nbTasks) {
+            const uint8_t* const weights = tasks[tk].weights;
+            HufScratch& S = *reinterpret_cast<HufScratch*>(smemHuf + areas + k * kHufAreaBytes);
+            tl = hufRankWarp(weights, tasks[tk].nbWeights, S);
+            if (tl && tl <= 11) hufFillWarp(S, tl, reinterpret_cast<uint16_t*>(smemHuf + k * kHufSlotBytes));
+            if (!tl && (threadIdx.x & 31) == 0) reportError(status, DERR_CORRUPTION);
+        }
+        if ((threadIdx.x & 31) == 0) sTl[k] = tl;
     }
-    __syncwarp();
+    __syncthreads();
+    if (wid != 0) return;
     // tableLog <= 11: each chunk in its own slot
-    uint32_t const tl = sTl[c];
-    bool const narrow = active && sOk[c] && tl <= 11;
-    uint16_t* const dt = reinterpret_cast<uint16_t*>(slot);
-    if (narrow) {
-        for (uint32_t s = sIdx; s < t.nbWeights; s += 4) {
-            uint32_t const w = t.weights[s];
-            if (!w) continue;
-            uint32_t const len = 1u << (w - 1);
-            uint16_t const e = uint16_t(s | ((tl + 1 - w) << 8));
-            uint32_t const f = first[s];
-            for (uint32_t u = 0; u < len; u++) dt[f + u] = e;
+    uint32_t const c = threadIdx.x >> 2, sIdx = threadIdx.x & 3; // chunk of this CTA, stream of the chunk
+    bool wide = false;
+    if (c < chunks) {
+        uint32_t const tl = sTl[c];
+        wide = tl > 11;
+        if (tl && !wide) {
+            HufTask const t = tasks[blockIdx.x * chunks + c];
+            hufDecodeStream(t, smemHuf, c * kHufSlotBytes, tl, sIdx, areas + c * kHufAreaBytes + sIdx * HufStream::kBytes,
+                            status);
         }
     }
-    __syncwarp();
-    uint32_t* const ring = reinterpret_cast<uint32_t*>(smemHuf + hufRingOff(chunks)) + threadIdx.x * 4 * kHufRing;
-    if (narrow) hufDecodeStream(t, dt, tl, sIdx, ring, status);
-    __syncwarp();
+    if (!__any_sync(0xffffffffu, wide)) return;
     // tableLog 12 (valid, but never emitted by the reference's encoder): one
-    // chunk at a time, its table across the first slots, ranks recomputed
-    // into the spare area after the slots
-    uint16_t* const wideFirst = reinterpret_cast<uint16_t*>(smemHuf + size_t(chunks) * kHufSlotBytes);
-    uint16_t* const wide = reinterpret_cast<uint16_t*>(smemHuf);
+    // chunk at a time, its table across the first two slots
     for (uint32_t k = 0; k < chunks; k++) {
-        if (!(sOk[k] && sTl[k] > 11)) continue; // warp-uniform
-        HufTask const tk = tasks[blockIdx.x * chunks + k];
-        if (threadIdx.x == 0) {
-            uint32_t tlk = 0;
-            hufRank(tk.weights, tk.nbWeights, wideFirst, tlk);
-        }
+        if (sTl[k] <= 11) continue; // warp-uniform
+        HufTask const t = tasks[blockIdx.x * chunks + k];
+        HufScratch& S = *reinterpret_cast<HufScratch*>(smemHuf + areas);
+        uint32_t const tl = hufRankWarp(t.weights, t.nbWeights, S);
+        hufFillWarp(S, tl, reinterpret_cast<uint16_t*>(smemHuf));
         __syncwarp();
-        uint32_t const tlk = sTl[k];
-        for (uint32_t s = threadIdx.x; s < tk.nbWeights; s += blockDim.x) { // 4 x chunks threads
-            uint32_t const w = tk.weights[s];
-            if (!w) continue;
-            uint32_t const len = 1u << (w - 1);
-            uint16_t const e = uint16_t(s | ((tlk + 1 - w) << 8));
-            uint32_t const f = wideFirst[s];
-            for (uint32_t u = 0; u < len; u++) wide[f + u] = e;
-        }
-        __syncwarp();
-        if (threadIdx.x < 4) hufDecodeStream(tk, wide, tlk, threadIdx.x, ring, status);
+        if (threadIdx.x < 4) hufDecodeStream(t, smemHuf, 0, tl, threadIdx.x, areas + threadIdx.x * HufStream::kBytes, status);
         __syncwarp();
     }
 }
 
-// Backward bit reader of the 16-bit Huffman decoder. The window is the three
-// stream words kb + 2 (top), kb + 1 and kb, loaded through the read-only data
-// cache at each step (a lane walks down one 128-byte line every few dozen
-// steps, so nearly all loads hit L1), and g = 32 * (kb + 3) - pos in
-// [0, 32): the 64 bits just below pos, most significant first, are two
-// funnel shifts of them. A step reads at most 48 bits; advance() drops them
-// with three integer operations. Word indices are clamped at 0, the 16-byte
-// block that holds the stream's first byte: words below the stream are never
-// consumed by a valid stream (finished() checks that the stream ends exactly
-// at its first bit), so any word may stand in for them, and nothing outside
-// the stream's blocks is read.
-struct BitLdg {
-    const uint32_t* base; // the 16-byte block holding the stream's first byte
-    int32_t kb, g, end;
-
-    __device__ __forceinline__ bool init(const uint8_t* p, uint32_t size)
-    {
-        int32_t pos;
-        const uint8_t* g16;
-        if (!streamStart(p, size, g16, pos, end)) return false;
-        base = reinterpret_cast<const uint32_t*>(g16);
-        int32_t const jt = (pos - 1) >> 5;
-        kb = jt - 2;
-        g = (kb + 3) * 32 - pos;
-        return true;
-    }
-    // the 64 bits below pos, most significant first
-    __device__ __forceinline__ void window(uint32_t& hi, uint32_t& lo) const
-    {
-        uint32_t const c = __ldg(base + max(kb, 0)), b = __ldg(base + max(kb + 1, 0)), a = __ldg(base + max(kb + 2, 0));
-        hi = __funnelshift_l(b, a, uint32_t(g));
-        lo = __funnelshift_l(c, b, uint32_t(g));
-    }
-    __device__ __forceinline__ void advance(uint32_t n)
-    {
-        g += int32_t(n);
-        kb -= g >> 5;
-        g &= 31;
-    }
-    // one field of nb bits (nb <= 12) just below pos
-    __device__ __forceinline__ uint32_t read(uint32_t nb)
-    {
-        uint32_t hi, lo;
-        window(hi, lo);
-        advance(nb);
-        return __funnelshift_l(hi, 0u, nb);
-    }
-    __device__ __forceinline__ bool finished() const { return (kb + 3) * 32 - g == end; }
-};
-
 // ---------------------------------------------------------------------------
-// 16-bit-symbol Huffman (huffman_struct_v2), one CTA per chunk. Tables reach
-// 2^20 cells (tableLog <= 20), so instead of a cell table the CTA keeps, per
+// 16-bit-symbol Huffman (huffman_struct_v2), one CTA per chunk. Codes reach 20
+// bits, so a cell table of them would take 2^20 cells. The CTA keeps, per
 // weight, the first cell and the first index into the symbols sorted by
 // (weight, value): the cell range of weight w spans count[w] << (w - 1)
 // cells, weight 1 (the longest code) first, and a symbol of weight w spans
 // 2^(w-1) consecutive cells and codes on tableLog + 1 - w bits
-// (decode_huffman_kernel.c:35-71). Decoding a symbol peeks tableLog bits,
-// finds the weight whose cell range holds them (binary search over at most
-// 20 ranks) and indexes the sorted symbols. The validity rules of
-// decode_entropy_binding.c:349-412 apply: weights at most 20, at least two
-// of them non-zero, the sum of 2^(w-1) a power of two. One lane decodes each
-// of the one or four streams; like the reference, a stream is not required
-// to end exactly at its first bit (the planner checked that the stream table
-// fills the input exactly).
-__global__ void __launch_bounds__(128) kHuf16(const Huf16Task* __restrict__ tasks, uint32_t* __restrict__ status)
+// (decode_huffman_kernel.c:35-71). The weight of a code is its place among at
+// most 20 ranges, so a table over its top kHuf16Log bits knows it but where a
+// bucket holds a range's start (at most 20 of 4096 buckets). An entry holds
+// the code length and what to add to the code to get its place among the
+// sorted symbols (a range's start is a multiple of its symbols' span, since
+// the ranges above it fill the rest). Codes of the other buckets find their
+// range by binary search. The validity rules of
+// decode_entropy_binding.c:349-412 apply: weights at most 20, at least two of
+// them non-zero, the sum of 2^(w-1) a power of two. One lane decodes each of
+// the one or four streams; like the reference, a stream is not required to end
+// exactly at its first bit (the planner checked that the stream table fills
+// the input exactly).
+//
+// What bounds it: each stream is a serial chain, a lookup and a shift a symbol
+// (four symbols per 64-bit window where codes have at most 16 bits, else
+// three). The search and three cached stream loads for every symbol took about
+// 550 cycles. A table of whole symbols over 12 bits was no help (5.99 ms):
+// 13-bit codes are the ordinary ones of large alphabets. The symbols' loads
+// (L1) leave the chain: they are stored a window later.
+// 98,304 symbols in four streams, geometric with mean 3000: 7.06 ms before,
+// 1.41 ms now.
+constexpr uint32_t kHuf16Log = 12, kHuf16Threads = 256, kHuf16Warps = kHuf16Threads / 32;
+using Huf16Stream = PosStream<16, 12>;
+
+__global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restrict__ tasks, uint32_t* __restrict__ status)
 {
-    __shared__ uint32_t sCount[32], sStart[32], sBase[32], sNext[32];
+    __shared__ uint32_t sCount[kHuf16Warps][32], sStart[32], sBase[32];
     __shared__ uint32_t sTl, sOk;
-    __shared__ unsigned long long sSum;
+    __shared__ uint32_t sTab[1u << kHuf16Log];
+    __shared__ __align__(16) uint8_t sRing[4 * Huf16Stream::kBytes];
     Huf16Task const t = tasks[blockIdx.x];
-    uint32_t const tid = threadIdx.x, lane = tid & 31;
-    if (tid < 32) sCount[tid] = 0;
-    if (tid == 0) {
-        sSum = 0;
-        sOk = 1;
-    }
+    uint32_t const tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    sCount[wid][lane] = 0;
+    if (tid == 0) sOk = 1;
     __syncthreads();
-    unsigned long long part = 0;
+    // every warp takes a run of symbols: counts per weight, then each warp's
+    // first place among the symbols of a weight, then the places
+    uint32_t const run = ((t.nbWeights + kHuf16Threads - 1) / kHuf16Threads) * 32;
+    uint32_t const b0 = min(t.nbWeights, wid * run), b1 = min(t.nbWeights, b0 + run);
     bool bad = false;
-    for (uint32_t s = tid; s < t.nbWeights; s += blockDim.x) {
-        uint32_t const w = t.weights[s];
+    for (uint32_t b = b0; b < b1; b += 32) {
+        uint32_t w = b + lane < b1 ? t.weights[b + lane] : 0u;
         if (w > 20) {
             bad = true;
-        } else if (w) {
-            atomicAdd(&sCount[w], 1u);
-            part += 1ull << (w - 1);
+            w = 0;
         }
+        uint32_t const m = __match_any_sync(0xffffffffu, w);
+        if (lane == 31u - __clz(m)) sCount[wid][w] += __popc(m);
+        __syncwarp();
     }
     if (bad) sOk = 0;
-    if (part) atomicAdd(&sSum, part);
     __syncthreads();
     if (tid == 0) {
-        uint64_t const sum = sSum;
-        uint32_t nz = 0;
-        for (int w = 1; w <= 20; w++) nz += sCount[w];
+        uint64_t sum = 0;
+        uint32_t nz = 0, total[21];
+        for (uint32_t w = 1; w <= 20; w++) {
+            total[w] = 0;
+            for (uint32_t k = 0; k < kHuf16Warps; k++) total[w] += sCount[k][w];
+            nz += total[w];
+            sum += uint64_t(total[w]) << (w - 1);
+        }
         uint32_t tl = 0;
         while (tl < 63 && (2ull << tl) <= sum) tl++;
         bool const ok = sOk && nz >= 2 && sum != 0 && !(sum & (sum - 1)) && tl <= 20;
@@ -1789,9 +1738,12 @@ __global__ void __launch_bounds__(128) kHuf16(const Huf16Task* __restrict__ task
             for (uint32_t w = 1; w <= tl; w++) {
                 sStart[w] = pos;
                 sBase[w] = base;
-                sNext[w] = base;
-                pos += sCount[w] << (w - 1);
-                base += sCount[w];
+                pos += total[w] << (w - 1);
+                for (uint32_t k = 0; k < kHuf16Warps; k++) {
+                    uint32_t const c = sCount[k][w];
+                    sCount[k][w] = base;
+                    base += c;
+                }
             }
             sStart[tl + 1] = 1u << tl;
         }
@@ -1804,51 +1756,142 @@ __global__ void __launch_bounds__(128) kHuf16(const Huf16Task* __restrict__ task
         return;
     }
     uint32_t const tl = sTl;
-    // symbols sorted by (weight, value): 32 at a time, ranked among the lanes
-    // holding the same weight
-    if (tid < 32) {
-        for (uint32_t b0 = 0; b0 < t.nbWeights; b0 += 32) {
-            uint32_t const s = b0 + lane;
-            uint32_t const w = s < t.nbWeights ? t.weights[s] : 0u;
-            uint32_t const m = __match_any_sync(0xffffffffu, w);
-            uint32_t const base = w ? sNext[w] : 0u;
-            __syncwarp();
-            if (w) {
-                if (lane == 31u - __clz(m)) sNext[w] = base + __popc(m);
-                t.sorted[base + __popc(m & ((1u << lane) - 1u))] = uint16_t(s);
-            }
-            __syncwarp();
+    for (uint32_t b = b0; b < b1; b += 32) {
+        uint32_t const w = b + lane < b1 ? t.weights[b + lane] : 0u;
+        uint32_t const m = __match_any_sync(0xffffffffu, w);
+        uint32_t const base = sCount[wid][w];
+        __syncwarp();
+        if (w) {
+            if (lane == 31u - __clz(m)) sCount[wid][w] = base + __popc(m);
+            t.sorted[base + __popc(m & ((1u << lane) - 1u))] = uint16_t(b + lane);
         }
+        __syncwarp();
     }
     __syncthreads();
-    if (tid >= t.nbStreams) return;
-    BitLdg br;
-    if (!br.init(t.stream[tid], t.streamSize[tid])) {
-        reportError(status, DERR_CORRUPTION);
-        return;
-    }
-    uint8_t* const out = t.out + 2ull * t.dstOff[tid];
-    bool const al = !(reinterpret_cast<uintptr_t>(out) & 1);
-    uint32_t const n = t.count[tid];
-    for (uint32_t i = 0; i < n; i++) {
-        uint32_t hi, lo;
-        br.window(hi, lo);
-        uint32_t const v = hi >> (32 - tl);
+    // the weight whose cell range holds cell v
+    auto weightOf = [&](uint32_t v) -> uint32_t {
         uint32_t a = 1, b = tl;
         while (a < b) {
             uint32_t const mid = (a + b + 1) >> 1;
             if (sStart[mid] <= v) a = mid;
             else b = mid - 1;
         }
-        uint32_t const sym = t.sorted[sBase[a] + ((v - sStart[a]) >> (a - 1))];
-        if (al) {
-            reinterpret_cast<uint16_t*>(out)[i] = uint16_t(sym);
-        } else {
-            out[2 * i] = uint8_t(sym);
-            out[2 * i + 1] = uint8_t(sym >> 8);
-        }
-        br.advance(tl + 1 - a);
+        return a;
+    };
+    // (place - code) << 5 | length of the codes of weight a
+    auto entryOf = [&](uint32_t a) -> uint32_t {
+        return ((sBase[a] - (sStart[a] >> (a - 1))) << 5) | (tl + 1 - a);
+    };
+    uint32_t const pl = min(tl, kHuf16Log);
+    for (uint32_t j = tid; j < (1u << pl); j += kHuf16Threads) {
+        uint32_t const a = weightOf(j << (tl - pl)), b = weightOf(((j + 1) << (tl - pl)) - 1);
+        sTab[j] = a == b ? entryOf(a) : 0u;
     }
+    __syncthreads();
+    if (tid >= t.nbStreams) return;
+    Huf16Stream br;
+    if (!br.init(t.stream[tid], t.streamSize[tid], sRing, tid * Huf16Stream::kBytes)) {
+        reportError(status, DERR_CORRUPTION);
+        return;
+    }
+    auto symbol = [&](uint32_t hi, uint32_t e) -> uint32_t {
+        return t.sorted[uint32_t(int32_t(e) >> 5) + __funnelshift_l(hi, 0u, e)];
+    };
+    uint8_t* const out = t.out + 2ull * t.dstOff[tid];
+    uint32_t const n = t.count[tid];
+    uint32_t i = 0;
+    auto put = [&](uint32_t k, uint32_t y) {
+        if (!(reinterpret_cast<uintptr_t>(out) & 1)) {
+            reinterpret_cast<uint16_t*>(out)[k] = uint16_t(y);
+        } else {
+            out[2 * k] = uint8_t(y);
+            out[2 * k + 1] = uint8_t(y >> 8);
+        }
+    };
+    // N codes at the position, N times the longest at most 64 bits: first as if
+    // the table knew them all (an entry 0 shifts by nothing), with the search
+    // only when one was not known, so that a window takes one branch
+    auto codes = [&](auto& y) {
+        constexpr int N = int(sizeof(y) / sizeof(y[0]));
+        uint32_t hi, lo, used = 0, least = ~0u;
+        br.window(hi, lo);
+        uint32_t const hi0 = hi, lo0 = lo;
+#pragma unroll
+        for (int k = 0; k < N; k++) { // an entry's low five bits are the shift amount
+            uint32_t const e = sTab[hi >> (32 - pl)];
+            y[k] = symbol(hi, e);
+            used += e & 31u;
+            least = min(least, e);
+            hi = __funnelshift_l(lo, hi, e);
+            lo = __funnelshift_l(0u, lo, e);
+        }
+        if (least == 0) {
+            hi = hi0;
+            lo = lo0;
+            used = 0;
+#pragma unroll 1
+            for (int k = 0; k < N; k++) {
+                uint32_t e = sTab[hi >> (32 - pl)];
+                if (e == 0) e = entryOf(weightOf(hi >> (32 - tl)));
+                uint32_t const z = symbol(hi, e);
+#pragma unroll
+                for (int m = 0; m < N; m++)
+                    if (m == k) y[m] = z;
+                used += e & 31u;
+                hi = __funnelshift_l(lo, hi, e);
+                lo = __funnelshift_l(0u, lo, e);
+            }
+        }
+        br.pos -= int32_t(used);
+    };
+    auto single = [&]() {
+        br.refill<1>();
+        uint32_t y[1];
+        codes(y);
+        put(i, y[0]);
+    };
+    if (tl <= 16 && !(reinterpret_cast<uintptr_t>(out) & 1)) {
+        // four codes a window, sixteen symbols (32 bytes at most) a refill
+        uint32_t const head = min(n, uint32_t((8 - (reinterpret_cast<uintptr_t>(out) & 7)) & 7) >> 1);
+        for (; i < head; i++) single();
+        uint32_t y[4], i0 = i;
+        auto store = [&](uint32_t k) {
+            *reinterpret_cast<uint2*>(out + 2 * k) = make_uint2(__byte_perm(y[0], y[1], 0x5410), __byte_perm(y[2], y[3], 0x5410));
+        };
+        for (; i + 16 <= n; i += 16) {
+            br.refill<3>();
+#pragma unroll
+            for (uint32_t q = 0; q < 16; q += 4) {
+                uint32_t z[4];
+                codes(z);
+                if (i + q > i0) store(i + q - 4);
+#pragma unroll
+                for (int k = 0; k < 4; k++) y[k] = z[k];
+            }
+        }
+        if (i > i0) store(i - 4);
+    } else {
+        // three codes a window, fifteen symbols (38 bytes at most) a refill
+        uint32_t y[3], i0 = i;
+        auto store = [&](uint32_t k) {
+#pragma unroll
+            for (int m = 0; m < 3; m++) put(k + m, y[m]);
+        };
+        for (; i + 15 <= n; i += 15) {
+            br.refill<3>();
+#pragma unroll
+            for (uint32_t q = 0; q < 15; q += 3) {
+                uint32_t z[3];
+                codes(z);
+                if (i + q > i0) store(i + q - 3);
+#pragma unroll
+                for (int k = 0; k < 3; k++) y[k] = z[k];
+            }
+        }
+        if (i > i0) store(i - 3);
+    }
+    for (; i < n; i++) single();
+    br.close();
 }
 
 // ---------------------------------------------------------------------------
@@ -2231,7 +2274,13 @@ FseShape fseShape(const Launch& l)
     s.lanes = std::max(1u, std::min(s.lanes, maxLanes));
     return s;
 }
-uint32_t hufSmem(uint32_t chunks) { return hufRingOff(chunks) + 4 * chunks * 16 * kHufRing; }
+// Chunks per CTA of an untuned Huffman launch: spread over the SMs first, up
+// to eight (a full warp), of which six CTAs fit an SM.
+uint32_t hufDefaultChunks(uint32_t nbTasks)
+{
+    uint32_t const sms = uint32_t(smCount()), perSm = (nbTasks + sms - 1) / sms;
+    return std::max(1u, std::min(kHufChunks, (perSm + 5) / 6));
+}
 // kHashBlocks grid: one warp per block up to eight full CTAs per SM, then
 // grid-stride (any grid size is correct)
 uint32_t hashGrid(uint32_t nbBlocks)
@@ -2318,9 +2367,9 @@ long runOneLaunch(const DeviceLayout& L, size_t li, uint8_t* dPool, uint8_t* dSc
                 break;
             }
             case KIND_HUF: {
-                uint32_t const chunks = l.tune && l.tune <= kHufChunks ? l.tune : kHufChunks;
+                uint32_t const chunks = l.tune && l.tune <= kHufChunks ? l.tune : hufDefaultChunks(l.nbTasks);
                 uint32_t const grid = (l.nbTasks + chunks - 1) / chunks;
-                kHuf<<<grid, 4 * chunks, hufSmem(chunks), s>>>(static_cast<const HufTask*>(tasks), l.nbTasks, chunks,
+                kHuf<<<grid, 64, hufSmem(chunks), s>>>(static_cast<const HufTask*>(tasks), l.nbTasks, chunks,
                                                                dStatus);
                 break;
             }
@@ -2328,7 +2377,7 @@ long runOneLaunch(const DeviceLayout& L, size_t li, uint8_t* dPool, uint8_t* dSc
                 kFlatpack<<<l.nbTiles, 256, 0, s>>>(static_cast<const FlatpackTask*>(tasks), tiles, dStatus);
                 break;
             case KIND_HUF16:
-                if (l.nbTasks) kHuf16<<<l.nbTasks, 128, 0, s>>>(static_cast<const Huf16Task*>(tasks), dStatus);
+                if (l.nbTasks) kHuf16<<<l.nbTasks, kHuf16Threads, 0, s>>>(static_cast<const Huf16Task*>(tasks), dStatus);
                 break;
             case KIND_WIDEN:
                 kWiden<<<l.nbTiles, 256, 0, s>>>(static_cast<const WidenTask*>(tasks), tiles, dStatus);

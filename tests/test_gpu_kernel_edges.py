@@ -73,3 +73,40 @@ def test_fse_blocks_alignments_and_table_forms(gpu_lib):
     many = [np.minimum(rng.geometric(0.04, 4097 + k % 300), 255).astype(np.uint8) for k in range(6000)]
     out, _ = _round_trip(many, 7, 0, [k % 16 for k in range(len(many))])
     assert all(g.tobytes() == a.tobytes() for a, g in zip(many, out))
+
+
+def test_huf16_code_lengths_and_stream_tails(gpu_lib):
+    """16-bit Huffman: codes within and beyond the lookup table's bits and
+    beyond 16, every length around the four-symbol windows and the refills, one
+    and four streams."""
+    rng = np.random.default_rng(16)
+    arrays = []
+    for n in [260 + k for k in range(20)] + [1000 + k for k in range(24)] + [20000, 65537, 99999, 100001]:
+        arrays.append(np.minimum(rng.geometric(1 / 3000, n), 65535).astype(np.uint16))
+        arrays.append((rng.zipf(1.3, n) % 3000).astype(np.uint16))
+        # half of the weight on few values, the rest spread thin: long codes
+        k = np.minimum(rng.geometric(0.5, n), 19) - 1
+        arrays.append(np.where(rng.random(n) < 0.9, k, rng.integers(0, 65536, n)).astype(np.uint16))
+    out, frames = _round_trip(arrays, 8, 2, [16 * (k % 2) for k in range(len(arrays))])
+    for a, g, f in zip(arrays, out, frames):
+        assert g.tobytes() == a.tobytes() == oracle.decompress(f)[0].tobytes(), a.size
+
+
+def test_huf_windows_alignments_and_table_logs(gpu_lib):
+    """8-bit Huffman: one and four streams, every stream length around the
+    sixteen-symbol blocks at every destination alignment, codes from one bit to
+    the longest."""
+    rng = np.random.default_rng(8)
+    arrays = []
+    for n in [20 + k for k in range(70)] + [255 + k for k in range(70)] + [4000 + k for k in range(20)] + [32768, 99999, 100001]:
+        kind = n % 3
+        if kind == 0:
+            a = np.minimum(rng.geometric(0.3, n), 255).astype(np.uint8)
+        elif kind == 1:
+            a = np.minimum(np.abs(rng.normal(100, 40, n)), 255).astype(np.uint8)
+        else:
+            a = np.where(rng.random(n) < 0.95, 7, rng.integers(0, 256, n)).astype(np.uint8)
+        arrays.append(a)
+    out, frames = _round_trip(arrays, 8, 0, [k % 16 for k in range(len(arrays))])
+    for a, g, f in zip(arrays, out, frames):
+        assert g.tobytes() == a.tobytes() == oracle.decompress(f)[0].tobytes(), a.size
