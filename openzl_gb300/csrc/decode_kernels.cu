@@ -85,21 +85,6 @@ __device__ __forceinline__ uint64_t widthMask(uint32_t w)
 // ---------------------------------------------------------------------------
 // copy / constant: tiles of kTileBytes output bytes
 
-// 16 bytes starting `off` bytes (1..15) into the 32 bytes (u0, u1); q and r
-// are off / 4 and (off % 4) * 8, uniform across the block
-__device__ __forceinline__ uint4 shiftCombine(uint4 u0, uint4 u1, uint32_t q, uint32_t r)
-{
-    uint32_t y0, y1, y2, y3, y4;
-    switch (q) {
-        case 0: y0 = u0.x; y1 = u0.y; y2 = u0.z; y3 = u0.w; y4 = u1.x; break;
-        case 1: y0 = u0.y; y1 = u0.z; y2 = u0.w; y3 = u1.x; y4 = u1.y; break;
-        case 2: y0 = u0.z; y1 = u0.w; y2 = u1.x; y3 = u1.y; y4 = u1.z; break;
-        default: y0 = u0.w; y1 = u1.x; y2 = u1.y; y3 = u1.z; y4 = u1.w; break;
-    }
-    return make_uint4(__funnelshift_r(y0, y1, r), __funnelshift_r(y1, y2, r), __funnelshift_r(y2, y3, r),
-                      __funnelshift_r(y3, y4, r));
-}
-
 // Copies one tile: bytes up to the destination's 16-byte boundary, then
 // 16-byte stores, each from the two aligned 16-byte source blocks that hold
 // its bytes (both blocks hold bytes of the source, so nothing outside the

@@ -70,11 +70,11 @@ struct FseEncTask {
     uint32_t tableLog;
     uint16_t* fields;        // chunks of kFseLongMin symbols or more: fseFieldBytes(n) of scratch
 };
-// Chunks of four states and at least this many symbols encode with one lane
-// per state (kFseEncStates, then kFseEncPack); shorter ones one lane each.
+// Chunks of four states and at least this many symbols take a CTA each, their
+// chains cut into segments (kFseEncLong); shorter ones one lane each.
 constexpr uint32_t kFseLongMin = 4096;
-// scratch of a long chunk: one 16-bit entry per field, padded to 8 bytes
-inline size_t fseFieldBytes(uint32_t n) { return 2 * ((size_t(n) + 3) & ~size_t(3)) + 16; }
+// scratch of a long chunk: one 16-bit entry per field, up to three before the first
+inline size_t fseFieldBytes(uint32_t n) { return 2 * ((size_t(n) + 3 + 3) & ~size_t(3)) + 16; }
 
 struct HufEncTask {
     const uint8_t* src;

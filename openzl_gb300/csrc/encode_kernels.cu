@@ -672,172 +672,268 @@ __global__ void __launch_bounds__(32) kFseEnc(const FseEncTask* __restrict__ tas
     sizes[t.sizeSlot] = bo.close();
 }
 
-// FSE, long chunks (four states, kFseLongMin symbols or more), in two
-// launches. The four states' chains are independent: only the order in which
-// their fields are appended couples them.
-//  - kFseEncStates: four lanes per chunk, lane k running state k's chain. It
-//    writes one 16-bit entry per transition (the field in bits 0-11, its
-//    width in bits 12-15) at the field's index in append order, and after its
-//    last transition its state's flush (tableLog bits) at index n - 4 + k. A
-//    chunk's n entries are then its bitstream's fields in order.
-//  - kFseEncPack: one warp per chunk appends the entries, 128 per round (four
-//    per lane): a warp scan of the lanes' widths places them, they are ORed
-//    into a window of words in shared memory, and the complete words go out
-//    (a word only when it fits the capacity, as in the one-lane encoder);
-//    then the end mark and the last bytes.
+// FSE, long chunks (four states, kFseLongMin symbols or more), one CTA each.
+// The four states' chains are independent (only the order in which their
+// fields are appended couples them), and a chain forgets where it came from:
+// after a symbol that holds c of the table's cells only c states remain, so
+// two unlike states meet with a probability of about (symbols present) / (table
+// size) a step. So each chain is cut into up to 32 segments run at once, lane k
+// of a group of four running state k:
+//  1. A segment starts some steps early from an arbitrary state (six times the
+//     mean to a meeting; from the true state where that reaches the chain's
+//     start), records the state it enters its own steps with, and writes one
+//     16-bit entry per transition (the field in bits 0-11, its width in bits
+//     12-15) at the field's index in append order. Segments are no shorter
+//     than that run-up, so few symbols mean few segments, and two or three one.
+//  2. A segment whose entry state is not the end state of the segment before
+//     it runs again from that state, until it meets its own earlier state at a
+//     quarter of the segment, or its end; this repeats until all agree.
+//  3. The entries are then the chunk's fields in order. Their widths, summed
+//     per segment, give each warp's first bit; a warp appends its quarter of
+//     the segments, 128 entries a round (a scan of the lanes' widths places
+//     them, they are ORed into a window of words in shared memory, complete
+//     words go out; only those that fit the capacity are written, as in the
+//     one-lane encoder). The words that two warps share meet in shared memory.
 // The bytes equal kFseEnc's for the same chunk.
-constexpr uint32_t kFseStChunks = 8; // chunks per CTA (one warp, four lanes each)
-constexpr uint32_t kFseStSlot = kFseLaneTables + 4 * 16 * kEncRing;
-static_assert(kFseStSlot % 16 == 0, "16-byte aligned rings");
+//
+// What bounds it: a transition's chain (two adds, two shifts and a shared
+// load, about 45 cycles); with one lane a chain it was 8,192 of them for a
+// chunk of 32 K symbols, at 290 cycles, in 24 lanes per SM. The segments give
+// an SM 16 chunks of 128 lanes. 32 K symbols: 1.19 ms and 0.11 ms of packing
+// before, 0.06 ms now (a plane of about 200 symbols); a stream of 100,000
+// symbols of which few values occur (one segment): about 2.5 and 1.1 ms.
+constexpr uint32_t kFseSegs = 32, kFseLongThreads = 4 * kFseSegs, kFseLongWarps = kFseLongThreads / 32;
+constexpr uint32_t kFseSegBatches = 16; // fewest batches (of four steps) in a segment, if there are several
 
-__global__ void __launch_bounds__(32) kFseEncStates(const FseEncTask* __restrict__ tasks, uint32_t nbTasks)
+__global__ void __launch_bounds__(kFseLongThreads) kFseEncLong(const FseEncTask* __restrict__ tasks,
+                                                               uint32_t* __restrict__ sizes)
 {
-    extern __shared__ __align__(16) uint8_t smemFseSt[];
-    uint32_t const lane = threadIdx.x, g = lane >> 2, k = lane & 3u;
-    uint32_t const ti = blockIdx.x * kFseStChunks + g;
-    if (ti >= nbTasks) return; // the four lanes of a group leave together
-    unsigned const gm = 0xFu << (4 * g);
-    FseEncTask const t = tasks[ti];
-    uint8_t* const base = smemFseSt + size_t(g) * kFseStSlot;
-    uint32_t* const dnb = reinterpret_cast<uint32_t*>(base);
-    int32_t* const dfs = reinterpret_cast<int32_t*>(base + 1024);
-    uint16_t* const st = reinterpret_cast<uint16_t*>(base + 2048);
-    const ent::FseCTable* ct = reinterpret_cast<const ent::FseCTable*>(t.ctable);
-    for (uint32_t y = k; y < 256; y += 4) {
-        dnb[y] = ct->deltaNbBits[y];
-        dfs[y] = ct->deltaFindState[y];
-    }
+    __shared__ uint2 tt[256];      // per symbol: deltaNbBits, deltaFindState
+    __shared__ uint16_t st[2048];
+    __shared__ uint32_t endState[kFseSegs][4], segBits[kFseSegs];
+    __shared__ uint32_t win[kFseLongWarps][64];
+    __shared__ uint32_t edgeWord[kFseLongWarps][2], edgeAt[kFseLongWarps][2]; // first and last word of each warp
+    FseEncTask const t = tasks[blockIdx.x];
+    uint32_t const tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, g = tid >> 2, k = tid & 3u;
+    const ent::FseCTable* const ct = reinterpret_cast<const ent::FseCTable*>(t.ctable);
     uint32_t const size = 1u << t.tableLog;
-    for (uint32_t u = k; u < size; u += 4) st[u] = ct->state[u];
-    __syncwarp(gm);
+    for (uint32_t y = tid; y < 256; y += kFseLongThreads) tt[y] = make_uint2(ct->deltaNbBits[y], uint32_t(ct->deltaFindState[y]));
+    for (uint32_t u = tid; u < size; u += kFseLongThreads) st[u] = ct->state[u];
+    // symbols present (an absent one's pair asks for tableLog + 1 bits)
+    uint32_t const absent = ((t.tableLog + 1) << 16) - size;
+    uint32_t const symbols = __syncthreads_count(tt[2 * tid].x != absent) + __syncthreads_count(tt[2 * tid + 1].x != absent);
 
-    uint32_t const n = t.n, r = n & 3u, s0 = 4u - r;
-    // the c-th symbol from the end belongs to state (s0 + c) % 4; the last
-    // four symbols start the states and emit nothing
-    uint32_t const cInit = (k + 4u - (s0 & 3u)) & 3u;
-    uint32_t v;
+    // The c-th symbol from the end belongs to state (s0 + c) % 4; the last
+    // four symbols start the states and emit nothing. Then the r = n % 4
+    // single symbols (fields 0 .. r - 1), then steps of four symbols: step i
+    // takes the bytes [ip - 4 i - 4, ip - 4 i), the top one for state 0, and
+    // state k's field is r + 4 i + k.
+    uint32_t const n = t.n, r = n & 3u, s0 = 4u - r, ip = n - 4 - r;
+    uint32_t const pad = (4u - r) & 3u; // entries start here, so that steps start at multiples of four
+    uint16_t* const fo = t.fields + pad;
+    uint32_t const steps = ip >> 2, batches = steps >> 2; // batches of four steps: 16 bytes of the source
+    uint32_t const warm = max(kFseSegBatches, (6 * size / symbols + 3) >> 2); // run-up, in batches
+    uint32_t const segs = min(kFseSegs, max(1u, batches / warm));
+    uint32_t bits = 0, v;
     {
-        uint32_t const y = t.src[n - 1 - cInit];
-        uint32_t const nbOut = (dnb[y] + (1u << 15)) >> 16;
-        uint32_t const x = (nbOut << 16) - dnb[y];
-        v = st[(x >> nbOut) + dfs[y]];
+        uint32_t const y = t.src[n - 1 - ((k + 4u - (s0 & 3u)) & 3u)];
+        uint32_t const nb = (tt[y].x + (1u << 15)) >> 16, x = (nb << 16) - tt[y].x;
+        v = st[(x >> nb) + tt[y].y];
     }
-    auto trans = [&](uint32_t y) -> uint32_t {
-        uint32_t const nb = (v + dnb[y]) >> 16;
-        uint32_t const e = (v & ((1u << nb) - 1u)) | (nb << 12);
-        v = st[(v >> nb) + dfs[y]];
+    // one transition with the symbol's pair; returns the entry
+    auto trans = [&](uint2 d) -> uint32_t {
+        uint32_t const nb = (v + d.x) >> 16, q = v >> nb;
+        uint32_t const e = (v - (q << nb)) + (nb << 12);
+        v = st[q + d.y];
+        bits += nb;
         return e;
     };
-    uint16_t* const fo = t.fields;
-    for (uint32_t c = 4; c < 4 + r; c++) // the n % 4 single symbols, fields 0 .. r - 1
-        if (((s0 + c) & 3u) == k) fo[c - 4] = uint16_t(trans(t.src[n - 1 - c]));
-    // then four symbols per word (its top byte for state 0), fields
-    // r + 4 t + k of step t. The next step's symbol and its two per-symbol
-    // entries do not depend on the state: they load while the state's
-    // next-state load is in flight, so a transition's chain is one shared
-    // load and a few integer operations.
-    uint32_t ip = n - 4 - r;
-    if (ip) {
-        BackWords bw;
-        bw.start(t.src, n, ip, reinterpret_cast<uint32_t*>(base + kFseLaneTables) + k * 4 * kEncRing);
-        uint32_t const shift = 24 - 8 * k;
-        uint32_t y = (bw.next() >> shift) & 0xffu;
-        uint32_t a = dnb[y];
-        int32_t b = dfs[y];
-        for (uint32_t f = r + k;; f += 4) {
-            uint32_t const nb = (v + a) >> 16;
-            uint32_t const e = (v & ((1u << nb) - 1u)) | (nb << 12);
-            uint32_t const next = (v >> nb) + b;
-            ip -= 4;
-            if (ip) {
-                y = (bw.next() >> shift) & 0xffu;
-                a = dnb[y];
-                b = dfs[y];
-            }
-            v = st[next];
-            fo[f] = uint16_t(e);
-            if (!ip) break;
+    for (uint32_t c = 4; c < 4 + r; c++)
+        if (((s0 + c) & 3u) == k) {
+            uint32_t const e = trans(tt[t.src[n - 1 - c]]);
+            if (g == 0) fo[c - 4] = uint16_t(e);
         }
-        asm volatile("cp.async.wait_all;" ::: "memory"); // no copy outlives the lane
+    if (g) bits = 0;
+
+    // Batches [from, to) from state v. A batch's 16 source bytes come from
+    // the one or two aligned blocks that hold them, three batches ahead.
+    uintptr_t const top = reinterpret_cast<uintptr_t>(t.src) + ip;
+    uint32_t const off = uint32_t(top & 15);
+    auto run = [&](uint32_t from, uint32_t to, bool write) {
+        if (from >= to) return;
+        const uint4* a = reinterpret_cast<const uint4*>(top - off) - (from + 1); // lower block of batch `from`
+        uint4 const zero = make_uint4(0, 0, 0, 0);
+        uint4 up = off ? __ldg(a + 1) : zero, lo = __ldg(a);
+        uint4 n1 = from + 1 < to ? __ldg(a - 1) : zero, n2 = from + 2 < to ? __ldg(a - 2) : zero;
+        for (uint32_t b = from; b < to; b++) {
+            a--;
+            uint4 const n3 = b + 3 < to ? __ldg(a - 2) : zero;
+            uint4 const w = off ? shiftCombine(lo, up, off >> 2, (off & 3) * 8) : lo;
+            uint32_t const sel = 0x4443u - k;
+            uint2 const d0 = tt[__byte_perm(w.w, 0, sel)], d1 = tt[__byte_perm(w.z, 0, sel)],
+                        d2 = tt[__byte_perm(w.y, 0, sel)], d3 = tt[__byte_perm(w.x, 0, sel)];
+            uint32_t const e0 = trans(d0), e1 = trans(d1), e2 = trans(d2), e3 = trans(d3);
+            if (write) {
+                uint16_t* const f = fo + r + 16 * b + k;
+                f[0] = uint16_t(e0);
+                f[4] = uint16_t(e1);
+                f[8] = uint16_t(e2);
+                f[12] = uint16_t(e3);
+            }
+            up = lo;
+            lo = n1;
+            n1 = n2;
+            n2 = n3;
+        }
+    };
+    uint32_t const b0 = g < segs ? batches * g / segs : 0, b1 = g < segs ? batches * (g + 1) / segs : 0;
+    uint32_t const singles = bits;
+    if (g && g < segs) {
+        uint32_t const w0 = b0 > warm ? b0 - warm : 0;
+        if (w0) v = size;
+        run(w0, b0, false);
     }
-    fo[n - 4 + k] = uint16_t((v & (size - 1u)) | (t.tableLog << 12));
-}
+    uint32_t entry = v, check[4], quarterBits[4];
+    auto quarter = [&](uint32_t q) { return b0 + (b1 - b0) * q / 4; };
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+        bits = 0;
+        run(quarter(q), quarter(q + 1), true);
+        check[q] = v;
+        quarterBits[q] = bits;
+    }
+    if (g < segs) endState[g][k] = v;
+    __syncthreads();
+    for (;;) {
+        uint32_t const want = g && g < segs ? endState[g - 1][k] : entry;
+        bool const bad = want != entry;
+        if (!__syncthreads_or(bad)) break;
+        if (bad) {
+            entry = v = want;
+            bool met = false;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; q++)
+                if (!met) {
+                    bits = 0;
+                    run(quarter(q), quarter(q + 1), true);
+                    quarterBits[q] = bits;
+                    met = v == check[q];
+                    check[q] = v;
+                }
+            endState[g][k] = check[3];
+        }
+        __syncthreads();
+    }
+    bits = singles + quarterBits[0] + quarterBits[1] + quarterBits[2] + quarterBits[3];
+    if (g == segs - 1) { // the steps past the last batch, then the state's flush
+        v = check[3];
+        for (uint32_t i = 4 * batches; i < steps; i++) fo[r + 4 * i + k] = uint16_t(trans(tt[t.src[ip - 4 * i - 1 - k]]));
+        fo[n - 4 + k] = uint16_t((v & (size - 1u)) | (t.tableLog << 12));
+        bits += t.tableLog;
+    }
+    bits += __shfl_xor_sync(0xffffffffu, bits, 1);
+    bits += __shfl_xor_sync(0xffffffffu, bits, 2);
+    if (k == 0) segBits[g] = g < segs ? bits : 0u;
+    __syncthreads();
 
-constexpr uint32_t kFsePackWarps = 4;
-
-__global__ void __launch_bounds__(32 * kFsePackWarps) kFseEncPack(const FseEncTask* __restrict__ tasks,
-                                                                   uint32_t nbTasks, uint32_t* __restrict__ sizes)
-{
-    // 64-word windows: a round places at most 128 x 12 bits (48 words) above
-    // the partial word carried from the round before
-    __shared__ uint32_t win[kFsePackWarps][64];
-    uint32_t const lane = threadIdx.x & 31u, wi = threadIdx.x >> 5;
-    uint32_t const ti = blockIdx.x * kFsePackWarps + wi;
-    if (ti >= nbTasks) return; // the whole warp
-    FseEncTask const t = tasks[ti];
-    uint32_t* const w = win[wi];
+    // 3. the warp's segments [sg0, sg1), entries [j0, j1) from `fields` on
+    uint32_t const cap = n + n / 128 + 512; // the one-lane encoder's capacity
+    uint8_t* const out = t.out;
+    uint32_t* const w = win[wid];
     w[lane] = 0;
     w[lane + 32] = 0;
     __syncwarp();
-    uint32_t const n = t.n, cap = t.n + t.n / 128 + 512; // the one-lane encoder's capacity
-    uint8_t* const out = t.out;
-    uint32_t B = 0, wb = 0; // bits placed; first word not written yet
-    auto flushWords = [&](uint32_t upTo) { // words [wb, upTo) are complete
+    uint32_t const sg0 = segs * wid / kFseLongWarps, sg1 = segs * (wid + 1) / kFseLongWarps;
+    uint32_t before = lane < sg0 ? segBits[lane] : 0u, total = segBits[lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        before += __shfl_xor_sync(0xffffffffu, before, o);
+        total += __shfl_xor_sync(0xffffffffu, total, o);
+    }
+    uint32_t B = before, wb = before >> 5; // bits placed; first word not written yet
+    auto startOf = [&](uint32_t sg) { return sg == 0 ? 0u : sg >= segs ? pad + n : pad + r + 16 * (batches * sg / segs); };
+    uint32_t const j0 = startOf(sg0), j1 = startOf(sg1);
+    if (lane == 0) {
+        edgeAt[wid][0] = edgeAt[wid][1] = before >> 5;
+        edgeWord[wid][0] = edgeWord[wid][1] = 0;
+    }
+    auto flushWords = [&](uint32_t upTo) { // words [wb, upTo) are complete but for the warp's first one
         for (uint32_t q = wb + lane; q < upTo; q += 32) {
             uint32_t const x = w[q & 63u];
             w[q & 63u] = 0;
-            if (4 * q + 4 <= cap) *reinterpret_cast<uint32_t*>(out + 4 * q) = x;
+            if (q == before >> 5) edgeWord[wid][0] = x;
+            else if (4 * q + 4 <= cap) *reinterpret_cast<uint32_t*>(out + 4 * q) = x;
         }
         __syncwarp();
         wb = upTo;
     };
     const uint2* const src = reinterpret_cast<const uint2*>(t.fields);
-    uint32_t const nw = (n + 3) >> 2; // entries in groups of four
-    uint2 d = lane < nw ? src[lane] : make_uint2(0u, 0u);
-    for (uint32_t i0 = 0; i0 < nw; i0 += 32) {
+    uint32_t const g1 = (j1 + 3) >> 2; // entries in groups of four (j0 is a multiple of four)
+    uint32_t gi = (j0 >> 2) + lane;
+    uint2 d = gi < g1 ? src[gi] : make_uint2(0u, 0u);
+    for (uint32_t i0 = j0 >> 2; i0 < g1; i0 += 32) {
         uint2 const cur = d;
-        uint32_t const inext = i0 + 32 + lane;
-        d = inext < nw ? src[inext] : make_uint2(0u, 0u); // the next round's entries, in flight
         uint32_t const j = 4 * (i0 + lane);
+        gi = i0 + 32 + lane;
+        d = gi < g1 ? src[gi] : make_uint2(0u, 0u); // the next round's entries, in flight
         uint32_t e0 = cur.x & 0xffffu, e1 = cur.x >> 16, e2 = cur.y & 0xffffu, e3 = cur.y >> 16;
-        if (j + 0 >= n) e0 = 0;
-        if (j + 1 >= n) e1 = 0;
-        if (j + 2 >= n) e2 = 0;
-        if (j + 3 >= n) e3 = 0;
-        uint32_t const sum = (e0 >> 12) + (e1 >> 12) + (e2 >> 12) + (e3 >> 12);
+        if (j < pad || j + 4 > pad + n) { // entries outside the chunk's
+            if (j + 0 < pad || j + 0 >= pad + n) e0 = 0;
+            if (j + 1 < pad || j + 1 >= pad + n) e1 = 0;
+            if (j + 2 < pad || j + 2 >= pad + n) e2 = 0;
+            if (j + 3 < pad || j + 3 >= pad + n) e3 = 0;
+        }
+        uint32_t const n0 = e0 >> 12, n01 = n0 + (e1 >> 12), n012 = n01 + (e2 >> 12), sum = n012 + (e3 >> 12);
         uint32_t inc = sum;
 #pragma unroll
         for (uint32_t o = 1; o < 32; o <<= 1) {
             uint32_t const y = __shfl_up_sync(0xffffffffu, inc, o);
             if (lane >= o) inc += y;
         }
-        uint32_t p = B + inc - sum;
-        auto place = [&](uint32_t e) {
-            uint32_t const nb = e >> 12, f = e & 0xfffu;
-            if (nb) {
-                uint32_t const q = p >> 5, sh = p & 31u;
-                atomicOr(&w[q & 63u], f << sh);
-                if (sh + nb > 32) atomicOr(&w[(q + 1) & 63u], f >> (32 - sh));
-            }
-            p += nb;
-        };
-        place(e0);
-        place(e1);
-        place(e2);
-        place(e3);
+        uint32_t const p = B + inc - sum, q = p >> 5, sh = p & 31u;
+        if (sum) { // at most 48 bits, from bit sh of word q
+            uint64_t const f = uint64_t(e0 & 0xfffu) | (uint64_t(e1 & 0xfffu) << n0) | (uint64_t(e2 & 0xfffu) << n01)
+                               | (uint64_t(e3 & 0xfffu) << n012);
+            uint64_t const lo = f << sh;
+            atomicOr(&w[q & 63u], uint32_t(lo));
+            if (sh + sum > 32) atomicOr(&w[(q + 1) & 63u], uint32_t(lo >> 32));
+            if (sh + sum > 64) atomicOr(&w[(q + 2) & 63u], uint32_t(f >> (64 - sh)));
+        }
         B += __shfl_sync(0xffffffffu, inc, 31);
         __syncwarp();
         flushWords(B >> 5);
     }
-    // the end mark; a word it completes goes out as a word, then the bytes
-    if (lane == 0) w[(B >> 5) & 63u] |= 1u << (B & 31u);
-    B += 1;
-    __syncwarp();
-    flushWords(B >> 5);
-    uint32_t const bytes = (B + 7) >> 3;
-    for (uint32_t b = 4 * wb + lane; b < bytes; b += 32)
-        if (b < cap) out[b] = uint8_t(w[(b >> 2) & 63u] >> (8 * (b & 3u)));
-    if (lane == 0) sizes[t.sizeSlot] = bytes;
+    if (lane == 0 && sg0 < sg1) {
+        edgeAt[wid][1] = B >> 5;
+        edgeWord[wid][1] = w[(B >> 5) & 63u]; // the warp's last word, not complete (its first one, if it has no other)
+    }
+    __syncthreads();
+    // the words at the warps' edges, then the end mark: the word it completes
+    // goes out as a word, then the bytes
+    if (tid == 0) {
+        uint32_t at = 0, x = 0;
+        auto put = [&](uint32_t pos, uint32_t word) {
+            if (pos != at) {
+                if (4 * at + 4 <= cap) *reinterpret_cast<uint32_t*>(out + 4 * at) = x;
+                at = pos;
+                x = 0;
+            }
+            x |= word;
+        };
+        for (uint32_t q = 0; q < kFseLongWarps; q++) {
+            put(edgeAt[q][0], edgeWord[q][0]);
+            put(edgeAt[q][1], edgeWord[q][1]);
+        }
+        put(total >> 5, 1u << (total & 31u));
+        uint32_t const bytes = (total + 1 + 7) >> 3;
+        if (((total + 1) & 31u) == 0) {
+            put(at + 1, 0);
+        } else {
+            for (uint32_t b = 4 * at; b < bytes; b++)
+                if (b < cap) out[b] = uint8_t(x >> (8 * (b & 3u)));
+        }
+        sizes[t.sizeSlot] = bytes;
+    }
 }
 
 // Huffman: one lane per stream (4 per chunk for 4X); symbols are appended
@@ -1197,11 +1293,7 @@ __global__ void __launch_bounds__(256) kTokEmit(const TokTask* __restrict__ task
 
 cudaError_t prepareEncodeKernels()
 {
-    cudaError_t const e = cudaFuncSetAttribute(kFseEnc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               int(kFseEncLanes * kFseLaneBytes));
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(kFseEncStates, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                int(kFseStChunks * kFseStSlot));
+    return cudaFuncSetAttribute(kFseEnc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFseEncLanes * kFseLaneBytes));
 }
 
 uint32_t hufEncStreamCap(uint32_t seg) { return ((seg + (seg >> 3) + 64) + 15) & ~15u; }
@@ -1239,9 +1331,7 @@ void launchFseEnc(const FseEncTask* t, uint32_t n, uint32_t* sizes, cudaStream_t
 }
 void launchFseEncLong(const FseEncTask* t, uint32_t n, uint32_t* sizes, cudaStream_t s)
 {
-    if (!n) return;
-    kFseEncStates<<<(n + kFseStChunks - 1) / kFseStChunks, 32, kFseStChunks * kFseStSlot, s>>>(t, n);
-    kFseEncPack<<<(n + kFsePackWarps - 1) / kFsePackWarps, 32 * kFsePackWarps, 0, s>>>(t, n, sizes);
+    if (n) kFseEncLong<<<n, kFseLongThreads, 0, s>>>(t, sizes);
 }
 void launchHufEnc(const HufEncTask* t, uint32_t n, uint32_t* sizes, cudaStream_t s)
 {

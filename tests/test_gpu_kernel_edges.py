@@ -110,3 +110,37 @@ def test_huf_windows_alignments_and_table_logs(gpu_lib):
     out, frames = _round_trip(arrays, 8, 0, [k % 16 for k in range(len(arrays))])
     for a, g, f in zip(arrays, out, frames):
         assert g.tobytes() == a.tobytes() == oracle.decompress(f)[0].tobytes(), a.size
+
+
+def _frames(arrays, recipe, width):
+    import torch
+    import openzl_gb300 as oz
+
+    enc, n = oz.GpuEncoder(), len(arrays)
+    srcs = [torch.from_numpy(np.concatenate([np.zeros(k % 16, np.uint8), a.view(np.uint8)])).cuda() for k, a in enumerate(arrays)]
+    caps = [enc.bound(a.nbytes) for a in arrays]
+    dsts = [torch.zeros(c, dtype=torch.uint8, device="cuda") for c in caps]
+    sizes = enc.compress_batch([s.data_ptr() + k % 16 for k, s in enumerate(srcs)], [a.size for a in arrays], [width] * n,
+                               [recipe] * n, [d.data_ptr() for d in dsts], caps, checksums=True)
+    return [d[:s].cpu().numpy().tobytes() for d, s in zip(dsts, sizes)]
+
+
+def test_fse_encoder_segments(gpu_lib):
+    """Long FSE chunks cut into one to 32 segments: from two symbols (one
+    segment) to 256, chains that forget their start at once and chains that
+    hardly do, lengths around the batches, sources at every alignment. Frames
+    equal the oracle's."""
+    rng = np.random.default_rng(31)
+    arrays = []
+    for n in [4096 + k for k in range(34)] + [8191, 12345, 32768, 65536, 99999]:
+        for symbols in (2, 3, 5, 20, 60, 256):
+            kind = rng.integers(0, 3)
+            if kind == 0:  # one dominant symbol
+                a = np.where(rng.random(n) < 0.97, 0, rng.integers(0, symbols, n))
+            elif kind == 1:
+                a = np.minimum(rng.geometric(min(0.9, 3.0 / symbols), n) - 1, symbols - 1)
+            else:  # two halves that differ
+                a = np.concatenate([rng.integers(0, symbols, n // 2), np.minimum(rng.geometric(0.5, n - n // 2) - 1, symbols - 1)])
+            arrays.append(a.astype(np.uint8))
+    for a, f in zip(arrays, _frames(arrays, 7, 0)):
+        assert f == oracle.compress(7, a, 0).tobytes(), a.size
