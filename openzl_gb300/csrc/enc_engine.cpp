@@ -801,10 +801,6 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
 {
     Impl& I = *impl_;
     launches_ = 0;
-    static std::once_flag prepOnce;
-    static cudaError_t prepErr = cudaSuccess;
-    std::call_once(prepOnce, [] { prepErr = prepareEncodeKernels(); });
-    if (prepErr != cudaSuccess) { err = "kernel attributes"; return 1; }
     size_t const nf = frames.size();
     sizes.assign(nf, 0);
     std::vector<Front> fronts(nf);
@@ -1689,11 +1685,11 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
         Bump stg{ I.bufE.data() + stageOff, 0 };
         layoutE(b, stg, true);
         if (b.used > stageOff) { err = "encode layout overflow"; return 1; }
-        // longest chunks first: one lane encodes a chunk serially, so the
-        // longest chains start at once and the short ones fill around them
-        // (each task writes its own output and size slot)
+        // longest chunks first: the longest chains start at once and the
+        // short ones fill around them (each task writes its own output and
+        // size slot)
         std::stable_sort(fseT.begin(), fseT.end(), [](const FseEncTask& a, const FseEncTask& c) { return a.n > c.n; });
-        // long chunks (one lane per state) are the first nbLong of fseT
+        // long chunks (a CTA each) are the first nbLong of fseT
         size_t nbLong = 0;
         while (nbLong < fseT.size() && fseT[nbLong].fields) nbLong++;
         std::stable_sort(hufT.begin(), hufT.end(), [](const HufEncTask& a, const HufEncTask& c) { return a.n > c.n; });
@@ -1749,7 +1745,7 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
         launchFseEnc(dFse + nbLong, uint32_t(fseT.size() - nbLong), dSizes, st);
         launchHufEnc(dHuf, uint32_t(hufT.size()), dSizes, st);
         launchPack(dPack, dPackTiles, uint32_t(packTiles.size()), st);
-        launches_ += (fseT.empty() ? 0 : 1) + (nbLong ? 2 : 0) + (fseT.size() > nbLong ? 1 : 0)
+        launches_ += (fseT.empty() ? 0 : 1) + (nbLong ? 1 : 0) + (fseT.size() > nbLong ? 1 : 0)
                      + (hufT.empty() ? 0 : 1) + (packTiles.empty() ? 0 : 1);
         std::vector<uint32_t> hs(nbSizes + 1);
         uint32_t tabErr = 0;

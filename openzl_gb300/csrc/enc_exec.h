@@ -6,7 +6,6 @@
 
 namespace ozl {
 
-cudaError_t prepareEncodeKernels();
 uint32_t hufEncStreamCap(uint32_t segmentSize);
 void launchEncMax(const EncNumTask* t, const TileRef* tiles, uint32_t nbTiles, unsigned long long* maxima,
                   cudaStream_t s);
@@ -31,7 +30,7 @@ void launchTokCount(const TokTask* t, uint32_t nbTasks, const TileRef* tiles, ui
 void launchHist16(const Hist16Task* t, const TileRef* tiles, uint32_t nbTiles, cudaStream_t s);
 // 16-bit chunks: tokenize indices.
 void launchTok16(const Tok16Task* t, const TileRef* tiles, uint32_t nbTiles, cudaStream_t s);
-// 16-bit-symbol Huffman streams, one thread per stream.
+// 16-bit-symbol Huffman streams, one warp per stream.
 void launchHuf16Enc(const Huf16EncTask* t, uint32_t n, uint32_t* sizes, cudaStream_t s);
 // Sorted tokenize: indices renumbered to the sorted alphabet.
 void launchRemap(const RemapTask* t, const TileRef* tiles, uint32_t nbTiles, cudaStream_t s);

@@ -144,3 +144,26 @@ def test_fse_encoder_segments(gpu_lib):
             arrays.append(a.astype(np.uint8))
     for a, f in zip(arrays, _frames(arrays, 7, 0)):
         assert f == oracle.compress(7, a, 0).tobytes(), a.size
+
+
+@pytest.mark.parametrize("recipe,width", [(7, 0), (8, 0), (8, 2)])
+def test_warp_written_bitstreams(gpu_lib, recipe, width):
+    """Short FSE chunks and Huffman streams of 8- and 16-bit symbols, which a
+    warp writes in rounds: every length around the rounds (256 bytes, 128
+    values, one and four streams), sources at every alignment, codes from one
+    bit to the longest. Frames equal the oracle's."""
+    rng = np.random.default_rng(256 + recipe + width)
+    arrays = []
+    for n in list(range(10, 60)) + [k * 128 + d for k in (1, 2, 4, 7) for d in range(-3, 4)] + [
+            k * 1024 + d for k in (1, 2) for d in range(-5, 6)] + [997, 998, 999, 1000, 1001, 4095, 32768, 99999]:
+        if width == 2:
+            a = (rng.zipf(1.3, n) % 3000 if n % 2 else np.minimum(rng.geometric(1 / 3000, n), 65535)).astype(np.uint16)
+        elif n % 3 == 0:
+            a = np.where(rng.random(n) < 0.9, 3, rng.integers(0, 256, n)).astype(np.uint8)
+        elif n % 3 == 1:
+            a = np.minimum(rng.geometric(0.2, n), 255).astype(np.uint8)
+        else:
+            a = np.minimum(np.abs(rng.normal(100, 30, n)), 255).astype(np.uint8)
+        arrays.append(a)
+    for a, f in zip(arrays, _frames(arrays, recipe, width)):
+        assert f == oracle.compress(recipe, a, width).tobytes(), a.size
