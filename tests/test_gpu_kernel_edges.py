@@ -167,3 +167,27 @@ def test_warp_written_bitstreams(gpu_lib, recipe, width):
         arrays.append(a)
     for a, f in zip(arrays, _frames(arrays, recipe, width)):
         assert f == oracle.compress(recipe, a, width).tobytes(), a.size
+
+
+@pytest.mark.parametrize("width", [1, 2, 4, 8])
+def test_front_end_tiles_and_vectors(gpu_lib, width):
+    """Every front end (planes, packed at small, odd and full widths, plain)
+    around the 4,096-element tiles, the 16- and 32-element rounds and the
+    16-byte vectors, sources on and off a 16-byte boundary. Frames equal the
+    oracle's."""
+    rng = np.random.default_rng(4096 + width)
+    dt = {1: np.uint8, 2: np.uint16, 4: np.uint32, 8: np.uint64}[width]
+    sizes = [12, 15, 16, 17, 31, 33, 63, 4095, 4096, 4097, 4098, 8191 + 16, 8192 + 1, 8192 + 33, 3 * 4096 + 2]
+    for recipe in (1, 2, 3, 4, 9, 10, 11, 12):
+        arrays = []
+        for k, n in enumerate(sizes):
+            step = [1, 3, 50, 3000, 1 << 20, 1 << 40][k % 6]
+            arrays += [(1000 + np.cumsum(rng.integers(-step, step + 1, n))).astype(dt)] * 2
+        if width > 1:  # _frames offsets sources by bytes: keep them on element boundaries
+            arrays = [a for a in arrays for _ in range(width)]
+        frames = _frames(arrays, recipe, width)
+        for k, (a, f) in enumerate(zip(arrays, frames)):
+            if k and arrays[k - 1] is a and k % width:
+                assert f == frames[k - 1]
+            else:
+                assert f == oracle.compress(recipe, a, width).tobytes(), (recipe, a.size)
