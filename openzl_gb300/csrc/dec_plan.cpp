@@ -1380,6 +1380,8 @@ int layoutPlan(const DecodePlan& plan, const uint8_t* const* dFrames, uint8_t* c
                 t.w = O.w;
                 t.srcMode = nd.srcMode;
                 t.nbBits = nd.nbBits;
+                // fields of the full width are little-endian elements
+                if (t.srcMode == SRC_BITPACK && t.nbBits == 8 * t.w) t.srcMode = SRC_PLAIN;
                 t.zigzag = nd.zigzag;
                 t.delta = nd.delta;
                 if (nd.delta && O.n) {
@@ -1509,8 +1511,10 @@ int layoutPlan(const DecodePlan& plan, const uint8_t* const* dFrames, uint8_t* c
     auto addTiled = [&](int kind, int lv, auto& tasks, auto tilesOf) {
         if (tasks.empty()) return;
         std::vector<TileRef> tiles;
+        uint32_t mostTiles = 0;
         for (size_t i = 0; i < tasks.size(); i++) {
             uint32_t nt = tilesOf(tasks[i]);
+            mostTiles = std::max(mostTiles, nt);
             tasks[i].tileBase = uint32_t(tiles.size());
             for (uint32_t k = 0; k < nt; k++) tiles.push_back(TileRef{ uint32_t(i), k });
         }
@@ -1523,6 +1527,7 @@ int layoutPlan(const DecodePlan& plan, const uint8_t* const* dFrames, uint8_t* c
         L.tileOff = pool.put(tiles);
         L.nbTiles = uint32_t(tiles.size());
         if (kind == KIND_NUMPIPE) {
+            L.param0 = mostTiles;
             bool anyDelta = false;
             for (auto& t : tasks) anyDelta |= reinterpret_cast<const NumPipeTask&>(t).delta != 0;
             if (anyDelta) {
