@@ -962,17 +962,28 @@ struct PosStream {
                      "@q cp.async.ca.shared.global.L2::128B [s + %5], [a], 16;\n\t}"
                      : "+r"(low) : "r"(goal), "r"(ringAddr), "l"(g16), "n"(16 * RING - 16), "n"(-16 * RING) : "memory");
     }
-    // `area`: byte of the kBytes of shared memory
-    __device__ __forceinline__ bool init(const uint8_t* p, uint32_t size, const uint8_t* sm, uint32_t area)
+    // the stream's top bit and its first; `area`: byte of the kBytes of shared memory
+    __device__ __forceinline__ bool open(const uint8_t* p, uint32_t size, const uint8_t* sm, uint32_t area)
     {
-        if (!streamStart(p, size, g16, pos, end)) return false;
         smem = sm;
         ring = area + 16;
         ringAddr = uint32_t(__cvta_generic_to_shared(sm + ring));
+        return streamStart(p, size, g16, pos, end);
+    }
+    // goes on from position `to`: fills the ring below it
+    __device__ __forceinline__ void seek(int32_t to)
+    {
+        close(); // a copy in flight may be to the same place
+        pos = to;
         int32_t const first = ((pos - 1) >> 7) * 16, goal = max(first - 16 * AHEAD, 0);
         low = first + 16;
         while (low > goal) next(goal);
         asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    }
+    __device__ __forceinline__ bool init(const uint8_t* p, uint32_t size, const uint8_t* sm, uint32_t area)
+    {
+        if (!open(p, size, sm, area)) return false;
+        seek(pos);
         return true;
     }
     // Keeps AHEAD chunks below the position's in the ring, given that at most
@@ -1449,41 +1460,126 @@ __global__ void __launch_bounds__(32) kFse4(const FseTask* __restrict__ tasks, u
 }
 
 // ---------------------------------------------------------------------------
+// One Huffman stream on several lanes. A decoder that starts inside a code
+// soon meets the true code boundaries, so the stream's bits are cut into S
+// runs of equal length:
+//  1. each lane counts the codes of its run from its first bit, noting its
+//     place kMeetBits into the run and where the last code ends;
+//  2. a lane whose run truly starts elsewhere (where the run before it ended)
+//     counts again from there, up to the noted place if it comes by it, else
+//     to the run's end; this repeats until all agree (codes whose lengths have
+//     a common factor may need all runs one after another, as one lane would);
+//  3. the counts give each run's place in the output (the caller decodes again
+//     from the true starts, and stores).
+// Decoding twice costs less than what it buys: a chunk's streams were four
+// chains on four lanes of its table's shared memory, which bounds how many
+// tables an SM holds.
+constexpr int32_t kMeetBits = 256;
+template <int T>
+struct SplitShared {
+    int32_t pos[T];
+    uint32_t count[T];
+};
+struct SplitRun {
+    int32_t start;          // the run's first bit (top)
+    uint32_t count, before; // its codes, the codes of the stream's runs before it
+    bool ok;                // the stream holds n codes and ends at its first bit
+};
+// Runs of at least 1,024 bits, at most `lanes`.
+__device__ __forceinline__ uint32_t splitRuns(int32_t bits, uint32_t lanes)
+{
+    return max(1u, min(lanes, uint32_t(max(bits, 0)) >> 10));
+}
+// Every thread of the CTA calls it. j < S: the thread's run of its stream
+// (br, opened), whose first run is thread tid - j's; run(bound): decodes codes
+// until the position is at or below `bound` and returns their number.
+template <int T, class Stream, class Run>
+__device__ __forceinline__ SplitRun splitStream(Stream& br, Run run, uint32_t j, uint32_t S, uint32_t n, SplitShared<T>& sh)
+{
+    uint32_t const tid = threadIdx.x;
+    bool const mine = j < S;
+    int32_t p = 0, e = 0, c = 0, meet = 0;
+    uint32_t upToMeet = 0, count = 0;
+    if (mine) {
+        int32_t const top = br.pos, bits = top - br.end;
+        p = top - int32_t(int64_t(bits) * j / S);
+        e = top - int32_t(int64_t(bits) * (j + 1) / S);
+        c = max(p - kMeetBits, e);
+        br.seek(p);
+        upToMeet = run(c);
+        meet = br.pos;
+        count = upToMeet + run(e);
+        sh.pos[tid] = br.pos;
+    }
+    __syncthreads();
+    int32_t used = p;
+    for (;;) {
+        int32_t const want = mine && j ? sh.pos[tid - 1] : used;
+        bool const differs = want != used;
+        if (!__syncthreads_or(differs)) break;
+        if (differs) {
+            used = want;
+            br.seek(want);
+            uint32_t const m = run(c);
+            if (br.pos == meet) {
+                count += m - upToMeet;
+            } else {
+                meet = br.pos;
+                count = m + run(e);
+                sh.pos[tid] = br.pos;
+            }
+            upToMeet = m;
+        }
+        __syncthreads();
+    }
+    sh.count[tid] = mine ? count : 0;
+    __syncthreads();
+    SplitRun r{ used, count, 0, false };
+    if (mine) {
+        uint32_t total = 0;
+        for (uint32_t k = 0; k < S; k++) {
+            if (k == j) r.before = total;
+            total += sh.count[tid - j + k];
+        }
+        r.ok = total == n && sh.pos[tid - j + S - 1] == br.end;
+    }
+    return r;
+}
+
 // Huffman: weights -> canonical table (symbols ranked by weight then value;
 // weight w spans 2^(w-1) cells, nbBits = tableLog + 1 - w), after
-// src/openzl/fse/decompress/huf_decompress.c:342-454. The first warp of a CTA
-// decodes up to eight chunks, four lanes per chunk (one per stream of a 4X
-// chunk; lane 0 alone for 1X) sharing the chunk's table (16-bit cells: symbol
-// << 8 | nbBits); both warps build the tables. Table slots hold tableLog 11,
-// the largest the reference's encoder emits (encode_entropy_binding.c:222,
-// HUF_TABLELOG_DEFAULT); chunks with tableLog 12 take two slots, one chunk at
-// a time after the others.
+// src/openzl/fse/decompress/huf_decompress.c:342-454. One CTA of T threads per
+// chunk: T / 4 lanes for each stream of a 4X chunk, all for a 1X one
+// (splitStream). The table (16-bit cells: symbol << 8 | nbBits) has room for
+// tableLog 11, the largest the reference's encoder emits
+// (encode_entropy_binding.c:222, HUF_TABLELOG_DEFAULT); at tableLog 12 it takes
+// the rings' room too, and one lane a stream decodes.
 //
-// What bounds it: a symbol's code length comes from a table lookup, so a
-// stream is a chain of lookups (shift, address, shared-memory load, shift: 35
-// cycles), and the tables limit an SM to 48 chunks, six warps of 32 streams,
-// which do not hide it. So everything else leaves the chain: the window is
-// loaded by position once per four symbols (PosStream), a cell's low five bits
-// are its shift amount, ring refills are two predicated copies per 16 symbols
-// without a branch, and 16 symbols share a store. A warp builds a table in a
-// few thousand cycles: symbols ranked 32 at a time, then one weight's cells
-// after another (one lane ranking all symbols and filling runs of unequal
-// length took longer than 1,000 symbols' decoding).
-// A 256 MiB timestamp frame (4,224 chunks of 32 KiB): 0.46 ms before, 0.33 now;
-// one chunk of about 100,000 symbols, a stream of 25,000: 1.12 and 0.75 ms.
+// What bounds it: a symbol's code length comes from a table lookup, so a lane
+// is a chain of lookups (shift, address, shared-memory load, shift: 43
+// cycles). With four lanes a chunk, 48 chunks an SM held six warps, each
+// stalled five cycles of six, and a lone chunk left the SM idle. Several lanes
+// a stream end both, at two decodes; where chunks fill the GPU the lookups'
+// bank conflicts (each of a warp's 32 hits about 3.4 deep) bound it instead.
+// What leaves the chain: the window is loaded by position once per four
+// symbols (PosStream), a cell's low five bits are the shift amount, refills are
+// a predicated copy per eight symbols, 16 symbols share a store.
+// A 256 MiB timestamp frame (4,224 chunks of 32 KiB): 0.46 ms with a register
+// window and one lane a stream, 0.33 with the present step, 0.32 now; one
+// chunk of about 100,000 symbols: 1.12, 0.75 and 0.095 ms.
 constexpr uint32_t kHufTableLog = 12;
-constexpr uint32_t kHufChunks = 8;
-constexpr uint32_t kHufSlotBytes = 2u << 11;
 using HufStream = PosStream<8, 4>;
-constexpr uint32_t kHufAreaBytes = 4 * HufStream::kBytes; // a chunk's four rings; the table build's scratch before
 struct HufScratch {
     uint32_t count[16], next[16];
     uint8_t sorted[256];
 };
-static_assert(sizeof(HufScratch) <= kHufAreaBytes && kHufAreaBytes % 16 == 0, "the scratch lies in the rings' memory");
-// tables (two slots at least, for a tableLog-12 chunk), then the rings
-__host__ __device__ __forceinline__ uint32_t hufAreaOff(uint32_t chunks) { return (chunks < 2 ? 2 : chunks) * kHufSlotBytes; }
-__host__ __device__ __forceinline__ uint32_t hufSmem(uint32_t chunks) { return hufAreaOff(chunks) + chunks * kHufAreaBytes; }
+// table, rings (or a tableLog-12 table and the rings of four lanes), scratch
+template <int T>
+struct HufSmem {
+    static constexpr uint32_t kRings = 2u << 11, kWideRings = 2u << 12;
+    static constexpr uint32_t kUsed = kRings + T * HufStream::kBytes, kWide = kWideRings + 4 * HufStream::kBytes;
+    static constexpr uint32_t kScratch = kUsed > kWide ? kUsed : kWide, kBytes = kScratch + sizeof(HufScratch);
+};
 
 // Ranks the symbols by weight (every lane of the warp calls it): count[w]
 // symbols of weight w in `sorted`, from the sum of the counts below w.
@@ -1535,18 +1631,19 @@ __device__ __forceinline__ uint32_t hufRankWarp(const uint8_t* weights, uint32_t
 }
 
 // Fills the cells of a table from the ranked symbols, one weight after another
-// (every lane of the warp calls it); two cells a store where a symbol has them.
-__device__ __forceinline__ void hufFillWarp(const HufScratch& S, uint32_t tl, uint16_t* tab)
+// (every thread of the CTA calls it); two cells a store where a symbol has them.
+template <int T>
+__device__ __forceinline__ void hufFill(const HufScratch& S, uint32_t tl, uint16_t* tab)
 {
-    uint32_t const lane = threadIdx.x & 31;
+    uint32_t const lane = threadIdx.x;
     uint32_t base = 0, start = 0;
     for (uint32_t w = 1; w <= tl; w++) {
         uint32_t const c = S.count[w], nb = tl + 1 - w;
         if (w == 1) {
-            for (uint32_t j = lane; j < c; j += 32) tab[j] = uint16_t((uint32_t(S.sorted[j]) << 8) | nb);
+            for (uint32_t j = lane; j < c; j += T) tab[j] = uint16_t((uint32_t(S.sorted[j]) << 8) | nb);
         } else { // the weight's first cell is a multiple of its symbols' spans
             uint32_t* const d = reinterpret_cast<uint32_t*>(tab + start);
-            for (uint32_t j = lane; j < c << (w - 2); j += 32)
+            for (uint32_t j = lane; j < c << (w - 2); j += T)
                 d[j] = ((uint32_t(S.sorted[base + (j >> (w - 2))]) << 8) | nb) * 0x10001u;
         }
         base += c;
@@ -1554,41 +1651,54 @@ __device__ __forceinline__ void hufFillWarp(const HufScratch& S, uint32_t tl, ui
     }
 }
 
-__device__ __forceinline__ void hufDecodeStream(const HufTask& t, const uint8_t* smem, uint32_t tab, uint32_t tl,
-                                                uint32_t sIdx, uint32_t area, uint32_t* status)
+template <int T>
+__global__ void __launch_bounds__(T) kHuf(const HufTask* __restrict__ tasks, uint32_t* __restrict__ status)
 {
-    const uint8_t* sp;
-    uint32_t ssize, n, o0;
-    if (t.x4) {
-        if (t.bitsSize < 10) { if (sIdx == 0) reportError(status, DERR_CORRUPTION); return; }
-        uint32_t const l1 = t.bits[0] | (t.bits[1] << 8);
-        uint32_t const l2 = t.bits[2] | (t.bits[3] << 8);
-        uint32_t const l3 = t.bits[4] | (t.bits[5] << 8);
-        if (6ull + l1 + l2 + l3 > t.bitsSize) { if (sIdx == 0) reportError(status, DERR_CORRUPTION); return; }
-        uint32_t const l4 = t.bitsSize - 6 - l1 - l2 - l3;
-        uint32_t const seg = (t.dstSize + 3) / 4;
-        if (3ull * seg > t.dstSize) { if (sIdx == 0) reportError(status, DERR_CORRUPTION); return; }
-        uint32_t off = 6;
-        off += sIdx > 0 ? l1 : 0;
-        off += sIdx > 1 ? l2 : 0;
-        off += sIdx > 2 ? l3 : 0;
-        sp = t.bits + off;
-        ssize = sIdx == 0 ? l1 : (sIdx == 1 ? l2 : (sIdx == 2 ? l3 : l4));
-        o0 = seg * sIdx;
-        n = sIdx == 3 ? t.dstSize - 3 * seg : seg;
-    } else {
-        if (sIdx != 0) return;
-        sp = t.bits;
-        ssize = t.bitsSize;
-        o0 = 0;
-        n = t.dstSize;
+    using M = HufSmem<T>;
+    __shared__ __align__(16) uint8_t smem[M::kBytes];
+    __shared__ SplitShared<T> split;
+    __shared__ uint32_t sTl;
+    HufTask const t = tasks[blockIdx.x];
+    HufScratch& S = *reinterpret_cast<HufScratch*>(smem + M::kScratch);
+    uint32_t const tid = threadIdx.x;
+    if (tid < 32) {
+        uint32_t const r = hufRankWarp(t.weights, t.nbWeights, S);
+        if (tid == 0) sTl = r;
     }
+    __syncthreads();
+    uint32_t const tl = sTl;
+    // the streams' places (the whole CTA agrees on them)
+    bool ok = tl != 0;
+    uint32_t const lanes = t.x4 ? T / 4 : T, sIdx = tid / lanes, j = tid % lanes; // lanes of a stream, stream, run
+    uint32_t size = t.bitsSize, off = 0, o0 = 0, n = t.dstSize;
+    if (t.x4 && ok) {
+        ok = t.bitsSize >= 10;
+        if (ok) {
+            uint32_t const l1 = t.bits[0] | (t.bits[1] << 8);
+            uint32_t const l2 = t.bits[2] | (t.bits[3] << 8);
+            uint32_t const l3 = t.bits[4] | (t.bits[5] << 8);
+            uint32_t const seg = (t.dstSize + 3) / 4;
+            ok = 6ull + l1 + l2 + l3 <= t.bitsSize && 3ull * seg <= t.dstSize;
+            off = 6 + (sIdx > 0 ? l1 : 0) + (sIdx > 1 ? l2 : 0) + (sIdx > 2 ? l3 : 0);
+            size = sIdx == 0 ? l1 : sIdx == 1 ? l2 : sIdx == 2 ? l3 : t.bitsSize - 6 - l1 - l2 - l3;
+            o0 = seg * sIdx;
+            n = sIdx == 3 ? t.dstSize - 3 * seg : seg;
+        }
+    }
+    if (!ok) {
+        if (tid == 0) reportError(status, DERR_CORRUPTION);
+        return;
+    }
+    hufFill<T>(S, tl, reinterpret_cast<uint16_t*>(smem));
+    bool const wide = tl > 11;
     HufStream br;
-    if (!br.init(sp, ssize, smem, area)) { reportError(status, DERR_CORRUPTION); return; }
-    uint8_t* const out = t.out + o0;
+    uint32_t const area = wide ? M::kWideRings + (sIdx & 3) * HufStream::kBytes : M::kRings + tid * HufStream::kBytes;
+    bool const opened = br.open(t.bits + off, size, smem, area);
+    uint32_t const runs = !opened ? 0 : wide ? 1 : splitRuns(br.pos - br.end, lanes);
+    __syncthreads(); // the table is filled
     uint32_t const sh = 32u - tl;
     // the cell of the code at the top of hi; its low five bits are the shift amount
-    auto cell = [&](uint32_t hi) -> uint32_t { return *reinterpret_cast<const uint16_t*>(smem + tab + 2 * (hi >> sh)); };
+    auto cell = [&](uint32_t hi) -> uint32_t { return *reinterpret_cast<const uint16_t*>(smem + 2 * (hi >> sh)); };
     auto four = [&]() -> uint32_t {
         uint32_t hi, lo, c[4];
         br.window(hi, lo);
@@ -1604,18 +1714,45 @@ __device__ __forceinline__ void hufDecodeStream(const HufTask& t, const uint8_t*
         br.pos -= int32_t((c[0] + c[1] + c[2] + c[3]) & 255u);
         return __byte_perm(__byte_perm(c[0], c[1], 0x0051), __byte_perm(c[2], c[3], 0x0051), 0x5410);
     };
-    uint32_t i = 0;
-    auto single = [&]() {
-        br.refill<1>();
+    auto one = [&]() -> uint32_t {
         uint32_t hi, lo;
+        br.refill<1>();
         br.window(hi, lo);
         uint32_t const c = cell(hi);
-        out[i] = uint8_t(c >> 8);
         br.pos -= int32_t(c & 31u);
+        return c >> 8;
     };
-    uint32_t const head = min(n, uint32_t((16 - (reinterpret_cast<uintptr_t>(out) & 15)) & 15));
-    for (; i < head; i++) single();
-    for (; i + 16 <= n; i += 16) { // eight codes are at most 12 bytes
+    auto run = [&](int32_t bound) -> uint32_t { // eight codes are at most 96 bits, twelve bytes
+        uint32_t m = 0;
+        for (; br.pos - bound >= 96; m += 8) {
+            br.refill<1>();
+            four();
+            four();
+        }
+        if (br.pos - bound >= 48) {
+            br.refill<1>();
+            four();
+            m += 4;
+        }
+        for (; br.pos > bound; m++) one();
+        return m;
+    };
+    SplitRun const r = splitStream<T>(br, run, j, runs, n, split);
+    if (j >= runs) {
+        if (!opened && j == 0) reportError(status, DERR_CORRUPTION);
+        return;
+    }
+    if (!r.ok) {
+        if (j == 0) reportError(status, DERR_CORRUPTION);
+        br.close();
+        return;
+    }
+    br.seek(r.start);
+    uint8_t* const out = t.out + o0 + r.before;
+    uint32_t const cnt = r.count, head = min(cnt, uint32_t((16 - (reinterpret_cast<uintptr_t>(out) & 15)) & 15));
+    uint32_t i = 0;
+    for (; i < head; i++) out[i] = uint8_t(one());
+    for (; i + 16 <= cnt; i += 16) {
         uint4 v;
         br.refill<1>();
         v.x = four();
@@ -1625,56 +1762,8 @@ __device__ __forceinline__ void hufDecodeStream(const HufTask& t, const uint8_t*
         v.w = four();
         *reinterpret_cast<uint4*>(out + i) = v;
     }
-    for (; i < n; i++) single();
+    for (; i < cnt; i++) out[i] = uint8_t(one());
     br.close();
-    if (!br.finished()) reportError(status, DERR_CORRUPTION);
-}
-
-__global__ void __launch_bounds__(64) kHuf(const HufTask* __restrict__ tasks, uint32_t nbTasks, uint32_t chunks,
-                                           uint32_t* __restrict__ status)
-{
-    extern __shared__ __align__(16) uint8_t smemHuf[];
-    __shared__ uint32_t sTl[kHufChunks];
-    uint32_t const wid = threadIdx.x >> 5, areas = hufAreaOff(chunks);
-    for (uint32_t k = wid; k < chunks; k += 2) {
-        uint32_t const tk = blockIdx.x * chunks + k;
-        uint32_t tl = 0;
-        if (tk < nbTasks) {
-            const uint8_t* const weights = tasks[tk].weights;
-            HufScratch& S = *reinterpret_cast<HufScratch*>(smemHuf + areas + k * kHufAreaBytes);
-            tl = hufRankWarp(weights, tasks[tk].nbWeights, S);
-            if (tl && tl <= 11) hufFillWarp(S, tl, reinterpret_cast<uint16_t*>(smemHuf + k * kHufSlotBytes));
-            if (!tl && (threadIdx.x & 31) == 0) reportError(status, DERR_CORRUPTION);
-        }
-        if ((threadIdx.x & 31) == 0) sTl[k] = tl;
-    }
-    __syncthreads();
-    if (wid != 0) return;
-    // tableLog <= 11: each chunk in its own slot
-    uint32_t const c = threadIdx.x >> 2, sIdx = threadIdx.x & 3; // chunk of this CTA, stream of the chunk
-    bool wide = false;
-    if (c < chunks) {
-        uint32_t const tl = sTl[c];
-        wide = tl > 11;
-        if (tl && !wide) {
-            HufTask const t = tasks[blockIdx.x * chunks + c];
-            hufDecodeStream(t, smemHuf, c * kHufSlotBytes, tl, sIdx, areas + c * kHufAreaBytes + sIdx * HufStream::kBytes,
-                            status);
-        }
-    }
-    if (!__any_sync(0xffffffffu, wide)) return;
-    // tableLog 12 (valid, but never emitted by the reference's encoder): one
-    // chunk at a time, its table across the first two slots
-    for (uint32_t k = 0; k < chunks; k++) {
-        if (sTl[k] <= 11) continue; // warp-uniform
-        HufTask const t = tasks[blockIdx.x * chunks + k];
-        HufScratch& S = *reinterpret_cast<HufScratch*>(smemHuf + areas);
-        uint32_t const tl = hufRankWarp(t.weights, t.nbWeights, S);
-        hufFillWarp(S, tl, reinterpret_cast<uint16_t*>(smemHuf));
-        __syncwarp();
-        if (threadIdx.x < 4) hufDecodeStream(t, smemHuf, 0, tl, threadIdx.x, areas + threadIdx.x * HufStream::kBytes, status);
-        __syncwarp();
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1692,28 +1781,28 @@ __global__ void __launch_bounds__(64) kHuf(const HufTask* __restrict__ tasks, ui
 // the ranges above it fill the rest). Codes of the other buckets find their
 // range by binary search. The validity rules of
 // decode_entropy_binding.c:349-412 apply: weights at most 20, at least two of
-// them non-zero, the sum of 2^(w-1) a power of two. One lane decodes each of
-// the one or four streams; like the reference, a stream is not required to end
-// exactly at its first bit (the planner checked that the stream table fills
-// the input exactly).
+// them non-zero, the sum of 2^(w-1) a power of two. Each of the one or four
+// streams is decoded by several lanes (splitStream); a stream that does not
+// hold its symbols exactly, which the reference does not refuse, by one.
 //
-// What bounds it: each stream is a serial chain, a lookup and a shift a symbol
+// What bounds it: a lane is a serial chain, a lookup and a shift a symbol
 // (four symbols per 64-bit window where codes have at most 16 bits, else
 // three). The search and three cached stream loads for every symbol took about
 // 550 cycles. A table of whole symbols over 12 bits was no help (5.99 ms):
 // 13-bit codes are the ordinary ones of large alphabets. The symbols' loads
 // (L1) leave the chain: they are stored a window later.
-// 98,304 symbols in four streams, geometric with mean 3000: 7.06 ms before,
-// 1.41 ms now.
-constexpr uint32_t kHuf16Log = 12, kHuf16Threads = 256, kHuf16Warps = kHuf16Threads / 32;
-using Huf16Stream = PosStream<16, 12>;
+// 98,304 symbols in four streams, geometric with mean 3000: 7.06 ms with one
+// lane a stream and the search, 1.41 with the table, 0.55 now.
+constexpr uint32_t kHuf16Log = 12, kHuf16Threads = 128, kHuf16Warps = kHuf16Threads / 32;
+using Huf16Stream = PosStream<8, 4>;
 
 __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restrict__ tasks, uint32_t* __restrict__ status)
 {
     __shared__ uint32_t sCount[kHuf16Warps][32], sStart[32], sBase[32];
     __shared__ uint32_t sTl, sOk;
     __shared__ uint32_t sTab[1u << kHuf16Log];
-    __shared__ __align__(16) uint8_t sRing[4 * Huf16Stream::kBytes];
+    __shared__ __align__(16) uint8_t sRing[kHuf16Threads * Huf16Stream::kBytes];
+    __shared__ SplitShared<kHuf16Threads> split;
     Huf16Task const t = tasks[blockIdx.x];
     uint32_t const tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     sCount[wid][lane] = 0;
@@ -1721,8 +1810,8 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
     __syncthreads();
     // every warp takes a run of symbols: counts per weight, then each warp's
     // first place among the symbols of a weight, then the places
-    uint32_t const run = ((t.nbWeights + kHuf16Threads - 1) / kHuf16Threads) * 32;
-    uint32_t const b0 = min(t.nbWeights, wid * run), b1 = min(t.nbWeights, b0 + run);
+    uint32_t const share = ((t.nbWeights + kHuf16Threads - 1) / kHuf16Threads) * 32;
+    uint32_t const b0 = min(t.nbWeights, wid * share), b1 = min(t.nbWeights, b0 + share);
     bool bad = false;
     for (uint32_t b = b0; b < b1; b += 32) {
         uint32_t w = b + lane < b1 ? t.weights[b + lane] : 0u;
@@ -1803,38 +1892,26 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
         sTab[j] = a == b ? entryOf(a) : 0u;
     }
     __syncthreads();
-    if (tid >= t.nbStreams) return;
+    uint32_t const lanes = t.nbStreams == 4 ? kHuf16Threads / 4 : kHuf16Threads, sIdx = tid / lanes, j = tid % lanes;
     Huf16Stream br;
-    if (!br.init(t.stream[tid], t.streamSize[tid], sRing, tid * Huf16Stream::kBytes)) {
-        reportError(status, DERR_CORRUPTION);
-        return;
-    }
+    bool const opened = br.open(t.stream[sIdx], t.streamSize[sIdx], sRing, tid * Huf16Stream::kBytes);
+    uint32_t const runs = opened ? splitRuns(br.pos - br.end, lanes) : 0, n = t.count[sIdx];
+    int32_t const top = br.pos;
     auto symbol = [&](uint32_t hi, uint32_t e) -> uint32_t {
         return t.sorted[uint32_t(int32_t(e) >> 5) + __funnelshift_l(hi, 0u, e)];
     };
-    uint8_t* const out = t.out + 2ull * t.dstOff[tid];
-    uint32_t const n = t.count[tid];
-    uint32_t i = 0;
-    auto put = [&](uint32_t k, uint32_t y) {
-        if (!(reinterpret_cast<uintptr_t>(out) & 1)) {
-            reinterpret_cast<uint16_t*>(out)[k] = uint16_t(y);
-        } else {
-            out[2 * k] = uint8_t(y);
-            out[2 * k + 1] = uint8_t(y >> 8);
-        }
-    };
     // N codes at the position, N times the longest at most 64 bits: first as if
     // the table knew them all (an entry 0 shifts by nothing), with the search
-    // only when one was not known, so that a window takes one branch
-    auto codes = [&](auto& y) {
-        constexpr int N = int(sizeof(y) / sizeof(y[0]));
+    // only when one was not known, so that a window takes one branch. `get`
+    // takes each code's place, top bits and entry.
+    auto codes = [&](auto N, auto get) {
         uint32_t hi, lo, used = 0, least = ~0u;
         br.window(hi, lo);
         uint32_t const hi0 = hi, lo0 = lo;
 #pragma unroll
-        for (int k = 0; k < N; k++) { // an entry's low five bits are the shift amount
+        for (int k = 0; k < decltype(N)::value; k++) { // an entry's low five bits are the shift amount
             uint32_t const e = sTab[hi >> (32 - pl)];
-            y[k] = symbol(hi, e);
+            get(k, hi, e);
             used += e & 31u;
             least = min(least, e);
             hi = __funnelshift_l(lo, hi, e);
@@ -1844,14 +1921,11 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
             hi = hi0;
             lo = lo0;
             used = 0;
-#pragma unroll 1
-            for (int k = 0; k < N; k++) {
+#pragma unroll
+            for (int k = 0; k < decltype(N)::value; k++) {
                 uint32_t e = sTab[hi >> (32 - pl)];
                 if (e == 0) e = entryOf(weightOf(hi >> (32 - tl)));
-                uint32_t const z = symbol(hi, e);
-#pragma unroll
-                for (int m = 0; m < N; m++)
-                    if (m == k) y[m] = z;
+                get(k, hi, e);
                 used += e & 31u;
                 hi = __funnelshift_l(lo, hi, e);
                 lo = __funnelshift_l(0u, lo, e);
@@ -1859,26 +1933,75 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
         }
         br.pos -= int32_t(used);
     };
+    using One = std::integral_constant<int, 1>;
+    using Three = std::integral_constant<int, 3>;
+    using Four = std::integral_constant<int, 4>;
+    auto none = [](int, uint32_t, uint32_t) {};
+    bool const narrow = tl <= 16; // four codes a window, else three
+    // two windows are at most 16 bytes
+    auto run = [&](int32_t bound) -> uint32_t {
+        uint32_t m = 0;
+        while (br.pos - bound >= 128) {
+            br.refill<1>();
+            if (narrow) {
+                codes(Four(), none);
+                codes(Four(), none);
+                m += 8;
+            } else {
+                codes(Three(), none);
+                codes(Three(), none);
+                m += 6;
+            }
+        }
+        for (; br.pos > bound; m++) {
+            br.refill<1>();
+            codes(One(), none);
+        }
+        return m;
+    };
+    SplitRun r = splitStream<int(kHuf16Threads)>(br, run, j, runs, n, split);
+    if (j >= runs) {
+        if (!opened && j == 0 && sIdx < t.nbStreams) reportError(status, DERR_CORRUPTION);
+        return;
+    }
+    if (!r.ok) { // not exactly n symbols: the first lane decodes n
+        if (j) {
+            br.close();
+            return;
+        }
+        r = SplitRun{ top, n, 0, true };
+    }
+    br.seek(r.start);
+    uint8_t* const out = t.out + 2ull * (t.dstOff[sIdx] + r.before);
+    uint32_t const cnt = r.count;
+    uint32_t i = 0;
+    auto put = [&](uint32_t k, uint32_t y) {
+        if (!(reinterpret_cast<uintptr_t>(out) & 1)) {
+            reinterpret_cast<uint16_t*>(out)[k] = uint16_t(y);
+        } else {
+            out[2 * k] = uint8_t(y);
+            out[2 * k + 1] = uint8_t(y >> 8);
+        }
+    };
     auto single = [&]() {
         br.refill<1>();
-        uint32_t y[1];
-        codes(y);
-        put(i, y[0]);
+        uint32_t y = 0;
+        codes(One(), [&](int, uint32_t hi, uint32_t e) { y = symbol(hi, e); });
+        put(i, y);
     };
-    if (tl <= 16 && !(reinterpret_cast<uintptr_t>(out) & 1)) {
-        // four codes a window, sixteen symbols (32 bytes at most) a refill
-        uint32_t const head = min(n, uint32_t((8 - (reinterpret_cast<uintptr_t>(out) & 7)) & 7) >> 1);
+    if (narrow && !(reinterpret_cast<uintptr_t>(out) & 1)) {
+        uint32_t const head = min(cnt, uint32_t((8 - (reinterpret_cast<uintptr_t>(out) & 7)) & 7) >> 1);
         for (; i < head; i++) single();
         uint32_t y[4], i0 = i;
         auto store = [&](uint32_t k) {
             *reinterpret_cast<uint2*>(out + 2 * k) = make_uint2(__byte_perm(y[0], y[1], 0x5410), __byte_perm(y[2], y[3], 0x5410));
         };
-        for (; i + 16 <= n; i += 16) {
-            br.refill<3>();
+        for (; i + 8 <= cnt; i += 8) {
+            br.refill<1>();
 #pragma unroll
-            for (uint32_t q = 0; q < 16; q += 4) {
+            for (uint32_t q = 0; q < 8; q += 4) {
                 uint32_t z[4];
-                codes(z);
+                codes(Four(), [&](int k, uint32_t hi, uint32_t e) { z[k] = symbol(hi, e); });
                 if (i + q > i0) store(i + q - 4);
 #pragma unroll
                 for (int k = 0; k < 4; k++) y[k] = z[k];
@@ -1886,18 +2009,17 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
         }
         if (i > i0) store(i - 4);
     } else {
-        // three codes a window, fifteen symbols (38 bytes at most) a refill
         uint32_t y[3], i0 = i;
         auto store = [&](uint32_t k) {
 #pragma unroll
             for (int m = 0; m < 3; m++) put(k + m, y[m]);
         };
-        for (; i + 15 <= n; i += 15) {
-            br.refill<3>();
+        for (; i + 6 <= cnt; i += 6) {
+            br.refill<1>();
 #pragma unroll
-            for (uint32_t q = 0; q < 15; q += 3) {
+            for (uint32_t q = 0; q < 6; q += 3) {
                 uint32_t z[3];
-                codes(z);
+                codes(Three(), [&](int k, uint32_t hi, uint32_t e) { z[k] = symbol(hi, e); });
                 if (i + q > i0) store(i + q - 3);
 #pragma unroll
                 for (int k = 0; k < 3; k++) y[k] = z[k];
@@ -1905,7 +2027,7 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
         }
         if (i > i0) store(i - 3);
     }
-    for (; i < n; i++) single();
+    for (; i < cnt; i++) single();
     br.close();
 }
 
@@ -2289,12 +2411,14 @@ FseShape fseShape(const Launch& l)
     s.lanes = std::max(1u, std::min(s.lanes, maxLanes));
     return s;
 }
-// Chunks per CTA of an untuned Huffman launch: spread over the SMs first, up
-// to eight (a full warp), of which six CTAs fit an SM.
-uint32_t hufDefaultChunks(uint32_t nbTasks)
+// Threads per chunk of an untuned Huffman launch: four warps while all chunks
+// run at once (eight CTAs an SM by shared memory and threads; a round of
+// host-buffer decoding took 0.2 ms where one lane a stream took 0.9), a warp
+// from there on, which holds 26 chunks an SM.
+uint32_t hufThreads(const Launch& l)
 {
-    uint32_t const sms = uint32_t(smCount()), perSm = (nbTasks + sms - 1) / sms;
-    return std::max(1u, std::min(kHufChunks, (perSm + 5) / 6));
+    if (l.tune) return l.tune >= 128 ? 128 : 32;
+    return l.nbTasks <= 8 * uint32_t(smCount()) ? 128 : 32;
 }
 // kHashBlocks grid: one warp per block up to eight full CTAs per SM, then
 // grid-stride (any grid size is correct)
@@ -2304,7 +2428,6 @@ uint32_t hashGrid(uint32_t nbBlocks)
     uint32_t const cap = uint32_t(smCount()) * 8;
     return want < cap ? (want ? want : 1) : cap;
 }
-static_assert(2 * kHufSlotBytes >= (2u << kHufTableLog), "a tableLog-12 table fits two slots");
 } // namespace
 
 cudaError_t prepareKernels()
@@ -2316,7 +2439,7 @@ cudaError_t prepareKernels()
     }
     e = cudaFuncSetAttribute(kFse4, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFseCtaSmem));
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(kHuf, cudaFuncAttributeMaxDynamicSharedMemorySize, int(hufSmem(kHufChunks)));
+    return cudaSuccess;
 }
 
 uint32_t tuneCandidates(const Launch& l, uint32_t* out, uint32_t cap)
@@ -2329,7 +2452,7 @@ uint32_t tuneCandidates(const Launch& l, uint32_t* out, uint32_t cap)
         for (uint32_t c : { 8u, 6u, 4u }) // kFse4: streams per warp
             if (c <= mx && n < cap) out[n++] = kFse4Variant | c;
     } else if (l.kind == KIND_HUF) {
-        for (uint32_t c : { 8u, 6u, 4u, 2u })
+        for (uint32_t c : { 32u, 128u }) // threads per chunk
             if (n < cap) out[n++] = c;
     }
     return n;
@@ -2382,10 +2505,9 @@ long runOneLaunch(const DeviceLayout& L, size_t li, uint8_t* dPool, uint8_t* dSc
                 break;
             }
             case KIND_HUF: {
-                uint32_t const chunks = l.tune && l.tune <= kHufChunks ? l.tune : hufDefaultChunks(l.nbTasks);
-                uint32_t const grid = (l.nbTasks + chunks - 1) / chunks;
-                kHuf<<<grid, 64, hufSmem(chunks), s>>>(static_cast<const HufTask*>(tasks), l.nbTasks, chunks,
-                                                               dStatus);
+                const HufTask* const huf = static_cast<const HufTask*>(tasks);
+                if (hufThreads(l) == 128) kHuf<128><<<l.nbTasks, 128, 0, s>>>(huf, dStatus);
+                else kHuf<32><<<l.nbTasks, 32, 0, s>>>(huf, dStatus);
                 break;
             }
             case KIND_FLATPACK:

@@ -191,3 +191,23 @@ def test_front_end_tiles_and_vectors(gpu_lib, width):
                 assert f == frames[k - 1]
             else:
                 assert f == oracle.compress(recipe, a, width).tobytes(), (recipe, a.size)
+
+
+def test_huf_streams_that_do_not_fall_into_step(gpu_lib):
+    """Codes whose lengths are all even (a decoder started on an odd bit never
+    meets the true boundaries), codes of one length but for a few, and long
+    runs of one symbol: few chunks (four warps each) and more than the SMs hold
+    at once (a warp each)."""
+    rng = np.random.default_rng(77)
+    even = np.array([0, 1, 2] * 4 + [3, 4, 5, 6], np.uint8)
+    arrays = []
+    for n in (2000, 9000, 32768, 65536, 99999, 100001):
+        arrays.append(even[rng.integers(0, 16, n)])
+        arrays.append(np.where(rng.random(n) < 0.02, 255, rng.integers(0, 127, n)).astype(np.uint8))
+        arrays.append(np.where(rng.random(n) < 0.999, 9, rng.integers(0, 256, n)).astype(np.uint8))
+    out, frames = _round_trip(arrays, 8, 0, [k % 16 for k in range(len(arrays))])
+    for a, g, f in zip(arrays, out, frames):
+        assert g.tobytes() == a.tobytes() == oracle.decompress(f)[0].tobytes(), a.size
+    many = [a[:5000 + k] for k in range(500) for a in arrays if a.size >= 9000][:1600]
+    out, _ = _round_trip(many, 8, 0, [k % 16 for k in range(len(many))])
+    assert all(g.tobytes() == a.tobytes() for a, g in zip(many, out))
