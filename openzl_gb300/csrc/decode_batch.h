@@ -84,13 +84,13 @@ cudaError_t prepareOnce();
 // latency-bound entropy decoding. All parts share the plan's arena and
 // parameter block; each has its own descriptor pool and scratch.
 struct DecodeBatch {
-    static constexpr int kMaxParts = 17; // the critical part plus 8 runs of each of two kinds
+    static constexpr int kMaxParts = 18; // long checksums, the critical part, 8 runs of each of two kinds
     struct Part {
         DeviceLayout layout;
         DevBuf pool, scratch;
         std::vector<char> mask;   // frames of this part
-        bool critical = false;    // frames with a long FSE stream: highest stream priority
-        int run = 0;              // index of this run within its kind
+        bool longChecksum = false; // frames whose content checksum is the batch's longest chain
+        int rank = 0;              // stream priority, 0 the highest
     };
     bool checkContent = true;
     bool checkCompressed = true;
@@ -103,6 +103,13 @@ struct DecodeBatch {
     // kind; smaller ones into the Huffman frames and the others.
     static constexpr uint64_t kSplitBytes = 512ull << 20;
     static constexpr uint32_t kCriticalDefault = 16000;
+    // A frame of at least this many decoded bytes, and of at least half the
+    // batch's largest, is decoded ahead of the others: its content checksum is
+    // a serial chain (12.4 ns a KiB: 0.4 ms for 32 MiB, 3.3 ms for 256 MiB) that
+    // starts when the frame is decoded and then leaves the SMs to the rest. A
+    // 256 MiB column beside 0.43 GB of weight matrices: 5.23 ms before, when
+    // the column waited behind the matrices' entropy decoding, 4.33 now.
+    static constexpr uint64_t kLongChecksum = 32ull << 20;
     int schedule = 0;             // OZL_DParam_schedule: priority policy of the branches
     DecodePlan plan;
     std::vector<Part> parts;
@@ -221,22 +228,29 @@ struct DecodeBatch {
         uint64_t const critical = criticalSymbols >= 0 ? uint64_t(criticalSymbols) : big ? kCriticalDefault : 0;
         std::vector<char> kindOf(n, 0);
         for (const PlanNode& nd : plan.nodes)
-            if (!nd.dead && nd.id == 50 && nd.frame >= 0) kindOf[size_t(nd.frame)] = 1;
+            if (!nd.dead && (nd.id == 50 || nd.id == 51) && nd.frame >= 0) kindOf[size_t(nd.frame)] = 1;
         if (critical)
             for (const PlanNode& nd : plan.nodes)
                 if (!nd.dead && nd.id == 49 && nd.frame >= 0 && nd.out >= 0
                     && plan.streams[size_t(nd.out)].n >= critical)
                     kindOf[size_t(nd.frame)] = 2;
+        size_t largest = 0;
+        for (size_t x : sizes) largest = std::max(largest, x);
+        if (checkContent && largest >= kLongChecksum)
+            for (const PlanHash& h : plan.hashes)
+                if (h.err == DERR_CONTENT_CK && sizes[size_t(h.frame)] >= std::max<size_t>(kLongChecksum, largest / 2))
+                    kindOf[size_t(h.frame)] = 3;
         // the parts' device buffers outlive the plan: a new plan reuses them
         // (no allocation, and so no device-wide synchronization, per batch)
         struct Spec {
             std::vector<char> mask;
-            bool critical;
-            int run;
+            bool longChecksum;
+            int rank;
         };
         std::vector<Spec> specs;
+        int ahead = 0; // kinds ahead of the runs
         if (splitParts) {
-            for (char kind : { char(2), char(1), char(0) }) {
+            for (char kind : { char(3), char(2), char(1), char(0) }) {
                 std::vector<size_t> fr;
                 uint64_t total = 0;
                 for (size_t i = 0; i < n; i++)
@@ -245,9 +259,10 @@ struct DecodeBatch {
                         total += sizes[i];
                     }
                 if (fr.empty()) continue;
-                size_t const g = kind == 2 ? 1 : std::min<size_t>(size_t(runs), fr.size());
+                size_t const g = kind >= 2 ? 1 : std::min<size_t>(size_t(runs), fr.size());
                 size_t const first = specs.size();
-                for (size_t k = 0; k < g; k++) specs.push_back(Spec{ std::vector<char>(n, 0), kind == 2, int(k) });
+                for (size_t k = 0; k < g; k++) specs.push_back(Spec{ std::vector<char>(n, 0), kind == 3, ahead + int(k) });
+                if (kind >= 2) ahead++;
                 uint64_t acc = 0;
                 size_t k = 0;
                 for (size_t i : fr) {
@@ -265,8 +280,8 @@ struct DecodeBatch {
         parts.resize(specs.size());
         for (size_t p = 0; p < specs.size(); p++) {
             parts[p].mask = std::move(specs[p].mask);
-            parts[p].critical = specs[p].critical;
-            parts[p].run = specs[p].run;
+            parts[p].longChecksum = specs[p].longChecksum;
+            parts[p].rank = specs[p].rank;
             parts[p].layout = DeviceLayout();
         }
         if (!arena.reserve(plan.arenaBytes) || !params.reserve(plan.params.size()) || !status.reserve(64)) {
@@ -384,10 +399,11 @@ struct DecodeBatch {
     // Enqueues the plan on `s` as a DAG: each part (branch) runs its
     // dependency levels in order, and the launches of one level, which do not
     // depend on one another, on streams of their own. Stream priorities
-    // order the block scheduler's work. Schedule 0: a branch's launches share
-    // its rank: the critical part (the longest chains) first, then each
-    // kind's runs in order, so that a run's element-wise work shares the SMs
-    // with the next run's entropy decoding. Schedule 1: every element-wise
+    // order the block scheduler's work. A part of long checksums decodes alone:
+    // the others wait until only its checksums are left. Schedule 0: a branch's
+    // launches share its rank: long checksums and the critical part (the
+    // longest chains) first, then each kind's runs in order, so that a run's
+    // element-wise work shares the SMs with the next run's entropy decoding. Schedule 1: every element-wise
     // launch (short, memory-bound) ahead of all entropy decoding, which keeps
     // the branch ranks. `marks` (timeline runs): a timing event before and
     // after every launch, in part order, on its stream.
@@ -409,10 +425,8 @@ struct DecodeBatch {
         }
         int least = 0, greatest = 0;
         if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess) least = greatest = 0;
-        bool anyCritical = false;
-        for (const Part& p : parts) anyCritical = anyCritical || p.critical;
         auto prioOf = [&](const Part& p, int kind) {
-            int const branch = p.critical ? 0 : p.run + (anyCritical ? 1 : 0);
+            int const branch = p.rank;
             bool const entropy = kind == KIND_FSE || kind == KIND_HUF || kind == KIND_HUF16;
             int const rank = schedule == 1 ? (entropy ? 1 + branch : 0) : branch;
             return std::min(least, greatest + rank); // greatest is the numerically smallest
@@ -423,10 +437,12 @@ struct DecodeBatch {
         long total = 0;
         size_t mark = 0;
         std::vector<cudaEvent_t> ends;
+        cudaEvent_t others = start; // what the parts after a long-checksum part wait for
         for (size_t p = 0; p < parts.size(); p++) {
             const DeviceLayout& L = parts[p].layout;
-            cudaEvent_t ready = start; // everything the next level waits for
+            cudaEvent_t ready = parts[p].longChecksum ? start : others; // everything the next level waits for
             for (size_t a = 0; a < L.launches.size();) {
+                if (parts[p].longChecksum && L.launches[a].kind == KIND_HASH) others = ready;
                 size_t b = a;
                 while (b < L.launches.size() && L.launches[b].level == L.launches[a].level) b++;
                 std::vector<cudaStream_t> used;
