@@ -2222,28 +2222,18 @@ __global__ void __launch_bounds__(256) kHashBlocks(const HashTask* __restrict__ 
 }
 
 
-// The block chain acc = scramble(acc + sum), scramble(x) = ((x ^ (x >> 47)) ^
-// key) * PRIME32_1, of accumulator i over nb blocks, starting from init, with
-// key words (klo, khi); bs: 8 sums a block. Returns the accumulator after the
-// last block.
+// One step of the block chain acc = scramble(acc + sum), scramble(x) = ((x ^
+// (x >> 47)) ^ key) * PRIME32_1, on y = acc + sum of the block about to be
+// scrambled, in 32-bit halves; nv: the next block's sum.
 //
-// The chain is serial, so its latency per block is what bounds a long input's
-// checksum. It runs on y = acc + sum of the block about to be scrambled, in
-// 32-bit halves: x >> 47 only reaches the low half, so with t = y.lo ^
-// (y.hi >> 15) ^ key.lo and u = y.hi ^ key.hi the next y is t * P + C with
-// C = next sum + ((u * P) << 32). C needs only u and is ready before t, which
-// leaves a shift, a xor, the low product (whose addition of C.lo sets the
-// carry) and the high product with C.hi and that carry: 4 + 4 + 4 + 9 cycles
-// (dependent-issue latencies measured one by one). One 64-bit multiply-add
-// instead of the pair measured 27, and the product added to in two steps 23.
-// Each lane reads its accumulator's sums straight into registers, a batch of
-// 48 blocks ahead: 48 steps cover the load's way to L2, and no barrier or
-// shared-memory round trip stands on the path (batches of 32 measured 28.7
-// cycles a block, 48 measured 22.8).
-// 262,144 blocks (a 256 MiB input): 4.71 ms before (a warp staged the sums of
-// 32 blocks in shared memory, two-step product), 3.25 ms now.
-constexpr int kChainBatch = 48;
-constexpr uint32_t kChainAhead = 512; // blocks fetched into L2 ahead of the chain
+// The chain is serial, so its latency per block bounds a long input's
+// checksum. x >> 47 only reaches the low half, so with t = y.lo ^ (y.hi >> 15)
+// ^ key.lo and u = y.hi ^ key.hi the next y is t * P + C with C = next sum +
+// ((u * P) << 32). C needs only u and is ready before t, which leaves a shift,
+// a xor, the low product (whose addition of C.lo sets the carry) and the high
+// product with C.hi and that carry: 4 + 4 + 4 + 9 cycles (dependent-issue
+// latencies measured one by one). One 64-bit multiply-add instead of the pair
+// measured 27, and the product added to in two steps 23.
 __device__ __forceinline__ void xxhChainStep(uint32_t& ylo, uint32_t& yhi, uint32_t klo, uint32_t khi, uint64_t nv)
 {
     uint32_t const c = (yhi ^ khi) * XP32_1 + uint32_t(nv >> 32);
@@ -2251,76 +2241,59 @@ __device__ __forceinline__ void xxhChainStep(uint32_t& ylo, uint32_t& yhi, uint3
     asm("mad.lo.cc.u32 %0, %2, %3, %4;\n\tmadc.hi.u32 %1, %2, %3, %5;"
         : "=&r"(ylo), "=r"(yhi) : "r"(t), "r"(XP32_1), "r"(uint32_t(nv)), "r"(c));
 }
-__device__ __noinline__ uint64_t xxhBlockChain(const uint64_t* __restrict__ bs, uint32_t nb, uint64_t init,
-                                               uint32_t klo, uint32_t khi, uint32_t i)
-{
-    if (nb == 0) return init;
-    uint64_t const y0 = init + __ldg(bs + i); // init + sum of block 0
-    uint32_t ylo = uint32_t(y0), yhi = uint32_t(y0 >> 32);
-    uint32_t const m = nb - 1; // steps that add a next sum; the last block's step adds none
-    const uint64_t* p = bs + 8 + i;
-    uint64_t cur[kChainBatch], nxt[kChainBatch];
-    uint32_t b = 0;
-    // a lane fetches one line of two blocks into L2, `ahead` blocks on
-    auto fetchL2 = [&](uint32_t from) {
-        uint32_t const blk = from + 2 * (threadIdx.x & 31);
-        if (blk < nb) asm volatile("prefetch.global.L2 [%0];" ::"l"(bs + 8ull * blk));
-    };
-    for (uint32_t f = kChainBatch; f < kChainAhead; f += 64) fetchL2(f);
-    if (m >= kChainBatch) {
-#pragma unroll
-        for (int k = 0; k < kChainBatch; k++) cur[k] = __ldg(p + 8 * k);
-        for (; b + 2 * kChainBatch <= m; b += kChainBatch) {
-            p += 8 * kChainBatch;
-            fetchL2(b + kChainAhead);
-#pragma unroll
-            for (int k = 0; k < kChainBatch; k++) nxt[k] = __ldg(p + 8 * k);
-#pragma unroll
-            for (int k = 0; k < kChainBatch; k++) xxhChainStep(ylo, yhi, klo, khi, cur[k]);
-#pragma unroll
-            for (int k = 0; k < kChainBatch; k++) cur[k] = nxt[k];
-        }
-        p += 8 * kChainBatch;
-    }
-    // the last full batch, if any, while the sums after it load; then those
-    uint32_t const rest = m - b - (m >= kChainBatch ? kChainBatch : 0); // below kChainBatch
-#pragma unroll
-    for (int k = 0; k < kChainBatch; k++) nxt[k] = uint32_t(k) < rest ? __ldg(p + 8 * k) : 0;
-    if (m >= kChainBatch) {
-#pragma unroll
-        for (int k = 0; k < kChainBatch; k++) xxhChainStep(ylo, yhi, klo, khi, cur[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < kChainBatch; k++)
-        if (uint32_t(k) <= rest) xxhChainStep(ylo, yhi, klo, khi, nxt[k]); // step `rest` adds 0: the last block
-    return (uint64_t(yhi) << 32) | ylo;
-}
 
-// Phase 2: one warp per task. Lane i (and its copies i + 8, i + 16, i + 24)
-// runs the block chain of accumulator i, then the trailing partial stripes
-// and the final stripe, and lane 0 merges. The trailing stripes add to the
-// accumulators without a chain: the four groups of 8 lanes take every fourth
-// one (at most 15, and the final stripe as the sixteenth), loaded before the
-// chain starts.
-constexpr uint32_t kFinishWarps = 4;
-__global__ void __launch_bounds__(32 * kFinishWarps) kHashFinish(const HashTask* __restrict__ tasks, uint32_t nbTasks,
-                                                                 uint32_t* __restrict__ status)
+// Phase 2: a CTA of two warps per task. Lane i of the first (and its copies
+// i + 8, i + 16, i + 24) runs the block chain of accumulator i, then the
+// trailing partial stripes and the final stripe, and lane 0 merges. The second
+// warp brings the block sums into a ring of batches of 64 blocks in shared
+// memory, three ahead, so that the first does nothing but steps and a barrier
+// a batch. (Sums read by the chain's own warp, 48 blocks ahead into registers,
+// measured 24.2 cycles a block; staged in shared memory by that warp, 31.)
+// 262,144 blocks (a 256 MiB input): 4.71 ms with two dependent multiply-adds
+// and the sums staged by the warp, 2.77 ms now (20.9 cycles a block).
+// The trailing stripes add to the accumulators without a chain: the four groups
+// of 8 lanes take every fourth one (at most 15, and the final stripe as the
+// sixteenth), loaded before the chain starts.
+constexpr uint32_t kChainBatch = 64, kChainSlots = 4, kFinishThreads = 64;
+__global__ void __launch_bounds__(kFinishThreads) kHashFinish(const HashTask* __restrict__ tasks, uint32_t* __restrict__ status)
 {
-    uint32_t const ti = blockIdx.x * kFinishWarps + (threadIdx.x >> 5);
-    uint32_t const lane = threadIdx.x & 31;
-    if (ti >= nbTasks) return;
-    HashTask const t = tasks[ti];
+    __shared__ __align__(16) uint64_t ring[kChainSlots][8 * kChainBatch];
+    uint32_t const lane = threadIdx.x & 31, i = lane & 7, g = lane >> 3;
+    HashTask const t = tasks[blockIdx.x];
+    uint32_t const nb = t.len > 240 ? t.nbBlocks : 0;
+    // steps that add a next sum (that of block k + 1, step k); the last block's adds none
+    uint32_t const m = nb ? nb - 1 : 0, batches = (m + kChainBatch - 1) / kChainBatch;
+    if (threadIdx.x >= 32) {
+        auto issue = [&](uint32_t b) {
+            const uint64_t* const src = t.blockSums + 8 + 8ull * kChainBatch * b;
+            uint32_t const words = 8 * min(kChainBatch, b < batches ? m - kChainBatch * b : 0);
+#pragma unroll
+            for (uint32_t k = 2 * lane; k < 8 * kChainBatch; k += 64)
+                if (k < words) {
+                    uint32_t const d = uint32_t(__cvta_generic_to_shared(&ring[b % kChainSlots][k]));
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + k) : "memory");
+                }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        for (uint32_t b = 0; b + 1 < kChainSlots; b++) issue(b);
+        for (uint32_t b = 0; b < batches; b++) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kChainSlots - 2) : "memory");
+            __syncthreads(); // batch b is there; batch b - 1 has been read
+            issue(b + kChainSlots - 1);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return;
+    }
     bool const al = t.aligned8 != 0;
     uint64_t h;
     if (t.len <= 240) {
         if (lane != 0) return;
         h = xxh3Short(t.data, t.len, al);
     } else {
-        uint32_t const i = lane & 7, g = lane >> 3;
         uint64_t const init = i == 0 ? XP32_3 : i == 1 ? XP64_1 : i == 2 ? XP64_2 : i == 3 ? XP64_3
                             : i == 4 ? XP64_4 : i == 5 ? XP32_2 : i == 6 ? XP64_5 : XP32_1;
         uint64_t const key = kXxhWords.w8[16 + i];
-        uint32_t const nb = t.nbBlocks;
+        uint32_t const klo = uint32_t(key), khi = uint32_t(key >> 32);
         uint64_t const len = t.len;
         uint32_t const nbStripes = uint32_t(((len - 1) - uint64_t(kHashBlock) * nb) / 64);
         const uint8_t* const last = t.data + uint64_t(kHashBlock) * nb;
@@ -2331,7 +2304,21 @@ __global__ void __launch_bounds__(32 * kFinishWarps) kHashFinish(const HashTask*
             const uint8_t* const p = st == 15 ? t.data + len - 64 : last + 64 * st;
             v[j] = st < nbStripes || st == 15 ? ldData(p + 8 * i, al) : 0;
         }
-        uint64_t acc = xxhBlockChain(t.blockSums, nb, init, uint32_t(key), uint32_t(key >> 32), i);
+        uint64_t const y0 = init + (nb ? t.blockSums[i] : 0); // init + sum of block 0
+        uint32_t ylo = uint32_t(y0), yhi = uint32_t(y0 >> 32);
+        for (uint32_t b = 0; b < batches; b++) {
+            __syncthreads();
+            const uint64_t* const s = ring[b % kChainSlots] + i;
+            uint32_t const cnt = min(kChainBatch, m - kChainBatch * b);
+            if (cnt == kChainBatch) {
+#pragma unroll
+                for (uint32_t k = 0; k < kChainBatch; k++) xxhChainStep(ylo, yhi, klo, khi, s[8 * k]);
+            } else {
+                for (uint32_t k = 0; k < cnt; k++) xxhChainStep(ylo, yhi, klo, khi, s[8 * k]);
+            }
+        }
+        if (nb) xxhChainStep(ylo, yhi, klo, khi, 0); // the last block
+        uint64_t acc = (uint64_t(yhi) << 32) | ylo;
         uint64_t part = 0;
 #pragma unroll
         for (uint32_t j = 0; j < 4; j++) {
@@ -2549,8 +2536,7 @@ long runOneLaunch(const DeviceLayout& L, size_t li, uint8_t* dPool, uint8_t* dSc
                                                                    l.nbTiles);
                     count++;
                 }
-                uint32_t const grid = (l.nbTasks + kFinishWarps - 1) / kFinishWarps;
-                kHashFinish<<<grid, 32 * kFinishWarps, 0, s>>>(static_cast<const HashTask*>(tasks), l.nbTasks, dStatus);
+                kHashFinish<<<l.nbTasks, kFinishThreads, 0, s>>>(static_cast<const HashTask*>(tasks), dStatus);
                 break;
             }
             default:
@@ -2576,7 +2562,7 @@ void launchHash(const HashTask* tasks, uint32_t nbTasks, const TileRef* blocks, 
                 cudaStream_t s)
 {
     if (nbBlocks) kHashBlocks<<<hashGrid(nbBlocks), 256, 0, s>>>(tasks, blocks, nbBlocks);
-    if (nbTasks) kHashFinish<<<(nbTasks + kFinishWarps - 1) / kFinishWarps, 32 * kFinishWarps, 0, s>>>(tasks, nbTasks, status);
+    if (nbTasks) kHashFinish<<<nbTasks, kFinishThreads, 0, s>>>(tasks, status);
 }
 
 cudaError_t xxh3Device(const uint8_t* data, uint64_t len, uint64_t* dHashOut, uint8_t* dScratch,
@@ -2603,7 +2589,7 @@ cudaError_t xxh3Device(const uint8_t* data, uint64_t len, uint64_t* dHashOut, ui
         if (e != cudaSuccess) return e;
         kHashBlocks<<<hashGrid(nbBlocks), 256, 0, s>>>(dTask, dTiles, nbBlocks);
     }
-    kHashFinish<<<1, 32, 0, s>>>(dTask, 1, nullptr);
+    kHashFinish<<<1, kFinishThreads, 0, s>>>(dTask, nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return cudaStreamSynchronize(s);
@@ -2679,7 +2665,7 @@ extern "C" ZL_Report ozl_gpu_xxh3_64_static(const void* d_data, size_t len, void
     uint32_t const stageThreads = nbBlocks > 0 ? nbBlocks : 1;
     kStageHashStatic<<<(stageThreads + 255) / 256, 256, 0, s>>>(t, dTask, dBlocks, nbBlocks, dResult);
     if (nbBlocks) ozl::kHashBlocks<<<ozl::hashGrid(nbBlocks), 256, 0, s>>>(dTask, dBlocks, nbBlocks);
-    ozl::kHashFinish<<<1, 32, 0, s>>>(dTask, 1, nullptr);
+    ozl::kHashFinish<<<1, ozl::kFinishThreads, 0, s>>>(dTask, nullptr);
     if (cudaGetLastError() != cudaSuccess) return ZL_Report{ ZL_ErrorCode_GENERIC, 0 };
     uint64_t h = 0;
     if (cudaMemcpyAsync(&h, dResult, 8, cudaMemcpyDeviceToHost, s) != cudaSuccess
