@@ -20,11 +20,17 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <condition_variable>
 #include <cstddef>
 #include <cstring>
+#include <exception>
+#include <functional>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
+
+#include <unistd.h>
 
 #include "dec_exec.h"
 #include "enc_exec.h"
@@ -85,6 +91,30 @@ struct Piece {
     const uint8_t* dev = nullptr;
     const uint8_t* host = nullptr;
     uint64_t bytes = 0;
+};
+
+// A stream's pieces; nearly all streams have one, which takes no allocation.
+struct Pieces {
+    Piece one;
+    std::vector<Piece> many; // two or more
+    size_t n = 0;
+    void push_back(const Piece& p)
+    {
+        if (n == 0) {
+            one = p;
+        } else {
+            if (n == 1) {
+                many.reserve(6);
+                many.push_back(one);
+            }
+            many.push_back(p);
+        }
+        n++;
+    }
+    bool empty() const { return n == 0; }
+    const Piece* begin() const { return n > 1 ? many.data() : &one; }
+    const Piece* end() const { return begin() + n; }
+    const Piece& operator[](size_t k) const { return begin()[k]; }
 };
 
 enum : int { M_FSE = 0, M_HUF, M_CONSTANT, M_FLATPACK, M_BITPACK, M_ANY };
@@ -166,7 +196,7 @@ struct RStream {
     int type;
     uint32_t w;
     uint64_t n;
-    std::vector<Piece> pieces; // content (contiguous device pointer is pieces[0] when single)
+    Pieces pieces; // content (contiguous device pointer is pieces[0] when single)
     bool store = false;
     uint64_t bytes() const { return n * w; }
 };
@@ -223,28 +253,112 @@ struct PinnedBuf {
     }
 };
 
-// host threads of the calling compress() (0: the machine's, at most 16)
-thread_local unsigned tlHostThreads = 0;
+// Helper threads of one encoder's host loops, kept for its lifetime: a loop
+// wakes them, and starting fifteen threads took 0.8 ms, longer than any loop.
+// One loop runs at a time (an encoder runs one compress() at a time). A forked
+// child has no such threads: there nothing is waited for, and the copied
+// state, whose condition variables still count them as waiting, is left alone.
+class HostPool {
+  public:
+    ~HostPool()
+    {
+        if (!s_ || pid_ != getpid()) return;
+        {
+            std::lock_guard<std::mutex> l(s_->m);
+            s_->stop = true;
+        }
+        s_->wake.notify_all();
+        for (std::thread& t : s_->threads) t.join();
+        delete s_;
+    }
+    // work() on the calling thread and on up to `helpers` others; returns when
+    // no thread runs it any more. It must not throw.
+    void run(unsigned helpers, const std::function<void()>& work)
+    {
+        if (!s_ || pid_ != getpid()) {
+            s_ = new State;
+            pid_ = getpid();
+        }
+        State& s = *s_;
+        {
+            std::lock_guard<std::mutex> l(s.m);
+            try {
+                while (s.threads.size() < helpers) s.threads.emplace_back([&s] { loop(s); });
+            } catch (const std::system_error&) { // as many as there are
+            }
+            s.work = &work;
+            s.open = unsigned(std::min<size_t>(helpers, s.threads.size()));
+            s.generation++;
+        }
+        s.wake.notify_all();
+        work();
+        std::unique_lock<std::mutex> l(s.m);
+        s.open = 0; // a helper that has not begun stays out
+        s.idle.wait(l, [&] { return s.running == 0; });
+        s.work = nullptr;
+    }
 
-// fn(i) for i < n on up to 16 host threads (chunks of 64 indices)
+  private:
+    struct State {
+        std::mutex m;
+        std::condition_variable wake, idle;
+        std::vector<std::thread> threads;
+        const std::function<void()>* work = nullptr;
+        uint64_t generation = 0;
+        unsigned open = 0, running = 0;
+        bool stop = false;
+    };
+    static void loop(State& s)
+    {
+        uint64_t seen = 0;
+        std::unique_lock<std::mutex> l(s.m);
+        for (;;) {
+            s.wake.wait(l, [&] { return s.stop || (s.open && s.generation != seen); });
+            if (s.stop) return;
+            seen = s.generation;
+            s.open--;
+            s.running++;
+            const std::function<void()>* const w = s.work;
+            l.unlock();
+            (*w)();
+            l.lock();
+            if (--s.running == 0) s.idle.notify_one();
+        }
+    }
+    State* s_ = nullptr;
+    pid_t pid_ = 0;
+};
+
+// host threads and helpers of the calling compress() (0: the machine's, at most 16)
+thread_local unsigned tlHostThreads = 0;
+thread_local HostPool* tlPool = nullptr;
+
+// fn(i) for i < n on up to 16 host threads, in chunks of `grain` indices;
+// fewer than four chunks run on the calling thread
 template <class F>
-void parallelFor(size_t n, F fn)
+void parallelFor(size_t n, F fn, size_t grain = 64)
 {
     unsigned const hw = std::thread::hardware_concurrency();
-    unsigned const nt = std::min(tlHostThreads ? tlHostThreads : 16u, hw ? hw : 1u);
-    if (n < 256 || nt < 2) {
+    size_t const chunks = (n + grain - 1) / grain;
+    unsigned const nt = unsigned(std::min<size_t>(std::min(tlHostThreads ? tlHostThreads : 16u, hw ? hw : 1u), chunks));
+    if (chunks < 4 || nt < 2 || !tlPool) {
         for (size_t i = 0; i < n; i++) fn(i);
         return;
     }
     std::atomic<size_t> next{ 0 };
-    auto work = [&] {
-        for (size_t i; (i = next.fetch_add(64)) < n;)
-            for (size_t k = i; k < std::min(n, i + 64); k++) fn(k);
-    };
-    std::vector<std::thread> th;
-    for (unsigned t = 1; t < nt; t++) th.emplace_back(work);
-    work();
-    for (auto& x : th) x.join();
+    std::mutex m;
+    std::exception_ptr failed; // the first exception, thrown on the calling thread
+    tlPool->run(nt - 1, [&] {
+        try {
+            for (size_t i; (i = next.fetch_add(grain)) < n;)
+                for (size_t k = i; k < std::min(n, i + grain); k++) fn(k);
+        } catch (...) {
+            next.store(n); // no further chunks
+            std::lock_guard<std::mutex> l(m);
+            if (!failed) failed = std::current_exception();
+        }
+    });
+    if (failed) std::rethrow_exception(failed);
 }
 
 struct EncodeBatch::Impl {
@@ -261,7 +375,8 @@ struct EncodeBatch::Impl {
         if (hashStart) cudaEventDestroy(hashStart);
         if (hashDone) cudaEventDestroy(hashDone);
     }
-    PinnedBuf stage, stageH;
+    PinnedBuf stage, stageH, hists;
+    HostPool pool;
     std::vector<Job> jobs;           // data chunks (discovery order), then nested weights jobs
     size_t nbDataJobs = 0;
     bool checksums = true;
@@ -302,10 +417,10 @@ struct Engine {
         nd.push_back(x);
         return nd.back();
     }
-    static std::vector<Piece> slice(const std::vector<Piece>& p, uint64_t off, uint64_t len)
+    static Pieces slice(const Pieces& p, uint64_t off, uint64_t len)
     {
         // contiguous single-piece sources only
-        std::vector<Piece> r;
+        Pieces r;
         if (p.empty()) return r;
         Piece x = p[0];
         if (x.dev) x.dev += off;
@@ -542,7 +657,10 @@ struct Engine {
             newNode(type == T_STRUCT ? TR_SPLITN_STRUCT : TR_SPLITN, sid, 0);
             int const first = int(s.size());
             uint64_t pos = 0;
-            std::vector<Piece> src = s[sid].pieces;
+            Pieces const src = s[sid].pieces;
+            size_t const room = s.size() + 6 * size_t(nb); // what the chunks add
+            if (room > s.capacity()) s.reserve(std::max(room, 2 * s.capacity()));
+            if (room > nd.capacity()) nd.reserve(std::max(room, 2 * nd.capacity()));
             for (uint64_t k = 0; k < nb; k++) {
                 uint64_t const len = k + 1 < nb ? kChunk : n - pos;
                 int o = newStream(type, w, len);
@@ -786,11 +904,14 @@ void pushBits(std::vector<uint8_t>& o, const std::vector<uint32_t>& v, int nbBit
 {
     size_t const base = o.size();
     o.resize(base + (v.size() * size_t(nbBits) + 7) / 8, 0);
-    for (size_t i = 0; i < v.size(); i++) {
-        size_t bit = i * size_t(nbBits);
-        for (int b = 0; b < nbBits; b++, bit++)
-            if ((v[i] >> b) & 1) o[base + (bit >> 3)] |= uint8_t(1u << (bit & 7));
+    uint64_t acc = 0, mask = (1ull << nbBits) - 1;
+    int nb = 0; // bits in acc, below 8 between values
+    size_t at = base;
+    for (uint32_t x : v) {
+        acc |= (x & mask) << nb;
+        for (nb += nbBits; nb >= 8; nb -= 8, acc >>= 8) o[at++] = uint8_t(acc);
     }
+    if (nb) o[at] = uint8_t(acc);
 }
 
 } // namespace
@@ -805,6 +926,10 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
     sizes.assign(nf, 0);
     std::vector<Front> fronts(nf);
     tlHostThreads = hostThreads_;
+    tlPool = &I.pool;
+    struct NoPool {
+        ~NoPool() { tlPool = nullptr; }
+    } const noPool;
     for (double& m : phaseMs_) m = 0;
     auto clock0 = std::chrono::steady_clock::now();
     int phase = 0;
@@ -1267,7 +1392,6 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
     endPhase();
     // ---- phase C: histograms ------------------------------------------------------
     size_t const nj = I.nbDataJobs;
-    std::vector<uint32_t> hists(nj * 256);
     std::vector<HistTask> ht;
     for (size_t j = 0; j < nj; j++)
         if (!I.jobs[j].wide) ht.push_back(HistTask{ I.jobs[j].dsrc, uint32_t(I.jobs[j].n), uint32_t(j) });
@@ -1280,7 +1404,8 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
         cudaMemcpyAsync(dHt, ht.data(), ht.size() * sizeof(HistTask), cudaMemcpyHostToDevice, st);
         launchHist(dHt, uint32_t(ht.size()), dH, st);
         launches_++;
-        cudaMemcpyAsync(hists.data(), dH, nj * 1024, cudaMemcpyDeviceToHost, st);
+        if (!I.hists.reserve(nj * 1024)) { err = "allocation failed"; return 70; }
+        cudaMemcpyAsync(I.hists.p, dH, nj * 1024, cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device error in histograms"; return 1; }
     }
     // 16-bit chunks: value counts, first occurrences and maxima on the
@@ -1371,9 +1496,8 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
     };
     // 16-bit chunks (encode_entropy_binding.c:612-681); tokenize adds the
     // Huffman-graph job of the indices, whose histogram follows from the
-    // value counts
-    auto decide16 = [&](size_t ji) -> bool {
-        Job& J = I.jobs[ji];
+    // value counts (left in `idx`, to be appended to the job list)
+    auto decide16 = [&](Job& J, std::unique_ptr<Job>& idx) -> bool {
         unsigned const m = J.maxSym16;
         J.card16 = 0;
         for (uint32_t c : J.count16) J.card16 += c != 0;
@@ -1408,14 +1532,12 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
                 }
                 J.alphaBits = 1 + (m ? unsigned(31 - __builtin_clz(m)) : 0);
                 J.alphaBytes = (order.size() * J.alphaBits + 7) / 8;
-                Job W;
-                W.n = J.n;
-                W.mode = M_HUF;
-                std::memset(W.hist.count, 0, sizeof(W.hist.count));
-                for (size_t k = 0; k < order.size(); k++) W.hist.count[k] = J.count16[order[k]];
-                decide(W);
-                I.jobs.push_back(std::move(W));
-                I.jobs[ji].idxJob = int(I.jobs.size() - 1);
+                idx.reset(new Job);
+                idx->n = J.n;
+                idx->mode = M_HUF;
+                std::memset(idx->hist.count, 0, sizeof(idx->hist.count));
+                for (size_t k = 0; k < order.size(); k++) idx->hist.count[k] = J.count16[order[k]];
+                decide(*idx);
                 return true;
             }
             case ent::CC_HUF16: {
@@ -1434,13 +1556,26 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
             default: return true;
         }
     };
-    // 16-bit chunks first (they append nested jobs), then the others on
-    // host threads
-    for (size_t j = 0; j < nj; j++)
-        if (I.jobs[j].wide && !decide16(j)) { err = "16-bit Huffman table construction failed"; return 1; }
+    // All on host threads: 16-bit chunks one by one (a table of a large
+    // alphabet takes about 0.4 ms), the others by the chunk; then the 16-bit
+    // chunks' nested jobs, in the chunks' order.
+    {
+        std::vector<size_t> wide;
+        for (size_t j = 0; j < nj; j++)
+            if (I.jobs[j].wide) wide.push_back(j);
+        std::vector<std::unique_ptr<Job>> idx(wide.size());
+        std::vector<char> built(wide.size(), 0);
+        parallelFor(wide.size(), [&](size_t k) { built[k] = decide16(I.jobs[wide[k]], idx[k]); }, 1);
+        for (size_t k = 0; k < wide.size(); k++) {
+            if (!built[k]) { err = "16-bit Huffman table construction failed"; return 1; }
+            if (!idx[k]) continue;
+            I.jobs[wide[k]].idxJob = int(I.jobs.size());
+            I.jobs.push_back(std::move(*idx[k]));
+        }
+    }
     parallelFor(nj, [&](size_t j) {
         if (I.jobs[j].wide) return;
-        std::memcpy(I.jobs[j].hist.count, &hists[j * 256], 1024);
+        std::memcpy(I.jobs[j].hist.count, I.hists.p + j * 1024, 1024);
         decide(I.jobs[j]);
     });
     // Huffman tables on the device: every 8-bit Huffman chunk's code lengths
@@ -1486,33 +1621,28 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
         }
     }
     // nested weights jobs (FSE graph of Huffman weights): decided on the host
-    // histogram of the weights, encoded on the device with the data jobs
-    for (size_t j = 0; j < I.jobs.size(); j++) {
-        Job& J = I.jobs[j];
-        if (J.codec != ent::CC_HUF && J.codec != ent::CC_HUF16) continue;
-        // weights stream: numeric u8; under 10 bytes it is stored, else the
-        // FSE graph gets it after a numeric->serial conversion
-        if (J.weights.size() < kMinStream) continue;
-        Job W;
-        W.hsrc = J.weights;
-        W.n = J.weights.size();
-        W.mode = M_FSE;
-        std::memset(W.hist.count, 0, sizeof(W.hist.count));
-        for (uint8_t x : W.hsrc) W.hist.count[x]++;
-        J.weightsJob = int(I.jobs.size());
-        I.jobs.push_back(std::move(W));
-    }
+    // histogram of the weights, encoded on the device with the data jobs.
+    // A weights stream is numeric u8: under 10 bytes it is stored, else the
+    // FSE graph gets it after a numeric->serial conversion. The jobs are filled
+    // where they lie, on host threads.
     {
-        // the weights jobs created above, decided on host threads
-        size_t first = I.jobs.size();
-        for (size_t j = 0; j < I.jobs.size(); j++)
-            if (!I.jobs[j].hsrc.empty()) {
-                first = j;
-                break;
-            }
-        parallelFor(I.jobs.size() - first, [&](size_t k) {
+        std::vector<size_t> owners;
+        size_t const first = I.jobs.size();
+        for (size_t j = 0; j < first; j++) {
+            Job& J = I.jobs[j];
+            if ((J.codec != ent::CC_HUF && J.codec != ent::CC_HUF16) || J.weights.size() < kMinStream) continue;
+            J.weightsJob = int(first + owners.size());
+            owners.push_back(j);
+        }
+        I.jobs.resize(first + owners.size());
+        parallelFor(owners.size(), [&](size_t k) {
             Job& W = I.jobs[first + k];
-            if (!W.hsrc.empty()) decide(W);
+            W.hsrc = I.jobs[owners[k]].weights;
+            W.n = W.hsrc.size();
+            W.mode = M_FSE;
+            std::memset(W.hist.count, 0, sizeof(W.hist.count));
+            for (uint8_t x : W.hsrc) W.hist.count[x]++;
+            decide(W);
         });
     }
 
