@@ -119,7 +119,7 @@ typedef enum {
     OZL_DParam_hostRounds = 1004,
     /* batch API only: rounds of ozl_gpu_batch_run_host that decode at once
      * (round r starts after round r - depth has decoded; 0 = all at once;
-     * default 6) */
+     * default 8) */
     OZL_DParam_hostDepth = 1005,
 } ZL_DParam;
 

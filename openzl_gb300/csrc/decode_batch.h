@@ -132,7 +132,11 @@ struct DecodeBatch {
     // as soon as it is done, so both copy directions overlap the decode.
     unsigned planThreads = 0; // host threads of the plan build (0: the machine's, at most 8)
     int hostRounds = 16;     // OZL_DParam_hostRounds
-    int hostDepth = 6;       // OZL_DParam_hostDepth: rounds decoding at once (0 = all)
+    // OZL_DParam_hostDepth: rounds decoding at once (0 = all). A round's FSE
+    // streams take over a millisecond while its copies take 0.3, so the copy
+    // streams starve with few (1024 mixed frames: 4 at once 6.9 ms, 6 6.0, 8 and
+    // 9 5.0, 12 5.2, all 16 5.5, because early rounds then end late).
+    int hostDepth = 8;
     struct HostPipe {
         static constexpr int kRounds = 16;
         std::vector<Part> rounds;
