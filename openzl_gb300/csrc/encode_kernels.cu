@@ -698,53 +698,81 @@ __global__ void __launch_bounds__(32) kFseEnc(const FseEncTask* __restrict__ tas
 
 // FSE, long chunks (four states, kFseLongMin symbols or more), one CTA each.
 // The four states' chains are independent (only the order in which their
-// fields are appended couples them), and a chain forgets where it came from:
-// after a symbol that holds c of the table's cells only c states remain, so
-// two unlike states meet with a probability of about (symbols present) / (table
-// size) a step. So each chain is cut into up to 32 segments run at once, lane k
-// of a group of four running state k:
-//  1. A segment starts some steps early from an arbitrary state (six times the
-//     mean to a meeting; from the true state where that reaches the chain's
-//     start), records the state it enters its own steps with, and writes one
-//     16-bit entry per transition (the field in bits 0-11, its width in bits
-//     12-15) at the field's index in append order. Segments are no shorter
-//     than that run-up, so few symbols mean few segments, and two or three one.
+// fields are appended couples them), and a chain forgets where it came from,
+// so each is cut into up to 32 segments run at once, lane k of a group of four
+// running state k:
+//  1. A segment starts some steps early from an arbitrary state (from the true
+//     state where that reaches the chain's start) and records, for each batch
+//     of four steps, the state that enters it.
 //  2. A segment whose entry state is not the end state of the segment before
 //     it runs again from that state, until it meets its own earlier state at a
 //     quarter of the segment, or its end; this repeats until all agree.
-//  3. The entries are then the chunk's fields in order. Their widths, summed
-//     per segment, give each warp's first bit; a warp appends its quarter of
-//     the segments, 128 entries a round (a scan of the lanes' widths places
-//     them, they are ORed into a window of words in shared memory, complete
-//     words go out; only those that fit the capacity are written, as in the
-//     one-lane encoder). The words that two warps share meet in shared memory.
+//  3. All threads replay the batches from their recorded states and write one
+//     16-bit entry per transition (the field in bits 0-11, its width in bits
+//     12-15) at the field's index in append order.
+//  4. The entries are then the chunk's fields in order. Their widths give each
+//     warp's first bit; a warp appends its quarter of the batches, 128 entries
+//     a round (a scan of the lanes' widths places them, they are ORed into a
+//     window of words in shared memory, complete words go out; only those that
+//     fit the capacity are written, as in the one-lane encoder). The words that
+//     two warps share meet in shared memory.
+//
+// The run-up, and the shortest segment, is four times the mean number of steps
+// in which two unlike states meet. A symbol that holds c of the table's cells
+// maps a state's logarithm by a rotation and rounds it to c values, so two
+// states drift apart or together only by that rounding: the mean is about
+// 300 / (sum of 1 / c) plus (table size) / (symbols present) (simulated for 36
+// distributions of 2 to 200 symbols; within a factor of two of the former term
+// or their sum). With few symbols that is longer than the chunk and one
+// segment is left; a run-up too short for them cost twelve repeats of step 2.
 //
 // What bounds it: a transition's chain (two adds, two shifts and a shared
-// load, about 45 cycles); with one lane a chain it was 8,192 of them for a
-// chunk of 32 K symbols, at 290 cycles, in 24 lanes per SM. The segments give
-// an SM 16 chunks of 128 lanes. 32 K symbols: 1.19 ms and 0.11 ms of packing
-// before, 0.06 ms now (a plane of about 200 symbols); a stream of 100,000
-// symbols of which few values occur (one segment): about 2.5 and 1.1 ms.
+// load, 47 cycles; 57 in step 1, whose loads run three batches ahead and
+// lookups one). With one lane a chain it was 8,192 of them for a chunk of 32 K
+// symbols, at 290 cycles, in 24 lanes per SM. Writing the entries inside the
+// chain (as before step 3 was split off) took 115 cycles a transition. 32 K
+// symbols, a plane of about 200 symbols: 1.19 ms and 0.11 ms of packing with
+// one lane a chain, 0.062 ms with entries in the chain, 0.056 ms now; two
+// symbols (one segment) 1.3, 0.58 and 0.27 ms. Encoder batch of 64 messages,
+// this launch: 0.59 ms before the split, 0.39 now; of 2048 mixed frames, in
+// one part: 3.3 and 2.5 ms.
 constexpr uint32_t kFseSegs = 32, kFseLongThreads = 4 * kFseSegs, kFseLongWarps = kFseLongThreads / 32;
-constexpr uint32_t kFseSegBatches = 16; // fewest batches (of four steps) in a segment, if there are several
+constexpr uint32_t kFseSegBatches = 16; // fewest batches in a segment, if there are several
 
 __global__ void __launch_bounds__(kFseLongThreads) kFseEncLong(const FseEncTask* __restrict__ tasks,
                                                                uint32_t* __restrict__ sizes)
 {
     __shared__ uint2 tt[256];      // per symbol: deltaNbBits, deltaFindState
     __shared__ uint16_t st[2048];
-    __shared__ uint32_t endState[kFseSegs][4], segBits[kFseSegs];
+    __shared__ uint32_t endState[kFseSegs][4], warpBits[kFseLongWarps];
+    __shared__ uint16_t check[4][kFseLongThreads]; // per thread and quarter of its segment: the state after it
     __shared__ uint32_t win[kFseLongWarps][64];
     __shared__ uint32_t edgeWord[kFseLongWarps][2], edgeAt[kFseLongWarps][2]; // first and last word of each warp
+    __shared__ float warpInv[kFseLongWarps];
     FseEncTask const t = tasks[blockIdx.x];
-    uint32_t const tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, g = tid >> 2, k = tid & 3u;
+    uint32_t const tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, k = tid & 3u;
+    // the first segments are not those of the first warp in every CTA: with few
+    // segments the SM's CTAs would all run them on one of its schedulers
+    uint32_t const g = (tid / 4 + 8 * (blockIdx.x * 0x9E3779B1u >> 30)) & (kFseSegs - 1);
     const ent::FseCTable* const ct = reinterpret_cast<const ent::FseCTable*>(t.ctable);
     uint32_t const size = 1u << t.tableLog;
+    if (tid < kFseLongWarps) warpBits[tid] = 0;
     for (uint32_t y = tid; y < 256; y += kFseLongThreads) tt[y] = make_uint2(ct->deltaNbBits[y], uint32_t(ct->deltaFindState[y]));
     for (uint32_t u = tid; u < size; u += kFseLongThreads) st[u] = ct->state[u];
-    // symbols present (an absent one's pair asks for tableLog + 1 bits)
+    // symbols present (an absent one's pair asks for tableLog + 1 bits), and
+    // the sum over them of 1 / cells
     uint32_t const absent = ((t.tableLog + 1) << 16) - size;
+    float inv = 0;
+#pragma unroll
+    for (uint32_t h = 0; h < 2; h++) {
+        uint32_t const d = tt[tid + kFseLongThreads * h].x, mb = (d + 0xffffu) >> 16;
+        if (d != absent) inv += 1.f / float(((mb << 16) - d) >> mb);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) inv += __shfl_xor_sync(0xffffffffu, inv, o);
+    if (lane == 0) warpInv[wid] = inv;
     uint32_t const symbols = __syncthreads_count(tt[2 * tid].x != absent) + __syncthreads_count(tt[2 * tid + 1].x != absent);
+    inv = warpInv[0] + warpInv[1] + warpInv[2] + warpInv[3];
 
     // The c-th symbol from the end belongs to state (s0 + c) % 4; the last
     // four symbols start the states and emit nothing. Then the r = n % 4
@@ -754,128 +782,192 @@ __global__ void __launch_bounds__(kFseLongThreads) kFseEncLong(const FseEncTask*
     uint32_t const n = t.n, r = n & 3u, s0 = 4u - r, ip = n - 4 - r;
     uint32_t const pad = (4u - r) & 3u; // entries start here, so that steps start at multiples of four
     uint16_t* const fo = t.fields + pad;
-    uint32_t const steps = ip >> 2, batches = steps >> 2; // batches of four steps: 16 bytes of the source
-    uint32_t const warm = max(kFseSegBatches, (6 * size / symbols + 3) >> 2); // run-up, in batches
+    uint32_t const steps = ip >> 2;
+    // batches of four steps: 16 bytes of the source, the first ones after so
+    // many single steps (i1) that they start in a block's first word
+    uint32_t const i1 = uint32_t(reinterpret_cast<uintptr_t>(t.src + ip) & 15) >> 2, r1 = r + 4 * i1;
+    uint32_t const batches = (steps - i1) >> 2;
+    uintptr_t const top = reinterpret_cast<uintptr_t>(t.src) + ip - 4 * i1;
+    uint32_t const off = uint32_t(top & 3);
+    uint32_t const warm = max(kFseSegBatches, uint32_t(min(300.f / inv + float(size) / float(symbols), 1e6f)));
     uint32_t const segs = min(kFseSegs, max(1u, batches / warm));
-    uint32_t bits = 0, v;
+    uint32_t v;
     {
         uint32_t const y = t.src[n - 1 - ((k + 4u - (s0 & 3u)) & 3u)];
         uint32_t const nb = (tt[y].x + (1u << 15)) >> 16, x = (nb << 16) - tt[y].x;
         v = st[(x >> nb) + tt[y].y];
     }
-    // one transition with the symbol's pair; returns the entry
-    auto trans = [&](uint2 d) -> uint32_t {
-        uint32_t const nb = (v + d.x) >> 16, q = v >> nb;
-        uint32_t const e = (v - (q << nb)) + (nb << 12);
-        v = st[q + d.y];
-        bits += nb;
-        return e;
+    // one transition of state x with the symbol's pair; the entry of one
+    auto trans = [&](uint32_t x, uint2 d) -> uint32_t { return st[(x >> ((x + d.x) >> 16)) + d.y]; };
+    auto entryOf = [&](uint32_t x, uint2 d) -> uint32_t {
+        uint32_t const nb = (x + d.x) >> 16;
+        return (x & ((1u << nb) - 1u)) + (nb << 12);
     };
+    uint32_t head = 0, tail = 0; // bits of the fields that this thread writes here
     for (uint32_t c = 4; c < 4 + r; c++)
         if (((s0 + c) & 3u) == k) {
-            uint32_t const e = trans(tt[t.src[n - 1 - c]]);
-            if (g == 0) fo[c - 4] = uint16_t(e);
-        }
-    if (g) bits = 0;
-
-    // Batches [from, to) from state v. A batch's 16 source bytes come from
-    // the one or two aligned blocks that hold them, three batches ahead.
-    uintptr_t const top = reinterpret_cast<uintptr_t>(t.src) + ip;
-    uint32_t const off = uint32_t(top & 15);
-    auto run = [&](uint32_t from, uint32_t to, bool write) {
-        if (from >= to) return;
-        const uint4* a = reinterpret_cast<const uint4*>(top - off) - (from + 1); // lower block of batch `from`
-        uint4 const zero = make_uint4(0, 0, 0, 0);
-        uint4 up = off ? __ldg(a + 1) : zero, lo = __ldg(a);
-        uint4 n1 = from + 1 < to ? __ldg(a - 1) : zero, n2 = from + 2 < to ? __ldg(a - 2) : zero;
-        for (uint32_t b = from; b < to; b++) {
-            a--;
-            uint4 const n3 = b + 3 < to ? __ldg(a - 2) : zero;
-            uint4 const w = off ? shiftCombine(lo, up, off >> 2, (off & 3) * 8) : lo;
-            uint32_t const sel = 0x4443u - k;
-            uint2 const d0 = tt[__byte_perm(w.w, 0, sel)], d1 = tt[__byte_perm(w.z, 0, sel)],
-                        d2 = tt[__byte_perm(w.y, 0, sel)], d3 = tt[__byte_perm(w.x, 0, sel)];
-            uint32_t const e0 = trans(d0), e1 = trans(d1), e2 = trans(d2), e3 = trans(d3);
-            if (write) {
-                uint16_t* const f = fo + r + 16 * b + k;
-                f[0] = uint16_t(e0);
-                f[4] = uint16_t(e1);
-                f[8] = uint16_t(e2);
-                f[12] = uint16_t(e3);
+            uint2 const d = tt[t.src[n - 1 - c]];
+            if (g == 0) {
+                uint32_t const e = entryOf(v, d);
+                fo[c - 4] = uint16_t(e);
+                head += e >> 12;
             }
-            up = lo;
-            lo = n1;
+            v = trans(v, d);
+        }
+    for (uint32_t i = 0; i < i1; i++) {
+        uint2 const d = tt[t.src[ip - 4 * i - 1 - k]];
+        if (g == 0) {
+            uint32_t const e = entryOf(v, d);
+            fo[r + 4 * i + k] = uint16_t(e);
+            head += e >> 12;
+        }
+        v = trans(v, d);
+    }
+
+    // Batches [from, to) from state v. A batch's 16 source bytes are loaded
+    // three batches ahead and its pairs one ahead, in between the transitions,
+    // so that only the chain itself is left between two states. `record`: the
+    // states that enter a batch go to its first four entries.
+    uint4 const zero = make_uint4(0, 0, 0, 0);
+    // the 16 bytes from byte `off` (0 to 3) of block lo on, up the block above it
+    auto window = [&](const uint4& lo, uint32_t up) -> uint4 {
+        return make_uint4(__funnelshift_r(lo.x, lo.y, 8 * off), __funnelshift_r(lo.y, lo.z, 8 * off),
+                          __funnelshift_r(lo.z, lo.w, 8 * off), __funnelshift_r(lo.w, up, 8 * off));
+    };
+    auto fetch = [](const uint4* p) -> uint4 {
+        uint4 x;
+        asm volatile("ld.global.nc.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "l"(p));
+        return x;
+    };
+    auto run = [&](uint32_t from, uint32_t to, bool record) {
+        if (from >= to) return;
+        uint32_t left = to - from; // batches from the one that p is at on
+        const uint4* p = reinterpret_cast<const uint4*>(top - off) - (from + 1);
+        auto down = [&] { // past the last batch, its block is loaded again
+            if (left > 1) {
+                left--;
+                p--;
+            }
+        };
+        uint32_t const sel = 0x4443u - k;
+        uint4 cur = __ldg(p), w = window(cur, off ? __ldg(reinterpret_cast<const uint32_t*>(p + 1)) : 0u);
+        uint32_t up = cur.x;
+        uint2 d[4] = { tt[__byte_perm(w.w, 0, sel)], tt[__byte_perm(w.z, 0, sel)], tt[__byte_perm(w.y, 0, sel)],
+                       tt[__byte_perm(w.x, 0, sel)] };
+        down();
+        uint4 n1 = fetch(p);
+        down();
+        uint4 n2 = fetch(p);
+        down();
+        uint4 n3 = fetch(p);
+        down();
+        uint4 n4 = fetch(p);
+        uint16_t* f = fo + r1 + 16 * from + k;
+        for (uint32_t b = from; b < to; b++, f += 16) {
+            if (record) *f = uint16_t(v);
+            down();
+            uint4 const n5 = fetch(p);
+            w = window(n1, up);
+            v = trans(v, d[0]);
+            d[0] = tt[__byte_perm(w.w, 0, sel)];
+            v = trans(v, d[1]);
+            d[1] = tt[__byte_perm(w.z, 0, sel)];
+            v = trans(v, d[2]);
+            d[2] = tt[__byte_perm(w.y, 0, sel)];
+            v = trans(v, d[3]);
+            d[3] = tt[__byte_perm(w.x, 0, sel)];
+            up = n1.x;
             n1 = n2;
             n2 = n3;
+            n3 = n4;
+            n4 = n5;
         }
     };
     uint32_t const b0 = g < segs ? batches * g / segs : 0, b1 = g < segs ? batches * (g + 1) / segs : 0;
-    uint32_t const singles = bits;
     if (g && g < segs) {
         uint32_t const w0 = b0 > warm ? b0 - warm : 0;
         if (w0) v = size;
         run(w0, b0, false);
     }
-    uint32_t entry = v, check[4], quarterBits[4];
-    auto quarter = [&](uint32_t q) { return b0 + (b1 - b0) * q / 4; };
-#pragma unroll
-    for (uint32_t q = 0; q < 4; q++) {
-        bits = 0;
-        run(quarter(q), quarter(q + 1), true);
-        check[q] = v;
-        quarterBits[q] = bits;
-    }
-    if (g < segs) endState[g][k] = v;
-    __syncthreads();
-    for (;;) {
-        uint32_t const want = g && g < segs ? endState[g - 1][k] : entry;
-        bool const bad = want != entry;
+    uint32_t entry = 0; // the state that the recorded ones follow from
+    for (uint32_t want = v;;) {
+        bool const bad = g < segs && want != entry;
         if (!__syncthreads_or(bad)) break;
         if (bad) {
-            entry = v = want;
             bool met = false;
-#pragma unroll
-            for (uint32_t q = 0; q < 4; q++)
-                if (!met) {
-                    bits = 0;
-                    run(quarter(q), quarter(q + 1), true);
-                    quarterBits[q] = bits;
-                    met = v == check[q];
-                    check[q] = v;
-                }
-            endState[g][k] = check[3];
+            v = want;
+            for (uint32_t q = 0; q < 4 && !met; q++) {
+                run(b0 + (b1 - b0) * q / 4, b0 + (b1 - b0) * (q + 1) / 4, true);
+                met = entry && v == check[q][tid];
+                check[q][tid] = uint16_t(v);
+            }
+            entry = want;
+            endState[g][k] = check[3][tid];
         }
         __syncthreads();
+        if (g && g < segs) want = endState[g - 1][k];
     }
-    bits = singles + quarterBits[0] + quarterBits[1] + quarterBits[2] + quarterBits[3];
     if (g == segs - 1) { // the steps past the last batch, then the state's flush
-        v = check[3];
-        for (uint32_t i = 4 * batches; i < steps; i++) fo[r + 4 * i + k] = uint16_t(trans(tt[t.src[ip - 4 * i - 1 - k]]));
+        v = check[3][tid];
+        for (uint32_t i = i1 + 4 * batches; i < steps; i++) {
+            uint2 const d = tt[t.src[ip - 4 * i - 1 - k]];
+            uint32_t const e = entryOf(v, d);
+            fo[r + 4 * i + k] = uint16_t(e);
+            tail += e >> 12;
+            v = trans(v, d);
+        }
         fo[n - 4 + k] = uint16_t((v & (size - 1u)) | (t.tableLog << 12));
-        bits += t.tableLog;
+        tail += t.tableLog;
     }
-    bits += __shfl_xor_sync(0xffffffffu, bits, 1);
-    bits += __shfl_xor_sync(0xffffffffu, bits, 2);
-    if (k == 0) segBits[g] = g < segs ? bits : 0u;
+    if (head) atomicAdd(&warpBits[0], head);
+    if (tail) atomicAdd(&warpBits[kFseLongWarps - 1], tail);
+
+    // 2. the warp's quarter of the batches, one per lane: four steps from the
+    // recorded states, whose entries take their place
+    uint32_t const B0 = batches * wid / kFseLongWarps, B1 = batches * (wid + 1) / kFseLongWarps;
+    uint32_t bits = 0;
+    for (uint32_t b = B0 + lane; b < B1; b += 32) {
+        const uint4* const a = reinterpret_cast<const uint4*>(top - off) - (b + 1);
+        uint4 const lo = __ldg(a);
+        uint4 const w = window(lo, off ? __ldg(reinterpret_cast<const uint32_t*>(a + 1)) : 0u);
+        uint2* const f = reinterpret_cast<uint2*>(fo + r1 + 16 * b);
+        uint2 const in = *f;
+        uint32_t x[4] = { in.x & 0xffffu, in.x >> 16, in.y & 0xffffu, in.y >> 16 };
+#pragma unroll
+        for (uint32_t i = 0; i < 4; i++) {
+            uint32_t const y = i == 0 ? w.w : i == 1 ? w.z : i == 2 ? w.y : w.x;
+            uint32_t e[4];
+#pragma unroll
+            for (uint32_t m = 0; m < 4; m++) {
+                uint2 const d = tt[__byte_perm(y, 0, 0x4443u - m)];
+                e[m] = entryOf(x[m], d);
+                bits += e[m] >> 12;
+                if (i < 3) x[m] = trans(x[m], d);
+            }
+            f[i] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) bits += __shfl_xor_sync(0xffffffffu, bits, o);
+    if (lane == 0) atomicAdd(&warpBits[wid], bits);
     __syncthreads();
 
-    // 3. the warp's segments [sg0, sg1), entries [j0, j1) from `fields` on
+    // 3. the warp's entries [j0, j1) from `fields` on
     uint32_t const cap = n + n / 128 + 512;
     uint8_t* const out = t.out;
     uint32_t* const w = win[wid];
     w[lane] = 0;
     w[lane + 32] = 0;
     __syncwarp();
-    uint32_t const sg0 = segs * wid / kFseLongWarps, sg1 = segs * (wid + 1) / kFseLongWarps;
-    uint32_t before = lane < sg0 ? segBits[lane] : 0u, total = segBits[lane];
+    uint32_t before = 0, total = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        before += __shfl_xor_sync(0xffffffffu, before, o);
-        total += __shfl_xor_sync(0xffffffffu, total, o);
+    for (uint32_t q = 0; q < kFseLongWarps; q++) {
+        before += q < wid ? warpBits[q] : 0u;
+        total += warpBits[q];
     }
     uint32_t B = before, wb = before >> 5; // bits placed; first word not written yet
-    auto startOf = [&](uint32_t sg) { return sg == 0 ? 0u : sg >= segs ? pad + n : pad + r + 16 * (batches * sg / segs); };
-    uint32_t const j0 = startOf(sg0), j1 = startOf(sg1);
+    uint32_t const j0 = wid == 0 ? 0u : pad + r1 + 16 * B0,
+                   j1 = wid == kFseLongWarps - 1 ? pad + n : pad + r1 + 16 * B1;
     if (lane == 0) {
         edgeAt[wid][0] = edgeAt[wid][1] = before >> 5;
         edgeWord[wid][0] = edgeWord[wid][1] = 0;
@@ -926,7 +1018,7 @@ __global__ void __launch_bounds__(kFseLongThreads) kFseEncLong(const FseEncTask*
         __syncwarp();
         flushWords(B >> 5);
     }
-    if (lane == 0 && sg0 < sg1) {
+    if (lane == 0 && j0 < j1) {
         edgeAt[wid][1] = B >> 5;
         edgeWord[wid][1] = w[(B >> 5) & 63u]; // the warp's last word, not complete (its first one, if it has no other)
     }
