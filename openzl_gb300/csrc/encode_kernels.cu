@@ -413,57 +413,187 @@ __global__ void __launch_bounds__(256) kHist(const HistTask* __restrict__ tasks,
     hists[uint64_t(t.outIndex) * 256 + tid] = s;
 }
 
-// FSE coding tables on the device, one warp per chunk: lane 0 normalizes the
-// histogram and writes the normalized-count header (fse_norm.h, serial as in
-// the reference); the warp builds the encoding table (FSE_buildCTable_wksp,
-// fse_compress.c:69-207). Cells: the count -1 symbols take the top cells in
+// FSE coding tables on the device, a warp or a CTA of four per chunk: the
+// histogram is normalized (fse_norm.h; a lane has eight symbols, a sum and a
+// maximum over the warp give the remainder and the symbol that takes it; the
+// rare second method runs on one lane), the encoding table is built
+// (FSE_buildCTable_wksp, fse_compress.c:69-207) and the normalized-count
+// header written (fseHeader). Cells: the count -1 symbols take the top cells in
 // symbol order; occurrence k of the other symbols (in symbol order, each
 // repeated count times) goes to the k-th cell of the sequence 0, step,
 // 2 step, ... (mod size) below the top cells, 32 positions per round ranked
 // by a ballot. States: a symbol's state slots, from its cumulative count,
 // take its cells in increasing order, ranked within the round by
-// __match_any_sync. The result equals the serial construction.
+// __match_any_sync; with four warps, each takes a quarter of the rounds, from
+// the occurrences before it (counted) and from the symbols' cells in the
+// quarters before it (a count in shared memory first). The result equals the
+// serial construction.
+//
+// What bounds it: the chain of rounds, each a ballot or match and dependent
+// shared loads (64 and 64 at table log 11). With normalization and header on
+// one lane a chunk took 72 us, a quarter of a small encode call; on 32 lanes
+// 35 us, with four warps 15.7 us.
 constexpr int kFseTabWarps = 4;
+// Up to this many chunks take a CTA each, beyond it a warp each (chunks of 32 K
+// symbols; a warp and a CTA each): 4 chunks 37 and 18 us, 1,024 44 and 35, 2,048
+// 60 and 60, 4,096 91 and 106, where the repeated normalization costs more
+// than the shorter rounds give.
+constexpr uint32_t kFseTabWide = 2048;
 struct FseBuildSmem {
     uint32_t count[256];
     int16_t norm[256];
     uint16_t posCum[260];  // occurrences before each symbol (positive counts)
     uint16_t cumul[260];   // state slots before each symbol (count -1 takes one)
-    uint16_t next[256];
+    uint32_t header[132]; // at most 2 + 2 * 256 + 2 bytes
     uint8_t symbolAt[2048];
 };
 
+// The normalized-count header (fseWriteNCountTo) by a whole warp: lane j holds
+// the normalized counts v of symbols 8j .. 8j + 7 and `slots`, the table's
+// cells before them. What a symbol writes depends on those before it by that
+// sum alone: the field's width follows from the cells that remain, and the
+// first zero of a run writes the run. Returns the bytes.
+__device__ __forceinline__ uint32_t fseHeader(uint32_t* header, const int (&v)[8], uint32_t slots, uint32_t maxSym,
+                                              uint32_t tl)
+{
+    uint32_t const lane = threadIdx.x & 31;
+    for (uint32_t i = lane; i < 132; i += 32) header[i] = i == 0 ? tl - 5 : 0u;
+    // the first symbol from the lane's last on that is not zero
+    int next = 512;
+#pragma unroll
+    for (int k = 7; k >= 0; k--) next = v[k] ? int(8 * lane + k) : next;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { // the least of the lane's and those above
+        int const y = __shfl_down_sync(0xffffffffu, next, o);
+        if (lane + o < 32) next = min(next, y);
+    }
+    next = __shfl_down_sync(0xffffffffu, next, 1);
+    if (lane == 31) next = 512;
+    bool zero = __shfl_up_sync(0xffffffffu, v[7], 1) == 0 && lane > 0; // the symbol before is zero
+    // fields (bits 0-11), their widths (12-16), and for a run's first zero the zeros that follow, plus 1 (17 on)
+    uint32_t f[8], bits = 0;
+    int remaining = int((1u << tl) + 1 - slots);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        f[k] = 0;
+        uint32_t const sy = 8 * lane + k;
+        if (sy <= maxSym && remaining > 1 && (v[k] || !zero)) {
+            int const lg = ent::highbit32v(uint32_t(remaining)), threshold = 1 << lg, most = 2 * threshold - 1 - remaining;
+            int c = v[k] + 1;
+            if (c >= threshold) c += most;
+            uint32_t const w = uint32_t(lg) + 1 - uint32_t(c < most);
+            f[k] = uint32_t(c) | (w << 12);
+            bits += w;
+            if (!v[k]) {
+                int to = next;
+#pragma unroll
+                for (int j = 7; j > 0; j--)
+                    if (j > k && v[j]) to = int(8 * lane + j);
+                if (to == 512) to = int(sy) + 1; // (no symbol at all)
+                uint32_t const run = uint32_t(to) - sy - 1;
+                f[k] |= (run + 1) << 17;
+                bits += 16 * (run / 24) + 2 * (run % 24 / 3) + 2;
+            }
+        }
+        zero = v[k] == 0;
+        remaining -= v[k] < 0 ? 1 : v[k];
+    }
+    uint32_t at = bits;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        uint32_t const y = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= uint32_t(o)) at += y;
+    }
+    uint32_t const total = 4 + __shfl_sync(0xffffffffu, at, 31);
+    at += 4 - bits;
+    __syncwarp();
+    auto put = [&](uint32_t x, uint32_t n) {
+        atomicOr(&header[at >> 5], x << (at & 31));
+        if ((at & 31) + n > 32) atomicOr(&header[(at >> 5) + 1], x >> (32 - (at & 31)));
+        at += n;
+    };
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        uint32_t const w = (f[k] >> 12) & 31u;
+        if (w) put(f[k] & 0xfffu, w);
+        if (f[k] >> 17) {
+            uint32_t const run = (f[k] >> 17) - 1;
+            for (uint32_t i = 0; i < run / 24; i++) put(0xffffu, 16);
+            uint32_t const threes = run % 24 / 3;
+            put((1u << (2 * threes)) - 1 + ((run % 3) << (2 * threes)), 2 * threes + 2);
+        }
+    }
+    __syncwarp();
+    return (total + 7) >> 3;
+}
+
+template <int W>
 __global__ void __launch_bounds__(32 * kFseTabWarps) kFseTables(const FseTableTask* __restrict__ tasks, uint32_t nbTasks,
                                                                 uint32_t* __restrict__ sizes,
                                                                 uint32_t* __restrict__ errors)
 {
-    __shared__ FseBuildSmem sm[kFseTabWarps];
+    static_assert(W == 1 || W == kFseTabWarps, "warps of a chunk: one, or the CTA");
+    __shared__ FseBuildSmem sm[kFseTabWarps / W];
+    __shared__ uint32_t nextSlot[kFseTabWarps][256];
     uint32_t const wid = threadIdx.x >> 5, lane = threadIdx.x & 31, lt = (1u << lane) - 1;
-    uint32_t const ti = blockIdx.x * kFseTabWarps + wid;
+    uint32_t const part = W == 1 ? 0 : wid; // the chunk's warp, which takes its share of the table's cells
+    uint32_t const ti = W == 1 ? blockIdx.x * kFseTabWarps + wid : blockIdx.x;
     if (ti >= nbTasks) return; // the whole warp
+    auto sync = [] {
+        if (W == 1) __syncwarp();
+        else __syncthreads();
+    };
     FseTableTask const t = tasks[ti];
-    FseBuildSmem& S = sm[wid];
+    FseBuildSmem& S = sm[W == 1 ? wid : 0];
+    uint32_t* const next = nextSlot[wid];
     uint32_t const tl = t.tableLog, maxSym = t.maxSym;
     uint32_t const size = 1u << tl, mask = size - 1, step = (size >> 1) + (size >> 3) + 3;
     if (tl < 5 || tl > 11 || maxSym > 255) { // outside what the encoder emits
         if (lane == 0) atomicOr(errors, 1u);
         return;
     }
-    for (uint32_t k = lane; k < 256; k += 32) {
+    for (uint32_t k = part * 32 + lane; k < 256; k += 32 * W) {
         S.count[k] = t.hist[k];
         S.norm[k] = 0;
     }
-    __syncwarp();
-    if (lane == 0 && !ent::fseNormalizeCounts(S.norm, tl, S.count, t.n, maxSym)) atomicOr(errors, 1u);
-    __syncwarp();
-    // lane j: symbols 8j .. 8j + 7; scans of occurrences, state slots and
-    // top cells
+    sync();
+    // (every warp of the chunk computes the same, the first one writes)
+    // lane j: symbols 8j .. 8j + 7
     int v[8];
+    {
+        ent::FseNormScale const normOf(tl, t.n);
+        uint32_t const low = uint32_t(t.n >> tl);
+        int still = 0, largest = 0; // largest: value, then 255 - symbol
+        bool one = false;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            uint32_t const sy = 8 * lane + k, c = sy <= maxSym ? S.count[sy] : 0u;
+            one |= c && c == t.n;
+            v[k] = c == 0 ? 0 : c <= low ? -1 : int(normOf(c));
+            still -= v[k] < 0 ? 1 : v[k];
+            if (v[k] > 0) largest = max(largest, (v[k] << 8) | int(255 - sy));
+        }
+        still = __reduce_add_sync(0xffffffffu, still) + int(size);
+        largest = __reduce_max_sync(0xffffffffu, largest);
+        one = __any_sync(0xffffffffu, one);
+        if (one || -still >= (largest >> 9)) { // one symbol, or the second method
+            if (part == 0 && lane == 0 && !ent::fseNormalizeCounts(S.norm, tl, S.count, t.n, maxSym)) atomicOr(errors, 1u);
+            sync();
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = 8 * lane + k <= maxSym ? int(S.norm[8 * lane + k]) : 0;
+        } else {
+            uint32_t const ls = largest ? 255u - uint32_t(largest & 255) : 0u;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                if (8 * lane + k == ls) v[k] += still;
+                if (part == 0) S.norm[8 * lane + k] = int16_t(v[k]);
+            }
+        }
+    }
+    // scans of occurrences, state slots and top cells
     uint32_t sp = 0, sc = 0, sn = 0;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        uint32_t const sy = 8 * lane + k;
-        v[k] = sy <= maxSym ? int(S.norm[sy]) : 0;
         sp += v[k] > 0 ? uint32_t(v[k]) : 0u;
         sc += v[k] == -1 ? 1u : (v[k] > 0 ? uint32_t(v[k]) : 0u);
         sn += v[k] == -1 ? 1u : 0u;
@@ -482,29 +612,45 @@ __global__ void __launch_bounds__(32 * kFseTabWarps) kFseTables(const FseTableTa
     uint32_t const totalNeg = __shfl_sync(0xffffffffu, in, 31);
     uint32_t const high = size - 1 - totalNeg;
     uint32_t p0 = ip - sp, c0 = ic - sc, n0 = in - sn;
+    if (part == 0) {
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        uint32_t const sy = 8 * lane + k;
-        S.posCum[sy] = uint16_t(p0);
-        S.cumul[sy] = uint16_t(c0);
-        S.next[sy] = uint16_t(c0);
-        p0 += v[k] > 0 ? uint32_t(v[k]) : 0u;
-        c0 += v[k] == -1 ? 1u : (v[k] > 0 ? uint32_t(v[k]) : 0u);
-        if (v[k] == -1) {
-            S.symbolAt[size - 1 - n0] = uint8_t(sy);
-            n0++;
+        for (int k = 0; k < 8; k++) {
+            uint32_t const sy = 8 * lane + k;
+            S.posCum[sy] = uint16_t(p0);
+            S.cumul[sy] = uint16_t(c0);
+            if (W == 1) next[sy] = c0;
+            p0 += v[k] > 0 ? uint32_t(v[k]) : 0u;
+            c0 += v[k] == -1 ? 1u : (v[k] > 0 ? uint32_t(v[k]) : 0u);
+            if (v[k] == -1) {
+                S.symbolAt[size - 1 - n0] = uint8_t(sy);
+                n0++;
+            }
+        }
+        if (lane == 31) {
+            S.posCum[256] = uint16_t(p0);
+            S.cumul[256] = uint16_t(c0);
         }
     }
-    if (lane == 31) {
-        S.posCum[256] = uint16_t(p0);
-        S.cumul[256] = uint16_t(c0);
+    if (W > 1)
+        for (uint32_t sy = lane; sy < 256; sy += 32) next[sy] = 0;
+    sync();
+    // spread: the warp's rounds of 32 positions
+    uint32_t const rounds = size / 32, r0 = rounds * part / W, r1 = rounds * (part + 1) / W;
+    bool const any = totalNeg < size;
+    uint32_t occBase = 0; // occurrences before the round
+    if (any)
+        for (uint32_t r = 0; r < r0; r++)
+            occBase += totalNeg ? __popc(__ballot_sync(0xffffffffu, (((32 * r + lane) * step) & mask) <= high)) : 32u;
+    uint32_t sCur = 0;
+    if (r0) { // the symbol of the warp's first occurrence
+#pragma unroll
+        for (uint32_t h = 128; h; h >>= 1)
+            if (S.posCum[sCur + h] <= occBase) sCur += h;
     }
-    __syncwarp();
-    // spread
-    uint32_t sCur = 0, cumNext = S.posCum[1], occBase = 0;
-    for (uint32_t b0 = 0; b0 < size; b0 += 32) {
-        uint32_t const pos = ((b0 + lane) * step) & mask;
-        bool const valid = totalNeg < size && pos <= high;
+    uint32_t cumNext = S.posCum[sCur + 1];
+    for (uint32_t r = r0; r < r1; r++) {
+        uint32_t const pos = ((32 * r + lane) * step) & mask;
+        bool const valid = any && pos <= high;
         uint32_t const bal = __ballot_sync(0xffffffffu, valid);
         if (valid) {
             uint32_t const occ = occBase + __popc(bal & lt);
@@ -513,28 +659,45 @@ __global__ void __launch_bounds__(32 * kFseTabWarps) kFseTables(const FseTableTa
         }
         occBase += __popc(bal);
     }
-    __syncwarp();
-    // state table
+    sync();
+    // state table; with several warps, each symbol's cells of each warp first
+    if (W > 1) {
+        for (uint32_t r = r0; r < r1; r++) atomicAdd(&next[S.symbolAt[32 * r + lane]], 1u);
+        sync();
+        for (uint32_t sy = threadIdx.x; sy < 256; sy += 32 * W) {
+            uint32_t slot = S.cumul[sy];
+#pragma unroll
+            for (int w = 0; w < W; w++) {
+                uint32_t const c = nextSlot[w][sy];
+                nextSlot[w][sy] = slot;
+                slot += c;
+            }
+        }
+        sync();
+    }
     ent::FseCTable* const ct = reinterpret_cast<ent::FseCTable*>(t.ctable);
-    for (uint32_t b0 = 0; b0 < size; b0 += 32) {
-        uint32_t const u = b0 + lane;
+    for (uint32_t r = r0; r < r1; r++) {
+        uint32_t const u = 32 * r + lane;
         uint32_t const sy = S.symbolAt[u];
         uint32_t const m = __match_any_sync(0xffffffffu, sy);
-        uint32_t const base = S.next[sy];
+        uint32_t const base = next[sy];
         __syncwarp();
-        if (lane == 31u - __clz(m)) S.next[sy] = uint16_t(base + __popc(m));
+        if (lane == 31u - __clz(m)) next[sy] = base + __popc(m);
         ct->state[base + __popc(m & lt)] = uint16_t(size + u);
         __syncwarp();
     }
-    for (uint32_t sy = lane; sy < 256; sy += 32) {
+    for (uint32_t sy = part * 32 + lane; sy < 256; sy += 32 * W) {
         int const c = sy <= maxSym ? int(S.norm[sy]) : 0;
         ent::fseSymbolDeltas(c, tl, S.cumul[sy], ct->deltaNbBits[sy], ct->deltaFindState[sy]);
+        if (sy <= maxSym) t.norm[sy] = S.norm[sy];
     }
-    for (uint32_t sy = lane; sy <= maxSym; sy += 32) t.norm[sy] = S.norm[sy];
+    if (part != W - 1) return;
+    uint32_t const headerBytes = fseHeader(S.header, v, ic - sc, maxSym, tl);
+    for (uint32_t i = lane; i < headerBytes; i += 32) t.ncount[i] = uint8_t(S.header[i >> 2] >> (8 * (i & 3)));
     if (lane == 0) {
         ct->tableLog = uint16_t(tl);
         ct->maxSym = uint16_t(maxSym);
-        sizes[t.sizeSlot] = uint32_t(ent::fseWriteNCountTo(t.ncount, S.norm, maxSym, tl));
+        sizes[t.sizeSlot] = headerBytes;
     }
 }
 
@@ -1449,7 +1612,9 @@ void launchHist(const HistTask* t, uint32_t n, uint32_t* hists, cudaStream_t s)
 }
 void launchFseTables(const FseTableTask* t, uint32_t n, uint32_t* sizes, uint32_t* errors, cudaStream_t s)
 {
-    if (n) kFseTables<<<(n + kFseTabWarps - 1) / kFseTabWarps, 32 * kFseTabWarps, 0, s>>>(t, n, sizes, errors);
+    if (!n) return;
+    if (n <= kFseTabWide) kFseTables<kFseTabWarps><<<n, 32 * kFseTabWarps, 0, s>>>(t, n, sizes, errors);
+    else kFseTables<1><<<(n + kFseTabWarps - 1) / kFseTabWarps, 32 * kFseTabWarps, 0, s>>>(t, n, sizes, errors);
 }
 
 void launchHufTables(const HufTableTask* t, uint32_t n, cudaStream_t s)

@@ -92,13 +92,35 @@ OZL_HD inline bool fseNormalizeM2(int16_t* norm, unsigned tl, const uint32_t* co
     return true;
 }
 
+// the first method's value of one count above the low threshold
+struct FseNormScale {
+    uint64_t scale, step, vStep;
+    OZL_HD FseNormScale(unsigned tl, uint64_t total)
+        : scale(62 - tl), step((uint64_t(1) << 62) / uint32_t(total)), vStep(uint64_t(1) << (62 - tl - 20))
+    {
+    }
+    OZL_HD int16_t operator()(uint32_t count) const
+    {
+        int16_t p = int16_t((count * step) >> scale);
+        if (p < 8) {
+            uint32_t const restToBeat = p <= 0   ? 0
+                                        : p == 1 ? 473195
+                                        : p == 2 ? 504333
+                                        : p == 3 ? 520860
+                                        : p == 4 ? 550000
+                                        : p == 5 ? 700000
+                                        : p == 6 ? 750000
+                                                 : 830000;
+            p = int16_t(p + ((count * step) - (uint64_t(p) << scale) > vStep * restToBeat));
+        }
+        return p;
+    }
+};
+
 // normalized counts with low-probability symbols (-1)
 OZL_HD inline bool fseNormalizeCounts(int16_t* norm, unsigned tl, const uint32_t* count, uint64_t total, unsigned maxSym)
 {
-    const uint32_t restToBeat[8] = { 0, 473195, 504333, 520860, 550000, 700000, 750000, 830000 };
-    uint64_t const scale = 62 - tl;
-    uint64_t const step = (uint64_t(1) << 62) / uint32_t(total);
-    uint64_t const vStep = uint64_t(1) << (scale - 20);
+    FseNormScale const normOf(tl, total);
     int still = 1 << tl;
     unsigned largest = 0;
     int16_t largestP = 0;
@@ -111,8 +133,7 @@ OZL_HD inline bool fseNormalizeCounts(int16_t* norm, unsigned tl, const uint32_t
             still--;
             continue;
         }
-        int16_t p = int16_t((count[s] * step) >> scale);
-        if (p < 8) p = int16_t(p + ((count[s] * step) - (uint64_t(p) << scale) > vStep * restToBeat[p]));
+        int16_t const p = normOf(count[s]);
         if (p > largestP) { largestP = p; largest = s; }
         norm[s] = p;
         still -= p;

@@ -211,3 +211,30 @@ def test_huf_streams_that_do_not_fall_into_step(gpu_lib):
     many = [a[:5000 + k] for k in range(500) for a in arrays if a.size >= 9000][:1600]
     out, _ = _round_trip(many, 8, 0, [k % 16 for k in range(len(many))])
     assert all(g.tobytes() == a.tobytes() for a, g in zip(many, out))
+
+
+@pytest.mark.parametrize("copies", [1, 9])
+def test_fse_tables_and_headers(gpu_lib, copies):
+    """FSE tables of histograms at the edges of their build: few and many
+    symbols, gaps of 0 to 200 absent ones (runs in the header), counts below
+    the low threshold, distributions for the second normalization, every table
+    log; few chunks (a CTA each) and more than 2,048 (a warp each). Frames
+    equal the oracle's."""
+    rng = np.random.default_rng(5 + copies)
+    arrays = []
+    for n in (40, 100, 300, 900, 2000, 5000, 32768):
+        for symbols in (2, 3, 8, 33, 100, 256):
+            for gap in (0, 1, 2, 3, 23, 24, 25, 27, 48, 51, 200):
+                if symbols - 1 + gap > 255:
+                    continue
+                alphabet = np.concatenate([np.arange(symbols // 2), np.arange(symbols // 2, symbols) + gap]).astype(np.uint8)
+                p = [np.ones(symbols), 0.7 ** np.arange(symbols), 1.0 / (1 + np.arange(symbols)) ** 2][len(arrays) % 3]
+                arrays.append(rng.choice(alphabet, n, p=p / p.sum()))
+    arrays += [np.where(np.arange(n) % 40 == 0, rng.integers(0, 256, n), 9).astype(np.uint8) for n in (500, 4000, 20000)]
+    if copies == 1:
+        arrays = arrays[::5] + arrays[-3:]
+    assert (len(arrays) * copies > 2048) == (copies > 1)
+    frames = _frames(arrays * copies, 7, 0)
+    want = [oracle.compress(7, a, 0).tobytes() for a in arrays]
+    for k, f in enumerate(frames):
+        assert f == want[k % len(arrays)], (arrays[k % len(arrays)].size, k)
