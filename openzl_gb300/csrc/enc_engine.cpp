@@ -169,7 +169,7 @@ struct Job {
     bool wide = false;
     unsigned width = 1; // element width in bytes
     unsigned maxSym16 = 0, card16 = 0;
-    std::vector<uint32_t> count16, first16; // values 0..maxSym16
+    const uint32_t *count16 = nullptr, *first16 = nullptr; // values 0..maxSym16 (pinned staging, until the decisions are made)
     uint8_t const16[2] = { 0, 0 };
     // huffman_struct_v2
     int tl16 = 0;
@@ -247,10 +247,46 @@ struct PinnedBuf {
         if (p) cudaFreeHost(p);
         p = nullptr;
         cap = 0;
+        bytes = std::max(bytes, size_t(256) << 10); // one allocation for all phases of a small call
         if (cudaHostAlloc(reinterpret_cast<void**>(&p), bytes, cudaHostAllocDefault) != cudaSuccess) return false;
         cap = bytes;
         return true;
     }
+};
+
+// The arrays that one phase brings to the device, in one copy: the device
+// range that holds them (in increasing order; what lies between them is not
+// used), staged in pinned memory from byte `at` on. A copy each cost a small
+// call 3 to 4 us of gaps, with 17 of them.
+class Upload {
+  public:
+    void add(void* dev, const void* host, size_t bytes) // host null: zeros
+    {
+        if (bytes) items_.push_back(Item{ static_cast<uint8_t*>(dev), host, bytes });
+    }
+    // false: out of pinned memory, or the copy failed. The staging is free again
+    // once `s` has passed the copy.
+    bool go(PinnedBuf& stage, size_t at, cudaStream_t s)
+    {
+        if (items_.empty()) return true;
+        uint8_t* const lo = items_.front().dev;
+        size_t const bytes = size_t(items_.back().dev - lo) + items_.back().bytes;
+        if (at == 0 ? !stage.reserve(bytes) : at + bytes > stage.cap) return false;
+        for (const Item& x : items_) {
+            if (x.host) std::memcpy(stage.p + at + (x.dev - lo), x.host, x.bytes);
+            else std::memset(stage.p + at + (x.dev - lo), 0, x.bytes);
+        }
+        items_.clear();
+        return cudaMemcpyAsync(lo, stage.p + at, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess;
+    }
+
+  private:
+    struct Item {
+        uint8_t* dev;
+        const void* host;
+        size_t bytes;
+    };
+    std::vector<Item> items_;
 };
 
 // Helper threads of one encoder's host loops, kept for its lifetime: a loop
@@ -1020,14 +1056,15 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
         Bump b{ I.bufSmall.data(), 0 };
         auto* dMaxTasks = reinterpret_cast<EncNumTask*>(b.take(maxTasks.size() * sizeof(EncNumTask) + 1));
         auto* dMaxTiles = reinterpret_cast<TileRef*>(b.take(maxTiles.size() * sizeof(TileRef) + 1));
-        auto* dMax = reinterpret_cast<unsigned long long*>(b.take(nbMax * 8 + 8));
+        auto* dFirstCopies = reinterpret_cast<CopyTask*>(b.take(nf * sizeof(CopyTask) + 8));
+        auto* dFirstTiles = reinterpret_cast<TileRef*>(b.take(nf * sizeof(TileRef) + 8));
+        // maxima and first elements: zeroed and brought back together
+        auto* dMax = reinterpret_cast<unsigned long long*>(b.take((nbMax + nf) * 8 + 8));
+        auto* dFirst = reinterpret_cast<uint64_t*>(dMax + nbMax);
         auto* dHashOut = reinterpret_cast<uint64_t*>(b.take(nf * 8 + 8));
         auto* dHashTasks = reinterpret_cast<HashTask*>(b.take(nf * sizeof(HashTask) + 1));
         auto* dSums = reinterpret_cast<uint64_t*>(b.take(blocks * 64 + 64));
         auto* dBlocks = reinterpret_cast<TileRef*>(b.take(blocks * sizeof(TileRef) + 8));
-        auto* dFirst = reinterpret_cast<uint64_t*>(b.take(nf * 8 + 8));
-        auto* dFirstCopies = reinterpret_cast<CopyTask*>(b.take(nf * sizeof(CopyTask) + 8));
-        auto* dFirstTiles = reinterpret_cast<TileRef*>(b.take(nf * sizeof(TileRef) + 8));
         // first elements of the delta inputs, gathered into one array
         std::vector<CopyTask> firstCopies;
         std::vector<TileRef> firstTiles;
@@ -1036,10 +1073,15 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
                 firstTiles.push_back(TileRef{ uint32_t(firstCopies.size()), 0 });
                 firstCopies.push_back(CopyTask{ reinterpret_cast<uint8_t*>(dFirst + f), frames[f].dIn, frames[f].w, 0 });
             }
+        size_t const nbBack = nbMax + (firstCopies.empty() ? 0 : nf); // values that come back
+        Upload up;
+        up.add(dMaxTasks, maxTasks.data(), maxTasks.size() * sizeof(EncNumTask));
+        up.add(dMaxTiles, maxTiles.data(), maxTiles.size() * sizeof(TileRef));
+        up.add(dFirstCopies, firstCopies.data(), firstCopies.size() * sizeof(CopyTask));
+        up.add(dFirstTiles, firstTiles.data(), firstTiles.size() * sizeof(TileRef));
+        up.add(dMax, nullptr, nbBack * 8);
+        if (!up.go(I.stage, 0, st)) { err = "allocation failed"; return 70; }
         if (!firstCopies.empty()) {
-            cudaMemsetAsync(dFirst, 0, nf * 8, st);
-            cudaMemcpyAsync(dFirstCopies, firstCopies.data(), firstCopies.size() * sizeof(CopyTask), cudaMemcpyHostToDevice, st);
-            cudaMemcpyAsync(dFirstTiles, firstTiles.data(), firstTiles.size() * sizeof(TileRef), cudaMemcpyHostToDevice, st);
             launchCopy(dFirstCopies, dFirstTiles, uint32_t(firstTiles.size()), st);
             launches_++;
         }
@@ -1059,9 +1101,6 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
             }
         }
         if (!maxTasks.empty()) {
-            cudaMemcpyAsync(dMaxTasks, maxTasks.data(), maxTasks.size() * sizeof(EncNumTask), cudaMemcpyHostToDevice, st);
-            cudaMemcpyAsync(dMaxTiles, maxTiles.data(), maxTiles.size() * sizeof(TileRef), cudaMemcpyHostToDevice, st);
-            cudaMemsetAsync(dMax, 0, nbMax * 8, st);
             launchEncMax(dMaxTasks, dMaxTiles, uint32_t(maxTiles.size()), dMax, st);
             launches_++;
         }
@@ -1081,13 +1120,11 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
             I.hashPending = true;
             launches_ += contentBlocks.empty() ? 1 : 2;
         }
-        std::vector<unsigned long long> maxima(nbMax);
-        if (nbMax) cudaMemcpyAsync(maxima.data(), dMax, nbMax * 8, cudaMemcpyDeviceToHost, st);
-        std::vector<uint64_t> firsts(firstCopies.empty() ? 0 : nf);
-        if (!firstCopies.empty()) cudaMemcpyAsync(firsts.data(), dFirst, nf * 8, cudaMemcpyDeviceToHost, st);
+        std::vector<uint64_t> maxima(nbBack);
+        if (nbBack) cudaMemcpyAsync(maxima.data(), dMax, nbBack * 8, cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device error in phase A"; return 1; }
         for (size_t f = 0; f < nf; f++)
-            if (fronts[f].needFirst) fronts[f].first = firsts[f];
+            if (fronts[f].needFirst) fronts[f].first = maxima[nbMax + f];
         for (size_t f = 0; f < nf; f++)
             if (fronts[f].needMax) {
                 uint64_t const mx = maxima[fronts[f].maxSlot];
@@ -1120,9 +1157,7 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
                     t.n = n;
                     t.w = w;
                     t.capMask = cap - 1;
-                    t.state = reinterpret_cast<uint32_t*>(b.take(4 * cap));
                     t.key = reinterpret_cast<uint64_t*>(b.take(8 * cap));
-                    t.first = reinterpret_cast<uint32_t*>(b.take(4 * cap));
                     t.slotOf = reinterpret_cast<uint32_t*>(b.take(4 * n + 64));
                     t.rank = reinterpret_cast<uint32_t*>(b.take(4 * n + 64));
                     t.alphabet = b.take(uint64_t(w) * n + 64);
@@ -1131,6 +1166,8 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
                     for (uint32_t j = 0; j < (n + kEncTile - 1) / kEncTile; j++) tiles.push_back(TileRef{ uint32_t(k), j });
                     fronts[f].tokSlot = uint32_t(k);
                 }
+                for (TokTask& t : tt) t.state = reinterpret_cast<uint32_t*>(b.take(4 * (t.capMask + 1)));
+                for (TokTask& t : tt) t.first = reinterpret_cast<uint32_t*>(b.take(4 * (t.capMask + 1)));
                 dTasks = b.take(tt.size() * sizeof(TokTask));
                 dTiles = b.take(tiles.size() * sizeof(TileRef));
                 dSums = b.take(tiles.size() * 8 + 8);
@@ -1142,10 +1179,9 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
             if (!I.bufT.reserve(sizeT.used)) { err = "device allocation failed"; return 70; }
             Bump realT{ I.bufT.data(), 0 };
             layoutT(realT);
-            for (const TokTask& t : tt) {
-                cudaMemsetAsync(t.state, 0, 4 * (t.capMask + 1), st);
-                cudaMemsetAsync(t.first, 0xff, 4 * (t.capMask + 1), st);
-            }
+            // (tables of a power of two of at least 1,024 cells: no gaps between them)
+            cudaMemsetAsync(tt[0].state, 0, size_t(tt[0].first - tt[0].state) * 4, st);
+            cudaMemsetAsync(tt[0].first, 0xff, size_t(tt[0].first - tt[0].state) * 4, st);
             uint32_t* const counts = reinterpret_cast<uint32_t*>(dCnt);
             uint32_t* const errors = counts + tt.size();
             cudaMemsetAsync(dCnt, 0, tt.size() * 4 + 8, st);
@@ -1305,15 +1341,17 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
             auto* dTi = reinterpret_cast<TileRef*>(b.take(tiles.size() * sizeof(TileRef)));
             auto* dB = reinterpret_cast<Bf16Task*>(b.take(bt.size() * sizeof(Bf16Task)));
             auto* dBi = reinterpret_cast<TileRef*>(b.take(btiles.size() * sizeof(TileRef)));
+            Upload up;
+            up.add(dT, tasks.data(), tasks.size() * sizeof(EncNumTask));
+            up.add(dTi, tiles.data(), tiles.size() * sizeof(TileRef));
+            up.add(dB, bt.data(), bt.size() * sizeof(Bf16Task));
+            up.add(dBi, btiles.data(), btiles.size() * sizeof(TileRef));
+            if (!up.go(I.stage, 0, st)) { err = "allocation failed"; return 70; }
             if (!tasks.empty()) {
-                cudaMemcpyAsync(dT, tasks.data(), tasks.size() * sizeof(EncNumTask), cudaMemcpyHostToDevice, st);
-                cudaMemcpyAsync(dTi, tiles.data(), tiles.size() * sizeof(TileRef), cudaMemcpyHostToDevice, st);
                 launchEncNum(dT, dTi, uint32_t(tiles.size()), st);
                 launches_++;
             }
             if (!bt.empty()) {
-                cudaMemcpyAsync(dB, bt.data(), bt.size() * sizeof(Bf16Task), cudaMemcpyHostToDevice, st);
-                cudaMemcpyAsync(dBi, btiles.data(), btiles.size() * sizeof(TileRef), cudaMemcpyHostToDevice, st);
                 launchBf16(dB, dBi, uint32_t(btiles.size()), st);
                 launches_++;
             }
@@ -1442,13 +1480,21 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
             std::vector<uint32_t> mx(nw);
             cudaMemcpyAsync(mx.data(), dMax, nw * 4, cudaMemcpyDeviceToHost, st);
             if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device error in 16-bit histograms"; return 1; }
+            // into pinned memory (a copy into a job's own arrays waited for the
+            // device each); decide16 takes them from there
+            size_t values = 0;
+            for (size_t k = 0; k < nw; k++) values += size_t(mx[k]) + 1;
+            if (!I.stage.reserve(values * 8)) { err = "allocation failed"; return 70; }
+            uint32_t* at = reinterpret_cast<uint32_t*>(I.stage.p);
             for (size_t k = 0; k < nw; k++) {
                 Job& J = I.jobs[wide[k]];
+                size_t const m = size_t(mx[k]) + 1;
                 J.maxSym16 = mx[k];
-                J.count16.resize(size_t(mx[k]) + 1);
-                J.first16.resize(size_t(mx[k]) + 1);
-                cudaMemcpyAsync(J.count16.data(), dCount + k * 65536, J.count16.size() * 4, cudaMemcpyDeviceToHost, st);
-                cudaMemcpyAsync(J.first16.data(), dFirst + k * 65536, J.first16.size() * 4, cudaMemcpyDeviceToHost, st);
+                J.count16 = at;
+                J.first16 = at + m;
+                cudaMemcpyAsync(at, dCount + k * 65536, m * 4, cudaMemcpyDeviceToHost, st);
+                cudaMemcpyAsync(at + m, dFirst + k * 65536, m * 4, cudaMemcpyDeviceToHost, st);
+                at += 2 * m;
             }
             if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device error in 16-bit histograms"; return 1; }
         }
@@ -1500,8 +1546,8 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
     auto decide16 = [&](Job& J, std::unique_ptr<Job>& idx) -> bool {
         unsigned const m = J.maxSym16;
         J.card16 = 0;
-        for (uint32_t c : J.count16) J.card16 += c != 0;
-        J.codec = ent::chooseCodec16(J.count16.data(), m, J.n, J.card16);
+        for (unsigned v = 0; v <= m; v++) J.card16 += J.count16[v] != 0;
+        J.codec = ent::chooseCodec16(J.count16, m, J.n, J.card16);
         switch (J.codec) {
             case ent::CC_CONSTANT:
                 J.const16[0] = uint8_t(m);
@@ -1543,7 +1589,7 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
             case ent::CC_HUF16: {
                 J.code16.assign(size_t(m) + 1, 0);
                 J.nbBits16.assign(size_t(m) + 1, 0);
-                J.tl16 = ent::huf16Build(J.code16.data(), J.nbBits16.data(), J.count16.data(), m);
+                J.tl16 = ent::huf16Build(J.code16.data(), J.nbBits16.data(), J.count16, m);
                 if (J.tl16 < 0) return false;
                 J.weights.resize(size_t(m) + 1);
                 for (unsigned v = 0; v <= m; v++)
@@ -1810,7 +1856,7 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
         size_t const stageOff = (sz.used + taskBytes + tilesGuess * sizeof(TileRef) + (nbSizes + 16) * 4 + 1024 + 255)
                 & ~size_t(255);
         size_t const total = stageOff + szStage.used + 256;
-        if (!I.bufE.reserve(total) || !I.stage.reserve(szStage.used + 256)) { err = "allocation failed"; return 70; }
+        if (!I.bufE.reserve(total) || !I.stage.reserve(szStage.used + stageOff + 512)) { err = "allocation failed"; return 70; }
         Bump b{ I.bufE.data(), 0 };
         Bump stg{ I.bufE.data() + stageOff, 0 };
         layoutE(b, stg, true);
@@ -1829,44 +1875,42 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
         if (stg.used)
             cudaMemcpyAsync(stg.base, I.stage.p, stg.used, cudaMemcpyHostToDevice, st);
         auto* dFseTab = reinterpret_cast<FseTableTask*>(b.take(fseTabT.size() * sizeof(FseTableTask) + 1));
-        auto* dTabErr = reinterpret_cast<uint32_t*>(b.take(16));
         auto* dFse = reinterpret_cast<FseEncTask*>(b.take(fseT.size() * sizeof(FseEncTask) + 1));
         auto* dHuf = reinterpret_cast<HufEncTask*>(b.take(hufT.size() * sizeof(HufEncTask) + 1));
         auto* dPack = reinterpret_cast<PackTask*>(b.take(packT.size() * sizeof(PackTask) + 1));
         auto* dPackTiles = reinterpret_cast<TileRef*>(b.take(packTiles.size() * sizeof(TileRef) + 1));
         auto* dSizes = reinterpret_cast<uint32_t*>(b.take((nbSizes + 1) * 4));
+        uint32_t* const dTabErr = dSizes + nbSizes;
         auto* dTok16 = reinterpret_cast<Tok16Task*>(b.take(tok16T.size() * sizeof(Tok16Task) + 1));
         auto* dTok16Tiles = reinterpret_cast<TileRef*>(b.take(tok16Tiles.size() * sizeof(TileRef) + 1));
         auto* dWideNum = reinterpret_cast<EncNumTask*>(b.take(wideNumT.size() * sizeof(EncNumTask) + 1));
         auto* dWideNumTiles = reinterpret_cast<TileRef*>(b.take(wideNumTiles.size() * sizeof(TileRef) + 1));
         auto* dHuf16 = reinterpret_cast<Huf16EncTask*>(b.take(huf16T.size() * sizeof(Huf16EncTask) + 1));
-        // uploads: the tasks (the staged blobs went up above)
-        if (!fseTabT.empty())
-            cudaMemcpyAsync(dFseTab, fseTabT.data(), fseTabT.size() * sizeof(FseTableTask), cudaMemcpyHostToDevice, st);
-        cudaMemsetAsync(dTabErr, 0, 4, st);
-        if (!fseT.empty()) cudaMemcpyAsync(dFse, fseT.data(), fseT.size() * sizeof(FseEncTask), cudaMemcpyHostToDevice, st);
-        if (!hufT.empty()) cudaMemcpyAsync(dHuf, hufT.data(), hufT.size() * sizeof(HufEncTask), cudaMemcpyHostToDevice, st);
-        if (!packT.empty()) {
-            cudaMemcpyAsync(dPack, packT.data(), packT.size() * sizeof(PackTask), cudaMemcpyHostToDevice, st);
-            cudaMemcpyAsync(dPackTiles, packTiles.data(), packTiles.size() * sizeof(TileRef), cudaMemcpyHostToDevice, st);
-        }
-        if (nbSizes) cudaMemsetAsync(dSizes, 0, nbSizes * 4, st);
+        // the tasks, and zeros for the sizes and the tables' error count behind them
+        Upload up;
+        up.add(dFseTab, fseTabT.data(), fseTabT.size() * sizeof(FseTableTask));
+        up.add(dFse, fseT.data(), fseT.size() * sizeof(FseEncTask));
+        up.add(dHuf, hufT.data(), hufT.size() * sizeof(HufEncTask));
+        up.add(dPack, packT.data(), packT.size() * sizeof(PackTask));
+        up.add(dPackTiles, packTiles.data(), packTiles.size() * sizeof(TileRef));
+        up.add(dSizes, nullptr, (nbSizes + 1) * 4);
+        up.add(dTok16, tok16T.data(), tok16T.size() * sizeof(Tok16Task));
+        up.add(dTok16Tiles, tok16Tiles.data(), tok16Tiles.size() * sizeof(TileRef));
+        up.add(dWideNum, wideNumT.data(), wideNumT.size() * sizeof(EncNumTask));
+        up.add(dWideNumTiles, wideNumTiles.data(), wideNumTiles.size() * sizeof(TileRef));
+        up.add(dHuf16, huf16T.data(), huf16T.size() * sizeof(Huf16EncTask));
+        if (!up.go(I.stage, (stg.used + 255) & ~size_t(255), st)) { err = "allocation failed"; return 70; }
         // 16-bit chunks first: the tokenize indices feed their Huffman-graph
         // jobs below
         if (!tok16T.empty()) {
-            cudaMemcpyAsync(dTok16, tok16T.data(), tok16T.size() * sizeof(Tok16Task), cudaMemcpyHostToDevice, st);
-            cudaMemcpyAsync(dTok16Tiles, tok16Tiles.data(), tok16Tiles.size() * sizeof(TileRef), cudaMemcpyHostToDevice, st);
             launchTok16(dTok16, dTok16Tiles, uint32_t(tok16Tiles.size()), st);
             launches_++;
         }
         if (!wideNumT.empty()) {
-            cudaMemcpyAsync(dWideNum, wideNumT.data(), wideNumT.size() * sizeof(EncNumTask), cudaMemcpyHostToDevice, st);
-            cudaMemcpyAsync(dWideNumTiles, wideNumTiles.data(), wideNumTiles.size() * sizeof(TileRef), cudaMemcpyHostToDevice, st);
             launchEncNum(dWideNum, dWideNumTiles, uint32_t(wideNumTiles.size()), st);
             launches_++;
         }
         if (!huf16T.empty()) {
-            cudaMemcpyAsync(dHuf16, huf16T.data(), huf16T.size() * sizeof(Huf16EncTask), cudaMemcpyHostToDevice, st);
             launchHuf16Enc(dHuf16, uint32_t(huf16T.size()), dSizes, st);
             launches_++;
         }
@@ -1878,11 +1922,9 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
         launches_ += (fseT.empty() ? 0 : 1) + (nbLong ? 1 : 0) + (fseT.size() > nbLong ? 1 : 0)
                      + (hufT.empty() ? 0 : 1) + (packTiles.empty() ? 0 : 1);
         std::vector<uint32_t> hs(nbSizes + 1);
-        uint32_t tabErr = 0;
-        if (nbSizes) cudaMemcpyAsync(hs.data(), dSizes, nbSizes * 4, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(&tabErr, dTabErr, 4, cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(hs.data(), dSizes, (nbSizes + 1) * 4, cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device error in entropy encoding"; return 1; }
-        if (tabErr) { err = "FSE normalization failed"; return 1; }
+        if (hs[nbSizes]) { err = "FSE normalization failed"; return 1; }
         for (Job& J : I.jobs) {
             if (J.wide && J.codec == ent::CC_HUF16) {
                 // the reference writes the streams into 2n + 32 bytes; each
@@ -2081,11 +2123,11 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
         auto* dCopies = reinterpret_cast<CopyTask*>(b.take(copies.size() * sizeof(CopyTask) + 1));
         auto* dTiles = reinterpret_cast<TileRef*>(b.take(tiles.size() * sizeof(TileRef) + 1));
         auto* dHT = reinterpret_cast<HashTask*>(b.take(blockHash.size() * sizeof(HashTask) + 1));
-        auto* dHOut = reinterpret_cast<uint64_t*>(b.take(blockHash.size() * 8 + 8));
-        auto* dSums = reinterpret_cast<uint64_t*>(b.take(nbBlocks * 64 + 64));
         auto* dBB = reinterpret_cast<TileRef*>(b.take(nbBlocks * sizeof(TileRef) + 8));
         auto* dPut1 = reinterpret_cast<PutTask*>(b.take(nf * sizeof(PutTask) + 1));
         auto* dPut2 = reinterpret_cast<PutTask*>(b.take(2 * nf * sizeof(PutTask) + 1));
+        auto* dHOut = reinterpret_cast<uint64_t*>(b.take(blockHash.size() * 8 + 8));
+        auto* dSums = reinterpret_cast<uint64_t*>(b.take(nbBlocks * 64 + 64));
         if (checksums) {
             uint64_t bb = 0;
             for (size_t i = 0; i < blockHash.size(); i++) {
@@ -2101,16 +2143,17 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
                 put2.push_back(PutTask{ dOut[f] + O.total - 1 - 4, dHOut + 2 * f + 1, 4 });
             }
         }
-        cudaMemcpyAsync(dStage, stage.data(), stage.size(), cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(dCopies, copies.data(), copies.size() * sizeof(CopyTask), cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(dTiles, tiles.data(), tiles.size() * sizeof(TileRef), cudaMemcpyHostToDevice, st);
+        Upload up;
+        up.add(dStage, stage.data(), stage.size());
+        up.add(dCopies, copies.data(), copies.size() * sizeof(CopyTask));
+        up.add(dTiles, tiles.data(), tiles.size() * sizeof(TileRef));
         if (checksums) {
-            cudaMemcpyAsync(dHT, blockHash.data(), blockHash.size() * sizeof(HashTask), cudaMemcpyHostToDevice, st);
-            if (!blockBlocks.empty())
-                cudaMemcpyAsync(dBB, blockBlocks.data(), blockBlocks.size() * sizeof(TileRef), cudaMemcpyHostToDevice, st);
-            cudaMemcpyAsync(dPut1, put1.data(), put1.size() * sizeof(PutTask), cudaMemcpyHostToDevice, st);
-            cudaMemcpyAsync(dPut2, put2.data(), put2.size() * sizeof(PutTask), cudaMemcpyHostToDevice, st);
+            up.add(dHT, blockHash.data(), blockHash.size() * sizeof(HashTask));
+            up.add(dBB, blockBlocks.data(), blockBlocks.size() * sizeof(TileRef));
+            up.add(dPut1, put1.data(), put1.size() * sizeof(PutTask));
+            up.add(dPut2, put2.data(), put2.size() * sizeof(PutTask));
         }
+        if (!up.go(I.stage, 0, st)) { err = "allocation failed"; return 70; }
         launchCopy(dCopies, dTiles, uint32_t(tiles.size()), st);
         launches_++;
         if (checksums) {
