@@ -238,3 +238,44 @@ def test_fse_tables_and_headers(gpu_lib, copies):
     want = [oracle.compress(7, a, 0).tobytes() for a in arrays]
     for k, f in enumerate(frames):
         assert f == want[k % len(arrays)], (arrays[k % len(arrays)].size, k)
+
+
+def test_flatpack_pairs_and_tails(gpu_lib):
+    """Flatpacked fields of every width (pairs of fields up to 5 bits, one field
+    above), alphabets that fill their width and that do not, lengths around the
+    eight fields of a thread and the 64 KiB tile."""
+    rng = np.random.default_rng(14)
+    arrays = []
+    for size in (2, 3, 4, 5, 8, 9, 16, 17, 31, 32, 33, 64, 65, 100, 200, 255, 256):
+        values = rng.permutation(256)[:size].astype(np.uint8)
+        for n in [size + d for d in range(9)] + [1000, 65535, 65536, 65537, 65543, 131073]:
+            a = values[rng.integers(0, size, n)]
+            a[:size] = values
+            arrays.append(a)
+    out, frames = _round_trip(arrays, 14, 0, [k % 16 for k in range(len(arrays))])
+    for a, g, f in zip(arrays, out, frames):
+        assert g.tobytes() == a.tobytes() == oracle.decompress(f)[0].tobytes(), a.size
+
+
+@pytest.mark.parametrize("size", [5, 9, 17, 33])
+def test_flatpack_field_outside_the_alphabet(gpu_lib, size):
+    """A field that no symbol has is refused, in pairs and alone."""
+    import torch
+    import openzl_gb300 as oz
+
+    enc, n = oz.GpuEncoder(), 999
+    a = (np.arange(n) % size).astype(np.uint8)
+    src, cap = torch.from_numpy(a).cuda(), enc.bound(n)
+    dst = torch.zeros(cap, dtype=torch.uint8, device="cuda")
+    used = enc.compress_batch([src.data_ptr()], [n], [0], [14], [dst.data_ptr()], [cap], checksums=False)[0]
+    frame = dst[:used].cpu().numpy().copy()
+    packed = -(-(n * int(size - 1).bit_length() + 1) // 8)
+    at = used - packed + packed // 2  # inside the packed fields, wherever the frame ends
+    frame[at - 8:at] = 255
+    out = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    with pytest.raises(oz.ZLError):
+        dev = torch.from_numpy(frame).cuda()
+        batch = oz.GpuBatch()
+        batch.plan([frame], [dev.data_ptr()], [out.data_ptr()], [n])
+        batch.run(0, graph=False)
+        batch.check(0)
