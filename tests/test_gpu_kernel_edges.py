@@ -25,7 +25,7 @@ def test_xxh3_around_the_chain_batches(gpu_lib, offset):
         assert oz.xxh3_64_device(dev.data_ptr() + offset, n) == want, n
 
 
-def _round_trip(arrays, recipe, width, dst_offsets):
+def _round_trip(arrays, recipe, width, dst_offsets, room=0):
     """Compresses on the device, decodes to destinations at the given offsets
     from a 16-byte boundary and returns the decoded bytes and the frames."""
     import torch
@@ -33,7 +33,7 @@ def _round_trip(arrays, recipe, width, dst_offsets):
 
     enc, n = oz.GpuEncoder(), len(arrays)
     srcs = [torch.from_numpy(a.view(np.uint8).copy()).cuda() for a in arrays]
-    caps = [enc.bound(a.nbytes) for a in arrays]
+    caps = [enc.bound(a.nbytes) + room * a.nbytes + room for a in arrays]
     dsts = [torch.zeros(c, dtype=torch.uint8, device="cuda") for c in caps]
     sizes = enc.compress_batch([s.data_ptr() for s in srcs], [a.size for a in arrays], [width] * n, [recipe] * n,
                                [d.data_ptr() for d in dsts], caps, checksums=True)
@@ -279,3 +279,27 @@ def test_flatpack_field_outside_the_alphabet(gpu_lib, size):
         batch.plan([frame], [dev.data_ptr()], [out.data_ptr()], [n])
         batch.run(0, graph=False)
         batch.check(0)
+
+
+@pytest.mark.parametrize("width", [1, 2, 4, 8])
+def test_tokenize_and_float_vectors(gpu_lib, width):
+    """Dictionary gathers with 1-, 2- and 4-byte indices and joined bfloat16
+    around the 4,096-element tiles and the 16-byte vectors, destinations and
+    stored alphabets (fractions) at every alignment."""
+    rng = np.random.default_rng(width)
+    for recipe in (5, 6) if width == 2 else (5,):
+        arrays = []
+        for n in [1, 2, 7, 15, 16, 17, 33, 500, 4095, 4096, 4097, 8191, 8193, 12345] + [100000, 300001] * (recipe == 5):
+            for values in (3, 200, 300, 90000):
+                if recipe == 6:
+                    a = rng.normal(0, 0.02, n).astype(np.float32).view(np.uint32) >> 16
+                    if values == 200:
+                        a = rng.integers(0, 65536, n)
+                else:
+                    size = min(values, 2 ** (8 * width))
+                    a = rng.integers(0, 2 ** (8 * width), size, dtype=np.uint64)[rng.integers(0, size, n)]
+                arrays.append(a.astype("u%d" % width))
+        out, frames = _round_trip(arrays, recipe, width, [(k * 8) % 16 if k % 3 else k % 16 for k in range(len(arrays))],
+                                  room=8)
+        for a, g, f in zip(arrays, out, frames):
+            assert g.tobytes() == a.tobytes() == oracle.decompress(f)[0].tobytes(), a.size
