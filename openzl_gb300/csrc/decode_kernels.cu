@@ -792,7 +792,8 @@ __global__ void kTranspose(const TransposeTask* __restrict__ tasks, const TileRe
 // What bounds it: memory, once a thread's loads and stores are whole vectors:
 // 16 bytes of output and their indices at a time where both are aligned (a
 // tile's first element is; tokenGather), element by element elsewhere. 256 MiB
-// of 4-byte elements with 16-bit indices: 181 us element by element, 101 now.
+// of 4-byte elements with 16-bit indices: 181 us element by element, 101 now, 135
+// with an unaligned alphabet (193 when its elements were read by bytes).
 //
 // Elements [e0, e1) of W bytes from IW-byte indices, 16 bytes of output a
 // thread and round; returns the first element left over.
@@ -829,7 +830,13 @@ __device__ __forceinline__ uint64_t tokenGather(const TokenizeTask& t, uint64_t 
                 k = 0;
             }
             uint64_t x;
-            if (!ALIGNED) x = ldElem(t.alphabet + uint64_t(k) * W, W);
+            if (!ALIGNED && W >= 4) { // the aligned words that hold the element
+                uint32_t const off = uint32_t(reinterpret_cast<uintptr_t>(t.alphabet) & 3);
+                const uint32_t* const p = reinterpret_cast<const uint32_t*>(t.alphabet - off) + uint64_t(k) * (W / 4);
+                uint32_t const a = __ldg(p), b = W == 8 || off ? __ldg(p + 1) : 0u;
+                x = __funnelshift_r(a, b, 8 * off);
+                if (W == 8) x |= uint64_t(__funnelshift_r(b, off ? __ldg(p + 2) : 0u, 8 * off)) << 32;
+            } else if (!ALIGNED) x = ldElem(t.alphabet + uint64_t(k) * W, W);
             else if (W == 8) x = __ldg(reinterpret_cast<const unsigned long long*>(t.alphabet) + k);
             else if (W == 4) x = __ldg(reinterpret_cast<const uint32_t*>(t.alphabet) + k);
             else if (W == 2) x = __ldg(reinterpret_cast<const uint16_t*>(t.alphabet) + k);
