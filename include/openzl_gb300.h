@@ -426,8 +426,8 @@ ZL_Report ozl_gpu_batch_host_timeline(OZL_GpuBatch* b, const void* h_in, size_t 
                                       size_t outBytes, void* stream, float* rows, size_t capacity);
 /* Name of a codec family reported by ozl_gpu_batch_profile. */
 const char* ozl_gpu_kind_name(int kind);
-/* Autotuner: times the candidate launch shapes (chunks per CTA of the FSE
- * and Huffman launches) of the planned batch on `stream`, best of `reps`,
+/* Autotuner: times the candidate launch shapes (streams per CTA of the FSE,
+ * threads per chunk of the Huffman launches) of the planned batch on `stream`, best of `reps`,
  * after one full run; keeps the fastest per launch for the following runs
  * (the next graph run recaptures). Writes the chosen shape of launch i to
  * shapes[i] (0 = not tunable) for i < capacity. Returns the number of

@@ -432,7 +432,7 @@ class GpuBatch:
         return rep.value
 
     def autotune(self, stream=0, reps=2, capacity=256):
-        """Picks the launch shapes (chunks per CTA) by timing; returns the
+        """Picks the launch shapes (FSE and Huffman) by timing; returns the
         chosen shape per launch (0 = not tunable)."""
         shapes = (ctypes.c_uint32 * capacity)()
         rep = self._lib.ozl_gpu_batch_autotune(self._h, stream, reps, shapes, capacity)

@@ -21,7 +21,8 @@ cudaError_t prepareKernels();
 // lane per stream (kFse).
 constexpr uint32_t kTuneFseLanePerState = 0x100;
 
-// Launch shapes the autotuner may try for a launch (chunks per CTA); 0 if none.
+// Launch shapes the autotuner may try for a launch (FSE: streams per CTA; Huffman:
+// threads per chunk); 0 if none.
 uint32_t tuneCandidates(const Launch& l, uint32_t* out, uint32_t cap);
 
 // Enqueues launch `i` of `layout` alone (the building block of runLaunches).

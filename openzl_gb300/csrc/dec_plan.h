@@ -33,11 +33,11 @@ struct Launch {
     uint32_t nbTasks;
     size_t tileOff;   // byte offset of the TileRef array (tiled kinds)
     uint32_t nbTiles;
-    size_t statusOff; // scratch offset of look-back status (NUMPIPE with delta)
+    size_t statusOff; // scratch offset of tile sums and prefixes (NUMPIPE with delta)
     size_t statusBytes;
     bool needsScan;
     uint32_t param0;  // kind-specific launch shape (FSE: max table log; NUMPIPE: most tiles of a task)
-    uint32_t tune;    // chunks per CTA chosen by the autotuner (FSE, Huffman); 0 = default
+    uint32_t tune;    // shape chosen by the autotuner (FSE: streams per CTA; Huffman: threads per chunk); 0 = default
     uint64_t algoBytes; // bytes the launch must read plus write (roofline numerator)
 };
 
@@ -185,7 +185,7 @@ struct DeviceLayout {
     std::vector<uint8_t> pool;     // task descriptors, tile lists, pointer arrays
     std::vector<Launch> launches;
     uint64_t arenaBytes = 0;       // intermediate streams
-    uint64_t scratchBytes = 0;     // look-back status + hash block sums
+    uint64_t scratchBytes = 0;     // tile sums + hash block sums
     uint64_t paramBytes = 0;
 };
 
