@@ -701,21 +701,189 @@ __global__ void __launch_bounds__(32 * kFseTabWarps) kFseTables(const FseTableTa
     }
 }
 
-// Huffman code lengths and codes on the device, one warp per chunk: the
-// build (huf_tree.h, as the reference's HUF_buildCTable) is serial, so lane 0
-// runs it on the warp's shared nodes; the warp loads the histogram and writes
-// the weights.
+// Huffman code lengths and codes on the device, one warp per chunk
+// (huf_tree.h, as the reference's HUF_buildCTable, has the serial form of every
+// step). The buckets are counted and filled 32 symbols a round, ranked by
+// __match_any_sync; each lane sorts a bucket of large counts of its own (the
+// quicksort's order of equal counts is part of the result, so a bucket is one
+// lane's); lane 0 joins the tree, with the two candidates' counts in registers,
+// and repairs its height; the depths follow by doubling the way to the root; the
+// codes are counted off by length as the buckets were.
+//
+// What bounds it: the join (two dependent shared loads a node) and the largest
+// bucket's quicksort, each one lane's chain. With every step on lane 0 the
+// launch over the 529 chunks of a 256 MiB timestamp array's tables took 220 us,
+// now 54 (64 messages: 155 and 54).
 constexpr int kHufTabWarps = 4;
 struct HufBuildSmem {
     ent::HufNode nodes[ent::kHufNodes];
     uint32_t count[256];
-    uint8_t nbBits[256];
+    uint16_t base[192], curr[192]; // symbols in bucket r or above; the next place of bucket r - 1
+    uint16_t rank[16], code[16];   // codes of a length; the next one
+    uint16_t up[256];              // inner nodes: the way to the root
+    uint8_t depth[256], nbBits[256];
 };
+
+// hufBuildCodes by the whole warp
+__device__ __forceinline__ uint32_t hufBuildWarp(HufBuildSmem& S, uint16_t* value, uint32_t maxSym, uint32_t maxNbBits)
+{
+    uint32_t const lane = threadIdx.x & 31, lt = (1u << lane) - 1;
+    ent::HufNode* const node = S.nodes + 1;
+    for (int k = lane; k < ent::kHufNodes; k += 32) S.nodes[k] = ent::HufNode{ 0, 0, 0, 0 };
+    for (uint32_t k = lane; k < 192; k += 32) S.base[k] = 0;
+    for (uint32_t k = lane; k < 256; k += 32) S.nbBits[k] = 0;
+    if (lane < 16) S.rank[lane] = 0;
+    __syncwarp();
+    // buckets: counts, then the symbols of higher buckets before each
+    for (uint32_t n0 = 0; n0 <= maxSym; n0 += 32) {
+        uint32_t const n = n0 + lane, bk = n <= maxSym ? ent::hufBucketOf(S.count[n]) : 192u;
+        uint32_t const m = __match_any_sync(0xffffffffu, bk);
+        if (bk < 192 && lane == 31u - __clz(m)) S.base[bk] = uint16_t(S.base[bk] + __popc(m));
+        __syncwarp();
+    }
+    {
+        uint32_t v[6], sum = 0; // lane j: buckets 6j .. 6j + 5
+#pragma unroll
+        for (int k = 5; k >= 0; k--) {
+            sum += S.base[6 * lane + k];
+            v[k] = sum;
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            uint32_t const y = __shfl_down_sync(0xffffffffu, incl, o);
+            if (lane + o < 32) incl += y;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 6; k++) S.base[6 * lane + k] = S.curr[6 * lane + k] = uint16_t(v[k] + incl - sum);
+    }
+    __syncwarp();
+    for (uint32_t n0 = 0; n0 <= maxSym; n0 += 32) {
+        uint32_t const n = n0 + lane, bk = n <= maxSym ? ent::hufBucketOf(S.count[n]) : 191u;
+        uint32_t const m = __match_any_sync(0xffffffffu, bk);
+        uint32_t const at = bk < 191 ? S.curr[bk + 1] : 0u;
+        __syncwarp();
+        if (bk < 191) {
+            uint32_t const pos = at + __popc(m & lt);
+            node[pos].count = S.count[n];
+            node[pos].byte = uint8_t(n);
+            if (lane == 31u - __clz(m)) S.curr[bk + 1] = uint16_t(at + __popc(m));
+        }
+        __syncwarp();
+    }
+    if (ent::kHufDistinctCutoff + lane < 191) {
+        uint32_t const r = ent::kHufDistinctCutoff + lane;
+        int const size = int(S.curr[r]) - int(S.base[r]);
+        if (size > 1) ent::hufQuickSortDesc(node + S.base[r], 0, size - 1);
+    }
+    __syncwarp();
+    // leaves 0 .. nonNull by decreasing count, inner nodes 256 .. root
+    uint32_t present = 0;
+    for (uint32_t n = lane; n <= maxSym; n += 32) present += node[n].count != 0;
+    present = __reduce_add_sync(0xffffffffu, present);
+    int const start = 256, nonNull = int(present) - 1, root = start + nonNull - 1;
+    if (lane == 0) {
+        int lowS = nonNull, nodeNb = start, lowN = start;
+        S.nodes[0].count = 1u << 31; // node[-1]: above every count
+        uint32_t cN = node[lowS].count + node[lowS - 1].count;
+        node[nodeNb].count = cN;
+        node[lowS].parent = node[lowS - 1].parent = uint16_t(nodeNb);
+        nodeNb++;
+        lowS -= 2;
+        uint32_t cS = node[lowS].count;
+        // the lesser of the next leaf and the next inner node; one not made yet
+        // counts 2^30, as there
+        auto take = [&](uint32_t& c) -> int {
+            int n;
+            if (cS < cN) {
+                c = cS;
+                n = lowS--;
+                cS = node[lowS].count;
+            } else {
+                c = cN;
+                n = lowN++;
+                cN = lowN < nodeNb ? node[lowN].count : 1u << 30;
+            }
+            return n;
+        };
+        while (nodeNb <= root) {
+            uint32_t c1, c2;
+            int const n1 = take(c1), n2 = take(c2);
+            node[nodeNb].count = c1 + c2;
+            node[n1].parent = node[n2].parent = uint16_t(nodeNb);
+            if (lowN == nodeNb) cN = c1 + c2;
+            nodeNb++;
+        }
+    }
+    __syncwarp();
+    for (int n = start + int(lane); n <= root; n += 32) {
+        S.up[n - start] = uint16_t(n == root ? root : node[n].parent);
+        S.depth[n - start] = n == root ? 0 : 1;
+    }
+    __syncwarp();
+    for (bool far = true; far;) { // (every way doubles: at most eight rounds)
+        uint32_t to[8], d[8];
+        far = false;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            int const n = 32 * k + int(lane);
+            if (start + n > root) continue;
+            uint32_t const u = S.up[n] - start;
+            d[k] = S.depth[n] + S.depth[u];
+            to[k] = S.up[u];
+            far |= int(to[k]) != root;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            int const n = 32 * k + int(lane);
+            if (start + n > root) continue;
+            S.depth[n] = uint8_t(d[k]);
+            S.up[n] = uint16_t(to[k]);
+        }
+        far = __any_sync(0xffffffffu, far);
+        __syncwarp();
+    }
+    for (int n = lane; n <= nonNull; n += 32) node[n].nbBits = uint8_t(S.depth[node[n].parent - start] + 1);
+    __syncwarp();
+    uint32_t maxBits = 0;
+    if (lane == 0) maxBits = ent::hufLimitHeight(node, uint32_t(nonNull), maxNbBits);
+    maxBits = __shfl_sync(0xffffffffu, maxBits, 0);
+    __syncwarp();
+    // codes of each length, in symbol order
+    for (uint32_t n0 = 0; n0 <= maxSym; n0 += 32) {
+        uint32_t const n = n0 + lane, nb = n <= maxSym ? node[n].nbBits : 0u;
+        uint32_t const m = __match_any_sync(0xffffffffu, nb);
+        if (nb && lane == 31u - __clz(m)) S.rank[nb] = uint16_t(S.rank[nb] + __popc(m));
+        if (n <= maxSym) S.nbBits[node[n].byte] = uint8_t(nb);
+        __syncwarp();
+    }
+    if (lane == 0) {
+        uint16_t mn = 0;
+        for (int n = int(maxBits); n > 0; n--) {
+            S.code[n] = mn;
+            mn = uint16_t((mn + S.rank[n]) >> 1);
+        }
+        S.code[0] = 0;
+    }
+    __syncwarp();
+    for (uint32_t n0 = 0; n0 < 256; n0 += 32) {
+        uint32_t const n = n0 + lane, nb = S.nbBits[n];
+        uint32_t const m = __match_any_sync(0xffffffffu, n <= maxSym ? nb : 16u);
+        uint32_t const at = S.code[nb];
+        __syncwarp();
+        // (absent symbols count off length 0's, as there)
+        value[n] = n <= maxSym ? uint16_t(at + __popc(m & lt)) : uint16_t(0);
+        if (n <= maxSym && lane == 31u - __clz(m)) S.code[nb] = uint16_t(at + __popc(m));
+        __syncwarp();
+    }
+    return maxBits;
+}
 
 __global__ void __launch_bounds__(32 * kHufTabWarps) kHufTables(const HufTableTask* __restrict__ tasks, uint32_t nbTasks)
 {
     __shared__ HufBuildSmem sm[kHufTabWarps];
-    __shared__ uint32_t sTl[kHufTabWarps];
     uint32_t const wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t const ti = blockIdx.x * kHufTabWarps + wid;
     if (ti >= nbTasks) return; // the whole warp
@@ -724,13 +892,8 @@ __global__ void __launch_bounds__(32 * kHufTabWarps) kHufTables(const HufTableTa
     for (uint32_t k = lane; k < 256; k += 32) S.count[k] = t.hist[k];
     __syncwarp();
     ent::HufCTable* const ct = reinterpret_cast<ent::HufCTable*>(t.ctable);
-    if (lane == 0) {
-        unsigned const tl = ent::hufBuildCodes(S.nodes, ct->value, S.nbBits, S.count, t.maxSym, t.maxNbBits);
-        ct->tableLog = tl;
-        sTl[wid] = tl;
-    }
-    __syncwarp();
-    uint32_t const tl = sTl[wid];
+    uint32_t const tl = hufBuildWarp(S, ct->value, t.maxSym, t.maxNbBits);
+    if (lane == 0) ct->tableLog = tl;
     for (uint32_t k = lane; k < 256; k += 32) {
         uint32_t const nb = S.nbBits[k];
         ct->nbBits[k] = uint8_t(nb);

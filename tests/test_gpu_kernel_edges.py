@@ -303,3 +303,36 @@ def test_tokenize_and_float_vectors(gpu_lib, width):
                                   room=8)
         for a, g, f in zip(arrays, out, frames):
             assert g.tobytes() == a.tobytes() == oracle.decompress(f)[0].tobytes(), a.size
+
+
+def test_huffman_tables_sorts_and_heights(gpu_lib):
+    """Code lengths of histograms at the edges of their build: counts around the
+    bucket cutoff (164, 165), large buckets of equal and of unlike counts,
+    counts that make the tree deeper than its limit, 2 to 256 symbols with gaps.
+    Frames equal the oracle's."""
+    rng = np.random.default_rng(11)
+    arrays = []
+    fib = [1, 1]
+    while len(fib) < 22:
+        fib.append(fib[-1] + fib[-2])
+
+    def add(counts):
+        counts = np.asarray(counts)
+        symbols = np.sort(rng.permutation(256)[:counts.size])
+        a = np.repeat(symbols, counts).astype(np.uint8)
+        arrays.append(rng.permutation(a))
+
+    for base in (1, 100, 163, 164, 165, 200, 255, 256, 511):
+        for symbols in (2, 3, 17, 60, 63):
+            add(np.full(symbols, base))
+            add(base + rng.integers(0, 3, symbols))
+    for symbols in (10, 64, 128, 200, 256):
+        add(rng.integers(128, 256, symbols) if symbols <= 128 else rng.integers(60, 128, symbols))
+        add(1 + rng.geometric(0.02, symbols))
+        add(np.maximum(1, (20000 * 0.9 ** np.arange(symbols) * 0.1).astype(int)))
+    for depth in (12, 16, 20):
+        add(fib[:depth])
+        add(fib[:depth] + [1] * 40)
+    arrays = [a for a in arrays if a.size <= 32768]
+    for a, f in zip(arrays, _frames(arrays, 8, 0)):
+        assert f == oracle.compress(8, a, 0).tobytes(), (a.size, np.bincount(a).tolist())
