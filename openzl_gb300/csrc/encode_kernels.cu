@@ -415,8 +415,8 @@ __global__ void __launch_bounds__(256) kHist(const HistTask* __restrict__ tasks,
 
 // FSE coding tables on the device, a warp or a CTA of four per chunk: the
 // histogram is normalized (fse_norm.h; a lane has eight symbols, a sum and a
-// maximum over the warp give the remainder and the symbol that takes it; the
-// rare second method runs on one lane), the encoding table is built
+// maximum over the warp give the remainder and the symbol that takes it, sums
+// and a scan the second method), the encoding table is built
 // (FSE_buildCTable_wksp, fse_compress.c:69-207) and the normalized-count
 // header written (fseHeader). Cells: the count -1 symbols take the top cells in
 // symbol order; occurrence k of the other symbols (in symbol order, each
@@ -432,7 +432,8 @@ __global__ void __launch_bounds__(256) kHist(const HistTask* __restrict__ tasks,
 // What bounds it: the chain of rounds, each a ballot or match and dependent
 // shared loads (64 and 64 at table log 11). With normalization and header on
 // one lane a chunk took 72 us, a quarter of a small encode call; on 32 lanes
-// 35 us, with four warps 15.7 us.
+// 35 us, with four warps 15.7 us. 64 messages, some for the second method: 84 us
+// while that ran on one lane, now 24.
 constexpr int kFseTabWarps = 4;
 // Up to this many chunks take a CTA each, beyond it a warp each (chunks of 32 K
 // symbols; a warp and a CTA each): 4 chunks 37 and 18 us, 1,024 44 and 35, 2,048
@@ -527,6 +528,99 @@ __device__ __forceinline__ uint32_t fseHeader(uint32_t* header, const int (&v)[8
     return (total + 7) >> 3;
 }
 
+// fseNormalizeM2 by a whole warp: lane j holds the counts c of symbols
+// 8j .. 8j + 7 (0 from maxSym + 1 on) and gets their normalized counts v. False
+// where the distribution cannot be normalized.
+__device__ __forceinline__ bool fseNormalizeSecond(int (&v)[8], const uint32_t (&c)[8], uint32_t tl, uint32_t total,
+                                                   uint32_t maxSym)
+{
+    uint32_t const lane = threadIdx.x & 31, size = 1u << tl, low = total >> tl;
+    uint32_t lowOne = uint32_t((uint64_t(total) * 3) >> (tl + 1));
+    uint32_t some = 0, used = 0; // symbols with their final count, and their occurrences
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        v[k] = c[k] == 0 ? 0 : c[k] <= low ? -1 : c[k] <= lowOne ? 1 : -2; // -2: not known yet
+        if (v[k] == 1 || v[k] == -1) {
+            some++;
+            used += c[k];
+        }
+    }
+    uint32_t distributed = __reduce_add_sync(0xffffffffu, some);
+    total -= __reduce_add_sync(0xffffffffu, used);
+    uint32_t left = size - distributed;
+    if (left == 0) return true;
+    if (total / left > lowOne) {
+        lowOne = uint32_t((uint64_t(total) * 3) / (left * 2));
+        some = used = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (v[k] == -2 && c[k] <= lowOne) {
+                v[k] = 1;
+                some++;
+                used += c[k];
+            }
+        distributed += __reduce_add_sync(0xffffffffu, some);
+        total -= __reduce_add_sync(0xffffffffu, used);
+        left = size - distributed;
+    }
+    if (distributed == maxSym + 1) { // the rest goes to the first of the most frequent symbols
+        uint32_t most = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) most = max(most, c[k]);
+        most = __reduce_max_sync(0xffffffffu, most);
+        uint32_t first = 256;
+#pragma unroll
+        for (int k = 7; k >= 0; k--) first = c[k] == most ? 8 * lane + k : first;
+        first = __reduce_min_sync(0xffffffffu, first);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (8 * lane + k == first) v[k] = int16_t(v[k] + int16_t(left));
+        return true;
+    }
+    if (total == 0) { // one each in turn to the symbols with a positive count
+        uint32_t mine = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) mine += v[k] > 0;
+        uint32_t at = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            uint32_t const y = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= uint32_t(o)) at += y;
+        }
+        uint32_t const all = __shfl_sync(0xffffffffu, at, 31);
+        if (all == 0) return false;
+        at -= mine;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (v[k] > 0) v[k] += int(left / all + (at++ < left % all ? 1u : 0u));
+        return true;
+    }
+    uint32_t const stepLog = 62 - tl;
+    uint64_t const mid = (uint64_t(1) << (stepLog - 1)) - 1, step = ((uint64_t(1) << stepLog) * left + mid) / total;
+    uint64_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        if (v[k] == -2) sum += c[k] * step;
+    uint64_t at = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        uint64_t const y = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= uint32_t(o)) at += y;
+    }
+    at += mid - sum;
+    bool bad = false;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        if (v[k] == -2) {
+            uint64_t const end = at + c[k] * step;
+            uint32_t const w = uint32_t(end >> stepLog) - uint32_t(at >> stepLog);
+            bad |= w < 1;
+            v[k] = int16_t(w);
+            at = end;
+        }
+    return !__any_sync(0xffffffffu, bad);
+}
+
 template <int W>
 __global__ void __launch_bounds__(32 * kFseTabWarps) kFseTables(const FseTableTask* __restrict__ tasks, uint32_t nbTasks,
                                                                 uint32_t* __restrict__ sizes,
@@ -554,7 +648,6 @@ __global__ void __launch_bounds__(32 * kFseTabWarps) kFseTables(const FseTableTa
     }
     for (uint32_t k = part * 32 + lane; k < 256; k += 32 * W) {
         S.count[k] = t.hist[k];
-        S.norm[k] = 0;
     }
     sync();
     // (every warp of the chunk computes the same, the first one writes)
@@ -563,31 +656,35 @@ __global__ void __launch_bounds__(32 * kFseTabWarps) kFseTables(const FseTableTa
     {
         ent::FseNormScale const normOf(tl, t.n);
         uint32_t const low = uint32_t(t.n >> tl);
+        uint32_t c[8];
         int still = 0, largest = 0; // largest: value, then 255 - symbol
         bool one = false;
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            uint32_t const sy = 8 * lane + k, c = sy <= maxSym ? S.count[sy] : 0u;
-            one |= c && c == t.n;
-            v[k] = c == 0 ? 0 : c <= low ? -1 : int(normOf(c));
+            uint32_t const sy = 8 * lane + k;
+            c[k] = sy <= maxSym ? S.count[sy] : 0u;
+            one |= c[k] && c[k] == t.n;
+            v[k] = c[k] == 0 ? 0 : c[k] <= low ? -1 : int(normOf(c[k]));
             still -= v[k] < 0 ? 1 : v[k];
             if (v[k] > 0) largest = max(largest, (v[k] << 8) | int(255 - sy));
         }
         still = __reduce_add_sync(0xffffffffu, still) + int(size);
         largest = __reduce_max_sync(0xffffffffu, largest);
         one = __any_sync(0xffffffffu, one);
-        if (one || -still >= (largest >> 9)) { // one symbol, or the second method
-            if (part == 0 && lane == 0 && !ent::fseNormalizeCounts(S.norm, tl, S.count, t.n, maxSym)) atomicOr(errors, 1u);
-            sync();
+        uint32_t const ls = largest ? 255u - uint32_t(largest & 255) : 0u;
+        if (one) { // (one symbol: no counts, as there)
 #pragma unroll
-            for (int k = 0; k < 8; k++) v[k] = 8 * lane + k <= maxSym ? int(S.norm[8 * lane + k]) : 0;
+            for (int k = 0; k < 8; k++) v[k] = 0;
+        } else if (-still >= (largest >> 9)) {
+            if (!fseNormalizeSecond(v, c, tl, uint32_t(t.n), maxSym) && part == 0 && lane == 0) atomicOr(errors, 1u);
         } else {
-            uint32_t const ls = largest ? 255u - uint32_t(largest & 255) : 0u;
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
+            for (int k = 0; k < 8; k++)
                 if (8 * lane + k == ls) v[k] += still;
-                if (part == 0) S.norm[8 * lane + k] = int16_t(v[k]);
-            }
+        }
+        if (part == 0) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) S.norm[8 * lane + k] = int16_t(v[k]);
         }
     }
     // scans of occurrences, state slots and top cells

@@ -336,3 +336,25 @@ def test_huffman_tables_sorts_and_heights(gpu_lib):
     arrays = [a for a in arrays if a.size <= 32768]
     for a, f in zip(arrays, _frames(arrays, 8, 0)):
         assert f == oracle.compress(8, a, 0).tobytes(), (a.size, np.bincount(a).tolist())
+
+
+def test_fse_second_normalization(gpu_lib):
+    """Histograms that the first normalization leaves unbalanced: many symbols
+    just above the low threshold beside few frequent ones, all symbols rare,
+    one that takes nearly all. Frames equal the oracle's."""
+    rng = np.random.default_rng(12)
+    arrays = []
+    for n in (300, 1000, 4000, 9999, 32768):
+        for rare in (1, 2, 3, 5, 9, 17, 40):
+            for symbols in (20, 100, 250):
+                if (rare + 1) * symbols > n * 9 // 10:
+                    continue
+                for heads in (1, 2, 5):
+                    counts = rng.integers(max(1, rare - 1), rare + 2, symbols)
+                    rest = n - counts.sum()
+                    head = np.diff(np.concatenate([[0], np.sort(rng.integers(0, rest, heads - 1)), [rest]]))
+                    a = np.repeat(np.arange(symbols + heads), np.concatenate([head, counts]))
+                    arrays.append(rng.permutation(a % 256).astype(np.uint8))
+        arrays.append((np.arange(n) % 256).astype(np.uint8))
+    for a, f in zip(arrays, _frames(arrays, 7, 0)):
+        assert f == oracle.compress(7, a, 0).tobytes(), (a.size, np.bincount(a).tolist())
