@@ -781,8 +781,10 @@ __global__ void __launch_bounds__(1024) kNumPrefix(const NumPipeTask* __restrict
     }
 }
 
-// pass 3: the output
-__global__ void __launch_bounds__(kNPThreads) kNumPipe(const NumPipeTask* __restrict__ tasks,
+// pass 3: the output. Six CTAs an SM (40 registers, no spills) where the
+// compiler's own choice of 48 gave five: 256 MiB of 8-byte elements 141 us with
+// five, 133 with six, 130 with seven, which spill and gain nothing in a batch.
+__global__ void __launch_bounds__(kNPThreads, 6) kNumPipe(const NumPipeTask* __restrict__ tasks,
                                                        const TileRef* __restrict__ tiles,
                                                        const uint64_t* __restrict__ prefix)
 {
