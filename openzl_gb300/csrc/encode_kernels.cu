@@ -14,6 +14,7 @@
 #include "enc_exec.h"
 #include "enc_tables.h"
 #include "fse_norm.h"
+#include "fse_segments.h"
 #include "huf_tree.h"
 #include "enc_tasks.h"
 #include "stream_ring.cuh"
@@ -1182,19 +1183,15 @@ __global__ void __launch_bounds__(kFseLongThreads) kFseEncLong(const FseEncTask*
     if (tid < kFseLongWarps) warpBits[tid] = 0;
     for (uint32_t y = tid; y < 256; y += kFseLongThreads) tt[y] = make_uint2(ct->deltaNbBits[y], uint32_t(ct->deltaFindState[y]));
     for (uint32_t u = tid; u < size; u += kFseLongThreads) st[u] = ct->state[u];
-    // symbols present (an absent one's pair asks for tableLog + 1 bits), and
-    // the sum over them of 1 / cells
-    uint32_t const absent = ((t.tableLog + 1) << 16) - size;
+    // symbols present and the sum over them of 1 / cells, each thread from the
+    // pairs that it put in place itself (the others' are not there yet)
     float inv = 0;
-#pragma unroll
-    for (uint32_t h = 0; h < 2; h++) {
-        uint32_t const d = tt[tid + kFseLongThreads * h].x, mb = (d + 0xffffu) >> 16;
-        if (d != absent) inv += 1.f / float(((mb << 16) - d) >> mb);
-    }
+    uint32_t const own = fseSymbolShare(tid, kFseLongThreads, t.tableLog, [&](uint32_t y) { return tt[y].x; }, inv);
+    static_assert(2 * kFseLongThreads == 256, "two symbols a thread");
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) inv += __shfl_xor_sync(0xffffffffu, inv, o);
     if (lane == 0) warpInv[wid] = inv;
-    uint32_t const symbols = __syncthreads_count(tt[2 * tid].x != absent) + __syncthreads_count(tt[2 * tid + 1].x != absent);
+    uint32_t const symbols = __syncthreads_count(own > 0) + __syncthreads_count(own > 1);
     inv = warpInv[0] + warpInv[1] + warpInv[2] + warpInv[3];
 
     // The c-th symbol from the end belongs to state (s0 + c) % 4; the last
@@ -1212,7 +1209,7 @@ __global__ void __launch_bounds__(kFseLongThreads) kFseEncLong(const FseEncTask*
     uint32_t const batches = (steps - i1) >> 2;
     uintptr_t const top = reinterpret_cast<uintptr_t>(t.src) + ip - 4 * i1;
     uint32_t const off = uint32_t(top & 3);
-    uint32_t const warm = max(kFseSegBatches, uint32_t(min(300.f / inv + float(size) / float(symbols), 1e6f)));
+    uint32_t const warm = fseRunUp(kFseSegBatches, size, symbols, inv);
     uint32_t const segs = min(kFseSegs, max(1u, batches / warm));
     uint32_t v;
     {
