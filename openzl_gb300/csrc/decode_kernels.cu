@@ -14,6 +14,7 @@
 
 #include "dec_tasks.h"
 #include "dec_exec.h"
+#include "huf_split.h"
 #include "stream_ring.cuh"
 
 namespace ozl {
@@ -1687,18 +1688,27 @@ __global__ void __launch_bounds__(32) kFse4(const FseTask* __restrict__ tasks, u
 // ---------------------------------------------------------------------------
 // One Huffman stream on several lanes. A decoder that starts inside a code
 // soon meets the true code boundaries, so the stream's bits are cut into S
-// runs of equal length:
+// runs of about equal length, which start at a multiple of the code lengths'
+// common divisor from the top, as every code does (splitStart):
 //  1. each lane counts the codes of its run from its first bit, noting its
 //     place kMeetBits into the run and where the last code ends;
 //  2. a lane whose run truly starts elsewhere (where the run before it ended)
 //     counts again from there, up to the noted place if it comes by it, else
-//     to the run's end; this repeats until all agree (codes whose lengths have
-//     a common factor may need all runs one after another, as one lane would);
+//     to the run's end; this repeats until all agree (at worst every run after
+//     the one before it, as one lane would);
 //  3. the counts give each run's place in the output (the caller decodes again
 //     from the true starts, and stores).
 // Decoding twice costs less than what it buys: a chunk's streams were four
 // chains on four lanes of its table's shared memory, which bounds how many
 // tables an SM holds.
+// From a first bit at any place, lanes whose codes all had lengths of a common
+// divisor never met the boundaries. 256 MiB of bytes, 64 MiB, 256 KiB: codes of
+// 2 and 4 bits 1.50, 0.48 and 0.385 ms so, 0.57, 0.17 and 0.063 from multiples
+// of 2 (0.94, 0.43 and 0.39 with one lane a stream); 4 and 8 bits 1.70, 0.51,
+// 0.386 and 0.69, 0.19, 0.053. Codes nearly all of one length (31 of 5 bits,
+// few of 9 to 11) meet late and stay the worst: 1.26, 0.50 and 0.21 ms (one
+// lane 1.09, 0.51 and 0.42). More places to meet at (two to four, up to 4,096
+// bits into the run) gained nothing.
 constexpr int32_t kMeetBits = 256;
 template <int T>
 struct SplitShared {
@@ -1710,16 +1720,13 @@ struct SplitRun {
     uint32_t count, before; // its codes, the codes of the stream's runs before it
     bool ok;                // the stream holds n codes and ends at its first bit
 };
-// Runs of at least 1,024 bits, at most `lanes`.
-__device__ __forceinline__ uint32_t splitRuns(int32_t bits, uint32_t lanes)
-{
-    return max(1u, min(lanes, uint32_t(max(bits, 0)) >> 10));
-}
 // Every thread of the CTA calls it. j < S: the thread's run of its stream
 // (br, opened), whose first run is thread tid - j's; run(bound): decodes codes
-// until the position is at or below `bound` and returns their number.
+// until the position is at or below `bound` and returns their number; step:
+// lengthStep of the codes.
 template <int T, class Stream, class Run>
-__device__ __forceinline__ SplitRun splitStream(Stream& br, Run run, uint32_t j, uint32_t S, uint32_t n, SplitShared<T>& sh)
+__device__ __forceinline__ SplitRun splitStream(Stream& br, Run run, uint32_t j, uint32_t S, uint32_t step, uint32_t n,
+                                                SplitShared<T>& sh)
 {
     uint32_t const tid = threadIdx.x;
     bool const mine = j < S;
@@ -1727,8 +1734,8 @@ __device__ __forceinline__ SplitRun splitStream(Stream& br, Run run, uint32_t j,
     uint32_t upToMeet = 0, count = 0;
     if (mine) {
         int32_t const top = br.pos, bits = top - br.end;
-        p = top - int32_t(int64_t(bits) * j / S);
-        e = top - int32_t(int64_t(bits) * (j + 1) / S);
+        p = top - splitStart(bits, j, S, step);
+        e = top - splitStart(bits, j + 1, S, step);
         c = max(p - kMeetBits, e);
         br.seek(p);
         upToMeet = run(c);
@@ -1796,6 +1803,7 @@ constexpr uint32_t kHufTableLog = 12;
 using HufStream = PosStream<8, 4>;
 struct HufScratch {
     uint32_t count[16], next[16];
+    uint32_t step; // lengthStep of the codes
     uint8_t sorted[256];
 };
 // table, rings (or a tableLog-12 table and the rings of four lanes), scratch
@@ -1841,6 +1849,9 @@ __device__ __forceinline__ uint32_t hufRankWarp(const uint8_t* weights, uint32_t
     if (sum == 0 || (sum & (sum - 1)) || nz < 2) return 0;
     uint32_t const tl = 31 - __clz(sum);
     if (tl > kHufTableLog) return 0;
+    // bit w of the ballot is length tl + 1 - w
+    uint32_t const used = __ballot_sync(0xffffffffu, c != 0);
+    if (lane == 0) S.step = lengthStep(__brev(used) >> (30 - tl));
     for (uint32_t b = 0; b < nbW; b += 32) {
         uint32_t const w = b + lane < nbW ? weights[b + lane] : 0u;
         uint32_t const m = __match_any_sync(0xffffffffu, w);
@@ -1962,7 +1973,7 @@ __global__ void __launch_bounds__(T) kHuf(const HufTask* __restrict__ tasks, uin
         for (; br.pos > bound; m++) one();
         return m;
     };
-    SplitRun const r = splitStream<T>(br, run, j, runs, n, split);
+    SplitRun const r = splitStream<T>(br, run, j, runs, S.step, n, split);
     if (j >= runs) {
         if (!opened && j == 0) reportError(status, DERR_CORRUPTION);
         return;
@@ -2024,7 +2035,7 @@ using Huf16Stream = PosStream<8, 4>;
 __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restrict__ tasks, uint32_t* __restrict__ status)
 {
     __shared__ uint32_t sCount[kHuf16Warps][32], sStart[32], sBase[32];
-    __shared__ uint32_t sTl, sOk;
+    __shared__ uint32_t sTl, sOk, sStep;
     __shared__ uint32_t sTab[1u << kHuf16Log];
     __shared__ __align__(16) uint8_t sRing[kHuf16Threads * Huf16Stream::kBytes];
     __shared__ SplitShared<kHuf16Threads> split;
@@ -2063,8 +2074,9 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
         while (tl < 63 && (2ull << tl) <= sum) tl++;
         bool const ok = sOk && nz >= 2 && sum != 0 && !(sum & (sum - 1)) && tl <= 20;
         if (ok) {
-            uint32_t pos = 0, base = 0;
+            uint32_t pos = 0, base = 0, lengths = 0;
             for (uint32_t w = 1; w <= tl; w++) {
+                lengths |= uint32_t(total[w] != 0) << (tl + 1 - w);
                 sStart[w] = pos;
                 sBase[w] = base;
                 pos += total[w] << (w - 1);
@@ -2075,6 +2087,7 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
                 }
             }
             sStart[tl + 1] = 1u << tl;
+            sStep = lengthStep(lengths);
         }
         sTl = tl;
         sOk = ok ? 1u : 0u;
@@ -2184,7 +2197,7 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
         }
         return m;
     };
-    SplitRun r = splitStream<int(kHuf16Threads)>(br, run, j, runs, n, split);
+    SplitRun r = splitStream<int(kHuf16Threads)>(br, run, j, runs, sStep, n, split);
     if (j >= runs) {
         if (!opened && j == 0 && sIdx < t.nbStreams) reportError(status, DERR_CORRUPTION);
         return;

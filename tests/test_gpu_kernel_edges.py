@@ -358,3 +358,35 @@ def test_fse_second_normalization(gpu_lib):
         arrays.append((np.arange(n) % 256).astype(np.uint8))
     for a, f in zip(arrays, _frames(arrays, 7, 0)):
         assert f == oracle.compress(7, a, 0).tobytes(), (a.size, np.bincount(a).tolist())
+
+
+def _symbols_of_lengths(rng, n, lengths):
+    """n symbols whose Huffman code has about these lengths."""
+    p = np.array([2.0 ** -l for l in lengths])
+    assert p.sum() == 1.0
+    return rng.choice(len(lengths), n, p=p)
+
+
+@pytest.mark.parametrize("lengths", [[2] * 3 + [4] * 4, [3] * 7 + [6] * 8, [4] * 15 + [8] * 16, [5] * 31 + [10] * 32,
+                                     [6] * 63 + [7] * 2, [7] * 127 + [8] * 2, [1] + [3] * 4],
+                         ids=lambda x: "-".join("%dx%d" % (x.count(l), l) for l in sorted(set(x))))
+def test_huf_code_lengths_with_a_common_divisor(gpu_lib, lengths):
+    """Streams whose codes all have lengths of a common divisor, and of two
+    neighbouring lengths: bytes and 16-bit symbols, one stream and four, few
+    chunks (four warps each) and more than the SMs hold at once (one warp)."""
+    rng = np.random.default_rng(len(lengths))
+    arrays = [_symbols_of_lengths(rng, n, lengths).astype(np.uint8) for n in
+              [100, 254, 1000, 1023, 1024, 4099, 30000, 32768, 99999]]
+    out, frames = _round_trip(arrays, 8, 0, [k % 16 for k in range(len(arrays))])
+    for a, g, f in zip(arrays, out, frames):
+        assert g.tobytes() == a.tobytes() == oracle.decompress(f)[0].tobytes(), a.size
+    many = [_symbols_of_lengths(rng, 20000 + 37 * k, lengths).astype(np.uint8) for k in range(13)] * 110
+    out, _ = _round_trip(many, 8, 0, [k % 16 for k in range(len(many))])
+    assert all(g.tobytes() == a.tobytes() for a, g in zip(many, out))
+    # 16-bit symbols: spread over more values, so that they stay 16-bit symbols
+    wide = [(300 + 256 * _symbols_of_lengths(rng, n, lengths)).astype(np.uint16) for n in [300, 1000, 30000, 32768, 99999]]
+    wide += [(7 * _symbols_of_lengths(rng, n, [l + 3 for l in lengths for _ in range(8)])).astype(np.uint16)
+             for n in [5000, 30000, 99999]]
+    out, frames = _round_trip(wide, 8, 2, [2 * (k % 8) for k in range(len(wide))])
+    for a, g, f in zip(wide, out, frames):
+        assert g.tobytes() == a.tobytes() == oracle.decompress(f)[0].tobytes(), a.size
