@@ -12,6 +12,7 @@
 
 #include "../../include/openzl_gb300.h"
 #include "dec_exec.h"
+#include "dec_parts.h"
 #include "dec_plan.h"
 #include "device_scope.h"
 
@@ -84,12 +85,12 @@ cudaError_t prepareOnce();
 // latency-bound entropy decoding. All parts share the plan's arena and
 // parameter block; each has its own descriptor pool and scratch.
 struct DecodeBatch {
-    static constexpr int kMaxParts = 18; // long checksums, the critical part, 8 runs of each of two kinds
+    static constexpr int kMaxParts = 20; // long checksums of three kinds, the critical part, 8 runs of each of two kinds
     struct Part {
         DeviceLayout layout;
         DevBuf pool, scratch;
         std::vector<char> mask;   // frames of this part
-        bool longChecksum = false; // frames whose content checksum is the batch's longest chain
+        bool longChecksum = false; // frames that decode ahead of the others (LongChecksums)
         int rank = 0;              // stream priority, 0 the highest
     };
     bool checkContent = true;
@@ -103,13 +104,7 @@ struct DecodeBatch {
     // kind; smaller ones into the Huffman frames and the others.
     static constexpr uint64_t kSplitBytes = 512ull << 20;
     static constexpr uint32_t kCriticalDefault = 16000;
-    // A frame of at least this many decoded bytes, and of at least half the
-    // batch's largest, is decoded ahead of the others: its content checksum is
-    // a serial chain (12.4 ns a KiB: 0.4 ms for 32 MiB, 3.3 ms for 256 MiB) that
-    // starts when the frame is decoded and then leaves the SMs to the rest. A
-    // 256 MiB column beside 0.43 GB of weight matrices: 5.23 ms before, when
-    // the column waited behind the matrices' entropy decoding, 4.33 now.
-    static constexpr uint64_t kLongChecksum = 32ull << 20;
+    bool longAlone = false;       // the parts of long checksums decode before the others begin
     int schedule = 0;             // OZL_DParam_schedule: priority policy of the branches
     DecodePlan plan;
     std::vector<Part> parts;
@@ -238,12 +233,21 @@ struct DecodeBatch {
                 if (!nd.dead && nd.id == 49 && nd.frame >= 0 && nd.out >= 0
                     && plan.streams[size_t(nd.out)].n >= critical)
                     kindOf[size_t(nd.frame)] = 2;
-        size_t largest = 0;
-        for (size_t x : sizes) largest = std::max(largest, x);
-        if (checkContent && largest >= kLongChecksum)
+        // frames of long checksums keep their kinds, in parts of their own
+        std::vector<char> checked(n, 0), fse(n, 0);
+        if (checkContent && splitParts) {
             for (const PlanHash& h : plan.hashes)
-                if (h.err == DERR_CONTENT_CK && sizes[size_t(h.frame)] >= std::max<size_t>(kLongChecksum, largest / 2))
-                    kindOf[size_t(h.frame)] = 3;
+                if (h.err == DERR_CONTENT_CK) checked[size_t(h.frame)] = 1;
+            for (const PlanNode& nd : plan.nodes)
+                if (!nd.dead && nd.id == 49 && nd.frame >= 0 && nd.out >= 0
+                    && plan.streams[size_t(nd.out)].n >= kCriticalDefault)
+                    fse[size_t(nd.frame)] = 1;
+        }
+        LongChecksums const longOnes(sizes, checked, fse);
+        longAlone = longOnes.alone;
+        constexpr char kLongKind = 3; // added to the kind
+        for (size_t i = 0; i < longOnes.of.size(); i++)
+            if (longOnes.of[i]) kindOf[i] = char(kindOf[i] + kLongKind);
         // the parts' device buffers outlive the plan: a new plan reuses them
         // (no allocation, and so no device-wide synchronization, per batch)
         struct Spec {
@@ -252,9 +256,9 @@ struct DecodeBatch {
             int rank;
         };
         std::vector<Spec> specs;
-        int ahead = 0; // kinds ahead of the runs
+        int ahead = longOnes.of.empty() ? 0 : 1; // ranks ahead of the runs: long checksums (of any kind), the critical part
         if (splitParts) {
-            for (char kind : { char(3), char(2), char(1), char(0) }) {
+            for (char kind : { char(5), char(4), char(3), char(2), char(1), char(0) }) {
                 std::vector<size_t> fr;
                 uint64_t total = 0;
                 for (size_t i = 0; i < n; i++)
@@ -265,8 +269,10 @@ struct DecodeBatch {
                 if (fr.empty()) continue;
                 size_t const g = kind >= 2 ? 1 : std::min<size_t>(size_t(runs), fr.size());
                 size_t const first = specs.size();
-                for (size_t k = 0; k < g; k++) specs.push_back(Spec{ std::vector<char>(n, 0), kind == 3, ahead + int(k) });
-                if (kind >= 2) ahead++;
+                bool const isLong = kind >= kLongKind;
+                int const rank = isLong ? 0 : ahead;
+                for (size_t k = 0; k < g; k++) specs.push_back(Spec{ std::vector<char>(n, 0), isLong, rank + int(k) });
+                if (kind == 2) ahead++;
                 uint64_t acc = 0;
                 size_t k = 0;
                 for (size_t i : fr) {
@@ -403,11 +409,12 @@ struct DecodeBatch {
     // Enqueues the plan on `s` as a DAG: each part (branch) runs its
     // dependency levels in order, and the launches of one level, which do not
     // depend on one another, on streams of their own. Stream priorities
-    // order the block scheduler's work. A part of long checksums decodes alone:
-    // the others wait until only its checksums are left. Schedule 0: a branch's
-    // launches share its rank: long checksums and the critical part (the
-    // longest chains) first, then each kind's runs in order, so that a run's
-    // element-wise work shares the SMs with the next run's entropy decoding. Schedule 1: every element-wise
+    // order the block scheduler's work. Where the parts of long checksums decode
+    // alone, the others wait until only their checksums are left. Schedule 0: a
+    // branch's launches share its rank: long checksums, then the critical part
+    // (the longest chains), then each kind's runs in order, so that a run's
+    // element-wise work shares the SMs with the next run's entropy decoding.
+    // Schedule 1: every element-wise
     // launch (short, memory-bound) ahead of all entropy decoding, which keeps
     // the branch ranks. `marks` (timeline runs): a timing event before and
     // after every launch, in part order, on its stream.
@@ -441,12 +448,13 @@ struct DecodeBatch {
         long total = 0;
         size_t mark = 0;
         std::vector<cudaEvent_t> ends;
-        cudaEvent_t others = start; // what the parts after a long-checksum part wait for
+        std::vector<cudaEvent_t> holds; // what the parts after those of long checksums wait for
         for (size_t p = 0; p < parts.size(); p++) {
             const DeviceLayout& L = parts[p].layout;
-            cudaEvent_t ready = parts[p].longChecksum ? start : others; // everything the next level waits for
+            cudaEvent_t ready = start; // everything the next level waits for
+            cudaEvent_t decoded = start; // what the part's last checksums wait for
             for (size_t a = 0; a < L.launches.size();) {
-                if (parts[p].longChecksum && L.launches[a].kind == KIND_HASH) others = ready;
+                if (L.launches[a].kind == KIND_HASH) decoded = ready;
                 size_t b = a;
                 while (b < L.launches.size() && L.launches[b].level == L.launches[a].level) b++;
                 std::vector<cudaStream_t> used;
@@ -456,7 +464,12 @@ struct DecodeBatch {
                                      || L.launches[li].kind == KIND_HUF16) ? 1 : 0;
                     cudaStream_t const x = slotStream(p, li - a, cls, prioOf(parts[p], L.launches[li].kind));
                     cudaEvent_t const e = nextEvent(ev);
-                    if (!x || !e || cudaStreamWaitEvent(x, ready, 0) != cudaSuccess) return reportFail(ZL_ErrorCode_GENERIC);
+                    if (!x || !e) return reportFail(ZL_ErrorCode_GENERIC);
+                    bool waits = true;
+                    if (a == 0 && !parts[p].longChecksum && !holds.empty()) // (each follows the start)
+                        for (cudaEvent_t h : holds) waits = waits && cudaStreamWaitEvent(x, h, 0) == cudaSuccess;
+                    else waits = cudaStreamWaitEvent(x, ready, 0) == cudaSuccess;
+                    if (!waits) return reportFail(ZL_ErrorCode_GENERIC);
                     if (marks) cudaEventRecord((*marks)[mark], x);
                     long const k = runOneLaunch(L, li, parts[p].pool.data(), parts[p].scratch.data(), st, x);
                     if (marks) cudaEventRecord((*marks)[mark + 1], x);
@@ -481,6 +494,7 @@ struct DecodeBatch {
                 a = b;
             }
             ends.push_back(ready);
+            if (longAlone && parts[p].longChecksum) holds.push_back(decoded);
         }
         for (cudaEvent_t e : ends)
             if (cudaStreamWaitEvent(s, e, 0) != cudaSuccess) return reportFail(ZL_ErrorCode_GENERIC);

@@ -390,3 +390,56 @@ def test_huf_code_lengths_with_a_common_divisor(gpu_lib, lengths):
     out, frames = _round_trip(wide, 8, 2, [2 * (k % 8) for k in range(len(wide))])
     for a, g, f in zip(wide, out, frames):
         assert g.tobytes() == a.tobytes() == oracle.decompress(f)[0].tobytes(), a.size
+
+
+# MiB of each frame, what decodes through FSE (1) and Huffman (2)
+LONG_CHECKSUMS = {
+    "Huffman alone before small ones": ([48, 1, 1, 4], [2, 1, 2, 1]),
+    "Huffman beside long work": ([48] + [22] * 10, [2] + [1, 2] * 5),
+    "FSE beside small ones": ([96, 1, 1, 4], [1, 1, 2, 2]),
+    "two kinds beside one small": ([96, 96, 1], [1, 2, 2]),
+    "all long": ([96, 96], [1, 2]),
+    "one frame": ([96], [1]),
+    "below the lines": ([95, 47, 1], [1, 2, 1]),
+}
+
+
+@pytest.mark.parametrize("name", list(LONG_CHECKSUMS))
+def test_long_checksums_beside_other_frames(gpu_lib, name):
+    """Batches with frames whose content checksums are long chains, as a
+    captured graph and as plain launches: outputs equal the inputs, and a wrong
+    checksum of the first or last frame is found."""
+    import torch
+    import openzl_gb300 as oz
+
+    sizes, recipes = LONG_CHECKSUMS[name]
+    gen = torch.Generator(device="cuda").manual_seed(len(sizes))
+    srcs = [torch.cumsum(torch.randint(-100, 101, (s << 18,), device="cuda", generator=gen), 0).to(torch.int32) for s in sizes]
+    enc, n = oz.GpuEncoder(), len(sizes)
+    nbytes = [s << 20 for s in sizes]
+    caps = [enc.bound(b) for b in nbytes]
+    dsts = [torch.empty(c, dtype=torch.uint8, device="cuda") for c in caps]
+    torch.cuda.synchronize()
+    got = enc.compress_batch([s.data_ptr() for s in srcs], [s << 18 for s in sizes], [4] * n, recipes,
+                             [d.data_ptr() for d in dsts], caps, checksums=True)
+    frames = [d[:g].cpu().numpy() for d, g in zip(dsts, got)]
+    side = torch.cuda.Stream()
+    for wrong in (None, 0, n - 1):
+        views = [f.copy() for f in frames]
+        if wrong is not None:
+            views[wrong][-9] ^= 1  # the content checksum that the plan expects
+        outs = [torch.zeros(b, dtype=torch.uint8, device="cuda") for b in nbytes]
+        batch = oz.GpuBatch()
+        batch.plan(views, [d.data_ptr() for d in dsts], [o.data_ptr() for o in outs], nbytes)
+        torch.cuda.synchronize()
+        for graph in (True, False, True):
+            for o in outs:
+                o.zero_()
+            torch.cuda.synchronize()
+            batch.run(side.cuda_stream, graph=graph)
+            if wrong is None:
+                batch.check(side.cuda_stream)
+            else:
+                with pytest.raises(oz.ZLError):
+                    batch.check(side.cuda_stream)
+            assert all(torch.equal(o, s.view(torch.uint8)) for o, s in zip(outs, srcs)), (wrong, graph)
