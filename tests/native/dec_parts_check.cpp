@@ -21,16 +21,25 @@ int main()
         for (char c : rule(b, fse).of) s += c ? '1' : '0';
         return s;
     };
+    // one frame just long enough beside a small one, and just not
+    CHECK(marks({ K, 4 * M }, 0) == "10" && rule({ K, 4 * M }, 0).alone);
+    CHECK(marks({ K - 1, 4 * M }, 0) == "" && !rule({ K - 1, 4 * M }, 0).alone);
+    // with long FSE streams, beside as much work in small frames, and a little less
+    std::vector<size_t> f(5, F / 4);
+    f[0] = F;
+    CHECK(marks(f, 1) == "10000" && !rule(f, 1).alone);
+    f[4]--;
+    CHECK(marks(f, 1) == "");
+    f[4]++;
+    f[0]--;
+    CHECK(marks(f, 1) == "");
     for (char fse : { char(0), char(1) }) {
         size_t const L = fse ? F : K;
-        // one frame just long enough beside a small one, and just not
-        CHECK(marks({ L, 4 * M }, fse) == "10" && rule({ L, 4 * M }, fse).alone == !fse);
-        CHECK(marks({ L - 1, 4 * M }, fse) == "" && !rule({ L - 1, 4 * M }, fse).alone);
         // every frame long: kinds and runs stay
         CHECK(marks({ L }, fse) == "" && marks({ L, L }, fse) == "");
         CHECK(marks(std::vector<size_t>(16, 2 * L), fse) == "");
         // at least half the longest
-        CHECK(marks({ 4 * L, 2 * L, 2 * L - 1, M }, fse) == "1100");
+        CHECK(marks({ 4 * L, 2 * L, 2 * L - 1, 3 * L / 2, 3 * L / 2 }, fse) == "11000");
     }
     CHECK(marks({ 32 * M, 4 * M, 4 * M }, 0) == "" && marks({ 64 * M, 64 * M, M }, 1) == "");
     // alone while the others are short beside the chain: 4.5 times the longest frame
@@ -45,10 +54,13 @@ int main()
     CHECK(c.of.size() == 3 && !c.of[0] && c.of[1] && !c.of[2] && c.alone);
     CHECK(LongChecksums({ K, M }, { 0, 0 }, { 0, 0 }).of.empty());
     CHECK(LongChecksums({}, {}, {}).of.empty() && LongChecksums({ 0, 0 }, { 1, 1 }, { 0, 0 }).of.empty());
-    // one kind of each: the long FSE frame goes ahead too, and nothing is held back
-    LongChecksums const d({ K, F + 2, F - 1, M }, { 1, 1, 1, 1 }, { 0, 1, 1, 1 });
-    CHECK(!d.of[0] && d.of[1] && !d.of[2] && !d.of[3] && !d.alone);
-    LongChecksums const e({ F, F, M }, { 1, 1, 1 }, { 0, 1, 0 });
+    // nothing goes ahead of a frame of half the longest that stays behind
+    CHECK(LongChecksums({ F, F - 1, M }, { 1, 1, 1 }, { 0, 1, 0 }).of.empty());
+    CHECK(LongChecksums({ F, F / 2, M }, { 1, 1, 1 }, { 0, 1, 0 }).of.empty());
+    LongChecksums const d({ F, F / 2 - 1, M }, { 1, 1, 1 }, { 0, 1, 0 });
+    CHECK(d.of[0] && !d.of[1] && !d.of[2] && d.alone);
+    // one kind of each
+    LongChecksums const e({ F, F, F / 3, F / 3, F / 3 }, { 1, 1, 1, 1, 1 }, { 0, 1, 0, 1, 0 });
     CHECK(e.of[0] && e.of[1] && !e.of[2] && !e.alone);
     std::printf("bad=%d\n", bad);
     return bad != 0;

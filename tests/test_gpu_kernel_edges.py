@@ -396,10 +396,10 @@ def test_huf_code_lengths_with_a_common_divisor(gpu_lib, lengths):
 LONG_CHECKSUMS = {
     "Huffman alone before small ones": ([48, 1, 1, 4], [2, 1, 2, 1]),
     "Huffman beside long work": ([48] + [22] * 10, [2] + [1, 2] * 5),
-    "FSE beside small ones": ([96, 1, 1, 4], [1, 1, 2, 2]),
-    "two kinds beside one small": ([96, 96, 1], [1, 2, 2]),
+    "FSE beside as much work": ([96] + [24] * 4, [1] + [1, 2] * 2),
+    "two kinds beside as much work": ([96, 96] + [24] * 4, [1, 2] + [1, 2] * 2),
     "all long": ([96, 96], [1, 2]),
-    "one frame": ([96], [1]),
+    "FSE of half the length stays behind": ([96, 48, 1], [2, 1, 1]),
     "below the lines": ([95, 47, 1], [1, 2, 1]),
 }
 
