@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include "dec_plan.h"
+#include "fse_shape.h" // kTuneFseLanePerState
 
 namespace ozl {
 
@@ -16,13 +17,8 @@ long runLaunches(const DeviceLayout& layout, uint8_t* dPool, uint8_t* dScratch, 
 // Applies the shared-memory carve-out attributes the entropy kernels need.
 // Call once per device before the first launch (and before graph capture).
 cudaError_t prepareKernels();
-// Launch::tune of an FSE launch: streams per CTA in the low byte; this flag
-// selects the kernel with one lane per decoder state (kFse4) instead of one
-// lane per stream (kFse).
-constexpr uint32_t kTuneFseLanePerState = 0x100;
-
 // Launch shapes the autotuner may try for a launch (FSE: streams per CTA; Huffman:
-// threads per chunk); 0 if none.
+// threads per chunk), the untuned one among them; 0 if none.
 uint32_t tuneCandidates(const Launch& l, uint32_t* out, uint32_t cap);
 
 // Enqueues launch `i` of `layout` alone (the building block of runLaunches).

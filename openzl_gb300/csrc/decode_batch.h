@@ -630,11 +630,12 @@ struct DecodeBatch {
     }
 
     // OZL_DParam_fseKernel: the FSE launches' kernel until the autotuner runs
+    // (one lane per stream is the untuned launches' kernel)
     void applyFseKernel(DeviceLayout& layout) const
     {
-        if (!fseKernel) return;
+        if (fseKernel != 2) return;
         for (Launch& l : layout.launches)
-            if (l.kind == KIND_FSE) l.tune = fseKernel == 2 ? (kTuneFseLanePerState | 8u) : (l.param0 <= 8 ? 32u : 6u);
+            if (l.kind == KIND_FSE) l.tune = kTuneFseLanePerState | 8u;
     }
 
     // Times every candidate launch shape of the tunable launches (one launch

@@ -14,6 +14,7 @@
 
 #include "dec_tasks.h"
 #include "dec_exec.h"
+#include "fse_shape.h"
 #include "huf_split.h"
 #include "stream_ring.cuh"
 
@@ -1250,34 +1251,8 @@ struct PosStream {
 // Table construction restates src/openzl/fse/decompress/fse_decompress.c:
 // 73-171; decode order restates fse_decompress.c:255-337 (state i % nbStates
 // emits symbol i; the last symbol of each state has no transition).
-enum FseCells : int { kCells32, kCells24, kCells24Wide };
-constexpr uint32_t kFseCtaSmem = 224 * 1024; // up to 32 tableLog-11 lanes per CTA (one decoding warp)
-
-constexpr uint32_t kFseQuarterSmem = 56 * 1024; // four CTAs of this much fit an SM
-constexpr int kFseRing = 16, kFseAhead = 12;   // stream ring: 256 bytes per lane, 192 bytes ahead
 using FseStream = PosStream<kFseRing, kFseAhead>;
-constexpr uint32_t kFseRingBytes = FseStream::kBytes;
-constexpr uint32_t kFseScratch = 260 * 2 + 256 * 2 + 8; // a warp's table-build scratch: cum[260], next[256]
-
-// warps that build a CTA's tables (the first one then decodes): a table takes
-// about 5 us, and the scratch of the builders is the rings' memory where it fits.
-// An odd number, so that the decoding warps of an SM's CTAs fall on different
-// schedulers (with two, on every other one: 5.2 against 5.0 ms as in fseShape).
-__host__ __device__ __forceinline__ uint32_t fseWarps(uint32_t lanes) { return lanes >= 2 ? 3 : 1; }
-__host__ __device__ __forceinline__ uint32_t fseRingOff(uint32_t lanes, uint32_t tlMax, int cells)
-{
-    return lanes * ((cells == kCells32 ? 4u : 3u) << tlMax);
-}
-// shared memory of a CTA: tables of all lanes, then the rings (kFse) or the
-// build scratch, whichever is larger
-__host__ __device__ __forceinline__ uint32_t fseSmemBytes(uint32_t lanes, uint32_t tlMax, int cells)
-{
-    uint32_t const rings = lanes * kFseRingBytes, scratch = fseWarps(lanes) * kFseScratch;
-    return fseRingOff(lanes, tlMax, cells) + (rings > scratch ? rings : scratch);
-}
-// per lane of kFse4: 16-bit entries, symbols, stream ring (16-byte aligned
-// for tableLog >= 4)
-__host__ __device__ __forceinline__ uint32_t fse4SlotBytes(uint32_t tlMax) { return (3u << tlMax) + 16u * kFseRing; }
+static_assert(FseStream::kBytes == kFseRingBytes, "a lane's ring as fse_shape.h has it");
 
 // Builds the decoding table of task t (cells or entries at tab, newStateBase
 // above the low NB bits of an entry; symbols at symOf, for kCells32 in the
@@ -1558,7 +1533,7 @@ __global__ void __launch_bounds__(96) kFse(const FseTask* __restrict__ tasks, ui
 // warp-uniform (streams of a CTA are of similar length: tasks are sorted
 // longest first) and ends when no lane of the warp has a symbol left. Tables
 // as kFse (one per stream, built by the whole warp).
-constexpr uint32_t kFse4Variant = kTuneFseLanePerState; // Launch::tune flag (dec_exec.h)
+constexpr uint32_t kFse4Variant = kTuneFseLanePerState; // Launch::tune flag (fse_shape.h)
 
 __global__ void __launch_bounds__(32) kFse4(const FseTask* __restrict__ tasks, uint32_t nbTasks, uint32_t streams,
                                             uint32_t tableLogMax, uint32_t* __restrict__ status)
@@ -2589,12 +2564,6 @@ __global__ void __launch_bounds__(kFinishThreads) kHashFinish(const HashTask* __
 namespace ozl {
 
 namespace {
-uint32_t fseLanes(uint32_t tlMax, int cells = kCells24)
-{
-    uint32_t lanes = 32;
-    while (lanes > 1 && fseSmemBytes(lanes, tlMax, cells) > kFseCtaSmem) lanes--;
-    return lanes;
-}
 int smCount()
 {
     static int sms = 0;
@@ -2605,39 +2574,6 @@ int smCount()
         if (sms <= 0) sms = 152;
     }
     return sms;
-}
-// Table form and streams per CTA of an FSE launch.
-// 32-bit cells step faster (96 against 115 cycles) but take a third more
-// shared memory: they are used while every stream of the launch fits the SMs
-// at once (24 per SM at tableLog 11), and for small tables; 24-bit cells where
-// the streams come in waves (32 per SM).
-// Untuned, small tables run as many lanes a CTA as fit. Large ones spread over
-// the SMs, one CTA on each, up to what four CTAs of an SM hold: one decoding
-// warp for each of its schedulers. (Spread over the four schedulers of an SM
-// as well, a stream steps a little faster alone, but each warp then issues for
-// fewer streams, which the launches beside it pay for: host-buffer decoding of
-// 1024 mixed frames, eight rounds at once, 5.6 ms against 5.0 ms.)
-struct FseShape {
-    int cells;
-    uint32_t lanes;
-};
-FseShape fseShape(const Launch& l)
-{
-    uint32_t const sms = uint32_t(smCount()), perSm = (l.nbTasks + sms - 1) / sms;
-    auto quarter = [&](int cells) { // streams of a CTA of which four fit an SM
-        uint32_t lanes = 32;
-        while (lanes > 1 && fseSmemBytes(lanes, l.param0, cells) > kFseQuarterSmem) lanes--;
-        return lanes;
-    };
-    FseShape s;
-    s.cells = l.param0 >= 12                                          ? kCells24Wide
-              : l.param0 <= 8 || perSm <= 4 * quarter(kCells32) ? kCells32
-                                                                      : kCells24;
-    uint32_t const maxLanes = fseLanes(l.param0, s.cells);
-    s.lanes = l.tune & 0xFFu;
-    if (!s.lanes) s.lanes = l.param0 <= 8 ? maxLanes : std::min(perSm, quarter(s.cells));
-    s.lanes = std::max(1u, std::min(s.lanes, maxLanes));
-    return s;
 }
 // Threads per chunk of an untuned Huffman launch: four warps while all chunks
 // run at once (eight CTAs an SM by shared memory and threads; a round of
@@ -2674,11 +2610,7 @@ uint32_t tuneCandidates(const Launch& l, uint32_t* out, uint32_t cap)
 {
     uint32_t n = 0;
     if (l.kind == KIND_FSE) {
-        uint32_t const mx = fseLanes(l.param0);
-        for (uint32_t c : { 32u, 17u, 11u, 8u, 6u, 5u, 4u, 2u })
-            if (c <= mx && n < cap) out[n++] = c;
-        for (uint32_t c : { 8u, 6u, 4u }) // kFse4: streams per warp
-            if (c <= mx && n < cap) out[n++] = kFse4Variant | c;
+        n = fseCandidates(l.nbTasks, l.param0, uint32_t(smCount()), out, cap);
     } else if (l.kind == KIND_HUF) {
         for (uint32_t c : { 32u, 128u }) // threads per chunk
             if (n < cap) out[n++] = c;
@@ -2713,7 +2645,7 @@ long runOneLaunch(const DeviceLayout& L, size_t li, uint8_t* dPool, uint8_t* dSc
                 kConst<<<l.nbTiles, 256, 0, s>>>(static_cast<const ConstTask*>(tasks), tiles);
                 break;
             case KIND_FSE: {
-                uint32_t const maxLanes = fseLanes(l.param0);
+                uint32_t const maxLanes = fseLanes(l.param0, kCells24);
                 if (l.tune & kFse4Variant) { // one lane per state, up to eight streams per warp
                     uint32_t streams = l.tune & 0xFFu;
                     if (streams > 8) streams = 8;
@@ -2724,7 +2656,7 @@ long runOneLaunch(const DeviceLayout& L, size_t li, uint8_t* dPool, uint8_t* dSc
                                                                             streams, l.param0, dStatus);
                     break;
                 }
-                FseShape const sh = fseShape(l);
+                FseShape const sh(l.nbTasks, l.param0, l.tune, uint32_t(smCount()));
                 uint32_t const grid = (l.nbTasks + sh.lanes - 1) / sh.lanes;
                 auto* const k = sh.cells == kCells32 ? kFse<kCells32> : sh.cells == kCells24 ? kFse<kCells24>
                                                                                               : kFse<kCells24Wide>;
