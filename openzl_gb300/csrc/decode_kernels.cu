@@ -1994,7 +1994,8 @@ __global__ void __launch_bounds__(T) kHuf(const HufTask* __restrict__ tasks, uin
 // decode_entropy_binding.c:349-412 apply: weights at most 20, at least two of
 // them non-zero, the sum of 2^(w-1) a power of two. Each of the one or four
 // streams is decoded by several lanes (splitStream); a stream that does not
-// hold its symbols exactly, which the reference does not refuse, by one.
+// hold its symbols exactly, which the reference does not refuse, by one, with
+// the search.
 //
 // What bounds it: a lane is a serial chain, a lookup and a shift a symbol
 // (four symbols per 64-bit window where codes have at most 16 bits, else
@@ -2172,22 +2173,12 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
         }
         return m;
     };
-    SplitRun r = splitStream<int(kHuf16Threads)>(br, run, j, runs, sStep, n, split);
+    SplitRun const r = splitStream<int(kHuf16Threads)>(br, run, j, runs, sStep, n, split);
     if (j >= runs) {
         if (!opened && j == 0 && sIdx < t.nbStreams) reportError(status, DERR_CORRUPTION);
         return;
     }
-    if (!r.ok) { // not exactly n symbols: the first lane decodes n
-        if (j) {
-            br.close();
-            return;
-        }
-        r = SplitRun{ top, n, 0, true };
-    }
-    br.seek(r.start);
-    uint8_t* const out = t.out + 2ull * (t.dstOff[sIdx] + r.before);
-    uint32_t const cnt = r.count;
-    uint32_t i = 0;
+    uint8_t* const out = t.out + 2ull * (t.dstOff[sIdx] + (r.ok ? r.before : 0));
     auto put = [&](uint32_t k, uint32_t y) {
         if (!(reinterpret_cast<uintptr_t>(out) & 1)) {
             reinterpret_cast<uint16_t*>(out)[k] = uint16_t(y);
@@ -2196,6 +2187,27 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
             out[2 * k + 1] = uint8_t(y >> 8);
         }
     };
+    if (!r.ok) { // not exactly n symbols: the first lane decodes n, one by one
+        br.close();
+        if (j) return;
+        // The words come from memory: a stream of too few bits reads below its
+        // first 16-byte block, where the ring would hold anything at all. There
+        // the block's first word stands in.
+        const uint32_t* const words = reinterpret_cast<const uint32_t*>(br.g16);
+        int32_t pos = top;
+        for (uint32_t i = 0; i < n; i++) {
+            int32_t const k = (pos - 1) >> 5;
+            uint32_t const a = __ldg(words + max(k, 0)), b = __ldg(words + max(k - 1, 0));
+            uint32_t const hi = __funnelshift_l(b, a, uint32_t(32 * (k + 1) - pos));
+            uint32_t const e = entryOf(weightOf(hi >> (32 - tl)));
+            put(i, symbol(hi, e));
+            pos -= int32_t(e & 31u);
+        }
+        return;
+    }
+    br.seek(r.start);
+    uint32_t const cnt = r.count;
+    uint32_t i = 0;
     auto single = [&]() {
         br.refill<1>();
         uint32_t y = 0;

@@ -443,3 +443,67 @@ def test_long_checksums_beside_other_frames(gpu_lib, name):
                 with pytest.raises(oz.ZLError):
                     batch.check(side.cuda_stream)
             assert all(torch.equal(o, s.view(torch.uint8)) for o, s in zip(outs, srcs)), (wrong, graph)
+
+
+def test_huf16_stream_of_too_few_bits_is_repeatable(gpu_lib):
+    """A 16-bit Huffman stream may hold fewer bits than its symbols take (only
+    the streams' sizes are checked, and there is no checksum): the symbols that
+    it holds are right, and the others do not depend on what ran before."""
+    import struct
+    import torch
+    import openzl_gb300 as oz
+
+    cut, rng, frames, wants, held = 16, np.random.default_rng(3), [], [], []
+    counts = [376, 376, 376, 1500 - 3 * 376]
+
+    def streams(f, at):
+        """(first byte, size) of the four streams from byte `at` on, or None."""
+        out = []
+        for n in counts:
+            if at < 0 or at + 8 > len(f) or struct.unpack_from("<I", f, at)[0] != n:
+                return None
+            out.append((at + 8, struct.unpack_from("<I", f, at + 4)[0]))
+            at += 8 + out[-1][1]
+        return out
+
+    while len(frames) < 16:
+        a = np.where(rng.random(1500) < 0.8, 5, rng.integers(0, 1000, 1500)).astype(np.uint16)
+        f = oracle.compress(8, a, 2, checksums=False).tobytes()
+        found = next((x for x in (streams(f, at) for at in range(len(f))) if x), None)
+        if not found or not 16 * 6 < found[0][1] < 16 * 8:
+            continue  # another codec, or a longer stream
+        # four streams, each its symbols' count, its size and its bits; the first
+        # one, of fewer bytes than the decoder's window, loses its last bits (its
+        # first bytes), which the last one gets as bits that nothing reads
+        bits = [f[p:p + s] for p, s in found]
+        bits[0], bits[3] = bits[0][cut:], bytes(cut) + bits[3]
+        body = b"".join(struct.pack("<II", n, len(b)) + b for n, b in zip(counts, bits))
+        frames.append(f[:found[0][0] - 8] + body + f[sum(found[3]):])
+        assert len(frames[-1]) == len(f)
+        wants.append(a)
+        held.append(376 - 8 * cut)  # codes have at least a bit
+    side = torch.cuda.Stream()
+    dfr = [torch.from_numpy(np.concatenate([np.zeros(k, np.uint8), np.frombuffer(f, np.uint8)])).cuda() for k, f in enumerate(frames)]
+    noise = [rng.integers(0, 4000, 30000).astype(np.uint16) for _ in range(400)]
+    nf = [oracle.compress(8, x, 2).tobytes() for x in noise[:40]]
+    dn = [torch.from_numpy(np.frombuffer(f, np.uint8).copy()).cuda() for f in nf]
+    nout = [torch.zeros(60000, dtype=torch.uint8, device="cuda") for _ in range(400)]
+    other = oz.GpuBatch()
+    other.plan([nf[k % 40] for k in range(400)], [dn[k % 40].data_ptr() for k in range(400)], [o.data_ptr() for o in nout],
+               [60000] * 400)
+    first = None
+    for rep in range(6):
+        if rep % 2:
+            other.run(side.cuda_stream, graph=False)
+        outs = [torch.zeros(3000, dtype=torch.uint8, device="cuda") for _ in frames]
+        batch = oz.GpuBatch()
+        batch.plan(frames, [d.data_ptr() + k for k, d in enumerate(dfr)], [o.data_ptr() for o in outs], [3000] * len(frames))
+        torch.cuda.synchronize()
+        batch.run(side.cuda_stream, graph=False)
+        batch.check(side.cuda_stream)
+        got = [o.cpu().numpy().view(np.uint16) for o in outs]
+        for g, a, n in zip(got, wants, held):
+            assert (g[:n] == a[:n]).all() and (g[376:] == a[376:]).all(), rep
+        if first is None:
+            first = got
+        assert all((g == x).all() for g, x in zip(got, first)), rep
