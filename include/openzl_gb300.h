@@ -476,6 +476,10 @@ typedef enum {
     OZL_GRAPH_ENTROPY = 17,         /* ZL_GRAPH_ENTROPY (FSE or Huffman per chunk) */
 } OZL_GraphRecipe;
 
+/* An encoder keeps until it is freed: its device buffers, pinned staging
+ * memory (some KiB for every entropy-coded chunk of the largest batch so far)
+ * and, once a batch has had enough chunks for several host threads, up to 15
+ * sleeping ones. A ZL_CCtx holds one encoder. */
 typedef struct OZL_GpuEncoder_s OZL_GpuEncoder;
 OZL_GpuEncoder* ozl_gpu_encoder_create(void);
 void ozl_gpu_encoder_free(OZL_GpuEncoder* e);

@@ -249,7 +249,11 @@ struct PinnedBuf {
         p = nullptr;
         cap = 0;
         bytes = std::max(bytes, size_t(256) << 10); // one allocation for all phases of a small call
-        if (cudaHostAlloc(reinterpret_cast<void**>(&p), bytes, cudaHostAllocDefault) != cudaSuccess) return false;
+        if (cudaHostAlloc(reinterpret_cast<void**>(&p), bytes, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError(); // (the caller may do without)
+            p = nullptr;
+            return false;
+        }
         cap = bytes;
         return true;
     }
@@ -261,7 +265,7 @@ struct PinnedBuf {
 // call 3 to 4 us of gaps, with 17 of them (64 KiB call: 266 us, now 243).
 // Ranges above kMost go up array by array: there the gaps do not count, and
 // growing the pinned staging to them took 15 ms of the first pass over 2048
-// mixed frames.
+// mixed frames. So they do where no memory can be pinned.
 class Upload {
   public:
     static constexpr size_t kMost = size_t(2) << 20;
@@ -269,14 +273,13 @@ class Upload {
     {
         if (bytes) items_.push_back(Item{ static_cast<uint8_t*>(dev), host, bytes });
     }
-    // false: out of pinned memory, or the copy failed. The staging is free again
-    // once `s` has passed the copy.
+    // false: a copy failed. The staging is free again once `s` has passed the copy.
     bool go(PinnedBuf& stage, size_t at, cudaStream_t s)
     {
         if (items_.empty()) return true;
         uint8_t* const lo = items_.front().dev;
         size_t const bytes = size_t(items_.back().dev - lo) + items_.back().bytes;
-        if (bytes > kMost) {
+        if (bytes > kMost || (at == 0 ? !stage.reserve(bytes) : at + bytes > stage.cap)) {
             bool ok = true;
             for (const Item& x : items_)
                 ok = (x.host ? cudaMemcpyAsync(x.dev, x.host, x.bytes, cudaMemcpyHostToDevice, s)
@@ -284,7 +287,6 @@ class Upload {
             items_.clear();
             return ok;
         }
-        if (at == 0 ? !stage.reserve(bytes) : at + bytes > stage.cap) return false;
         for (const Item& x : items_) {
             if (x.host) std::memcpy(stage.p + at + (x.dev - lo), x.host, x.bytes);
             else std::memset(stage.p + at + (x.dev - lo), 0, x.bytes);
@@ -423,12 +425,59 @@ struct EncodeBatch::Impl {
         if (hashStream) cudaStreamDestroy(hashStream);
         if (hashStart) cudaEventDestroy(hashStart);
         if (hashDone) cudaEventDestroy(hashDone);
+        for (cudaEvent_t e : histDone)
+            if (e) cudaEventDestroy(e);
     }
+    cudaEvent_t histDone[2] = {};
     PinnedBuf stage, stageH, hists;
     HostPool pool;
     std::vector<Job> jobs;           // data chunks (discovery order), then nested weights jobs
     size_t nbDataJobs = 0;
     bool checksums = true;
+
+    // Brings the histograms of the jobs [0, n) from the device and waits for
+    // them: up to 8 MiB of them into pinned memory, where the decisions take them
+    // from (histAt); more through two such blocks in turn into the jobs, one
+    // taken over by the host threads while the other is filled. Pageable memory
+    // where none can be pinned.
+    static constexpr size_t kHistBlock = 8192; // histograms of 1 KiB
+    const uint32_t* histAt = nullptr;
+    std::vector<uint32_t> histPageable;
+    bool histsToJobs(const uint32_t* dH, size_t n, cudaStream_t st)
+    {
+        size_t const block = std::min(n, kHistBlock), blocks = (n + block - 1) / block;
+        size_t const room = std::min(blocks, size_t(2)) * block * 256;
+        bool const pinned = hists.reserve(4 * room);
+        histPageable.resize(pinned ? 0 : room);
+        uint32_t* const at = pinned ? reinterpret_cast<uint32_t*>(hists.p) : histPageable.data();
+        if (blocks == 1) {
+            histAt = at;
+            return cudaMemcpyAsync(at, dH, n * 1024, cudaMemcpyDeviceToHost, st) == cudaSuccess
+                   && cudaStreamSynchronize(st) == cudaSuccess;
+        }
+        histAt = nullptr;
+        for (cudaEvent_t& e : histDone)
+            if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return false;
+        auto fetch = [&](size_t k) -> bool {
+            size_t const first = k * block, count = std::min(block, n - first);
+            return cudaMemcpyAsync(at + (k & 1) * block * 256, dH + first * 256, count * 1024, cudaMemcpyDeviceToHost, st)
+                           == cudaSuccess
+                   && cudaEventRecord(histDone[k & 1], st) == cudaSuccess;
+        };
+        bool ok = fetch(0);
+        for (size_t k = 0; ok && k < blocks; k++) {
+            if (k + 1 < blocks) ok = fetch(k + 1);
+            ok = ok && cudaEventSynchronize(histDone[k & 1]) == cudaSuccess;
+            if (!ok) break;
+            const uint32_t* const from = at + (k & 1) * block * 256;
+            Job* const to = jobs.data() + k * block;
+            parallelFor(std::min(block, n - k * block), [&](size_t j) {
+                if (!to[j].wide) std::memcpy(to[j].hist.count, from + j * 256, 1024);
+            }, 256);
+        }
+        if (!ok) cudaStreamSynchronize(st); // no copy outlives the blocks
+        return ok;
+    }
 };
 
 EncodeBatch::EncodeBatch() : impl_(new Impl) {}
@@ -1455,9 +1504,7 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
         cudaMemcpyAsync(dHt, ht.data(), ht.size() * sizeof(HistTask), cudaMemcpyHostToDevice, st);
         launchHist(dHt, uint32_t(ht.size()), dH, st);
         launches_++;
-        if (!I.hists.reserve(nj * 1024)) { err = "allocation failed"; return 70; }
-        cudaMemcpyAsync(I.hists.p, dH, nj * 1024, cudaMemcpyDeviceToHost, st);
-        if (cudaStreamSynchronize(st) != cudaSuccess) { err = "device error in histograms"; return 1; }
+        if (!I.histsToJobs(dH, nj, st)) { err = "device error in histograms"; return 1; }
     }
     // 16-bit chunks: value counts, first occurrences and maxima on the
     // device; the counts of values up to each chunk's maximum come back
@@ -1498,8 +1545,7 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
             // chunks: 1.1 ms, now 0.3). Up to 16 MiB, beyond it own arrays.
             size_t values = 0;
             for (size_t k = 0; k < nw; k++) values += size_t(mx[k]) + 1;
-            bool const pinned = values * 8 <= (size_t(16) << 20);
-            if (pinned && !I.stage.reserve(values * 8)) { err = "allocation failed"; return 70; }
+            bool const pinned = values * 8 <= (size_t(16) << 20) && I.stage.reserve(values * 8);
             uint32_t* at = reinterpret_cast<uint32_t*>(I.stage.p);
             for (size_t k = 0; k < nw; k++) {
                 Job& J = I.jobs[wide[k]];
@@ -1640,7 +1686,7 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
     }
     parallelFor(nj, [&](size_t j) {
         if (I.jobs[j].wide) return;
-        std::memcpy(I.jobs[j].hist.count, I.hists.p + j * 1024, 1024);
+        if (I.histAt) std::memcpy(I.jobs[j].hist.count, I.histAt + j * 256, 1024);
         decide(I.jobs[j]);
     });
     // Huffman tables on the device: every 8-bit Huffman chunk's code lengths
@@ -1875,7 +1921,12 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
         size_t const stageOff = (sz.used + taskBytes + tilesGuess * sizeof(TileRef) + (nbSizes + 16) * 4 + 1024 + 255)
                 & ~size_t(255);
         size_t const total = stageOff + szStage.used + 256;
-        if (!I.bufE.reserve(total) || !I.stage.reserve(szStage.used + 256 + std::min(stageOff - sz.used, Upload::kMost))) { err = "allocation failed"; return 70; }
+        if (!I.bufE.reserve(total)
+            || !(I.stage.reserve(szStage.used + 256 + std::min(stageOff - sz.used, Upload::kMost))
+                 || I.stage.reserve(szStage.used + 256))) {
+            err = "allocation failed";
+            return 70;
+        }
         Bump b{ I.bufE.data(), 0 };
         Bump stg{ I.bufE.data() + stageOff, 0 };
         layoutE(b, stg, true);

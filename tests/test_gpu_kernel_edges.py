@@ -507,3 +507,36 @@ def test_huf16_stream_of_too_few_bits_is_repeatable(gpu_lib):
         if first is None:
             first = got
         assert all((g == x).all() for g, x in zip(got, first)), rep
+
+
+@pytest.mark.parametrize("n", [8192, 8193, 16385, 25000])
+def test_encoder_histograms_in_blocks(gpu_lib, n):
+    """More chunks than the encoder brings back histograms of at once, 16-bit
+    chunks among them: frames equal the oracle's."""
+    rng = np.random.default_rng(n)
+    pool = []
+    for k in range(60):
+        m = 20 + 7 * (k % 13)
+        pool.append(((rng.geometric(0.2, m) % 256).astype(np.uint8), 0, (7, 8, 17)[k % 3]))
+    pool.append(((rng.zipf(1.3, 2000) % 3000).astype(np.uint16), 2, 8))
+    pool.append((np.minimum(rng.geometric(1 / 300, 3000), 65535).astype(np.uint16), 2, 17))
+    want = [oracle.compress(r, a, w).tobytes() for a, w, r in pool]
+    pick = [int(x) for x in rng.integers(0, len(pool) - 2, n - 5)] + [len(pool) - 2, len(pool) - 1, len(pool) - 2, 0, 1]
+    import torch
+    import openzl_gb300 as oz
+
+    enc = oz.GpuEncoder()
+    dev = [torch.from_numpy(a.view(np.uint8).copy()).cuda() for a, _, _ in pool]
+    caps = [enc.bound(a.nbytes) for a, _, _ in pool]
+    room = [(caps[k] + 255) // 256 * 256 for k in pick]
+    at = np.concatenate([[0], np.cumsum(room)[:-1]])
+    dst = torch.zeros(int(sum(room)), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        dst.zero_()
+        torch.cuda.synchronize()
+        sizes = enc.compress_batch([dev[k].data_ptr() for k in pick], [pool[k][0].size for k in pick],
+                                   [pool[k][1] for k in pick], [pool[k][2] for k in pick],
+                                   [dst.data_ptr() + int(o) for o in at], [caps[k] for k in pick], checksums=True)
+        host = dst.cpu().numpy()
+        assert all(host[o:o + s].tobytes() == want[k] for k, o, s in zip(pick, at, sizes))
