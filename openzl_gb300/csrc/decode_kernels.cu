@@ -2217,7 +2217,7 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
     if (narrow && !(reinterpret_cast<uintptr_t>(out) & 1)) {
         uint32_t const head = min(cnt, uint32_t((8 - (reinterpret_cast<uintptr_t>(out) & 7)) & 7) >> 1);
         for (; i < head; i++) single();
-        uint32_t y[4], i0 = i;
+        uint32_t y[4] = {}, i0 = i;
         auto store = [&](uint32_t k) {
             *reinterpret_cast<uint2*>(out + 2 * k) = make_uint2(__byte_perm(y[0], y[1], 0x5410), __byte_perm(y[2], y[3], 0x5410));
         };
@@ -2234,7 +2234,7 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
         }
         if (i > i0) store(i - 4);
     } else {
-        uint32_t y[3], i0 = i;
+        uint32_t y[3] = {}, i0 = i;
         auto store = [&](uint32_t k) {
 #pragma unroll
             for (int m = 0; m < 3; m++) put(k + m, y[m]);

@@ -136,6 +136,23 @@ def compress_huf_tablelog12(recipe, arr, elt_width, checksums=True):
         lib().ozo_test_set_huf_max_tablelog(11)
 
 
+def compress_float(elt_type, sign_frac, exponent):
+    """A frame (no checksums) of the float node's two streams: element type 0
+    (float32, 3 bytes of sign and fraction an element), 1 (bfloat16, 1) or 2
+    (float16, 2), one exponent byte each. Test frames: the reference's encoder
+    makes these of numbers, whose float16 exponents have 5 bits."""
+    sf, ex = np.ascontiguousarray(sign_frac, np.uint8), np.ascontiguousarray(exponent, np.uint8)
+    assert sf.size == ex.size * (3, 1, 2)[elt_type]
+    w = (4, 2, 2)[elt_type]
+    streams = lib().ozo_test_set_float
+    streams.restype, streams.argtypes = None, [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
+    streams(elt_type, sf.ctypes.data, ex.ctypes.data)
+    try:
+        return compress(6, np.zeros(ex.size, {4: np.uint32, 2: np.uint16}[w]), w, False)
+    finally:
+        streams(1, None, None)
+
+
 def xxh3_64(buf):
     b = np.frombuffer(bytes(buf), np.uint8)
     return lib().ozo_xxh3_64(b.ctypes.data, b.size)

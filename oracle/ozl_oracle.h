@@ -68,6 +68,10 @@ int64_t ozo_tokenize(const void* src, size_t n, int w, int sorted, void* alphaOu
  * reference encoder's) or 12 (the decoders' limit). Not thread-safe. */
 void ozo_test_set_fse_max_tablelog(unsigned tl);
 void ozo_test_set_huf_max_tablelog(unsigned tl);
+/* Test entry point: the streams of the next frames' float nodes, as element
+ * type 0 (float32), 1 (bfloat16) or 2 (float16); sf NULL: the input's own. Not
+ * thread-safe. */
+void ozo_test_set_float(int type, const uint8_t* sf, const uint8_t* ex);
 
 #ifdef __cplusplus
 }

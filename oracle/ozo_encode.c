@@ -1442,6 +1442,18 @@ static int node_tokenize(ECtx* c, int in, int sorted)
     return a;
 }
 
+/* Test hook: the next frames' float nodes take these streams (one exponent
+ * byte an element, and 3, 1 or 2 bytes of sign|fraction) as element type 0
+ * (float32), 1 (bfloat16) or 2 (float16) instead of the input's; NULL: off. */
+static int g_floatType = 1;
+static const uint8_t *g_floatSf = NULL, *g_floatEx = NULL;
+void ozo_test_set_float(int type, const uint8_t* sf, const uint8_t* ex)
+{
+    g_floatType = sf ? type : 1;
+    g_floatSf = sf;
+    g_floatEx = ex;
+}
+
 /* EI_bfloat16_deconstruct (encode_float_deconstruct_binding.c:14-80):
  * header = element type; outputs sign|fraction (struct, width 1) and
  * exponent (serial). */
@@ -1449,8 +1461,15 @@ static int node_bf16(ECtx* c, int in)
 {
     size_t const n = S(in)->n;
     ENode* nd = new_node(c, TR_FLOAT_DECONSTRUCT, in, 2);
-    nd->hdr[0] = 1;
+    nd->hdr[0] = (uint8_t)g_floatType;
     nd->hsz = 1;
+    if (g_floatSf) {
+        size_t const w = g_floatType == 0 ? 3 : (g_floatType == 1 ? 1 : 2);
+        int const sf = new_stream(c, OZO_TYPE_STRUCT, w, n, g_floatSf);
+        new_stream(c, OZO_TYPE_SERIAL, 1, n, g_floatEx);
+        nd->nbOut = 2;
+        return sf;
+    }
     int sf = new_stream(c, OZO_TYPE_STRUCT, 1, n, NULL);
     int ex = new_stream(c, OZO_TYPE_SERIAL, 1, n, NULL);
     for (size_t i = 0; i < n; i++) {

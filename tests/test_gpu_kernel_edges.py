@@ -540,3 +540,90 @@ def test_encoder_histograms_in_blocks(gpu_lib, n):
                                    [dst.data_ptr() + int(o) for o in at], [caps[k] for k in pick], checksums=True)
         host = dst.cpu().numpy()
         assert all(host[o:o + s].tobytes() == want[k] for k, o, s in zip(pick, at, sizes))
+
+
+@pytest.mark.parametrize("elt_type", [0, 1, 2], ids=["float32", "bfloat16", "float16"])
+def test_float_joins_of_every_type(gpu_lib, elt_type):
+    """Sign and fraction joined with the exponent around the vectors of 4 and 8
+    elements and the 4,096-element tile, any bit pattern (float16 exponents of
+    more than 5 bits among them), frames and destinations at every alignment.
+    The oracle's bytes, and for float32 and float16 numbers the numbers."""
+    import torch
+    import openzl_gb300 as oz
+
+    rng = np.random.default_rng(elt_type)
+    w, sw = (4, 2, 2)[elt_type], (3, 1, 2)[elt_type]
+    cases = []
+    for n in [5, 6, 7, 8, 9, 11, 12, 15, 16, 17, 31, 33, 100, 1000, 4095, 4096, 4097, 4100, 4104, 8191, 8192, 8193, 20001]:
+        for kind in range(3):
+            sf = rng.integers(0, 256, n * sw).astype(np.uint8)
+            ex = rng.integers(0, 256, n).astype(np.uint8)  # stored
+            if kind == 1:
+                ex = np.minimum(rng.geometric(0.3, n), 255).astype(np.uint8)  # entropy-coded
+            number = None
+            if kind == 2 and elt_type != 1:  # numbers, taken apart as the format has them
+                x = rng.normal(0, 1, n).astype(np.float32 if elt_type == 0 else np.float16)
+                bits = x.view("u%d" % w).astype(np.uint32)
+                frac = 23 if elt_type == 0 else 10
+                s = (bits >> (8 * w - 1)) | ((bits & ((1 << frac) - 1)) << 1)
+                sf = s.astype("<u4").view(np.uint8).reshape(n, 4)[:, :sw].copy().ravel()
+                ex = ((bits >> frac) & (255 if elt_type == 0 else 31)).astype(np.uint8)
+                number = x.tobytes()
+            f = oracle.compress_float(elt_type, sf, ex)
+            want = oracle.decompress(f)[0].tobytes()
+            assert number in (None, want) and len(want) == n * w
+            cases.append((f.tobytes(), want))
+    for shift in range(4):
+        src = [torch.from_numpy(np.frombuffer(b"\0" * ((k + 5 * shift) % 16) + f, np.uint8).copy()).cuda()
+               for k, (f, _) in enumerate(cases)]
+        outs = [torch.zeros(len(x) + 32, dtype=torch.uint8, device="cuda") for _, x in cases]
+        at = [w * ((k // 3 + shift) % (16 // w)) if shift else 16 * (k % 2) for k in range(len(cases))]
+        batch = oz.GpuBatch()
+        batch.plan([f for f, _ in cases], [t.data_ptr() + (k + 5 * shift) % 16 for k, t in enumerate(src)],
+                   [o.data_ptr() + a for o, a in zip(outs, at)], [len(x) for _, x in cases])
+        batch.run(0, graph=False)
+        batch.check(0)
+        for (_, x), o, a in zip(cases, outs, at):
+            g = o.cpu().numpy()
+            assert g[a:a + len(x)].tobytes() == x, (shift, len(x))
+            assert not g[:a].any() and not g[a + len(x):].any(), (shift, len(x))
+
+
+def _random_histogram(rng):
+    """Symbols of a random histogram: uniform, skewed, geometric, one dominant
+    symbol, few symbols, groups of equal counts around the Huffman sort's bucket
+    cutoff."""
+    most = 1 + int(rng.integers(0, 255))
+    n = 20 + int(rng.integers(0, 200 if rng.random() < 0.25 else 12000))
+    kind = int(rng.integers(0, 7))
+    if kind == 0:
+        a = rng.integers(0, most + 1, n)
+    elif kind == 1:
+        a = ((most + 1) * rng.random(n) ** (2 + 4 * rng.random())).astype(np.int64)
+    elif kind == 2:
+        a = np.minimum(rng.geometric(1 / 3, n) - 1, most)
+    elif kind == 3:
+        a = np.where(rng.random(n) < 0.95, 0, rng.integers(0, most + 1, n))
+    elif kind == 4:
+        few = rng.integers(0, most + 1, 2 + int(rng.integers(0, 6)))
+        a = few[np.minimum(rng.geometric(0.6, n) - 1, few.size - 1)]
+    elif kind == 5:
+        count = rng.integers(0, 3, most + 1) * int(rng.integers(1, 180)) + rng.integers(0, 2, most + 1)
+        a = np.repeat(np.arange(most + 1), count)
+    else:
+        count = np.where(rng.random(most + 1) < 0.5, rng.geometric(0.02, most + 1), 163 + rng.integers(0, 4, most + 1))
+        a = np.repeat(np.arange(most + 1), count)
+    a = rng.permutation(a.astype(np.uint8))[:32000]
+    return a if a.size >= 20 else (np.arange(40) % 7).astype(np.uint8)
+
+
+@pytest.mark.parametrize("recipe", [7, 8], ids=["fse", "huffman"])
+@pytest.mark.parametrize("n", [1500, 3500])
+def test_device_tables_on_random_histograms(gpu_lib, recipe, n):
+    """Normalized counts, headers, coding tables and code lengths that the
+    kernels build, on random histograms, as many chunks as take a CTA each for
+    their tables and more: frames equal the oracle's."""
+    rng = np.random.default_rng(recipe + n)
+    arrays = [_random_histogram(rng) for _ in range(n)]
+    for k, (a, f) in enumerate(zip(arrays, _frames(arrays, recipe, 0))):
+        assert f == oracle.compress(recipe, a, 0).tobytes(), (k, a.size)
