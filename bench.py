@@ -908,7 +908,7 @@ def main():
                          [d_out.data_ptr() + o for o in ooffs], osizes)
     assert planned == total_out, (planned, total_out)
 
-    # autotuner: launch shapes (chunks per CTA of the FSE and Huffman launches)
+    # autotuner: launch shapes (streams per CTA of the FSE launches, threads per chunk of the Huffman ones)
     prof0 = sum(ms for _, ms, _ in batch.profile(sptr, capacity=256))
     if args.fse_kernel is None:
         shapes = batch.autotune(sptr, reps=2)

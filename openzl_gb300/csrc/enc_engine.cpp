@@ -1878,8 +1878,7 @@ int EncodeBatch::compress(const std::vector<EncFrameSpec>& frames, uint8_t* cons
                             fseTabT.push_back(FseTableTask{ reinterpret_cast<const uint32_t*>(hist), J.n, table,
                                                             reinterpret_cast<int16_t*>(J.dNorm), J.dNcount,
                                                             J.hist.maxSym, J.tl, J.ncountSlot, 0 });
-                            fseT.push_back(FseEncTask{ src, J.out, J.dTable, uint32_t(J.n), J.sizeSlot, J.nbStates, J.tl,
-                                                       J.dFields });
+                            fseT.push_back(FseEncTask{ src, J.out, J.dTable, uint32_t(J.n), J.sizeSlot, J.tl, J.dFields });
                         }
                         break;
                     }

@@ -119,65 +119,9 @@ ChunkCodec chooseCodec(const Histo& h, int mode)
     return mode == EM_HUF ? CC_HUF : CC_FSE;
 }
 
-// FSE table log, normalization and header: the shared restatement in
-// fse_norm.h (the device table builder uses the same functions)
 unsigned fseTableLog(unsigned maxTL, uint64_t srcSize, unsigned maxSym, unsigned minus)
 {
     return fseTableLogOf(maxTL, srcSize, maxSym, minus);
-}
-
-bool fseNormalize(int16_t* norm, unsigned tl, const uint32_t* count, uint64_t total, unsigned maxSym)
-{
-    return fseNormalizeCounts(norm, tl, count, total, maxSym);
-}
-
-size_t fseWriteNCount(uint8_t* out, const int16_t* norm, unsigned maxSym, unsigned tl)
-{
-    return fseWriteNCountTo(out, norm, maxSym, tl);
-}
-
-// FSE_buildCTable_wksp (fse_compress.c:69-207)
-void fseBuildCTable(FseCTable& ct, const int16_t* norm, unsigned maxSym, unsigned tl)
-{
-    uint32_t const size = 1u << tl, mask = size - 1, step = (size >> 1) + (size >> 3) + 3;
-    uint16_t cumul[258];
-    uint8_t symbolAt[4096];
-    uint32_t high = size - 1;
-    ct.tableLog = uint16_t(tl);
-    ct.maxSym = uint16_t(maxSym);
-    cumul[0] = 0;
-    for (unsigned u = 1; u <= maxSym + 1; u++) {
-        if (norm[u - 1] == -1) {
-            cumul[u] = uint16_t(cumul[u - 1] + 1);
-            symbolAt[high--] = uint8_t(u - 1);
-        } else {
-            cumul[u] = uint16_t(cumul[u - 1] + uint16_t(norm[u - 1]));
-        }
-    }
-    uint32_t pos = 0;
-    for (unsigned s = 0; s <= maxSym; s++)
-        for (int i = 0; i < norm[s]; i++) {
-            symbolAt[pos] = uint8_t(s);
-            do { pos = (pos + step) & mask; } while (pos > high);
-        }
-    for (uint32_t u = 0; u < size; u++) ct.state[cumul[symbolAt[u]]++] = uint16_t(size + u);
-    unsigned total = 0;
-    for (unsigned s = 0; s < 256; s++) {
-        int const c = s <= maxSym ? norm[s] : 0;
-        fseSymbolDeltas(c, tl, total, ct.deltaNbBits[s], ct.deltaFindState[s]);
-        total += c == -1 ? 1u : unsigned(c);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Huffman code lengths and codes: the shared restatement in huf_tree.h (the
-// device table builder uses the same functions)
-unsigned hufBuild(HufCTable& ct, const uint32_t* count, unsigned maxSym, unsigned maxNbBits)
-{
-    HufNode all[kHufNodes];
-    unsigned const tl = hufBuildCodes(all, ct.value, ct.nbBits, count, maxSym, maxNbBits);
-    ct.tableLog = tl;
-    return tl;
 }
 
 // ---------------------------------------------------------------------------

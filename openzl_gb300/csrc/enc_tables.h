@@ -49,13 +49,11 @@ uint64_t hufSizeFast(double entropy, uint64_t n);
 uint64_t flatpackedSize(const Histo& h);
 uint64_t bitpackedSize(const Histo& h);
 
-// FSE: table log, normalized counts, encoding tables.
+// FSE and Huffman table log of a chunk.
 unsigned fseTableLog(unsigned maxTableLog, uint64_t srcSize, unsigned maxSym, unsigned minus);
-bool fseNormalize(int16_t* norm, unsigned tableLog, const uint32_t* count, uint64_t total, unsigned maxSym);
-size_t fseWriteNCount(uint8_t* out, const int16_t* norm, unsigned maxSym, unsigned tableLog);
 
-// Device-ready FSE encoding table: next-state table sorted by symbol, and
-// per-symbol (deltaNbBits, deltaFindState).
+// FSE encoding table in device memory (kFseTables): next-state table sorted by
+// symbol, and per-symbol (deltaNbBits, deltaFindState).
 struct FseCTable {
     uint16_t tableLog;
     uint16_t maxSym;
@@ -63,15 +61,13 @@ struct FseCTable {
     int32_t deltaFindState[256];
     uint16_t state[2048];
 };
-void fseBuildCTable(FseCTable& ct, const int16_t* norm, unsigned maxSym, unsigned tableLog);
 
-// Huffman: code lengths and canonical codes for a histogram.
+// Huffman code lengths and canonical codes of a chunk in device memory (kHufTables).
 struct HufCTable {
     uint16_t value[256];
     uint8_t nbBits[256];
     uint32_t tableLog;
 };
-unsigned hufBuild(HufCTable& ct, const uint32_t* count, unsigned maxSym, unsigned maxNbBits);
 
 // Chunk codec choice for a 16-bit struct chunk (the 2-byte branch of
 // entropyCompressChunk, encode_entropy_binding.c:612-681), whatever the

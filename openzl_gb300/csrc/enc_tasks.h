@@ -66,7 +66,6 @@ struct FseEncTask {
     const uint8_t* ctable;   // ent::FseCTable on the device
     uint32_t n;
     uint32_t sizeSlot;       // where the bitstream size is written
-    uint32_t nbStates;
     uint32_t tableLog;
     uint16_t* fields;        // chunks of kFseLongMin symbols or more: fseFieldBytes(n) of scratch
 };

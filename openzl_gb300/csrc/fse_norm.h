@@ -1,9 +1,15 @@
-// FSE table-log choice, count normalization and normalized-count header,
-// shared by the host path and the device table builder (kFseTables). They
+// FSE table-log choice, count normalization and normalized-count header. They
 // restate src/openzl/fse/compress/fse_compress.c exactly (the tables decide
 // the frame's bytes): FSE_optimalTableLog_internal (:379-396),
 // FSE_normalizeM2 (:400-470), FSE_normalizeCount (:472-520) and
 // FSE_writeNCount_generic (:226-338). Integer arithmetic only.
+//
+// The encoder uses fseTableLogOf, FseNormScale and fseSymbolDeltas; the table
+// kernel (kFseTables) does the rest with all lanes of a warp. The serial
+// fseNormalizeCounts, fseNormalizeM2 and fseWriteNCountTo state what those
+// lanes must equal, and are checked against the reference's functions on random
+// histograms (tests/native/tables_ref_check.cpp); the kernel's results are
+// compared as frames with the CPU oracle's on such histograms.
 #pragma once
 #include <cstddef>
 #include <cstdint>

@@ -1,5 +1,8 @@
-// Huffman code lengths and canonical codes of one chunk, shared by the host
-// path and the device table builder (kHufTables). They restate
+// Huffman code lengths and codes of one chunk. The table kernel (kHufTables)
+// uses the buckets, the quicksort and the height limit from here and does the
+// rest with all lanes of a warp; the serial hufSortByCount and hufBuildCodes
+// state what those lanes must equal, and are checked against the reference's
+// function on random histograms (tests/native/tables_ref_check.cpp). They restate
 // src/openzl/fse/compress/huf_compress.c exactly (the lengths decide the
 // frame's bytes): HUF_sort (:352-420, bucket sort with a quicksort of the
 // large-count buckets), HUF_buildTree (:580-640), HUF_setMaxHeight

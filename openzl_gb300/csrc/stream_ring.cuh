@@ -1,5 +1,5 @@
-// Device helpers shared by the decoders and the encoders: unaligned 16-byte
-// reads and the encoders' per-lane source ring (also kFse4's stream ring).
+// Device helpers: unaligned 16-byte reads (decoders and encoders) and kFse4's
+// stream ring.
 #pragma once
 #include <cstdint>
 
@@ -38,26 +38,6 @@ struct StreamRing {
             asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(g16 + 16 * size_t(m)) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    // Starts the ring for a stream whose top bit is at position pos (> 0).
-    __device__ __forceinline__ void start(int32_t pos)
-    {
-        int32_t const mt = (pos - 1) >> 7;
-        for (int32_t m = mt; m >= mt - AHEAD; m--) issue(m);
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        low = mt;
-    }
-    // Word k (descending order after start(); k may be negative: 0).
-    __device__ __forceinline__ uint32_t word(int32_t k)
-    {
-        if (k < 0) return 0u;
-        int32_t const m = k >> 2;
-        if (m < low) {
-            low = m;
-            issue(m - AHEAD);
-            asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
-        }
-        return ring[k & (4 * RING - 1)];
     }
 };
 
