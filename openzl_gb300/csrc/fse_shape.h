@@ -20,7 +20,7 @@ constexpr uint32_t kFseScratch = 260 * 2 + 256 * 2 + 8; // a warp's table-build 
 // warps that build a CTA's tables (the first one then decodes): a table takes
 // about 5 us, and the scratch of the builders is the rings' memory where it fits.
 // An odd number, so that the decoding warps of an SM's CTAs fall on different
-// schedulers (with two, on every other one: 5.2 against 5.0 ms as in fseShape).
+// schedulers (with two, on every other one: 5.2 against 5.0 ms as in FseShape).
 OZL_HD inline uint32_t fseWarps(uint32_t lanes) { return lanes >= 2 ? 3 : 1; }
 OZL_HD inline uint32_t fseRingOff(uint32_t lanes, uint32_t tlMax, int cells)
 {
