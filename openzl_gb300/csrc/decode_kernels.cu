@@ -2566,7 +2566,12 @@ __global__ void __launch_bounds__(kFinishThreads) kHashFinish(const HashTask* __
     }
     if (t.hashOut) *t.hashOut = h;
     bool const ok = t.low8 ? ((h & 255) == t.expected) : (uint32_t(h) == t.expected);
-    if (!ok && t.errCode) reportError(status, t.errCode);
+    if (!ok && t.errCode) {
+        // of a frame's two checksums the compressed one is the first to be
+        // verified, so its error stands whichever CTA ends first
+        uint32_t const before = atomicCAS(status, 0u, t.errCode);
+        if (t.errCode == DERR_COMPRESSED_CK && before == DERR_CONTENT_CK) atomicCAS(status, DERR_CONTENT_CK, DERR_COMPRESSED_CK);
+    }
 }
 
 } // namespace ozl

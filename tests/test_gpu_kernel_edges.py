@@ -627,3 +627,40 @@ def test_device_tables_on_random_histograms(gpu_lib, recipe, n):
     arrays = [_random_histogram(rng) for _ in range(n)]
     for k, (a, f) in enumerate(zip(arrays, _frames(arrays, recipe, 0))):
         assert f == oracle.compress(recipe, a, 0).tobytes(), (k, a.size)
+
+
+def test_compressed_checksum_error_stands_before_content(gpu_lib):
+    """A corrupted byte of a stored stream fails both checksums: the compressed
+    one is reported (it is verified first), however long the two take; a wrong
+    content checksum alone is reported as such."""
+    import torch
+    import openzl_gb300 as oz
+
+    rng = np.random.default_rng(5)
+    side = torch.cuda.Stream()
+    for n in [20, 200, 240, 241, 1000, 1024, 1025, 5000, 65536, 66000, 300000]:
+        for recipe, width in ((0, 0), (0, 1), (9, 4), (12, 2)):
+            a = rng.integers(0, 256, n * max(width, 1)).astype(np.uint8)
+            f = oracle.compress(recipe, a.view("u%d" % max(width, 1)), width)
+            for at, code in ((len(f) - 9 - n // 2, 13), (len(f) - 9, 13), (None, 14)):
+                bad = f.copy()
+                if at is not None:
+                    bad[at] ^= 0x10  # a payload byte; the content checksum (both hold it)
+                else:  # the compressed checksum made to hold the wrong content checksum
+                    bad[-9] ^= 0x10
+                    start = next(k for k in range(len(f)) if _xxh3_low32(f[k:-5]) == bytes(f[-5:-1]))
+                    bad[-5:-1] = np.frombuffer(_xxh3_low32(bad[start:-5]), np.uint8)
+                dev = torch.from_numpy(bad).cuda()
+                out = torch.zeros(a.nbytes + 64, dtype=torch.uint8, device="cuda")
+                batch = oz.GpuBatch()
+                batch.plan([bad.tobytes()], [dev.data_ptr()], [out.data_ptr()], [a.nbytes])
+                torch.cuda.synchronize()
+                for graph in (False, True):
+                    batch.run(side.cuda_stream, graph=graph)
+                    with pytest.raises(oz.ZLError) as e:
+                        batch.check(side.cuda_stream)
+                    assert e.value.code == code, (n, recipe, width, at)
+
+
+def _xxh3_low32(x):
+    return (oracle.xxh3_64(x.tobytes()) & 0xFFFFFFFF).to_bytes(4, "little")
