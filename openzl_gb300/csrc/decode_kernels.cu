@@ -1164,13 +1164,16 @@ __device__ __forceinline__ bool streamStart(const uint8_t* p, uint32_t size, con
 // wrap. Words below the stream are never consumed by a valid stream
 // (finished() checks that it ends exactly at its first bit), so the ring's
 // stale contents may stand in for them.
-template <int RING, int AHEAD>
+// SHIFT: spread() may move positions, so that lanes' windows fall on different
+// banks.
+template <int RING, int AHEAD, bool SHIFT = false>
 struct PosStream {
     static_assert((RING & (RING - 1)) == 0 && AHEAD + 4 <= RING, "ring shape");
     static constexpr uint32_t kBytes = 16 + 16 * RING; // mirror and ring, 16-byte aligned
     const uint8_t *g16, *smem;
     uint32_t ring, ringAddr;
     int32_t pos, end, low;
+    int32_t lowest = 0; // byte of the stream's first chunk
 
     // the next chunk below, unless `low` has reached `goal` (not below 0)
     __device__ __forceinline__ void next(int32_t goal)
@@ -1200,10 +1203,22 @@ struct PosStream {
     {
         close(); // a copy in flight may be to the same place
         pos = to;
-        int32_t const first = ((pos - 1) >> 7) * 16, goal = max(first - 16 * AHEAD, 0);
+        int32_t const first = ((pos - 1) >> 7) * 16, goal = max(first - 16 * AHEAD, SHIFT ? lowest : 0);
         low = first + 16;
         while (low > goal) next(goal);
         asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    }
+    // Counts positions from up to RING - 1 chunks before the first one, so that
+    // position p falls into the ring's first chunk; returns what it adds to them.
+    __device__ __forceinline__ int32_t spread(int32_t p)
+    {
+        static_assert(SHIFT, "a stream whose positions may move");
+        int32_t const k = -((p - 1) >> 7) & (RING - 1);
+        lowest = 16 * k;
+        g16 -= lowest;
+        pos += 128 * k;
+        end += 128 * k;
+        return 128 * k;
     }
     __device__ __forceinline__ bool init(const uint8_t* p, uint32_t size, const uint8_t* sm, uint32_t area)
     {
@@ -1218,7 +1233,7 @@ struct PosStream {
     __device__ __forceinline__ void refill()
     {
         static_assert(3 * N + 1 <= AHEAD, "a chunk is issued two calls before it is read");
-        int32_t const goal = max(((pos >> 3) & ~15) - 16 * AHEAD, 0);
+        int32_t const goal = max(((pos >> 3) & ~15) - 16 * AHEAD, SHIFT ? lowest : 0);
 #pragma unroll
         for (int k = 0; k < N; k++) next(goal);
         asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 2;" ::: "memory");
@@ -1678,12 +1693,16 @@ __global__ void __launch_bounds__(32) kFse4(const FseTask* __restrict__ tasks, u
 // tables an SM holds.
 // From a first bit at any place, lanes whose codes all had lengths of a common
 // divisor never met the boundaries. 256 MiB of bytes, 64 MiB, 256 KiB: codes of
-// 2 and 4 bits 1.50, 0.48 and 0.385 ms so, 0.57, 0.17 and 0.063 from multiples
+// 2 and 4 bits 1.50, 0.48 and 0.385 ms so, 0.57, 0.17 and 0.062 from multiples
 // of 2 (0.94, 0.43 and 0.39 with one lane a stream); 4 and 8 bits 1.70, 0.51,
-// 0.386 and 0.69, 0.19, 0.053. Codes nearly all of one length (31 of 5 bits,
-// few of 9 to 11) meet late and stay the worst: 1.26, 0.50 and 0.21 ms (one
+// 0.386 and 0.69, 0.19, 0.052. Codes nearly all of one length (31 of 5 bits,
+// few of 9 to 11) meet late and stay the worst: 1.11, 0.44 and 0.20 ms (one
 // lane 1.09, 0.51 and 0.42). More places to meet at (two to four, up to 4,096
 // bits into the run) gained nothing.
+// Lanes of about equal codes keep their windows' distance in the rings, so each
+// lane's positions are moved to begin in a bank group of its own (spread): runs
+// of 100 words, as codes of 3.125 bits make in a chunk of 32 K, had all lanes in
+// one bank, 1.14 ms for 256 MiB and 0.61 now (geometric bytes 0.83 and 0.81).
 constexpr int32_t kMeetBits = 256;
 template <int T>
 struct SplitShared {
@@ -1705,23 +1724,26 @@ __device__ __forceinline__ SplitRun splitStream(Stream& br, Run run, uint32_t j,
 {
     uint32_t const tid = threadIdx.x;
     bool const mine = j < S;
-    int32_t p = 0, e = 0, c = 0, meet = 0;
+    int32_t p = 0, e = 0, c = 0, meet = 0, shift = 0;
     uint32_t upToMeet = 0, count = 0;
     if (mine) {
         int32_t const top = br.pos, bits = top - br.end;
         p = top - splitStart(bits, j, S, step);
         e = top - splitStart(bits, j + 1, S, step);
+        shift = br.spread(p);
+        p += shift;
+        e += shift;
         c = max(p - kMeetBits, e);
         br.seek(p);
         upToMeet = run(c);
         meet = br.pos;
         count = upToMeet + run(e);
-        sh.pos[tid] = br.pos;
+        sh.pos[tid] = br.pos - shift;
     }
     __syncthreads();
     int32_t used = p;
     for (;;) {
-        int32_t const want = mine && j ? sh.pos[tid - 1] : used;
+        int32_t const want = mine && j ? sh.pos[tid - 1] + shift : used;
         bool const differs = want != used;
         if (!__syncthreads_or(differs)) break;
         if (differs) {
@@ -1733,7 +1755,7 @@ __device__ __forceinline__ SplitRun splitStream(Stream& br, Run run, uint32_t j,
             } else {
                 meet = br.pos;
                 count = m + run(e);
-                sh.pos[tid] = br.pos;
+                sh.pos[tid] = br.pos - shift;
             }
             upToMeet = m;
         }
@@ -1748,7 +1770,7 @@ __device__ __forceinline__ SplitRun splitStream(Stream& br, Run run, uint32_t j,
             if (k == j) r.before = total;
             total += sh.count[tid - j + k];
         }
-        r.ok = total == n && sh.pos[tid - j + S - 1] == br.end;
+        r.ok = total == n && sh.pos[tid - j + S - 1] == br.end - shift;
     }
     return r;
 }
@@ -1775,7 +1797,7 @@ __device__ __forceinline__ SplitRun splitStream(Stream& br, Run run, uint32_t j,
 // window and one lane a stream, 0.33 with the present step, 0.32 now; one
 // chunk of about 100,000 symbols: 1.12, 0.75 and 0.095 ms.
 constexpr uint32_t kHufTableLog = 12;
-using HufStream = PosStream<8, 4>;
+using HufStream = PosStream<8, 4, true>;
 struct HufScratch {
     uint32_t count[16], next[16];
     uint32_t step; // lengthStep of the codes
@@ -2006,7 +2028,7 @@ __global__ void __launch_bounds__(T) kHuf(const HufTask* __restrict__ tasks, uin
 // 98,304 symbols in four streams, geometric with mean 3000: 7.06 ms with one
 // lane a stream and the search, 1.41 with the table, 0.55 now.
 constexpr uint32_t kHuf16Log = 12, kHuf16Threads = 128, kHuf16Warps = kHuf16Threads / 32;
-using Huf16Stream = PosStream<8, 4>;
+using Huf16Stream = PosStream<8, 4, true>;
 
 __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restrict__ tasks, uint32_t* __restrict__ status)
 {
@@ -2111,6 +2133,7 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
     bool const opened = br.open(t.stream[sIdx], t.streamSize[sIdx], sRing, tid * Huf16Stream::kBytes);
     uint32_t const runs = opened ? splitRuns(br.pos - br.end, lanes) : 0, n = t.count[sIdx];
     int32_t const top = br.pos;
+    const uint32_t* const words = reinterpret_cast<const uint32_t*>(br.g16);
     auto symbol = [&](uint32_t hi, uint32_t e) -> uint32_t {
         return t.sorted[uint32_t(int32_t(e) >> 5) + __funnelshift_l(hi, 0u, e)];
     };
@@ -2193,7 +2216,6 @@ __global__ void __launch_bounds__(kHuf16Threads) kHuf16(const Huf16Task* __restr
         // The words come from memory: a stream of too few bits reads below its
         // first 16-byte block, where the ring would hold anything at all. There
         // the block's first word stands in.
-        const uint32_t* const words = reinterpret_cast<const uint32_t*>(br.g16);
         int32_t pos = top;
         for (uint32_t i = 0; i < n; i++) {
             int32_t const k = (pos - 1) >> 5;

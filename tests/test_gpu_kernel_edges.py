@@ -368,7 +368,7 @@ def _symbols_of_lengths(rng, n, lengths):
 
 
 @pytest.mark.parametrize("lengths", [[2] * 3 + [4] * 4, [3] * 7 + [6] * 8, [4] * 15 + [8] * 16, [5] * 31 + [10] * 32,
-                                     [6] * 63 + [7] * 2, [7] * 127 + [8] * 2, [1] + [3] * 4],
+                                     [6] * 63 + [7] * 2, [7] * 127 + [8] * 2, [1] + [3] * 4, [3] * 7 + [4] * 2],
                          ids=lambda x: "-".join("%dx%d" % (x.count(l), l) for l in sorted(set(x))))
 def test_huf_code_lengths_with_a_common_divisor(gpu_lib, lengths):
     """Streams whose codes all have lengths of a common divisor, and of two
